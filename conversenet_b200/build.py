@@ -84,6 +84,10 @@ def _units():
     units = [("converse_b200", "converse_b200.cu", []), ("k_dynamic", "k_dynamic.cu", []),
              ("k_strip", "k_strip.cu", []), ("k_block", "k_block.cu", []), ("k_block_tc", "k_block_tc.cu", []), ("k_block_tc2", "k_block_tc2.cu", []),
              ("k_block_tc3", "k_block_tc3.cu", [])]
+    units += [("k_rp", "k_rp.cu", []), ("k_rp_rows", "k_rp_rows.cu", [])]
+    for name, io in (("f32", "float"), ("bf16", "__nv_bfloat16")):
+        for unit in ("k_rp_cols", "k_rp_plane"):
+            units.append(("%s_%s" % (unit, name), unit + ".cu", ["-DCVB_IO=" + io, "-DCVB_IO_NAME=" + name]))
     for (a, b, c, d, nt, mb) in STATIC_PLANS:
         units.append(("k_static_%d_%d_%d_%d_%d_%d" % (a, b, c, d, nt, mb), "k_static.cu",
                       ["-DCVB_RY0=%d" % a, "-DCVB_RY1=%d" % b, "-DCVB_RX0=%d" % c, "-DCVB_RX1=%d" % d,

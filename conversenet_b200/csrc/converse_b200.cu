@@ -4,6 +4,7 @@
 #include "cvb_internal.h"
 #include "cvb_plan.h"
 #include "cvb_block.cuh"
+#include "cvb_rp_plan.h"
 
 #include <algorithm>
 #include <cstdlib>
@@ -138,6 +139,9 @@ static bool needs_strip(int h, int w, int k, bool big) {
   return big || smem_bytes_for(h, w, k) > kSmemLimit || option(CVB_OPT_MULTIPASS) != 0;
 }
 
+// chunk workspace of the multi-launch real-plane kernels
+constexpr size_t kRpWorkspace = (size_t)64 << 20;
+
 static int check_padding(int H, int W, int p, int pad_mode) {
   if (p < 0) return CVB_ERR_BAD_ARGUMENT;
   if (pad_mode < CVB_PAD_CIRCULAR || pad_mode > CVB_PAD_CONSTANT) return CVB_ERR_BAD_ARGUMENT;
@@ -217,7 +221,8 @@ size_t cvb_transfer_bytes(int C, int h, int w) {
   }
   RaderInfo ry, rx;
   rader_both(py, px, ry, rx);
-  return ((size_t)C * h * w + h + w + rader_blob_float2(ry) + rader_blob_float2(rx)) * sizeof(float2);
+  const size_t n = ((size_t)C * h * w + h + w + rader_blob_float2(ry) + rader_blob_float2(rx)) * sizeof(float2);
+  return std::max(n, rp::table_bytes(C, h, w));
 }
 
 static int build_table(const float* weight, const float* bias, int C, int k, int s, int h, int w, float eps,
@@ -238,6 +243,7 @@ static int build_table(const float* weight, const float* bias, int C, int k, int
   if (!weight || !bias || !table || C < 1 || k < 1 || s < 1 || h < 2 || w < 2) return CVB_ERR_BAD_ARGUMENT;
   // the tiled build keeps k-long arrays of kMaxTaps entries per thread and per block
   if (k > kMaxTaps || k > s * h || k > s * w) return CVB_ERR_KERNEL_TOO_LARGE;
+  if (rp::supported(h, w)) return rp::build_table(weight, bias, C, k, s, h, w, eps, kind, table, (cudaStream_t)stream);
   TransferParams T;
   if (!make_axis_plans(h, w, T.py, T.px)) return CVB_ERR_UNSUPPORTED_SIZE;
   T.weight = weight; T.bias = bias; T.table = (float2*)table;
@@ -271,6 +277,8 @@ size_t cvb_converse2d_workspace_bytes(int B, int C, int H, int W, int s, int p, 
   (void)io_dtype;
   if (B < 1 || C < 1 || H < 1 || W < 1 || p < 0 || s < 1) return 0;
   const int h = H + 2 * p, w = W + 2 * p;
+  if (rp::supported(h, w))
+    return rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0, std::max(kRpWorkspace, rp::ws_plane_bytes(h, w, s))).ws_bytes;
   Plan1D py, px;
   bool big = false;
   if (h < 2 || w < 2 || !make_axis_plans(h, w, py, px, &big)) return 0;
@@ -287,6 +295,15 @@ int cvb_converse2d_fwd(const void* x, void* out, const void* table, const float*
   if (k > kMaxTaps) return CVB_ERR_KERNEL_TOO_LARGE;
   int rc = check_padding(H, W, p, pad_mode);
   if (rc != CVB_OK) return rc;
+  if (H + 2 * p < 2 || W + 2 * p < 2) return CVB_ERR_BAD_ARGUMENT;
+  if (k > s * (H + 2 * p) || k > s * (W + 2 * p)) return CVB_ERR_KERNEL_TOO_LARGE;
+  rp::Params Q;
+  if (rp::fill_params(Q, table, B, C, H, W, k, s, p, pad_mode)) {
+    Q.x = x; Q.out = out; Q.weight = weight; Q.gelu = fuse_gelu ? 1 : 0;
+    const rp::Route r = rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0,
+                                  std::max(kRpWorkspace, rp::ws_plane_bytes(H + 2 * p, W + 2 * p, s)));
+    return rp::run(Q, r, io_dtype, workspace, workspace_bytes, (cudaStream_t)stream);
+  }
   FwdParams P;
   P.x = x; P.out = out; P.table = (const float2*)table; P.weight = weight;
   P.B = B; P.C = C; P.H = H; P.W = W; P.k = k; P.s = s; P.p = p; P.pad_mode = pad_mode;
@@ -331,7 +348,8 @@ int cvb_cross_spectrum(const float* x, const float* q, const void* table, void* 
   if (kind != 1 && kind != 2) return CVB_ERR_UNSUPPORTED_SIZE;
   Q.direct = kind == 2 ? 1 : 0;
   if (!make_plan(Q.h, Q.py) || !make_plan(Q.w, Q.px)) return CVB_ERR_UNSUPPORTED_SIZE;
-  Q.tw = (const float2*)table + (size_t)C * Q.h * Q.w;   // the twiddles behind the multiplier
+  // the twiddles behind the multiplier
+  Q.tw = (const float2*)table + (rp::supported(Q.h, Q.w) ? (size_t)C * Q.w * (Q.h / 2 + 1) : (size_t)C * Q.h * Q.w);
   return launch_xspec(Q, (cudaStream_t)stream);
 }
 
@@ -355,6 +373,16 @@ int cvb_converse2d_fwd_static_scratch(const void* x, void* out, const void* tabl
   if (k > kMaxTaps) return CVB_ERR_KERNEL_TOO_LARGE;
   const int rc = check_padding(H, W, p, pad_mode);
   if (rc != CVB_OK) return rc;
+  rp::Params Q;
+  if (k <= s * (H + 2 * p) && k <= s * (W + 2 * p) && rp::fill_params(Q, table, B, C, H, W, k, s, p, pad_mode)) {
+    if ((size_t)Q.h * Q.w * sizeof(float2) > CVB_STATIC_SCRATCH_BYTES) return CVB_ERR_TOO_LARGE;
+    Q.x = x; Q.out = out; Q.weight = weight; Q.gelu = fuse_gelu ? 1 : 0;
+    void* scratch = nullptr;
+    const int rs = static_scratch_address(&scratch);
+    if (rs != CVB_OK) return rs;
+    return rp::run(Q, rp::route(B, C, H, W, s, p, sm_count(), true, CVB_STATIC_SCRATCH_BYTES), io_dtype, scratch,
+                   CVB_STATIC_SCRATCH_BYTES, (cudaStream_t)stream);
+  }
   FwdParams P;
   P.x = x; P.out = out; P.table = (const float2*)table; P.weight = weight;
   P.B = B; P.C = C; P.H = H; P.W = W; P.k = k; P.s = s; P.p = p; P.pad_mode = pad_mode;

@@ -37,7 +37,18 @@ int launch_tap_gradient(const float* g, const float* r, float* out, int nseg, in
 // Multi-pass path through a workspace (k_strip.cu).
 int launch_strip(const FwdParams& P, int io_dtype, void* workspace, size_t ws_bytes, cudaStream_t st);
 // Same kernels, workspace = the library's own fixed device array (no allocation anywhere).
+int static_scratch_address(void** out);
 int launch_strip_static_scratch(const FwdParams& P, int io_dtype, cudaStream_t st);
+
+// Real-plane solve for every size with a two-stage plan (k_rp.cu).
+namespace rp {
+struct Params;
+struct Route;
+size_t table_bytes(int C, int h, int w);
+int build_table(const float* weight, const float* bias, int C, int k, int s, int h, int w, float eps, int kind,
+                void* table, cudaStream_t st);
+int run(Params& P, const Route& r, int io_dtype, void* workspace, size_t ws_bytes, cudaStream_t st);
+}  // namespace rp
 
 // Fused channel-mixing kernels of ConverseBlock (k_block.cu).
 struct BlockParams;

@@ -1200,9 +1200,8 @@ struct TransferParams {
 
 // One table entry, straightforward form (one sine / cosine pair per tap and alias); kept for
 // scales above kFastMaxScale.  fp64 throughout.
-__host__ __device__ inline void transfer_entry_slow(const TransferParams& T, int c, int posy, int posx) {
+__host__ __device__ inline void transfer_value_slow(const TransferParams& T, int c, int u, int v, double& tr, double& ti) {
   const int s = T.s, k = T.k, h = T.h, w = T.w, cc = T.k / 2;
-  const int u = pos_to_freq(T.py, posy), v = pos_to_freq(T.px, posx);
   const double lam = 1.0 / (1.0 + exp(-((double)T.bias[c] - 9.0))) + (double)T.eps;
   const int Nh = s * h, Nw = s * w;
   const float* K = T.weight + (size_t)c * k * k;
@@ -1250,8 +1249,6 @@ __host__ __device__ inline void transfer_entry_slow(const TransferParams& T, int
     }
   }
   const double inv_alias = 1.0 / (double)(s * s);
-  const double norm = 1.0 / ((double)h * (double)w);
-  double tr, ti;
   if (T.kind == 1) {
     tr = 1.0 / (den * inv_alias + lam);
     ti = 0.0;
@@ -1264,7 +1261,12 @@ __host__ __device__ inline void transfer_entry_slow(const TransferParams& T, int
     tr = (1.0 - num_r * inv_alias) / d;
     ti = (-num_i * inv_alias) / d;
   }
-  T.table[((size_t)c * w + posx) * h + posy] = make_float2((float)(tr * norm), (float)(ti * norm));
+}
+__host__ __device__ inline void transfer_entry_slow(const TransferParams& T, int c, int posy, int posx) {
+  const double norm = 1.0 / ((double)T.h * (double)T.w);
+  double tr, ti;
+  transfer_value_slow(T, c, pos_to_freq(T.py, posy), pos_to_freq(T.px, posx), tr, ti);
+  T.table[((size_t)c * T.w + posx) * T.h + posy] = make_float2((float)(tr * norm), (float)(ti * norm));
 }
 
 // exp(-2 pi i m / N) in fp64

@@ -1,0 +1,142 @@
+// Host side of the real-plane kernels (cvb_rp.cuh): axis plans, table layout, launch geometry.  Allocates nothing.
+#pragma once
+#include "cvb_plan.h"
+#include "cvb_rp.cuh"
+
+namespace cvb {
+namespace rp {
+
+constexpr int kMatrixMax = 127;   // largest R0 of the matrix stage
+constexpr int kMaxR1 = 26;        // (separating the spectra keeps 2 R1 values in a thread: small ones are cheaper)
+
+// N = R0 * R1 with the lowest estimated cost per point: packed butterfly operations plus about nine instructions of
+// loads, stores and twiddles a stage; a matrix stage costs R0 FMAs a point (two packed operations each, at the
+// efficiency measured for it).  Radices above 16 keep more values in registers than three blocks an SM allow.
+inline bool axis_plan(int n, int& r0, int& r1) {
+  double best = 1e30;
+  auto codelet = [](int r) { return register_radix(r); };
+  auto cost = [&](int r) { return 9.0 + kRadixOps[r] * 0.01 + (r > 16 ? 0.25 * (r - 16) : 0.0) + (r > kSmallRadix ? 2.0 : 0.0); };
+  for (int b = 1; b <= kMaxR1 && b <= n; ++b) {
+    if (n % b || (b > 1 && !codelet(b))) continue;
+    const int a = n / b;
+    if (a < 2) continue;
+    double c = b == 1 ? 6.0 : cost(b) + (b > 10 ? 0.3 * (b - 10) : 0.0);
+    if (codelet(a)) c += cost(a);
+    else if (a >= 3 && a <= kMatrixMax) c += 16.0 + 0.75 * a;
+    else continue;
+    if (c < best) { best = c; r0 = a; r1 = b; }
+  }
+  return best < 1e30;
+}
+
+inline bool supported(int h, int w) {
+  int a, b;
+  return h >= 2 && w >= 2 && axis_plan(h, a, b) && axis_plan(w, a, b);
+}
+
+inline int matrix_entries(int r0) { return ((r0 - 1) / 2) * matrix_groups(r0) * 8; }   // float2
+
+// Blob in float2 units: multiplier [C][w][hh]; twiddles of h and of w in natural order (tw), then in position order
+// (twy, twx); matrix rows of R0(h) and of R0(w)
+struct Blob { size_t tw, twy, twx, dmy, dmx, total; };
+inline Blob blob_layout(int C, int h, int w, int r0y, int r0x) {
+  Blob b;
+  b.tw = (size_t)C * w * (h / 2 + 1);
+  b.twy = (b.tw + h + w + 1) & ~(size_t)1;
+  b.twx = (b.twy + h + 1) & ~(size_t)1;
+  b.dmy = (b.twx + w + 1) & ~(size_t)1;
+  b.dmx = b.dmy + matrix_entries(r0y);
+  b.total = b.dmx + matrix_entries(r0x);
+  return b;
+}
+
+inline void fill_axis(Axis& a, int n, int r0, int r1, const float2* tw, const float2* dm) {
+  a.n = n; a.r0 = r0; a.r1 = r1;
+  a.nkg = matrix_groups(r0);
+  a.inv_r1 = 1.0f / (float)r1;
+  a.tw = tw; a.dm = dm;
+}
+
+inline int lines_log2(int bytes_per_line) {   // widest strip of 16 / 8 / 4 lines with two blocks on an SM
+  for (int s = 4; s > 2; --s)
+    if ((bytes_per_line << s) <= 104 * 1024) return s;
+  return 2;
+}
+inline size_t cols_smem(const Params& P) { return ((size_t)P.h << P.lsh_c) * sizeof(float2) + (size_t)P.h * sizeof(int); }
+inline size_t rows_smem(const Params& P) { return ((size_t)P.pitch << P.lsh_r) * sizeof(float2); }
+// kernels built for small radices serve an axis whose two radices are small
+inline bool small_axis(const Axis& a) { return a.nkg == 0 && a.r0 <= kSmallRadix && a.r1 <= kSmallRadix; }
+
+inline size_t plane_smem(int h, int w, int k) {
+  const int wc = (w + 1) / 2, hh = h / 2 + 1;
+  return ((size_t)h * wc + (size_t)hh * (w | 1) + (k * k + 1) / 2) * sizeof(float2) + (size_t)h * sizeof(int);
+}
+
+// Everything of Params that depends on the shape; false when an axis has no plan.
+inline bool fill_params(Params& P, const void* table, int B, int C, int H, int W, int k, int s, int p, int pad_mode) {
+  const int h = H + 2 * p, w = W + 2 * p;
+  int r0y, r1y, r0x, r1x;
+  if (h < 2 || w < 2 || !axis_plan(h, r0y, r1y) || !axis_plan(w, r0x, r1x)) return false;
+  const float2* t = (const float2*)table;
+  const Blob bl = blob_layout(C, h, w, r0y, r0x);
+  P.tab = t;
+  P.B = B; P.C = C; P.H = H; P.W = W; P.k = k; P.s = s; P.p = p; P.pad_mode = pad_mode;
+  P.h = h; P.w = w; P.hh = h / 2 + 1; P.wc = (w + 1) / 2; P.wp = 2 * P.wc;
+  P.pitch = w | 1;
+  P.inv_wc = 1.0f / (float)P.wc; P.inv_hh = 1.0f / (float)P.hh;
+  P.lsh_c = lines_log2(h * 8);
+  P.lsh_r = lines_log2(P.pitch * 8);
+  fill_axis(P.ay, h, r0y, r1y, t + bl.twy, t + bl.dmy);
+  fill_axis(P.ax, w, r0x, r1x, t + bl.twx, t + bl.dmx);
+  P.gelu = 0; P.conj = 0; P.plane0 = 0; P.nplane = 0; P.vec = 0;
+  P.ws = nullptr; P.r = nullptr; P.x = nullptr; P.out = nullptr; P.weight = nullptr;
+  return true;
+}
+
+// Bytes of workspace one plane takes in the multi-launch form
+inline size_t ws_plane_bytes(int h, int w, int s) {
+  const int wp = (w + 1) / 2 * 2;
+  const size_t spec = (size_t)(h / 2 + 1) * wp * sizeof(float2);
+  return s > 1 ? spec + ((size_t)h * wp * sizeof(float) + 15) / 16 * 16 : spec;
+}
+
+struct Route {
+  bool one_block;       // plane_body, no workspace
+  int threads;          //   its block size
+  int chunk;            // multi-launch form: planes per chunk
+  size_t ws_bytes;
+};
+// One block per plane while three of them share an SM's memory (or the planes are too few and small for launches of
+// strips to pay), else the multi-launch form over chunks of at most ws_cap bytes of workspace.
+inline Route route(int B, int C, int H, int W, int s, int p, int sms, bool force_multi, size_t ws_cap) {
+  const int h = H + 2 * p, w = W + 2 * p, planes = B * C;
+  Route r;
+  const size_t sm = plane_smem(h, w, kMaxTaps);
+  r.one_block = !force_multi && (sm <= 75 * 1024 && (planes >= sms || sm <= 24 * 1024));
+  r.threads = 256;
+  const size_t per = ws_plane_bytes(h, w, s);
+  size_t n = ws_cap / per;
+  if (n > (size_t)planes) n = planes;
+  r.chunk = (int)n;
+  r.ws_bytes = r.one_block ? 0 : n * per;
+  return r;
+}
+
+// block size of plane_body: the count that wastes the fewest thread slots over its stages
+inline int plane_threads(const Params& P) {
+  const Axis &y = P.ay, &x = P.ax;
+  const int items[4] = {y.r1 * P.wc, (y.r0 / 2 + 1) * P.wc, x.r1 * P.hh, x.r0 * P.hh};
+  const int cost[4] = {y.r0, 2 * y.r1, x.r0, x.r1};
+  double best = 1e30;
+  int bt = 64;
+  for (int t = 64; t <= 256; t += 32) {
+    double c = 0;
+    for (int i = 0; i < 4; ++i) c += (double)((items[i] + t - 1) / t) * t * (cost[i] + 2);
+    c *= 1.0 + 8.0 / t;      // fewer warps hide less latency
+    if (c < best - 1e-9) { best = c; bt = t; }
+  }
+  return bt;
+}
+
+}  // namespace rp
+}  // namespace cvb

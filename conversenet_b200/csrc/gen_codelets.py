@@ -21,6 +21,8 @@ import math
 import sys
 
 RADICES = [2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 18, 19, 20, 22, 23, 24, 26]
+# further butterflies of the two-stage plans (cvb_rp.cuh)
+RADICES2 = [21, 25, 27, 28, 29, 30, 31, 32]
 
 
 def is_prime(n):
@@ -264,6 +266,15 @@ def gen(R):
     return "\n".join(lines)
 
 
+def ops_per_point(R):
+    """Packed arithmetic instructions of Radix<R> per point, times 100 (the planner's cost)."""
+    if R not in RADICES and R not in RADICES2:
+        return 0
+    e = Emitter2()
+    e.dft([f"z{i}" for i in range(R)])
+    return 100 * sum(ln.count("p2_add(") + ln.count("p2_sub(") + ln.count("p2_mul(") + ln.count("p2_fma(") for ln in e.lines) // R
+
+
 def main():
     print("// GENERATED by gen_codelets.py -- do not edit.  Register-resident DFT butterflies.")
     print("#pragma once")
@@ -284,11 +295,14 @@ def main():
     print("template <int R> struct Radix;")
     print("template <> struct Radix<1> { static CVB_HD void fwd(float (&)[1], float (&)[1]) {} };")
     print()
-    for R in RADICES:
+    for R in RADICES + RADICES2:
         print(gen(R))
     print("#define CVB_FOR_EACH_RADIX(X) " + " ".join(f"X({R})" for R in RADICES))
     print("static const int kRadices[] = {" + ", ".join(str(R) for R in RADICES) + "};")
     print("static const int kNumRadices = %d;" % len(RADICES))
+    print("#define CVB_RP_EACH_RADIX(X) " + " ".join(f"X({R})" for R in sorted(RADICES + RADICES2)))
+    print("// packed operations per point of a butterfly, in hundredths; 0 = there is none")
+    print("static const int kRadixOps[33] = {" + ", ".join(str(ops_per_point(R)) for R in range(33)) + "};")
     print("}  // namespace cvb")
 
 

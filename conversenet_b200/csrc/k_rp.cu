@@ -1,0 +1,221 @@
+// Real-plane solve (cvb_rp.cuh): table build and launches.
+#include "../../include/converse_b200.h"
+#include "cvb_internal.h"
+#include "cvb_rp_plan.h"
+
+namespace cvb {
+namespace rp {
+
+int launch_cols_fwd_f32(const Params&, bool, int, size_t, cudaStream_t);
+int launch_cols_fwd_bf16(const Params&, bool, int, size_t, cudaStream_t);
+int launch_cols_inv_f32(const Params&, bool, int, size_t, cudaStream_t);
+int launch_cols_inv_bf16(const Params&, bool, int, size_t, cudaStream_t);
+int launch_epilogue_f32(const Params&, cudaStream_t);
+int launch_epilogue_bf16(const Params&, cudaStream_t);
+int launch_rows(const Params&, bool, int, size_t, cudaStream_t);
+int launch_plane_f32(const Params&, bool, int, size_t, cudaStream_t);
+int launch_plane_bf16(const Params&, bool, int, size_t, cudaStream_t);
+
+// ------------------------------------------------------------------ table
+struct TableParams {
+  const float* weight;   // (C,k,k)
+  const float* bias;     // (C)
+  float2* out;
+  int C, k, s, h, w, hh, kind;
+  float eps;
+  int tk, tf;            // tiles of 32 rows, of 16 frequencies along x
+  int r0y, r1y, r0x, r1x, ey, ex;  // plans; entries of the matrix stages (0 = none)
+  size_t tw, twy, twx, dmy, dmx;
+};
+constexpr int kTK = 32, kTF = 16;
+
+__device__ __forceinline__ double2 cmul(double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
+// exp(-2 pi i m / N)
+__device__ __forceinline__ double2 cis(long long m, int N) {
+  m %= N;
+  if (m < 0) m += N;
+  double2 r;
+  sincospi(-2.0 * (double)m / (double)N, &r.y, &r.x);
+  return r;
+}
+
+// twiddles and matrix rows behind the multiplier
+__device__ void table_tail(const TableParams& T, int i0, int step) {
+  const int nt = T.h + T.w;
+  for (int i = i0; i < 2 * nt + T.ey + T.ex; i += step) {
+    double sn, cs;
+    if (i < 2 * nt) {
+      const int t = i < nt ? i : i - nt, N = t < T.h ? T.h : T.w, n = t < T.h ? t : t - T.h;
+      const int r1 = t < T.h ? T.r1y : T.r1x, m = i < nt ? n : (n / r1) * (n % r1);   // position k0 r1 + j: k0 j
+      sincospi(2.0 * (double)m / (double)N, &sn, &cs);
+      T.out[(i < nt ? T.tw + (t < T.h ? 0 : T.h) : t < T.h ? T.twy : T.twx) + n] = make_float2((float)cs, (float)sn);
+    } else {
+      const bool y = i < 2 * nt + T.ey;
+      const int e = y ? i - 2 * nt : i - 2 * nt - T.ey, R = y ? T.r0y : T.r0x;
+      const int kp = matrix_groups(R) * 8, q = e / kp + 1, k = e % kp;
+      sincospi(2.0 * (double)((q * k) % R) / (double)R, &sn, &cs);
+      T.out[(y ? T.dmy : T.dmx) + e] = k <= R / 2 ? make_float2((float)cs, (float)sn) : make_float2(0.f, 0.f);
+    }
+  }
+}
+
+// Multiplier rows k = 0 .. h/2, [c][f][k], fp64, times 1 / (2 h w): the separated column spectra are twice the
+// transforms.  A block computes 32 rows x 16 frequencies of one channel from the separable exponentials
+//   FK[U,V] = sum_a ey^(a-c) ( sum_b K[a][b] ex^(b-c) ),  U = k + ia h, V = f + ib w,
+// whose two halves are computed once per block into shared memory.
+__global__ void __launch_bounds__(256) table_kernel(const TableParams T) {
+  extern __shared__ double2 tsm[];
+  const int tid = threadIdx.x, nb = T.C * T.tk * T.tf;
+  if (blockIdx.x >= nb) {
+    table_tail(T, (blockIdx.x - nb) * 256 + tid, (gridDim.x - nb) * 256);
+    return;
+  }
+  const int s = T.s, k = T.k, cc = k / 2, Nh = s * T.h, Nw = s * T.w;
+  const int c = blockIdx.x / (T.tk * T.tf), rest = blockIdx.x % (T.tk * T.tf);
+  const int k0 = (rest % T.tk) * kTK, f0 = (rest / T.tk) * kTF;
+  double2* tx = tsm;                       // [ib][f][a]
+  double2* ey = tx + s * kTF * k;          // [ia][row][a]
+  double2* dw = ey + s * kTK * k;          // [ib][f]
+  double2* dh = dw + s * kTF;              // [ia][row]
+  double2* lam = dh + s * kTK;
+  const float* K = T.weight + (size_t)c * k * k;
+  if (tid == 0) lam->x = 1.0 / (1.0 + exp(-((double)T.bias[c] - 9.0))) + (double)T.eps;
+  for (int i = tid; i < s * kTF * k; i += 256) {
+    const int a = i % k, f = (i / k) % kTF, ib = i / (k * kTF);
+    const int V = f0 + f + ib * T.w;
+    const double2 e = cis(V, Nw);
+    double2 p = cis(-(long long)cc * V, Nw), sum = make_double2(0.0, 0.0);
+    for (int b = 0; b < k; ++b) {
+      const double kv = (double)K[a * k + b];
+      sum.x += kv * p.x; sum.y += kv * p.y;
+      p = cmul(p, e);
+    }
+    tx[i] = sum;
+    if (a == 0) {
+      double2 d = make_double2(0.0, 0.0), q = make_double2(1.0, 0.0);
+      for (int b = 0; b < s; ++b) { d.x += q.x; d.y += q.y; q = cmul(q, e); }
+      dw[ib * kTF + f] = d;
+    }
+  }
+  for (int i = tid; i < s * kTK; i += 256) {
+    const int row = i % kTK, ia = i / kTK, U = k0 + row + ia * T.h;
+    const double2 e = cis(U, Nh);
+    double2 p = cis(-(long long)cc * U, Nh), d = make_double2(0.0, 0.0), q = make_double2(1.0, 0.0);
+    for (int a = 0; a < k; ++a) { ey[i * k + a] = p; p = cmul(p, e); }
+    for (int a = 0; a < s; ++a) { d.x += q.x; d.y += q.y; q = cmul(q, e); }
+    dh[i] = d;
+  }
+  __syncthreads();
+  const double norm = 0.5 / ((double)T.h * (double)T.w), ia2 = 1.0 / (double)(s * s);
+  for (int e = tid; e < kTK * kTF; e += 256) {
+    const int row = e % kTK, f = e / kTK;
+    if (k0 + row >= T.hh || f0 + f >= T.w) continue;
+    double nr = 0.0, ni = 0.0, den = 0.0;
+    for (int ia = 0; ia < s; ++ia)
+      for (int ib = 0; ib < s; ++ib) {
+        const double2* pe = ey + (ia * kTK + row) * k;
+        const double2* pt = tx + (ib * kTF + f) * k;
+        double fr = 0.0, fi = 0.0;
+        for (int a = 0; a < k; ++a) {
+          fr += pe[a].x * pt[a].x - pe[a].y * pt[a].y;
+          fi += pe[a].x * pt[a].y + pe[a].y * pt[a].x;
+        }
+        den += fr * fr + fi * fi;
+        if (s == 1) {
+          nr = fr; ni = -fi;
+        } else {
+          const double2 d = cmul(dh[ia * kTK + row], dw[ib * kTF + f]);
+          nr += fr * d.x - fi * d.y;
+          ni += fr * d.y + fi * d.x;
+        }
+      }
+    const double d = den * ia2 + lam->x, inv = norm / d;
+    double tr, ti;
+    if (T.kind == 1) { tr = inv; ti = 0.0; }
+    else if (s == 1) { tr = (nr + lam->x) * inv; ti = ni * inv; }
+    else { tr = (1.0 - nr * ia2) * inv; ti = -ni * ia2 * inv; }
+    T.out[((size_t)c * T.w + f0 + f) * T.hh + k0 + row] = make_float2((float)tr, (float)ti);
+  }
+}
+
+// scales whose alias arrays do not fit the tiled kernel's shared memory: one thread per entry
+__global__ void table_slow_kernel(const TransferParams S, const TableParams T) {
+  const size_t total = (size_t)T.C * T.w * T.hh;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+    const int k = (int)(i % T.hh);
+    const size_t rest = i / T.hh;
+    double tr, ti;
+    transfer_value_slow(S, (int)(rest / T.w), k, (int)(rest % T.w), tr, ti);
+    const double norm = 0.5 / ((double)T.h * (double)T.w);
+    T.out[i] = make_float2((float)(tr * norm), (float)(ti * norm));
+  }
+  table_tail(T, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
+size_t table_bytes(int C, int h, int w) {
+  int r0y, r1y, r0x, r1x;
+  if (!axis_plan(h, r0y, r1y) || !axis_plan(w, r0x, r1x)) return 0;
+  return blob_layout(C, h, w, r0y, r0x).total * sizeof(float2);
+}
+
+int build_table(const float* weight, const float* bias, int C, int k, int s, int h, int w, float eps, int kind,
+                void* table, cudaStream_t st) {
+  int r0y, r1y, r0x, r1x;
+  if (!axis_plan(h, r0y, r1y) || !axis_plan(w, r0x, r1x)) return CVB_ERR_UNSUPPORTED_SIZE;
+  const Blob bl = blob_layout(C, h, w, r0y, r0x);
+  TableParams T;
+  T.weight = weight; T.bias = bias; T.out = (float2*)table;
+  T.C = C; T.k = k; T.s = s; T.h = h; T.w = w; T.hh = h / 2 + 1; T.kind = kind; T.eps = eps;
+  T.tk = (T.hh + kTK - 1) / kTK; T.tf = (w + kTF - 1) / kTF;
+  T.r0y = r0y; T.r1y = r1y; T.r0x = r0x; T.r1x = r1x; T.ey = matrix_entries(r0y); T.ex = matrix_entries(r0x);
+  T.tw = bl.tw; T.twy = bl.twy; T.twx = bl.twx; T.dmy = bl.dmy; T.dmx = bl.dmx;
+  const int tail = (2 * (h + w) + T.ey + T.ex + 255) / 256;
+  const size_t smem = (size_t)(s * (kTF + kTK) * (k + 1) + 1) * sizeof(double2);
+  const long long nblk = (long long)C * T.tk * T.tf;
+  if (nblk + tail > 0x7fffffffLL) return CVB_ERR_TOO_LARGE;
+  if (smem <= 48 * 1024) {
+    table_kernel<<<(int)nblk + tail, 256, smem, st>>>(T);
+  } else {
+    TransferParams S;
+    memset(&S, 0, sizeof(S));
+    S.weight = weight; S.bias = bias; S.C = C; S.k = k; S.s = s; S.h = h; S.w = w; S.eps = eps; S.kind = kind;
+    table_slow_kernel<<<148 * 16, 128, 0, st>>>(S, T);
+  }
+  CVB_CUDA(cudaGetLastError());
+  return CVB_OK;
+}
+
+// ------------------------------------------------------------------ forward
+int run(Params& P, const Route& r, int io_dtype, void* workspace, size_t ws_bytes, cudaStream_t st) {
+  const bool f32 = io_dtype == CVB_F32;
+  const int planes = P.B * P.C;
+  P.vec = P.p % 2 == 0 && P.W % 2 == 0 && (((size_t)P.out) | ((size_t)P.x)) % (f32 ? 8 : 4) == 0;
+  if (r.one_block) {
+    P.plane0 = 0; P.nplane = planes;
+    const size_t smem = plane_smem(P.h, P.w, P.k);
+    const bool small = small_axis(P.ay) && small_axis(P.ax);
+    return f32 ? launch_plane_f32(P, small, plane_threads(P), smem, st) : launch_plane_bf16(P, small, plane_threads(P), smem, st);
+  }
+  if (r.chunk < 1) return CVB_ERR_TOO_LARGE;
+  if (!workspace || ws_bytes < r.ws_bytes) return CVB_ERR_WORKSPACE;
+  const size_t smem_c = cols_smem(P), smem_r = rows_smem(P);
+  if (smem_c > kSmemLimit || smem_r > kSmemLimit) return CVB_ERR_UNSUPPORTED_SIZE;
+  const bool sy = small_axis(P.ay) && P.lsh_c == 4, sx = small_axis(P.ax) && P.lsh_r == 4;
+  P.ws = (float2*)workspace;
+  for (int p0 = 0; p0 < planes; p0 += r.chunk) {
+    P.plane0 = p0;
+    P.nplane = planes - p0 < r.chunk ? planes - p0 : r.chunk;
+    if (P.s > 1) P.r = (float*)((char*)workspace + (size_t)P.nplane * P.hh * P.wp * sizeof(float2));
+    const int gc = (P.nplane * P.wc + (1 << P.lsh_c) - 1) >> P.lsh_c;
+    const int gr = (P.nplane * P.hh + (1 << P.lsh_r) - 1) >> P.lsh_r;
+    int rc = f32 ? launch_cols_fwd_f32(P, sy, gc, smem_c, st) : launch_cols_fwd_bf16(P, sy, gc, smem_c, st);
+    if (rc == CVB_OK) rc = launch_rows(P, sx, gr, smem_r, st);
+    if (rc == CVB_OK) rc = f32 ? launch_cols_inv_f32(P, sy, gc, smem_c, st) : launch_cols_inv_bf16(P, sy, gc, smem_c, st);
+    if (rc == CVB_OK && P.s > 1) rc = f32 ? launch_epilogue_f32(P, st) : launch_epilogue_bf16(P, st);
+    if (rc != CVB_OK) return rc;
+  }
+  return CVB_OK;
+}
+
+}  // namespace rp
+}  // namespace cvb

@@ -1,0 +1,33 @@
+// Row kernel of the real-plane solve (cvb_rp.cuh), multi-launch form.
+#include "../../include/converse_b200.h"
+#include "cvb_internal.h"
+#include "cvb_rp.cuh"
+
+namespace cvb {
+namespace rp {
+
+__global__ void __launch_bounds__(128, 6) rows_small_kernel(const __grid_constant__ Params P) {
+  extern __shared__ float2 smem[];
+  rows_body<kSmallRadix, 4>(P, smem);
+}
+template <int CSH>
+__global__ void __launch_bounds__(256, 2) rows_kernel(const __grid_constant__ Params P) {
+  extern __shared__ float2 smem[];
+  rows_body<kAnyRadix, CSH>(P, smem);
+}
+
+template <typename K>
+static int go(K kernel, const Params& P, int grid, int threads, size_t smem, cudaStream_t st) {
+  CVB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel<<<grid, threads, smem, st>>>(P);
+  CVB_CUDA(cudaGetLastError());
+  return CVB_OK;
+}
+int launch_rows(const Params& P, bool small, int grid, size_t smem, cudaStream_t st) {
+  if (small) return go(rows_small_kernel, P, grid, 128, smem, st);
+  if (P.lsh_r == 4) return go(rows_kernel<4>, P, grid, 256, smem, st);
+  return go(rows_kernel<-1>, P, grid, 256, smem, st);
+}
+
+}  // namespace rp
+}  // namespace cvb

@@ -199,7 +199,7 @@ int launch_t(const FwdParams& P, void* workspace, size_t ws_bytes, cudaStream_t 
 // device with that device current.
 static __device__ __align__(256) unsigned char g_static_scratch[CVB_STATIC_SCRATCH_BYTES];
 
-static int static_scratch_address(void** out) {
+int static_scratch_address(void** out) {
   static void* ptrs[64] = {nullptr};
   int dev = 0;
   CVB_CUDA(cudaGetDevice(&dev));
