@@ -43,6 +43,9 @@ STRIP2_PLANS = [
 # multi-pass kernels, and therefore not listed: 66 (264), 130 (520).
 GEMM_PLANS = [67, 128, 129]
 
+# Widths of the matrix stage (CVB_RP_EACH_WIDTH in cvb_rp.cuh)
+MATRIX_WIDTHS = [20, 24, 32, 36, 44, 56, 64]
+
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC"] + os.environ.get("CVB_NVCC_DEFS", "").split()   # e.g. -DCVB_TUNING for tuning builds
 
@@ -88,6 +91,8 @@ def _units():
     for name, io in (("f32", "float"), ("bf16", "__nv_bfloat16")):
         for unit in ("k_rp_cols", "k_rp_plane"):
             units.append(("%s_%s" % (unit, name), unit + ".cu", ["-DCVB_IO=" + io, "-DCVB_IO_NAME=" + name]))
+    for width in MATRIX_WIDTHS:
+        units.append(("k_rp_matrix_%d" % width, "k_rp_matrix.cu", ["-DCVB_MP=%d" % width]))
     for (a, b, c, d, nt, mb) in STATIC_PLANS:
         units.append(("k_static_%d_%d_%d_%d_%d_%d" % (a, b, c, d, nt, mb), "k_static.cu",
                       ["-DCVB_RY0=%d" % a, "-DCVB_RY1=%d" % b, "-DCVB_RX0=%d" % c, "-DCVB_RX1=%d" % d,

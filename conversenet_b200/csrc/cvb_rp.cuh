@@ -31,10 +31,10 @@ namespace rp {
 
 struct Axis {
   int n, r0, r1;
-  int nkg;              // 0: R0 is a register butterfly; else groups of 8 k of the matrix stage
+  int mp;               // 0: R0 is a register butterfly; else the width of the matrix stage's rows
   float inv_r1;
   const float2* tw;     // twiddles in position order: [k0 r1 + j] = (cos, sin)(2 pi k0 j / n)
-  const float2* dm;     // matrix stage: [q = 1 ..][k < 8 nkg] (cos, sin)(2 pi q k / R0)
+  const float* dm;      // matrix stage: cos(2 pi q k / R0) as [k = 0 .. R0/2][q = 1 .. mp], then sin likewise
 };
 
 struct Params {
@@ -46,7 +46,6 @@ struct Params {
   int h, w, hh, wc, wp; // hh = h / 2 + 1 rows, wc column pairs, wp = 2 wc
   int conj;             // 1: multiply by the conjugated table (the adjoint)
   int plane0, nplane;   // planes of this launch (plane = b * C + c)
-  int lsh_c, lsh_r;     // log2 of the lines per block, column / row kernels
   int vec;              // p and W even, pointers aligned: pairs of columns are loaded and stored at once
   float2* ws;           // [nplane][hh][wp]
   float* r;             // scale >= 2: [nplane][h][wp]
@@ -55,16 +54,26 @@ struct Params {
   Axis ay, ax;
 };
 
-// groups of 8 outputs of an R0-point matrix stage; 0: R0 has a register butterfly
 __host__ __device__ constexpr bool register_radix(int r) {
 #define CVB_RP_X(R) r == R ||
   return CVB_RP_EACH_RADIX(CVB_RP_X) false;
 #undef CVB_RP_X
 }
-__host__ __device__ constexpr int matrix_groups(int r0) { return register_radix(r0) ? 0 : (r0 / 2 + 1 + 7) / 8; }
+// Widths the matrix stage is built for (pairs q, R - q held in registers), and the one R0 takes: 0 = a register butterfly
+#define CVB_RP_EACH_WIDTH(X) X(20) X(24) X(32) X(36) X(44) X(56) X(64)
+__host__ __device__ constexpr int matrix_width(int r0) {
+  if (register_radix(r0)) return 0;
+#define CVB_RP_X(M) if (r0 / 2 <= M) return M;
+  CVB_RP_EACH_WIDTH(CVB_RP_X)
+#undef CVB_RP_X
+  return -1;
+}
 
-// Two builds of every kernel: radices up to kSmallRadix (80 registers a thread) and all radices.
-constexpr int kSmallRadix = 20, kAnyRadix = 32;
+// Builds of every kernel: both radices up to kSmallRadix (80 registers a thread); up to kAnyRadix; a matrix stage of a
+// given width with R1 up to kMatrixR1.
+constexpr int kSmallRadix = 20, kAnyRadix = 32, kMatrixR1 = 16;
+
+constexpr int kLinesLog2 = 4, kLines = 16;   // lines (column pairs, rows) of a block of the strip kernels
 
 template <int R> struct IC { static constexpr int value = R; };
 
@@ -106,88 +115,90 @@ __device__ __forceinline__ void twiddle(float (&re)[R], float (&im)[R], const fl
 }
 
 // ------------------------------------------------------------------ matrix stage
-// R-point transforms of nvec vectors: in(v, q) reads element q of vector v, put(v, k, value) takes element k.
-// A thread computes 8 outputs k and their mirrors R - k of VT vectors from the sums and differences of the pairs
-// (q, R - q): 4 FMAs per (k, q) and vector; the cosine / sine row of a q is the same for the whole warp and is
-// read through L1.  INPLACE: put overwrites what in reads, with a block barrier between (a round covers whole
-// vectors).
-template <bool INPLACE, int VT, class In, class Put>
-__device__ __forceinline__ void matrix_rounds(const Axis& ax, int nvec, In in, Put put) {
-  const int R = ax.r0, nkg = ax.nkg, tid = threadIdx.x, nthr = blockDim.x;
-  int vc = nthr / nkg;
-  if (vc >= 32) vc &= ~15;
-  const int want = ((nvec + VT - 1) / VT + 15) & ~15;
-  if (want < vc) vc = want;
-  const int kg = tid / vc, vl = tid - kg * vc;
-  const int QH = (R - 1) >> 1, KH = R >> 1;
-  const bool even = (R & 1) == 0;
-  for (int v0 = 0; v0 < nvec; v0 += VT * vc) {
-    int v[VT];
-    const bool act = kg < nkg && v0 + vl < nvec;
-    bool last = false;
+// R-point transforms of nvec vectors in shared memory, in place; vector v has its elements at base(v)[q * stride].
+// With p_q = x_q + x_(R-q), m_q = x_q - x_(R-q):  X_k = a_k - i b_k, X_(R-k) = a_k + i b_k,
+// a_k = x_0 + sum_q cos(2 pi q k / R) p_q,  b_k = sum_q sin(2 pi q k / R) m_q.  One thread keeps the p (or the m) of a
+// vector in registers and runs over the k: two FMAs per (k, q), the cosines four at a time from shared memory.  Element
+// k then holds a_k and element R - k holds b_k (matrix_value puts them together), so that the two threads of a vector
+// never have to meet.  FMA-bound by construction: about R FMAs per point.
+template <int MP, class Base>
+__device__ __forceinline__ void matrix_stage(int R, int nvec, int stride, const float* mats, Base base) {
+  const int tid = threadIdx.x, half = blockDim.x >> 1;
+  int nvr = (nvec + 15) & ~15;
+  if (nvr > half) nvr = half;
+  const int ng = half / nvr;                       // groups of k, when there are few vectors
+  const int g = tid / nvr, vl = tid - g * nvr, side = g & 1, kg = g >> 1;
+  const int KH = R >> 1, QH = (R - 1) >> 1;
+  const int kper = (KH + ng) / ng;                 // rows k = 0 .. KH over the groups
+  const float* mat = mats + (side ? (KH + 1) * MP : 0);
+  for (int v0 = 0; v0 < nvec; v0 += nvr) {
+    const bool act = v0 + vl < nvec && kg < ng;
+    float2* x = base(act ? v0 + vl : 0);
+    float2 p[MP];
+    const float2 x0 = side ? make_float2(0.f, 0.f) : x[0];
 #pragma unroll
-    for (int t = 0; t < VT; ++t) {
-      v[t] = v0 + vl + t * vc;
-      if (v[t] >= nvec) { v[t] = v0 + vl; last = true; }   // computed twice, written once
-    }
-    float ar[VT][8], ai[VT][8], br[VT][8], bi[VT][8];
-    if (act) {
-#pragma unroll
-      for (int t = 0; t < VT; ++t) {
-        const float2 x0 = in(v[t], 0);
-        float2 xh = make_float2(0.f, 0.f);
-        if (even) xh = in(v[t], KH);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float sg = (i & 1) ? -1.f : 1.f;
-          ar[t][i] = fmaf(sg, xh.x, x0.x); ai[t][i] = fmaf(sg, xh.y, x0.y);
-          br[t][i] = 0.f; bi[t][i] = 0.f;
-        }
-      }
-      const float4* d = (const float4*)(ax.dm + kg * 8);
-      const int dstep = nkg * 4;
-#pragma unroll 2
-      for (int q = 1; q <= QH; ++q, d += dstep) {
-        float pr[VT], pi[VT], mr[VT], mi[VT];
-#pragma unroll
-        for (int t = 0; t < VT; ++t) {
-          const float2 u = in(v[t], q), w = in(v[t], R - q);
-          pr[t] = u.x + w.x; pi[t] = u.y + w.y; mr[t] = u.x - w.x; mi[t] = u.y - w.y;
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 c = __ldg(d + i);
-#pragma unroll
-          for (int t = 0; t < VT; ++t) {
-            ar[t][2 * i] = fmaf(c.x, pr[t], ar[t][2 * i]);         ai[t][2 * i] = fmaf(c.x, pi[t], ai[t][2 * i]);
-            br[t][2 * i] = fmaf(c.y, mr[t], br[t][2 * i]);         bi[t][2 * i] = fmaf(c.y, mi[t], bi[t][2 * i]);
-            ar[t][2 * i + 1] = fmaf(c.z, pr[t], ar[t][2 * i + 1]); ai[t][2 * i + 1] = fmaf(c.z, pi[t], ai[t][2 * i + 1]);
-            br[t][2 * i + 1] = fmaf(c.w, mr[t], br[t][2 * i + 1]); bi[t][2 * i + 1] = fmaf(c.w, mi[t], bi[t][2 * i + 1]);
-          }
-        }
+    for (int q = 1; q <= MP; ++q) {
+      p[q - 1] = make_float2(0.f, 0.f);
+      if (q <= QH) {
+        const float2 u = x[q * stride], w = x[(R - q) * stride];
+        p[q - 1] = side ? make_float2(u.x - w.x, u.y - w.y) : make_float2(u.x + w.x, u.y + w.y);
+      } else if (q == KH) {                        // even R: the middle element, cosines only
+        if (!side) p[q - 1] = x[q * stride];
       }
     }
-    if (INPLACE) __syncthreads();
+    __syncthreads();
     if (act) {
+      const int k0 = kg * kper > side ? kg * kper : side, k1 = (kg + 1) * kper < KH + 1 ? (kg + 1) * kper : KH + 1;
+      const int kend = side && k1 > QH + 1 ? QH + 1 : k1;
+      for (int k = k0; k < kend; ++k) {
+        const float4* c4 = (const float4*)(mat + k * MP);
+        float r0 = x0.x, i0 = x0.y, r1 = 0.f, i1 = 0.f;
 #pragma unroll
-      for (int t = 0; t < VT; ++t) {
-        if (t > 0 && last && v[t] == v0 + vl) continue;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int k = kg * 8 + i;
-          if (k <= KH) {
-            put(v[t], k, make_float2(ar[t][i] + bi[t][i], ai[t][i] - br[t][i]));
-            if (k != 0 && 2 * k != R) put(v[t], R - k, make_float2(ar[t][i] - bi[t][i], ai[t][i] + br[t][i]));
-          }
+        for (int q = 0; q < MP; q += 4) {
+          const float4 c = c4[q >> 2];
+          r0 = fmaf(c.x, p[q].x, r0);     i0 = fmaf(c.x, p[q].y, i0);
+          r1 = fmaf(c.y, p[q + 1].x, r1); i1 = fmaf(c.y, p[q + 1].y, i1);
+          r0 = fmaf(c.z, p[q + 2].x, r0); i0 = fmaf(c.z, p[q + 2].y, i0);
+          r1 = fmaf(c.w, p[q + 3].x, r1); i1 = fmaf(c.w, p[q + 3].y, i1);
         }
+        x[(side ? R - k : k) * stride] = make_float2(r0 + r1, i0 + i1);
       }
     }
   }
 }
-template <bool INPLACE, class In, class Put>
-__device__ __forceinline__ void matrix_stage(const Axis& ax, int nvec, In in, Put put) {
-  if (nvec * ax.nkg > (int)blockDim.x) matrix_rounds<INPLACE, 2>(ax, nvec, in, put);
-  else matrix_rounds<INPLACE, 1>(ax, nvec, in, put);
+// element k of the transform from what matrix_stage leaves
+__device__ __forceinline__ float2 matrix_value(const float2* x, int R, int k, int stride) {
+  if (k == 0 || 2 * k == R) return x[k * stride];
+  const bool mir = 2 * k > R;
+  const float2 a = x[(mir ? R - k : k) * stride], b = x[(mir ? k : R - k) * stride];
+  return mir ? make_float2(a.x - b.y, a.y + b.x) : make_float2(a.x + b.y, a.y - b.x);
+}
+// the R elements j = 0 .. R-1 of position kk (side 0) or r0 - kk (side 1), elements j at x + (j << sh)
+template <int R>
+__device__ __forceinline__ void load_matrix(const float2* x, int r0, int kk, int side, int stride, int sh, bool in,
+                                            float (&re)[R], float (&im)[R]) {
+  if (!in || kk == 0 || 2 * kk == r0) {
+    const float2* a = x + (in ? kk : 0) * stride;
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const float2 v = a[j << sh];
+      re[j] = v.x; im[j] = v.y;
+    }
+  } else {
+    const float2* a = x + kk * stride;
+    const float2* b = x + (r0 - kk) * stride;
+    const float sg = side ? -1.f : 1.f;
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const float2 u = a[j << sh], v = b[j << sh];
+      re[j] = fmaf(sg, v.y, u.x); im[j] = fmaf(-sg, v.x, u.y);
+    }
+  }
+}
+template <int MP>
+__device__ __forceinline__ void copy_matrices(float* dst, const Axis& a) {
+  const int n = 2 * (a.r0 / 2 + 1) * MP / 4;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) ((float4*)dst)[i] = __ldg((const float4*)a.dm + i);
 }
 
 // Two adjacent padded columns of one plane: what a thread reads in every row it visits.
@@ -271,12 +282,13 @@ __device__ __forceinline__ void store_crop(const Params& P, IO* op, int y, int c
 }
 
 // ------------------------------------------------------------------ columns forward: x -> S^
-// CSH: log2 of the lines of a block, or -1 for the run-time value.  Shared memory: the tile [pos][line], then the row
-// offsets.  Lanes run along the lines, so every access of a half warp is one contiguous piece of a row.
-template <typename IO, int MAXR, int CSH>
+// A block takes 16 lines.  Shared memory: the tile [pos][line], then the row offsets.  Lanes run along the lines, so
+// every access of a half warp is one contiguous piece of a row.
+// MP > 0: the R0 points are a matrix stage of that width; its matrices follow the row offsets.
+template <typename IO, int MAXR, int MP>
 __device__ __forceinline__ void cols_fwd_body(const Params& P, float2* T) {
   const int tid = threadIdx.x, nthr = blockDim.x;
-  const int sh = CSH >= 0 ? CSH : P.lsh_c, NL = 1 << sh;
+  constexpr int sh = kLinesLog2, NL = kLines;
   const int l = tid & (NL - 1);
   const int gl = blockIdx.x * NL + l;
   const bool valid = gl < P.nplane * P.wc;
@@ -288,8 +300,10 @@ __device__ __forceinline__ void cols_fwd_body(const Params& P, float2* T) {
   float2* Tl = T + l;
   int* rowoff = (int*)(T + ((size_t)P.h << sh));
   for (int y = tid; y < P.h; y += nthr) rowoff[y] = row_offset(P, y);
+  float* mats = (float*)(rowoff + ((P.h + 3) & ~3));
+  if constexpr (MP > 0) copy_matrices<MP>(mats, ay);
   __syncthreads();
-  if (MAXR <= kSmallRadix || ay.nkg == 0) {
+  if constexpr (MP == 0) {
     dispatch<MAXR>(r0, [&](auto ic) {
       constexpr int R = decltype(ic)::value;
       for (int j = tid >> sh; j < r1; j += nthr >> sh) {
@@ -317,10 +331,8 @@ __device__ __forceinline__ void cols_fwd_body(const Params& P, float2* T) {
       }
     }
     __syncthreads();
-    // vector v = (j, line): elements (j + r1 q, line) in, (k r1 + j, line) out -- the same set of cells
-    matrix_stage<true>(ay, r1 << sh,
-                       [&](int v, int q) { return T[v + ((r1 * q) << sh)]; },
-                       [&](int v, int k, float2 z) { T[v + ((r1 * k) << sh)] = z; });
+    // vector v = (j, line): elements (j + r1 q, line) become (k r1 + j, line), the same cells
+    matrix_stage<MP>(r0, r1 << sh, r1 << sh, mats, [&](int v) { return T + v; });
   }
   __syncthreads();
   // radix R1; lanes with bit `sh` clear hold k0 = kk, those with it set R0 - kk, so that Z[k] and Z[-k] are
@@ -338,10 +350,14 @@ __device__ __forceinline__ void cols_fwd_body(const Params& P, float2* T) {
       const int k0 = !in || kk == 0 ? 0 : side ? r0 - kk : kk;
       float re[R], im[R];
       const float2* tp = Tl + ((k0 * r1) << sh);
+      if constexpr (MP == 0) {
 #pragma unroll
-      for (int j = 0; j < R; ++j) {
-        const float2 v = tp[j << sh];
-        re[j] = v.x; im[j] = v.y;
+        for (int j = 0; j < R; ++j) {
+          const float2 v = tp[j << sh];
+          re[j] = v.x; im[j] = v.y;
+        }
+      } else {
+        load_matrix<R>(Tl, r0, kk, side, r1 << sh, sh, in, re, im);
       }
       twiddle<R>(re, im, ay.tw + k0 * r1);
       Radix<R>::fwd(re, im);
@@ -351,8 +367,8 @@ __device__ __forceinline__ void cols_fwd_body(const Params& P, float2* T) {
       auto put = [&](int j2, float wx, float wy) {
         *(float4*)(wr + j2 * ws) = make_float4(re[j2] + wx, im[j2] - wy, im[j2] + wy, wx - re[j2]);
       };
-      // all 16 lines of a warp share kk when a block has 16 lines: the branches are then warp-uniform
-      if (CSH == 4 && self) {
+      if (self) {        // warp-uniform: a warp is 16 lines x 2 sides of one kk
+
         if (st) {
           if (kk == 0) {
 #pragma unroll
@@ -365,26 +381,21 @@ __device__ __forceinline__ void cols_fwd_body(const Params& P, float2* T) {
       } else {
 #pragma unroll
         for (int j2 = 0; j2 < JH; ++j2) {
-          float wx = __shfl_xor_sync(0xffffffffu, re[R - 1 - j2], NL);
-          float wy = __shfl_xor_sync(0xffffffffu, im[R - 1 - j2], NL);
-          if (CSH != 4) {
-            if (self) { wx = re[R - 1 - j2]; wy = im[R - 1 - j2]; }
-            if (kk == 0) { wx = re[(R - j2) % R]; wy = im[(R - j2) % R]; }
-          }
+          const float wx = __shfl_xor_sync(0xffffffffu, re[R - 1 - j2], NL);
+          const float wy = __shfl_xor_sync(0xffffffffu, im[R - 1 - j2], NL);
           if (st && !((R & 1) && j2 == JH - 1 && side)) put(j2, wx, wy);
         }
-        if (CSH != 4 && (R & 1) == 0 && kk == 0 && st) put(R / 2, re[R / 2], im[R / 2]);
       }
     }
   });
 }
 
 // ------------------------------------------------------------------ rows: S^ -> . table -> U, in place
-// R1-point butterfly of row `row` at k0, multiply, conjugate, R1-point butterfly, in place in shared memory
+// R1-point butterfly of a row at k0, multiply, conjugate, R1-point butterfly, to shared memory
 template <int R>
-__device__ __forceinline__ void rows_mid(const Params& P, float2* Tk, const float2* tab, int k0) {
+__device__ __forceinline__ void rows_mid(const Params& P, float (&re)[R], float (&im)[R], float2* Tk, const float2* tab,
+                                         int k0) {
   const Axis& ax = P.ax;
-  float re[R], im[R];
   const size_t ts = (size_t)ax.r0 * P.hh;
   const float2* tp = tab + (size_t)k0 * P.hh;
   const float2* tw = ax.tw + k0 * ax.r1;
@@ -393,11 +404,6 @@ __device__ __forceinline__ void rows_mid(const Params& P, float2* Tk, const floa
   if (kAhead) {
 #pragma unroll
     for (int j2 = 0; j2 < R; ++j2) g[j2] = __ldg(tp + j2 * ts);
-  }
-#pragma unroll
-  for (int j = 0; j < R; ++j) {
-    const float2 v = Tk[j];
-    re[j] = v.x; im[j] = v.y;
   }
   twiddle<R>(re, im, tw);
   Radix<R>::fwd(re, im);
@@ -418,17 +424,18 @@ __device__ __forceinline__ void rows_mid(const Params& P, float2* Tk, const floa
   for (int j = 0; j < R; ++j) Tk[j] = make_float2(re[j], im[j]);
 }
 
-template <int MAXR, int CSH>
+template <int MAXR, int MP>
 __device__ __forceinline__ void rows_body(const Params& P, float2* T) {
   const int tid = threadIdx.x, nthr = blockDim.x;
-  const int sh = CSH >= 0 ? CSH : P.lsh_r, NL = 1 << sh, pitch = P.pitch;
+  constexpr int sh = kLinesLog2, NL = kLines;
+  const int pitch = P.pitch;
   const Axis& ax = P.ax;
   const int r0 = ax.r0, r1 = ax.r1;
   const int row0 = blockIdx.x * NL, nrows = P.nplane * P.hh;
   const int nl = nrows - row0 < NL ? nrows - row0 : NL;
   float2* W = P.ws + (size_t)row0 * P.wp;
-  const bool matrix = MAXR > kSmallRadix && ax.nkg != 0;
-  if (!matrix) {
+  float* mats = (float*)(T + (((size_t)pitch << sh) + 1 & ~(size_t)1));
+  if constexpr (MP == 0) {
     dispatch<MAXR>(r0, [&](auto ic) {
       constexpr int R = decltype(ic)::value;
       for (int it = tid; it < nl * r1; it += nthr) {
@@ -448,6 +455,7 @@ __device__ __forceinline__ void rows_body(const Params& P, float2* T) {
       }
     });
   } else {
+    copy_matrices<MP>(mats, ax);
     // whole rows into shared memory, a warp per row
     for (int row = tid >> 5; row < nl; row += nthr >> 5) {
       const float2* src = W + (size_t)row * P.wp;
@@ -462,9 +470,7 @@ __device__ __forceinline__ void rows_body(const Params& P, float2* T) {
       }
     }
     __syncthreads();
-    matrix_stage<true>(ax, r1 << sh,
-                       [&](int v, int q) { return T[(v & (NL - 1)) * pitch + (v >> sh) + r1 * q]; },
-                       [&](int v, int k, float2 z) { T[(v & (NL - 1)) * pitch + (v >> sh) + r1 * k] = z; });
+    matrix_stage<MP>(r0, r1 << sh, r1, mats, [&](int v) { return T + (v & (NL - 1)) * pitch + (v >> sh); });
   }
   __syncthreads();
   {
@@ -475,12 +481,44 @@ __device__ __forceinline__ void rows_body(const Params& P, float2* T) {
       const float2* tab = P.tab + (size_t)c * P.w * P.hh + k;
       dispatch<MAXR>(r1, [&](auto ic) {
         constexpr int R = decltype(ic)::value;
-        for (int k0 = tid >> sh; k0 < r0; k0 += nthr >> sh) rows_mid<R>(P, T + row * pitch + k0 * r1, tab, k0);
+        if constexpr (MP == 0) {
+          for (int k0 = tid >> sh; k0 < r0; k0 += nthr >> sh) {
+            float2* Tk = T + row * pitch + k0 * r1;
+            float re[R], im[R];
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+              const float2 v = Tk[j];
+              re[j] = v.x; im[j] = v.y;
+            }
+            rows_mid<R>(P, re, im, Tk, tab, k0);
+          }
+        } else {
+          // positions kk and r0 - kk share what they read: one thread takes both
+          float2* Tr = T + row * pitch;
+          for (int kk = tid >> sh; kk <= r0 / 2; kk += nthr >> sh) {
+            const bool self = kk == 0 || 2 * kk == r0;
+            float ar[R], ai[R], br[R], bi[R];
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+              const float2 u = Tr[kk * r1 + j], v = self ? make_float2(0.f, 0.f) : Tr[(r0 - kk) * r1 + j];
+              ar[j] = u.x; ai[j] = u.y; br[j] = v.x; bi[j] = v.y;
+            }
+#pragma unroll 1
+            for (int side = 0; side < (self ? 1 : 2); ++side) {
+              const float sg = side ? -1.f : 1.f;
+              const int k0 = side ? r0 - kk : kk;
+              float re[R], im[R];
+#pragma unroll
+              for (int j = 0; j < R; ++j) { re[j] = fmaf(sg, bi[j], ar[j]); im[j] = fmaf(-sg, br[j], ai[j]); }
+              rows_mid<R>(P, re, im, Tr + k0 * r1, tab, k0);
+            }
+          }
+        }
       });
     }
   }
   __syncthreads();
-  if (!matrix) {
+  if constexpr (MP == 0) {
     dispatch<MAXR>(r0, [&](auto ic) {
       constexpr int R = decltype(ic)::value;
       for (int it = tid; it < nl * r1; it += nthr) {
@@ -500,22 +538,24 @@ __device__ __forceinline__ void rows_body(const Params& P, float2* T) {
       }
     });
   } else {
-    matrix_stage<true>(ax, r1 << sh,
-                       [&](int v, int q) { return T[(v & (NL - 1)) * pitch + (v >> sh) + r1 * q]; },
-                       [&](int v, int k, float2 z) { T[(v & (NL - 1)) * pitch + (v >> sh) + r1 * k] = z; });
+    matrix_stage<MP>(r0, r1 << sh, r1, mats, [&](int v) { return T + (v & (NL - 1)) * pitch + (v >> sh); });
     __syncthreads();
     for (int row = tid >> 5; row < nl; row += nthr >> 5) {
       float2* dst = W + (size_t)row * P.wp;
-      for (int x = tid & 31; x < P.w; x += 32) dst[x] = T[row * pitch + x];
+      for (int x = tid & 31; x < P.w; x += 32) {
+        int q, j;
+        divmod_small(x, r1, ax.inv_r1, q, j);
+        dst[x] = matrix_value(T + row * pitch + j, r0, q, r1);
+      }
     }
   }
 }
 
 // ------------------------------------------------------------------ columns inverse: U -> out (or r)
-template <typename IO, int MAXR, int CSH>
+template <typename IO, int MAXR, int MP>
 __device__ __forceinline__ void cols_inv_body(const Params& P, float2* T) {
   const int tid = threadIdx.x, nthr = blockDim.x;
-  const int sh = CSH >= 0 ? CSH : P.lsh_c, NL = 1 << sh;
+  constexpr int sh = kLinesLog2, NL = kLines;
   const int l = tid & (NL - 1);
   const int gl = blockIdx.x * NL + l;
   const bool valid = gl < P.nplane * P.wc;
@@ -524,6 +564,8 @@ __device__ __forceinline__ void cols_inv_body(const Params& P, float2* T) {
   const int r0 = ay.r0, r1 = ay.r1;
   float2* Tl = T + l;
   const float2* wl = P.ws + ((size_t)pl * P.hh) * P.wp + 2 * c;
+  float* mats = (float*)(T + ((size_t)P.h << sh));
+  if constexpr (MP > 0) copy_matrices<MP>(mats, ay);
   dispatch<MAXR>(r1, [&](auto ic) {
     constexpr int R = decltype(ic)::value;
     constexpr int JH = (R + 1) / 2;
@@ -551,7 +593,7 @@ __device__ __forceinline__ void cols_inv_body(const Params& P, float2* T) {
       auto v2y = [&](const float4& a) { return -a.y - a.z; };
 #pragma unroll
       for (int j2 = 0; j2 < JH; ++j2) { re[j2] = v1x(u[j2]); im[j2] = v1y(u[j2]); }
-      if (CSH == 4 && self) {            // warp-uniform: k0 = 0 or R0 / 2 is its own mirror
+      if (self) {            // warp-uniform: k0 = 0 or R0 / 2 is its own mirror
         if (kk == 0) {
           float4 uh = make_float4(0.f, 0.f, 0.f, 0.f);
           if ((R & 1) == 0) uh = *(const float4*)(wr + (R / 2) * ws);
@@ -563,21 +605,12 @@ __device__ __forceinline__ void cols_inv_body(const Params& P, float2* T) {
           for (int j2 = 0; j2 < R / 2; ++j2) { re[R - 1 - j2] = v2x(u[j2]); im[R - 1 - j2] = v2y(u[j2]); }
         }
       } else {
-        float4 uh = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (CSH != 4 && (R & 1) == 0 && kk == 0) uh = *(const float4*)(wr + (R / 2) * ws);
 #pragma unroll
         for (int j2 = 0; j2 < JH; ++j2) {
           const float ax_ = v2x(u[j2]), ay_ = v2y(u[j2]);
-          float wx = __shfl_xor_sync(0xffffffffu, ax_, NL);
-          float wy = __shfl_xor_sync(0xffffffffu, ay_, NL);
+          const float wx = __shfl_xor_sync(0xffffffffu, ax_, NL);
+          const float wy = __shfl_xor_sync(0xffffffffu, ay_, NL);
           if (R - 1 - j2 != j2) {
-            if (CSH != 4) {
-              const int n = j2 + 1 < JH ? j2 + 1 : j2;
-              float ox = v2x(u[n]), oy = v2y(u[n]);
-              if ((R & 1) == 0 && j2 == JH - 1) { ox = v1x(uh); oy = v1y(uh); }
-              if (self) { wx = ax_; wy = ay_; }
-              if (kk == 0) { wx = ox; wy = oy; }
-            }
             re[R - 1 - j2] = wx; im[R - 1 - j2] = wy;
           } else if (side && !self) {
             re[j2] = wx; im[j2] = wy;
@@ -594,10 +627,10 @@ __device__ __forceinline__ void cols_inv_body(const Params& P, float2* T) {
     }
   });
   __syncthreads();
-  if (MAXR <= kSmallRadix || ay.nkg == 0) {
+  IO* op = (IO*)P.out + (size_t)(P.plane0 + pl) * P.H * P.W;
+  float2* rl = (float2*)P.r + (size_t)pl * P.h * P.wc + c;
+  if constexpr (MP == 0) {
     if (!valid) return;
-    IO* op = (IO*)P.out + (size_t)(P.plane0 + pl) * P.H * P.W;
-    float2* rl = (float2*)P.r + (size_t)pl * P.h * P.wc + c;
     dispatch<MAXR>(r0, [&](auto ic) {
       constexpr int R = decltype(ic)::value;
       for (int j = tid >> sh; j < r1; j += nthr >> sh) {
@@ -618,18 +651,29 @@ __device__ __forceinline__ void cols_inv_body(const Params& P, float2* T) {
       }
     });
   } else {
-    // the matrix stage's vectors are (j, line) with any line of the block: line data are recomputed per vector
-    matrix_stage<false>(ay, r1 << sh,
-                        [&](int v, int q) { return T[v + ((q * r1) << sh)]; },
-                        [&](int v, int q, float2 z) {
-                          const int g = blockIdx.x * NL + (v & (NL - 1));
-                          if (g >= P.nplane * P.wc) return;
-                          const int vp = g / P.wc, vcol = g - vp * P.wc, y = (v >> sh) + r1 * q;
-                          if (P.s == 1)
-                            store_crop<IO>(P, (IO*)P.out + (size_t)(P.plane0 + vp) * P.H * P.W, y, vcol, z);
-                          else
-                            ((float2*)P.r)[((size_t)vp * P.h + y) * P.wc + vcol] = make_float2(z.x, -z.y);
-                        });
+    const int st = r1 << sh;
+    matrix_stage<MP>(r0, st, st, mats, [&](int v) { return T + v; });
+    __syncthreads();
+    if (!valid) return;
+    // rows q and r0 - q of a column pair from the same two cells
+    const int nq = (r0 / 2 + 1) * r1;
+    for (int it = tid >> sh; it < nq; it += nthr >> sh) {
+      int q, j;
+      divmod_small(it, r1, ay.inv_r1, q, j);
+      const float2* x = Tl + (j << sh);
+      const float2 a = x[q * st];
+      const bool self = q == 0 || 2 * q == r0;
+      const float2 b = self ? make_float2(0.f, 0.f) : x[(r0 - q) * st];
+      const float2 z0 = make_float2(a.x + b.y, a.y - b.x), z1 = make_float2(a.x - b.y, a.y + b.x);
+      const int y0 = j + r1 * q, y1 = j + r1 * (r0 - q);
+      if (P.s == 1) {
+        store_crop<IO>(P, op, y0, c, z0);
+        if (!self) store_crop<IO>(P, op, y1, c, z1);
+      } else {
+        rl[(size_t)y0 * P.wc] = make_float2(z0.x, -z0.y);
+        if (!self) rl[(size_t)y1 * P.wc] = make_float2(z1.x, -z1.y);
+      }
+    }
   }
 }
 
@@ -811,7 +855,6 @@ __device__ __forceinline__ void plane_body(const Params& P, float2* sm) {
   const IO* xp = (const IO*)P.x + (size_t)plane * P.H * P.W;
   const Axis& ay = P.ay;
   const Axis& ax = P.ax;
-  const bool my_ = MAXR > kSmallRadix && ay.nkg != 0, mx_ = MAXR > kSmallRadix && ax.nkg != 0;
   if (P.s > 1)
     for (int i = tid; i < P.k * P.k; i += nthr) wk[i] = P.weight[(size_t)ch * P.k * P.k + i];
   for (int y = tid; y < h; y += nthr) rowoff[y] = row_offset(P, y);
@@ -819,7 +862,6 @@ __device__ __forceinline__ void plane_body(const Params& P, float2* sm) {
   // ---- columns forward
   {
     const int r0 = ay.r0, r1 = ay.r1, st = r1 * wc;
-    if (!my_) {
       dispatch<MAXR>(r0, [&](auto ic) {
         constexpr int R = decltype(ic)::value;
         for (int it = tid; it < st; it += nthr) {
@@ -835,20 +877,6 @@ __device__ __forceinline__ void plane_body(const Params& P, float2* sm) {
           for (int k = 0; k < R; ++k) d[k * st] = make_float2(re[k], im[k]);
         }
       });
-    } else {
-      for (int it = tid; it < h * wc; it += nthr) {
-        int y, c;
-        divmod_small(it, wc, P.inv_wc, y, c);
-        ColumnPair<IO> cp;
-        cp.set(P, xp, c, true);
-        float re[1], im[1];
-        load_rows<1, IO>(P, cp, rowoff, y, 0, re, im);
-        T1[it] = make_float2(re[0], im[0]);
-      }
-      __syncthreads();
-      matrix_stage<true>(ay, st, [&](int v, int q) { return T1[v + q * st]; },
-                         [&](int v, int k, float2 z) { T1[v + k * st] = z; });
-    }
     __syncthreads();
     // radix R1 of k0 = kk and of its mirror R0 - kk in one thread, spectra of the two columns separated
     const int nkk = r0 / 2 + 1;
@@ -904,7 +932,6 @@ __device__ __forceinline__ void plane_body(const Params& P, float2* sm) {
     const int r0 = ax.r0, r1 = ax.r1;
     const float2* tab = P.tab + (size_t)ch * w * hh;
     auto outer = [&]() {
-      if (!mx_) {
         dispatch<MAXR>(r0, [&](auto ic) {
           constexpr int R = decltype(ic)::value;
           for (int it = tid; it < hh * r1; it += nthr) {
@@ -922,11 +949,6 @@ __device__ __forceinline__ void plane_body(const Params& P, float2* sm) {
             for (int k = 0; k < R; ++k) d[k * r1] = make_float2(re[k], im[k]);
           }
         });
-      } else {
-        matrix_stage<true>(ax, r1 * hh,
-                           [&](int v, int q) { int j, row; divmod_small(v, hh, P.inv_hh, j, row); return T2[row * pitch + j + r1 * q]; },
-                           [&](int v, int k, float2 z) { int j, row; divmod_small(v, hh, P.inv_hh, j, row); T2[row * pitch + j + r1 * k] = z; });
-      }
       __syncthreads();
     };
     // the two outer passes share one copy of the butterfly code
@@ -939,7 +961,14 @@ __device__ __forceinline__ void plane_body(const Params& P, float2* sm) {
           for (int it = tid; it < r0 * hh; it += nthr) {
             int k0, row;
             divmod_small(it, hh, P.inv_hh, k0, row);
-            rows_mid<R>(P, T2 + row * pitch + k0 * r1, tab + row, k0);
+            float2* Tk = T2 + row * pitch + k0 * r1;
+            float re[R], im[R];
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+              const float2 v = Tk[j];
+              re[j] = v.x; im[j] = v.y;
+            }
+            rows_mid<R>(P, re, im, Tk, tab + row, k0);
           }
         });
         __syncthreads();
@@ -1005,7 +1034,6 @@ __device__ __forceinline__ void plane_body(const Params& P, float2* sm) {
     });
     __syncthreads();
     IO* op = (IO*)P.out + (size_t)plane * P.H * P.W * P.s * P.s;
-    if (!my_) {
       dispatch<MAXR>(r0, [&](auto ic) {
         constexpr int R = decltype(ic)::value;
         for (int it = tid; it < st; it += nthr) {
@@ -1028,17 +1056,6 @@ __device__ __forceinline__ void plane_body(const Params& P, float2* sm) {
           }
         }
       });
-    } else if (P.s == 1) {
-      matrix_stage<false>(ay, st, [&](int v, int q) { return T1[v + q * st]; },
-                          [&](int v, int q, float2 z) {
-                            int j, c;
-                            divmod_small(v, wc, P.inv_wc, j, c);
-                            store_crop<IO>(P, op, j + r1 * q, c, z);
-                          });
-    } else {
-      matrix_stage<true>(ay, st, [&](int v, int q) { return T1[v + q * st]; },
-                         [&](int v, int q, float2 z) { T1[v + q * st] = make_float2(z.x, -z.y); });
-    }
     if (P.s > 1) {
       __syncthreads();
       epilogue<IO>(P, (const float*)T1, 2 * wc, wk, xp, op, tid, nthr, 0, P.H);

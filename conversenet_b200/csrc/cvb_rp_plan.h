@@ -7,22 +7,22 @@ namespace cvb {
 namespace rp {
 
 constexpr int kMatrixMax = 127;   // largest R0 of the matrix stage
+constexpr int kMatrixN = 1300;    //   and the longest axis whose tile and matrices fit shared memory
 constexpr int kMaxR1 = 26;        // (separating the spectra keeps 2 R1 values in a thread: small ones are cheaper)
 
 // N = R0 * R1 with the lowest estimated cost per point: packed butterfly operations plus about nine instructions of
-// loads, stores and twiddles a stage; a matrix stage costs R0 FMAs a point (two packed operations each, at the
-// efficiency measured for it).  Radices above 16 keep more values in registers than three blocks an SM allow.
+// loads, stores and twiddles a stage; a matrix stage costs R0 FMAs a point.  Radices above kSmallRadix take the
+// kernels with fewer resident warps.
 inline bool axis_plan(int n, int& r0, int& r1) {
   double best = 1e30;
-  auto codelet = [](int r) { return register_radix(r); };
   auto cost = [&](int r) { return 9.0 + kRadixOps[r] * 0.01 + (r > 16 ? 0.25 * (r - 16) : 0.0) + (r > kSmallRadix ? 2.0 : 0.0); };
   for (int b = 1; b <= kMaxR1 && b <= n; ++b) {
-    if (n % b || (b > 1 && !codelet(b))) continue;
+    if (n % b || (b > 1 && !register_radix(b))) continue;
     const int a = n / b;
     if (a < 2) continue;
     double c = b == 1 ? 6.0 : cost(b) + (b > 10 ? 0.3 * (b - 10) : 0.0);
-    if (codelet(a)) c += cost(a);
-    else if (a >= 3 && a <= kMatrixMax) c += 16.0 + 0.75 * a;
+    if (register_radix(a)) c += cost(a);
+    else if (a <= kMatrixMax && b <= kMatrixR1 && n <= kMatrixN) c += 20.0 + 1.2 * matrix_width(a) * 2;
     else continue;
     if (c < best) { best = c; r0 = a; r1 = b; }
   }
@@ -34,7 +34,7 @@ inline bool supported(int h, int w) {
   return h >= 2 && w >= 2 && axis_plan(h, a, b) && axis_plan(w, a, b);
 }
 
-inline int matrix_entries(int r0) { return ((r0 - 1) / 2) * matrix_groups(r0) * 8; }   // float2
+inline int matrix_entries(int r0) { return 2 * (r0 / 2 + 1) * matrix_width(r0); }   // floats, a multiple of 8
 
 // Blob in float2 units: multiplier [C][w][hh]; twiddles of h and of w in natural order (tw), then in position order
 // (twy, twx); matrix rows of R0(h) and of R0(w)
@@ -45,27 +45,27 @@ inline Blob blob_layout(int C, int h, int w, int r0y, int r0x) {
   b.twy = (b.tw + h + w + 1) & ~(size_t)1;
   b.twx = (b.twy + h + 1) & ~(size_t)1;
   b.dmy = (b.twx + w + 1) & ~(size_t)1;
-  b.dmx = b.dmy + matrix_entries(r0y);
-  b.total = b.dmx + matrix_entries(r0x);
+  b.dmx = b.dmy + matrix_entries(r0y) / 2;
+  b.total = b.dmx + matrix_entries(r0x) / 2;
   return b;
 }
 
 inline void fill_axis(Axis& a, int n, int r0, int r1, const float2* tw, const float2* dm) {
   a.n = n; a.r0 = r0; a.r1 = r1;
-  a.nkg = matrix_groups(r0);
+  a.mp = matrix_width(r0);
   a.inv_r1 = 1.0f / (float)r1;
-  a.tw = tw; a.dm = dm;
+  a.tw = tw; a.dm = (const float*)dm;
 }
 
-inline int lines_log2(int bytes_per_line) {   // widest strip of 16 / 8 / 4 lines with two blocks on an SM
-  for (int s = 4; s > 2; --s)
-    if ((bytes_per_line << s) <= 104 * 1024) return s;
-  return 2;
+inline size_t cols_smem(const Params& P) {
+  return (size_t)P.h * kLines * sizeof(float2) + (size_t)((P.h + 3) & ~3) * sizeof(int) +
+         (P.ay.mp ? matrix_entries(P.ay.r0) : 0) * sizeof(float);
 }
-inline size_t cols_smem(const Params& P) { return ((size_t)P.h << P.lsh_c) * sizeof(float2) + (size_t)P.h * sizeof(int); }
-inline size_t rows_smem(const Params& P) { return ((size_t)P.pitch << P.lsh_r) * sizeof(float2); }
+inline size_t rows_smem(const Params& P) {
+  return (((size_t)P.pitch * kLines + 1) & ~(size_t)1) * sizeof(float2) + (P.ax.mp ? matrix_entries(P.ax.r0) : 0) * sizeof(float);
+}
 // kernels built for small radices serve an axis whose two radices are small
-inline bool small_axis(const Axis& a) { return a.nkg == 0 && a.r0 <= kSmallRadix && a.r1 <= kSmallRadix; }
+inline bool small_axis(const Axis& a) { return a.mp == 0 && a.r0 <= kSmallRadix && a.r1 <= kSmallRadix; }
 
 inline size_t plane_smem(int h, int w, int k) {
   const int wc = (w + 1) / 2, hh = h / 2 + 1;
@@ -84,8 +84,6 @@ inline bool fill_params(Params& P, const void* table, int B, int C, int H, int W
   P.h = h; P.w = w; P.hh = h / 2 + 1; P.wc = (w + 1) / 2; P.wp = 2 * P.wc;
   P.pitch = w | 1;
   P.inv_wc = 1.0f / (float)P.wc; P.inv_hh = 1.0f / (float)P.hh;
-  P.lsh_c = lines_log2(h * 8);
-  P.lsh_r = lines_log2(P.pitch * 8);
   fill_axis(P.ay, h, r0y, r1y, t + bl.twy, t + bl.dmy);
   fill_axis(P.ax, w, r0x, r1x, t + bl.twx, t + bl.dmx);
   P.gelu = 0; P.conj = 0; P.plane0 = 0; P.nplane = 0; P.vec = 0;
@@ -112,7 +110,10 @@ inline Route route(int B, int C, int H, int W, int s, int p, int sms, bool force
   const int h = H + 2 * p, w = W + 2 * p, planes = B * C;
   Route r;
   const size_t sm = plane_smem(h, w, kMaxTaps);
-  r.one_block = !force_multi && (sm <= 75 * 1024 && (planes >= sms || sm <= 24 * 1024));
+  int a, b, c, d;
+  axis_plan(h, a, b);
+  axis_plan(w, c, d);
+  r.one_block = !force_multi && register_radix(a) && register_radix(c) && (sm <= 75 * 1024 && (planes >= sms || sm <= 24 * 1024));
   r.threads = 256;
   const size_t per = ws_plane_bytes(h, w, s);
   size_t n = ws_cap / per;

@@ -6,6 +6,7 @@
 namespace cvb {
 namespace rp {
 
+// generated launchers: register plans (k_rp_cols.cu, k_rp_rows.cu), matrix stages by width (k_rp_matrix.cu)
 int launch_cols_fwd_f32(const Params&, bool, int, size_t, cudaStream_t);
 int launch_cols_fwd_bf16(const Params&, bool, int, size_t, cudaStream_t);
 int launch_cols_inv_f32(const Params&, bool, int, size_t, cudaStream_t);
@@ -15,6 +16,24 @@ int launch_epilogue_bf16(const Params&, cudaStream_t);
 int launch_rows(const Params&, bool, int, size_t, cudaStream_t);
 int launch_plane_f32(const Params&, bool, int, size_t, cudaStream_t);
 int launch_plane_bf16(const Params&, bool, int, size_t, cudaStream_t);
+typedef int (*MatrixLauncher)(const Params&, int, int, size_t, cudaStream_t);   // (.., tensor type, grid, ..)
+struct MatrixEntry { int width; MatrixLauncher cols_fwd, rows, cols_inv; };
+#define CVB_RP_X(M)                                                            \
+  int launch_matrix_cols_fwd_##M(const Params&, int, int, size_t, cudaStream_t); \
+  int launch_matrix_rows_##M(const Params&, int, int, size_t, cudaStream_t);     \
+  int launch_matrix_cols_inv_##M(const Params&, int, int, size_t, cudaStream_t);
+CVB_RP_EACH_WIDTH(CVB_RP_X)
+#undef CVB_RP_X
+static const MatrixEntry kMatrix[] = {
+#define CVB_RP_X(M) {M, launch_matrix_cols_fwd_##M, launch_matrix_rows_##M, launch_matrix_cols_inv_##M},
+  CVB_RP_EACH_WIDTH(CVB_RP_X)
+#undef CVB_RP_X
+};
+static const MatrixEntry& matrix_entry(int width) {
+  int i = 0;
+  while (kMatrix[i].width != width) ++i;
+  return kMatrix[i];
+}
 
 // ------------------------------------------------------------------ table
 struct TableParams {
@@ -52,9 +71,10 @@ __device__ void table_tail(const TableParams& T, int i0, int step) {
     } else {
       const bool y = i < 2 * nt + T.ey;
       const int e = y ? i - 2 * nt : i - 2 * nt - T.ey, R = y ? T.r0y : T.r0x;
-      const int kp = matrix_groups(R) * 8, q = e / kp + 1, k = e % kp;
+      const int mp = matrix_width(R), n = (R / 2 + 1) * mp, sine = e >= n, f = sine ? e - n : e;
+      const int k = f / mp, q = f % mp + 1;
       sincospi(2.0 * (double)((q * k) % R) / (double)R, &sn, &cs);
-      T.out[(y ? T.dmy : T.dmx) + e] = k <= R / 2 ? make_float2((float)cs, (float)sn) : make_float2(0.f, 0.f);
+      ((float*)(T.out + (y ? T.dmy : T.dmx)))[e] = q > R / 2 ? 0.f : (float)(sine ? sn : cs);
     }
   }
 }
@@ -200,17 +220,22 @@ int run(Params& P, const Route& r, int io_dtype, void* workspace, size_t ws_byte
   if (!workspace || ws_bytes < r.ws_bytes) return CVB_ERR_WORKSPACE;
   const size_t smem_c = cols_smem(P), smem_r = rows_smem(P);
   if (smem_c > kSmemLimit || smem_r > kSmemLimit) return CVB_ERR_UNSUPPORTED_SIZE;
-  const bool sy = small_axis(P.ay) && P.lsh_c == 4, sx = small_axis(P.ax) && P.lsh_r == 4;
+  const bool sy = small_axis(P.ay), sx = small_axis(P.ax);
   P.ws = (float2*)workspace;
   for (int p0 = 0; p0 < planes; p0 += r.chunk) {
     P.plane0 = p0;
     P.nplane = planes - p0 < r.chunk ? planes - p0 : r.chunk;
     if (P.s > 1) P.r = (float*)((char*)workspace + (size_t)P.nplane * P.hh * P.wp * sizeof(float2));
-    const int gc = (P.nplane * P.wc + (1 << P.lsh_c) - 1) >> P.lsh_c;
-    const int gr = (P.nplane * P.hh + (1 << P.lsh_r) - 1) >> P.lsh_r;
-    int rc = f32 ? launch_cols_fwd_f32(P, sy, gc, smem_c, st) : launch_cols_fwd_bf16(P, sy, gc, smem_c, st);
-    if (rc == CVB_OK) rc = launch_rows(P, sx, gr, smem_r, st);
-    if (rc == CVB_OK) rc = f32 ? launch_cols_inv_f32(P, sy, gc, smem_c, st) : launch_cols_inv_bf16(P, sy, gc, smem_c, st);
+    const int gc = (P.nplane * P.wc + kLines - 1) / kLines, gr = (P.nplane * P.hh + kLines - 1) / kLines;
+    int rc = P.ay.mp ? matrix_entry(P.ay.mp).cols_fwd(P, io_dtype, gc, smem_c, st)
+             : f32   ? launch_cols_fwd_f32(P, sy, gc, smem_c, st)
+                     : launch_cols_fwd_bf16(P, sy, gc, smem_c, st);
+    if (rc == CVB_OK)
+      rc = P.ax.mp ? matrix_entry(P.ax.mp).rows(P, io_dtype, gr, smem_r, st) : launch_rows(P, sx, gr, smem_r, st);
+    if (rc == CVB_OK)
+      rc = P.ay.mp ? matrix_entry(P.ay.mp).cols_inv(P, io_dtype, gc, smem_c, st)
+           : f32   ? launch_cols_inv_f32(P, sy, gc, smem_c, st)
+                   : launch_cols_inv_bf16(P, sy, gc, smem_c, st);
     if (rc == CVB_OK && P.s > 1) rc = f32 ? launch_epilogue_f32(P, st) : launch_epilogue_bf16(P, st);
     if (rc != CVB_OK) return rc;
   }

@@ -14,22 +14,22 @@ namespace rp {
 template <typename IO>
 __global__ void __launch_bounds__(128, 6) cols_fwd_small_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
-  cols_fwd_body<IO, kSmallRadix, 4>(P, smem);
+  cols_fwd_body<IO, kSmallRadix, 0>(P, smem);
 }
 template <typename IO>
 __global__ void __launch_bounds__(128, 6) cols_inv_small_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
-  cols_inv_body<IO, kSmallRadix, 4>(P, smem);
+  cols_inv_body<IO, kSmallRadix, 0>(P, smem);
 }
-template <typename IO, int CSH>
-__global__ void __launch_bounds__(256, 2) cols_fwd_kernel(const __grid_constant__ Params P) {
+template <typename IO>
+__global__ void __launch_bounds__(128, 4) cols_fwd_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
-  cols_fwd_body<IO, kAnyRadix, CSH>(P, smem);
+  cols_fwd_body<IO, kAnyRadix, 0>(P, smem);
 }
-template <typename IO, int CSH>
-__global__ void __launch_bounds__(256, 2) cols_inv_kernel(const __grid_constant__ Params P) {
+template <typename IO>
+__global__ void __launch_bounds__(128, 4) cols_inv_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
-  cols_inv_body<IO, kAnyRadix, CSH>(P, smem);
+  cols_inv_body<IO, kAnyRadix, 0>(P, smem);
 }
 template <typename IO>
 __global__ void __launch_bounds__(128) epilogue_kernel(const __grid_constant__ Params P) {
@@ -45,13 +45,11 @@ static int go(K kernel, const Params& P, int grid, int threads, size_t smem, cud
 }
 int CVB_CAT(launch_cols_fwd, CVB_IO_NAME)(const Params& P, bool small, int grid, size_t smem, cudaStream_t st) {
   if (small) return go(cols_fwd_small_kernel<CVB_IO>, P, grid, 128, smem, st);
-  if (P.lsh_c == 4) return go(cols_fwd_kernel<CVB_IO, 4>, P, grid, 256, smem, st);
-  return go(cols_fwd_kernel<CVB_IO, -1>, P, grid, 256, smem, st);
+  return go(cols_fwd_kernel<CVB_IO>, P, grid, 128, smem, st);
 }
 int CVB_CAT(launch_cols_inv, CVB_IO_NAME)(const Params& P, bool small, int grid, size_t smem, cudaStream_t st) {
   if (small) return go(cols_inv_small_kernel<CVB_IO>, P, grid, 128, smem, st);
-  if (P.lsh_c == 4) return go(cols_inv_kernel<CVB_IO, 4>, P, grid, 256, smem, st);
-  return go(cols_inv_kernel<CVB_IO, -1>, P, grid, 256, smem, st);
+  return go(cols_inv_kernel<CVB_IO>, P, grid, 128, smem, st);
 }
 int CVB_CAT(launch_epilogue, CVB_IO_NAME)(const Params& P, cudaStream_t st) {
   epilogue_kernel<CVB_IO><<<dim3((P.H + kEpiRows - 1) / kEpiRows, P.nplane), 128, 0, st>>>(P);

@@ -1,0 +1,50 @@
+// Strip kernels of the real-plane solve whose R0-point transform is a matrix stage (lengths with a large prime).  Built
+// once per width with -DCVB_MP=..; 128 threads, as many blocks on an SM as the pairs held in registers allow.
+#include "../../include/converse_b200.h"
+#include "cvb_internal.h"
+#include "cvb_rp.cuh"
+
+#define CVB_CAT_(a, b) a##_##b
+#define CVB_CAT(a, b) CVB_CAT_(a, b)
+#define CVB_RP_BLOCKS (CVB_MP <= 36 ? 5 : CVB_MP <= 44 ? 4 : 3)
+
+namespace cvb {
+namespace rp {
+
+template <typename IO, int MP>
+__global__ void __launch_bounds__(128, CVB_RP_BLOCKS) matrix_cols_fwd_kernel(const __grid_constant__ Params P) {
+  extern __shared__ float2 smem[];
+  cols_fwd_body<IO, kMatrixR1, MP>(P, smem);
+}
+template <int MP>
+__global__ void __launch_bounds__(128, CVB_RP_BLOCKS) matrix_rows_kernel(const __grid_constant__ Params P) {
+  extern __shared__ float2 smem[];
+  rows_body<kMatrixR1, MP>(P, smem);
+}
+template <typename IO, int MP>
+__global__ void __launch_bounds__(128, CVB_RP_BLOCKS) matrix_cols_inv_kernel(const __grid_constant__ Params P) {
+  extern __shared__ float2 smem[];
+  cols_inv_body<IO, kMatrixR1, MP>(P, smem);
+}
+
+template <typename K>
+static int go(K kernel, const Params& P, int grid, size_t smem, cudaStream_t st) {
+  CVB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel<<<grid, 128, smem, st>>>(P);
+  CVB_CUDA(cudaGetLastError());
+  return CVB_OK;
+}
+int CVB_CAT(launch_matrix_cols_fwd, CVB_MP)(const Params& P, int io_dtype, int grid, size_t smem, cudaStream_t st) {
+  return io_dtype == CVB_F32 ? go(matrix_cols_fwd_kernel<float, CVB_MP>, P, grid, smem, st)
+                             : go(matrix_cols_fwd_kernel<__nv_bfloat16, CVB_MP>, P, grid, smem, st);
+}
+int CVB_CAT(launch_matrix_rows, CVB_MP)(const Params& P, int, int grid, size_t smem, cudaStream_t st) {
+  return go(matrix_rows_kernel<CVB_MP>, P, grid, smem, st);
+}
+int CVB_CAT(launch_matrix_cols_inv, CVB_MP)(const Params& P, int io_dtype, int grid, size_t smem, cudaStream_t st) {
+  return io_dtype == CVB_F32 ? go(matrix_cols_inv_kernel<float, CVB_MP>, P, grid, smem, st)
+                             : go(matrix_cols_inv_kernel<__nv_bfloat16, CVB_MP>, P, grid, smem, st);
+}
+
+}  // namespace rp
+}  // namespace cvb

@@ -8,12 +8,11 @@ namespace rp {
 
 __global__ void __launch_bounds__(128, 6) rows_small_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
-  rows_body<kSmallRadix, 4>(P, smem);
+  rows_body<kSmallRadix, 0>(P, smem);
 }
-template <int CSH>
-__global__ void __launch_bounds__(256, 2) rows_kernel(const __grid_constant__ Params P) {
+__global__ void __launch_bounds__(128, 4) rows_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
-  rows_body<kAnyRadix, CSH>(P, smem);
+  rows_body<kAnyRadix, 0>(P, smem);
 }
 
 template <typename K>
@@ -25,8 +24,7 @@ static int go(K kernel, const Params& P, int grid, int threads, size_t smem, cud
 }
 int launch_rows(const Params& P, bool small, int grid, size_t smem, cudaStream_t st) {
   if (small) return go(rows_small_kernel, P, grid, 128, smem, st);
-  if (P.lsh_r == 4) return go(rows_kernel<4>, P, grid, 256, smem, st);
-  return go(rows_kernel<-1>, P, grid, 256, smem, st);
+  return go(rows_kernel, P, grid, 128, smem, st);
 }
 
 }  // namespace rp
