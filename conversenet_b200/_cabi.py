@@ -36,6 +36,10 @@ SIGNATURES = {
     "cvb_ln_pw_gelu_fwd": (_c.c_int, [_c.c_void_p] * 4 + [_c.c_float] + [_c.c_void_p] * 2 + [_c.c_int] * 4 + [_c.c_void_p]),
     "cvb_pw_res_mlp_fwd": (_c.c_int, [_c.c_void_p] * 8 + [_c.c_float] + [_c.c_void_p] * 5 + [_c.c_int] * 4 + [_c.c_void_p]),
     "cvb_pw_res_fwd": (_c.c_int, [_c.c_void_p] * 6 + [_c.c_int] * 4 + [_c.c_void_p]),
+    "cvb_block_pack_bytes": (_c.c_size_t, []),
+    "cvb_block_pack": (_c.c_int, [_c.c_void_p] * 16),
+    "cvb_block_pre_fwd": (_c.c_int, [_c.c_void_p] * 3 + [_c.c_float] + [_c.c_int] * 3 + [_c.c_void_p]),
+    "cvb_block_post_fwd": (_c.c_int, [_c.c_void_p] * 4 + [_c.c_float] + [_c.c_int] * 3 + [_c.c_void_p]),
     "cvb_plan_radices": (_c.c_int, [_c.c_int, _c.POINTER(_c.c_int), _c.c_int]),
     "cvb_fits_shared": (_c.c_int, [_c.c_int, _c.c_int]),
     "cvb_cross_spectrum": (_c.c_int, [_c.c_void_p] * 4 + [_c.c_int] * 7 + [_c.c_void_p]),
@@ -66,6 +70,24 @@ def load():
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+_host = None
+
+
+def host():
+    """The native host module (`csrc/host.cpp`), bound to the loaded library."""
+    global _host
+    if _host is None:
+        lib = load()
+        try:
+            from . import _host as mod
+        except ImportError as e:
+            raise ConverseLibraryError("the host module of the package is not built (run `python -m "
+                                       "conversenet_b200.build`): %s" % e)
+        mod.init(*[_c.cast(getattr(lib, n), _c.c_void_p).value for n in mod.names])
+        _host = mod
+    return _host
 
 
 def check(status, what):

@@ -16,6 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libconverse_b200.so")
+HOST = os.path.join(HERE, "_host" + (__import__("sysconfig").get_config_var("EXT_SUFFIX") or ".so"))
 
 # Compile-time plans: (RY0, RY1, RX0, RX1, threads, min blocks per SM).
 # Padded plane = (RY0*RY1) x (RX0*RX1); radices in the order the planner emits.
@@ -38,10 +39,9 @@ STRIP2_PLANS = [
 ]
 
 # First factor R0 of the tensor-core multi-pass plans (padded length 4 * R0, both axes of a plane):
-# 268 (ConverseDnCNN), 512 (ConverseUSRNet data step) and 516 (ConverseUSRNet blocks: 2.65 ms per
-# 4 x 128 planes against 2.76 ms for the Rader plan 43 * 12).  Measured slower than the register-FFT
-# multi-pass kernels, and therefore not listed: 66 (264), 130 (520).
-GEMM_PLANS = [67, 128, 129]
+# 268 (ConverseDnCNN) and 516 (ConverseUSRNet blocks).  Measured slower than the register
+# transforms, and therefore not listed: 66 (264), 128 (512), 130 (520).
+GEMM_PLANS = [67, 129]
 
 # Widths of the matrix stage (CVB_RP_EACH_WIDTH in cvb_rp.cuh)
 MATRIX_WIDTHS = [20, 24, 32, 36, 44, 56, 64]
@@ -86,7 +86,7 @@ def generate_sources():
 def _units():
     units = [("converse_b200", "converse_b200.cu", []), ("k_dynamic", "k_dynamic.cu", []),
              ("k_strip", "k_strip.cu", []), ("k_block", "k_block.cu", []), ("k_block_tc", "k_block_tc.cu", []), ("k_block_tc2", "k_block_tc2.cu", []),
-             ("k_block_tc3", "k_block_tc3.cu", [])]
+             ("k_block_tc3", "k_block_tc3.cu", []), ("k_block_mlp", "k_block_mlp.cu", [])]
     units += [("k_rp", "k_rp.cu", []), ("k_rp_rows", "k_rp_rows.cu", [])]
     for name, io in (("f32", "float"), ("bf16", "__nv_bfloat16")):
         for unit in ("k_rp_cols", "k_rp_plane"):
@@ -115,6 +115,34 @@ def _stamp(defs):
     return h.hexdigest()
 
 
+def _host_command():
+    """g++ command of the native host module (csrc/host.cpp) against the installed torch."""
+    import sysconfig
+    import torch
+    inc = os.path.join(os.path.dirname(torch.__file__), "include")
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w", "-I" + sysconfig.get_paths()["include"], "-I" + inc,
+            "-I" + os.path.join(inc, "torch", "csrc", "api", "include"), "-I" + os.path.join(cuda, "include"),
+            "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
+            os.path.join(CSRC, "host.cpp"), "-o", HOST, "-L" + lib, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10",
+            "-lc10_cuda", "-Wl,-rpath," + lib]
+
+
+def build_host(force=False):
+    """The native host module next to this file; rebuilt when its source, the C ABI or torch changed."""
+    cmd = _host_command()
+    h = hashlib.sha1(" ".join(cmd).encode())
+    for path in (os.path.join(CSRC, "host.cpp"), os.path.join(HERE, "..", "include", "converse_b200.h")):
+        h.update(open(path, "rb").read())
+    stamp = os.path.join(OBJ, "host.stamp")
+    if not force and os.path.exists(HOST) and os.path.exists(stamp) and open(stamp).read() == h.hexdigest():
+        return
+    _run(cmd)
+    with open(stamp, "w") as f:
+        f.write(h.hexdigest())
+
+
 def build(force=False, ptxas_v=False, verbose=True):
     generate_sources()
     os.makedirs(OBJ, exist_ok=True)
@@ -131,6 +159,8 @@ def build(force=False, ptxas_v=False, verbose=True):
                   ["-c", os.path.join(CSRC, src), "-o", obj]
             jobs.append((name, cmd, stamp_path, stamp))
     logs = {}
+    host = ThreadPoolExecutor(max_workers=1)
+    host_done = host.submit(build_host, force)
     if jobs:
         with ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 4)) as ex:
             for (name, cmd, stamp_path, stamp), out in zip(jobs, ex.map(lambda j: _run(j[1]), jobs)):
@@ -140,6 +170,8 @@ def build(force=False, ptxas_v=False, verbose=True):
     if jobs or force or not os.path.exists(LIB):
         objs = [os.path.join(OBJ, name + ".o") for name, _, _ in units]
         _run([_nvcc(), "-shared", "-o", LIB] + objs + ["-lcudart"])
+    host_done.result()
+    host.shutdown()
     if verbose:
         for name, out in logs.items():
             if ptxas_v and out.strip():

@@ -142,6 +142,14 @@ static bool needs_strip(int h, int w, int k, bool big) {
 // chunk workspace of the multi-launch real-plane kernels
 constexpr size_t kRpWorkspace = (size_t)64 << 20;
 
+// Planes whose two lengths are in the tensor-core registry keep the tables of both kernel families: the tensor-core
+// kernels pack two planes that share their taps (two images of a batch) into one complex plane and win when there are
+// two (268 x 268, 8 x 128 planes: 1.01 ms against 1.55), the real-plane kernels when every pair would hold one (1 x 128
+// planes: 0.21 ms against 0.25).
+static bool dual_tables(int h, int w) { return gemm_axis(h) && gemm_axis(w) && rp::supported(h, w) && !gemm_disabled(); }
+static size_t dual_offset(int C, int h, int w) { return (rp::table_bytes(C, h, w) + 255) / 256 * 256; }
+static bool takes_tensor_cores(int B, int h, int w) { return B >= 2 && dual_tables(h, w); }
+
 static int check_padding(int H, int W, int p, int pad_mode) {
   if (p < 0) return CVB_ERR_BAD_ARGUMENT;
   if (pad_mode < CVB_PAD_CIRCULAR || pad_mode > CVB_PAD_CONSTANT) return CVB_ERR_BAD_ARGUMENT;
@@ -222,7 +230,7 @@ size_t cvb_transfer_bytes(int C, int h, int w) {
   RaderInfo ry, rx;
   rader_both(py, px, ry, rx);
   const size_t n = ((size_t)C * h * w + h + w + rader_blob_float2(ry) + rader_blob_float2(rx)) * sizeof(float2);
-  return std::max(n, rp::table_bytes(C, h, w));
+  return dual_tables(h, w) ? n + dual_offset(C, h, w) : std::max(n, rp::table_bytes(C, h, w));
 }
 
 static int build_table(const float* weight, const float* bias, int C, int k, int s, int h, int w, float eps,
@@ -243,7 +251,11 @@ static int build_table(const float* weight, const float* bias, int C, int k, int
   if (!weight || !bias || !table || C < 1 || k < 1 || s < 1 || h < 2 || w < 2) return CVB_ERR_BAD_ARGUMENT;
   // the tiled build keeps k-long arrays of kMaxTaps entries per thread and per block
   if (k > kMaxTaps || k > s * h || k > s * w) return CVB_ERR_KERNEL_TOO_LARGE;
-  if (rp::supported(h, w)) return rp::build_table(weight, bias, C, k, s, h, w, eps, kind, table, (cudaStream_t)stream);
+  if (rp::supported(h, w)) {
+    const int rc = rp::build_table(weight, bias, C, k, s, h, w, eps, kind, table, (cudaStream_t)stream);
+    if (rc != CVB_OK || !dual_tables(h, w)) return rc;
+    table = (char*)table + dual_offset(C, h, w);
+  }
   TransferParams T;
   if (!make_axis_plans(h, w, T.py, T.px)) return CVB_ERR_UNSUPPORTED_SIZE;
   T.weight = weight; T.bias = bias; T.table = (float2*)table;
@@ -277,7 +289,7 @@ size_t cvb_converse2d_workspace_bytes(int B, int C, int H, int W, int s, int p, 
   (void)io_dtype;
   if (B < 1 || C < 1 || H < 1 || W < 1 || p < 0 || s < 1) return 0;
   const int h = H + 2 * p, w = W + 2 * p;
-  if (rp::supported(h, w))
+  if (rp::supported(h, w) && !takes_tensor_cores(B, h, w))
     return rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0, std::max(kRpWorkspace, rp::ws_plane_bytes(h, w, s))).ws_bytes;
   Plan1D py, px;
   bool big = false;
@@ -298,7 +310,9 @@ int cvb_converse2d_fwd(const void* x, void* out, const void* table, const float*
   if (H + 2 * p < 2 || W + 2 * p < 2) return CVB_ERR_BAD_ARGUMENT;
   if (k > s * (H + 2 * p) || k > s * (W + 2 * p)) return CVB_ERR_KERNEL_TOO_LARGE;
   rp::Params Q;
-  if (rp::fill_params(Q, table, B, C, H, W, k, s, p, pad_mode)) {
+  if (takes_tensor_cores(B, H + 2 * p, W + 2 * p)) {
+    table = (const char*)table + dual_offset(C, H + 2 * p, W + 2 * p);
+  } else if (rp::fill_params(Q, table, B, C, H, W, k, s, p, pad_mode)) {
     Q.x = x; Q.out = out; Q.weight = weight; Q.gelu = fuse_gelu ? 1 : 0;
     const rp::Route r = rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0,
                                   std::max(kRpWorkspace, rp::ws_plane_bytes(H + 2 * p, W + 2 * p, s)));
@@ -450,6 +464,33 @@ int cvb_pw_res_fwd(const void* t, const void* res, void* out, const float* w, co
   return bk == 3   ? launch_pw_res_tc3(P, io_dtype, sm_count(), status_ptr(), (cudaStream_t)stream)
          : bk != 1 ? launch_pw_res_tc2(P, io_dtype, sm_count(), status_ptr(), (cudaStream_t)stream)
                    : launch_pw_res_tc(P, sm_count(), status_ptr(), (cudaStream_t)stream);
+}
+
+size_t cvb_block_pack_bytes(void) { return block_pack_bytes(); }
+
+int cvb_block_pack(const float* ln1_w, const float* ln1_b, const float* w1, const float* b1, const float* w2,
+                   const float* b2, const float* alpha1, const float* ln2_w, const float* ln2_b, const float* w3,
+                   const float* b3, const float* w4, const float* b4, const float* alpha2, void* pack, void* stream) {
+  if (!ln1_w || !ln1_b || !w1 || !b1 || !w2 || !b2 || !ln2_w || !ln2_b || !w3 || !b3 || !w4 || !b4 || !pack)
+    return CVB_ERR_BAD_ARGUMENT;
+  return launch_block_pack(ln1_w, ln1_b, w1, b1, w2, b2, alpha1, ln2_w, ln2_b, w3, b3, w4, b4, alpha2, pack,
+                           (cudaStream_t)stream);
+}
+
+int cvb_block_pre_fwd(const void* x, void* out, const void* pack, float ln_eps, int B, int HW, int io_dtype,
+                      void* stream) {
+  if (!x || !out || !pack || ((size_t)pack) % 16 || B < 1 || HW < 1) return CVB_ERR_BAD_ARGUMENT;
+  if (io_dtype != CVB_F32 && io_dtype != CVB_BF16) return CVB_ERR_BAD_ARGUMENT;
+  return launch_block_mix(false, x, nullptr, out, pack, ln_eps, B, HW, io_dtype, sm_count(), status_ptr(),
+                          (cudaStream_t)stream);
+}
+
+int cvb_block_post_fwd(const void* t, const void* x, void* out, const void* pack, float ln_eps, int B, int HW,
+                       int io_dtype, void* stream) {
+  if (!t || !x || !out || !pack || ((size_t)pack) % 16 || B < 1 || HW < 1) return CVB_ERR_BAD_ARGUMENT;
+  if (io_dtype != CVB_F32 && io_dtype != CVB_BF16) return CVB_ERR_BAD_ARGUMENT;
+  return launch_block_mix(true, x, t, out, pack, ln_eps, B, HW, io_dtype, sm_count(), status_ptr(),
+                          (cudaStream_t)stream);
 }
 
 }  // extern "C"

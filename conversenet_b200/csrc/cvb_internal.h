@@ -64,6 +64,14 @@ int launch_pw_res_tc2(const BlockParams& P, int io_dtype, int sms, int* status, 
 int launch_ln_pw_gelu_tc3(const BlockParams& P, int io_dtype, int sms, int* status, cudaStream_t st);
 int launch_pw_res_tc3(const BlockParams& P, int io_dtype, int sms, int* status, cudaStream_t st);
 
+// packed weights, both sides of the block (k_block_mlp.cu)
+size_t block_pack_bytes();
+int launch_block_pack(const float* ln1_w, const float* ln1_b, const float* w1, const float* b1, const float* w2,
+                      const float* b2, const float* a1, const float* ln2_w, const float* ln2_b, const float* w3,
+                      const float* b3, const float* w4, const float* b4, const float* a2, void* pack, cudaStream_t st);
+int launch_block_mix(bool post, const void* x, const void* t, void* out, const void* pack, float eps, int B, int HW,
+                     int io_dtype, int sms, int* status, cudaStream_t st);
+
 // Multi-pass kernels with a compile-time axis plan (k_strip2.cu, one object per registry line).
 struct StripParams;
 typedef int (*Strip2Launcher)(const StripParams& SP, int io_dtype, cudaStream_t st);

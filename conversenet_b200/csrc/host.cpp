@@ -1,0 +1,260 @@
+// Host side of the Python entry points: argument checks, allocation, stream look-up and the C ABI calls of one layer or
+// one block in a single native call.  A small layer runs in a few microseconds on the GPU; going through Python and
+// ctypes for every buffer and argument took 22 us a call, four times the kernel (24 x 20 planes, 64 channels).
+//
+// The C ABI is reached through the function addresses of the library that the package loaded (init()), so there is one
+// copy of it in the process.  Only tensors' public C++ interface is used.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <cstring>
+#include <stdexcept>
+#include <string>
+
+#include "../../include/converse_b200.h"
+
+namespace {
+
+struct Api {
+  decltype(&cvb_strerror) strerror_ = nullptr;
+  decltype(&cvb_last_cuda_error) last_cuda_error = nullptr;
+  decltype(&cvb_transfer_bytes) transfer_bytes = nullptr;
+  decltype(&cvb_build_transfer) build_transfer = nullptr;
+  decltype(&cvb_build_x0_table) build_x0_table = nullptr;
+  decltype(&cvb_converse2d_workspace_bytes) workspace_bytes = nullptr;
+  decltype(&cvb_converse2d_fwd) converse2d_fwd = nullptr;
+  decltype(&cvb_block_pack_bytes) block_pack_bytes = nullptr;
+  decltype(&cvb_block_pack) block_pack = nullptr;
+  decltype(&cvb_block_pre_fwd) block_pre = nullptr;
+  decltype(&cvb_block_post_fwd) block_post = nullptr;
+} api;
+
+struct Failed : std::runtime_error { using std::runtime_error::runtime_error; };
+
+void check(int rc, const char* what) {
+  if (rc == 0) return;
+  std::string m = std::string(what) + " failed: " + api.strerror_(rc);
+  if (rc == CVB_ERR_CUDA) m += " (cudaError " + std::to_string(api.last_cuda_error()) + ")";
+  throw Failed(m);
+}
+
+const at::Tensor& tensor(PyObject* o, const char* what) {
+  if (!THPVariable_Check(o)) throw Failed(std::string(what) + " must be a tensor");
+  return THPVariable_Unpack(o);
+}
+const at::Tensor& cuda_tensor(PyObject* o, const char* what) {
+  const at::Tensor& t = tensor(o, what);
+  if (!t.is_cuda()) throw Failed("Converse2D needs a CUDA tensor; this build has no CPU path");
+  return t;
+}
+long integer(PyObject* o) {
+  const long v = PyLong_AsLong(o);
+  if (v == -1 && PyErr_Occurred()) throw std::invalid_argument("");
+  return v;
+}
+double real(PyObject* o) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) throw std::invalid_argument("");
+  return v;
+}
+int io_type(const at::Tensor& t) {
+  if (t.scalar_type() == at::kFloat) return CVB_F32;
+  if (t.scalar_type() == at::kBFloat16) return CVB_BF16;
+  throw Failed("Converse2D supports float32 and bfloat16 tensors, got torch." + std::string(
+      t.scalar_type() == at::kHalf ? "float16" : t.scalar_type() == at::kDouble ? "float64" : toString(t.scalar_type())));
+}
+int pad_mode(PyObject* o) {
+  const char* s = PyUnicode_Check(o) ? PyUnicode_AsUTF8(o) : nullptr;
+  if (s) {
+    if (!std::strcmp(s, "circular")) return CVB_PAD_CIRCULAR;
+    if (!std::strcmp(s, "replicate")) return CVB_PAD_REPLICATE;
+    if (!std::strcmp(s, "reflect")) return CVB_PAD_REFLECT;
+    if (!std::strcmp(s, "constant")) return CVB_PAD_CONSTANT;
+  }
+  throw Failed("unknown padding_mode '" + std::string(s ? s : "?") + "'");
+}
+void* stream(const at::Tensor& t) { return (void*)c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+at::Tensor bytes_like(const at::Tensor& t, size_t n) {
+  return at::empty({(int64_t)n}, t.options().dtype(at::kByte).requires_grad(false));
+}
+// a parameter as contiguous fp32 (itself when it already is)
+at::Tensor f32(const at::Tensor& t) {
+  if (t.scalar_type() == at::kFloat && t.is_contiguous()) return t;
+  return t.detach().to(at::kFloat).contiguous();
+}
+
+at::Tensor forward(const at::Tensor& x, const at::Tensor& table, const at::Tensor& wf, int k, int s, int p, int mode,
+                   int gelu, at::Tensor out) {
+  const int B = (int)x.size(0), C = (int)x.size(1), H = (int)x.size(2), W = (int)x.size(3), io = io_type(x);
+  if (!out.defined()) out = at::empty({B, C, (int64_t)H * s, (int64_t)W * s}, x.options().requires_grad(false));
+  const size_t ws = api.workspace_bytes(B, C, H, W, s, p, io);
+  at::Tensor w;
+  if (ws) w = bytes_like(x, ws);
+  check(api.converse2d_fwd(x.data_ptr(), out.data_ptr(), table.data_ptr(), (const float*)wf.data_ptr(), B, C, H, W, k, s,
+                           p, mode, io, gelu, ws ? w.data_ptr() : nullptr, ws, stream(x)),
+        "cvb_converse2d_fwd");
+  return out;
+}
+
+template <class F>
+PyObject* guarded(F f) {
+  try {
+    return f();
+  } catch (const Failed& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+  } catch (const c10::Error& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
+  } catch (const std::exception& e) {
+    if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what());
+  }
+  return nullptr;
+}
+void want(Py_ssize_t n, Py_ssize_t m) {
+  if (n != m) throw Failed("wrong number of arguments");
+}
+
+// converse2d(x, table, weight_f32, kernel_size, scale, padding, padding_mode, fuse_gelu, out or None)
+PyObject* py_converse2d(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    want(n, 9);
+    const at::Tensor& x0 = cuda_tensor(a[0], "x");
+    if (x0.dim() != 4) throw Failed("x must be (B,C,H,W)");
+    const c10::cuda::CUDAGuard dev(x0.device());
+    const at::Tensor x = x0.is_contiguous() ? x0 : x0.contiguous();
+    at::Tensor out;
+    if (a[8] != Py_None) out = tensor(a[8], "out");
+    return THPVariable_Wrap(forward(x, tensor(a[1], "table"), tensor(a[2], "weight"), (int)integer(a[3]), (int)integer(a[4]),
+                                    (int)integer(a[5]), pad_mode(a[6]), PyObject_IsTrue(a[7]), std::move(out)));
+  });
+}
+
+// build_transfer(weight, bias, scale, eps, h, w, x0_term) -> (table, weight as contiguous fp32 (C,k,k))
+PyObject* py_build_transfer(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    want(n, 7);
+    const at::Tensor &w = tensor(a[0], "weight"), &b = tensor(a[1], "bias");
+    const long s = integer(a[2]), h = integer(a[4]), wd = integer(a[5]);
+    if (!w.is_cuda()) throw Failed("Converse2D parameters must live on a CUDA device");
+    if (w.dim() != 4 || w.size(0) != 1) throw Failed("weight must be (1,C,kh,kw)");
+    const int C = (int)w.size(1), k = (int)w.size(2);
+    if (w.size(3) != k) throw Failed("only square kernels are supported");
+    if (b.dim() != 4 || b.size(0) != 1 || b.size(1) != C || b.size(2) != 1 || b.size(3) != 1)
+      throw Failed("bias must be (1,C,1,1)");
+    if (s < 1) throw Failed("scale must be >= 1");
+    const size_t bytes = api.transfer_bytes(C, (int)h, (int)wd);
+    if (!bytes) throw Failed("padded plane " + std::to_string(h) + "x" + std::to_string(wd) + " is not supported by the FFT engine");
+    const c10::cuda::CUDAGuard dev(w.device());
+    const at::Tensor wf = f32(w.detach()).view({C, k, k}), bf = f32(b.detach());
+    at::Tensor table = bytes_like(w, bytes);
+    auto fn = PyObject_IsTrue(a[6]) ? api.build_x0_table : api.build_transfer;
+    check(fn((const float*)wf.data_ptr(), (const float*)bf.data_ptr(), C, k, (int)s, (int)h, (int)wd, (float)real(a[3]),
+             table.data_ptr(), stream(w)),
+          "cvb_build_transfer");
+    return Py_BuildValue("(NN)", THPVariable_Wrap(table), THPVariable_Wrap(wf));
+  });
+}
+
+// state(t, ...) -> bytes: storage addresses and version counters; equal bytes = unmodified tensors (None allowed)
+PyObject* py_state(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    PyObject* o = PyBytes_FromStringAndSize(nullptr, n * 16);
+    if (!o) return nullptr;
+    char* d = PyBytes_AS_STRING(o);
+    for (Py_ssize_t i = 0; i < n; ++i) {
+      int64_t v[2] = {0, 0};
+      if (a[i] != Py_None && THPVariable_Check(a[i])) {
+        const at::Tensor& t = THPVariable_Unpack(a[i]);
+        v[0] = (int64_t)t.data_ptr();
+        v[1] = t.is_inference() ? 0 : (int64_t)t._version();
+      }
+      std::memcpy(d + 16 * i, v, 16);
+    }
+    return o;
+  });
+}
+
+// block_pack(ln1.weight, ln1.bias, w1, b1, w2, b2, alpha1, ln2.weight, ln2.bias, w3, b3, w4, b4, alpha2) -> packed weights
+PyObject* py_block_pack(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    want(n, 14);
+    at::Tensor t[14];
+    const float* q[14];
+    for (int i = 0; i < 14; ++i) {
+      q[i] = nullptr;
+      if (a[i] == Py_None) continue;
+      t[i] = f32(cuda_tensor(a[i], "parameter"));
+      q[i] = (const float*)t[i].data_ptr();
+    }
+    const c10::cuda::CUDAGuard dev(t[2].device());
+    at::Tensor pack = bytes_like(t[2], api.block_pack_bytes());
+    check(api.block_pack(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7], q[8], q[9], q[10], q[11], q[12], q[13],
+                         pack.data_ptr(), stream(pack)),
+          "cvb_block_pack");
+    return THPVariable_Wrap(pack);
+  });
+}
+
+// block(x, table, weight_f32, pack, kernel_size, padding, padding_mode, eps1, eps2) -> ConverseBlock.forward(x)
+PyObject* py_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    want(n, 9);
+    const at::Tensor& x0 = cuda_tensor(a[0], "x");
+    if (x0.dim() != 4) throw Failed("x must be (B,C,H,W)");
+    const c10::cuda::CUDAGuard dev(x0.device());
+    const at::Tensor x = x0.is_contiguous() ? x0 : x0.contiguous();
+    const at::Tensor& pack = tensor(a[3], "pack");
+    const int B = (int)x.size(0), C = (int)x.size(1), H = (int)x.size(2), W = (int)x.size(3), io = io_type(x);
+    const auto opt = x.options().requires_grad(false);
+    void* st = stream(x);
+    at::Tensor t = at::empty({B, 2 * C, H, W}, opt);
+    check(api.block_pre(x.data_ptr(), t.data_ptr(), pack.data_ptr(), (float)real(a[7]), B, H * W, io, st), "cvb_block_pre_fwd");
+    t = forward(t, tensor(a[1], "table"), tensor(a[2], "weight"), (int)integer(a[4]), 1, (int)integer(a[5]), pad_mode(a[6]), 1,
+                at::Tensor());
+    at::Tensor out = at::empty({B, C, H, W}, opt);
+    check(api.block_post(t.data_ptr(), x.data_ptr(), out.data_ptr(), pack.data_ptr(), (float)real(a[8]), B, H * W, io, st),
+          "cvb_block_post_fwd");
+    return THPVariable_Wrap(out);
+  });
+}
+
+// init(address of each C ABI function in the order of `names`)
+PyObject* py_init(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    want(n, 11);
+    void* p[11];
+    for (int i = 0; i < 11; ++i) p[i] = PyLong_AsVoidPtr(a[i]);
+    int i = 0;
+    auto set = [&](auto& f) { f = (std::decay_t<decltype(f)>)p[i++]; };
+    set(api.strerror_); set(api.last_cuda_error); set(api.transfer_bytes); set(api.build_transfer); set(api.build_x0_table);
+    set(api.workspace_bytes); set(api.converse2d_fwd); set(api.block_pack_bytes); set(api.block_pack); set(api.block_pre);
+    set(api.block_post);
+    Py_RETURN_NONE;
+  });
+}
+
+PyMethodDef methods[] = {
+    {"init", (PyCFunction)(void (*)(void))py_init, METH_FASTCALL, nullptr},
+    {"converse2d", (PyCFunction)(void (*)(void))py_converse2d, METH_FASTCALL, nullptr},
+    {"build_transfer", (PyCFunction)(void (*)(void))py_build_transfer, METH_FASTCALL, nullptr},
+    {"state", (PyCFunction)(void (*)(void))py_state, METH_FASTCALL, nullptr},
+    {"block_pack", (PyCFunction)(void (*)(void))py_block_pack, METH_FASTCALL, nullptr},
+    {"block", (PyCFunction)(void (*)(void))py_block, METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host(void) {
+  PyObject* m = PyModule_Create(&module);
+  if (!m) return nullptr;
+  PyObject* names = Py_BuildValue("(sssssssssss)", "cvb_strerror", "cvb_last_cuda_error", "cvb_transfer_bytes",
+                                  "cvb_build_transfer", "cvb_build_x0_table", "cvb_converse2d_workspace_bytes",
+                                  "cvb_converse2d_fwd", "cvb_block_pack_bytes", "cvb_block_pack", "cvb_block_pre_fwd",
+                                  "cvb_block_post_fwd");
+  if (!names || PyModule_AddObject(m, "names", names) < 0) return nullptr;
+  return m;
+}

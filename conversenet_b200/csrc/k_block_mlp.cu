@@ -1,0 +1,340 @@
+// The channel-mixing parts of ConverseBlock on tcgen05, one kernel for each side of the Converse2D operator:
+//   PRE :  out = GELU( W1 . LN(x) + b1 )                                   64 -> 128 channels
+//   POST:  x1 = x + a1 (W2 . t + b2);  out = x1 + a2 (W4 . GELU( W3 . LN(x1) + b3 ) + b4)    t: 128, x, out: 64
+// (models/util_converse.py:278-293, 321-322).  A thread owns a pixel from its loads to its stores: LayerNorm, GELU,
+// residuals and the operands of all three contractions of POST stay inside one thread and its lane of tensor memory,
+// so the 128-channel hidden tensor and x1 never leave the SM.
+//
+// A block is two groups of 128 threads; each works on a 128-pixel tile of its own, so that one group's arithmetic
+// covers the other's MMAs.  Per contraction: the thread splits its values into TF32 hi + lo and writes them to its
+// lane of the group's operand columns (tcgen05.st, 64 channels at a time); after a barrier of the group one thread
+// issues hi hi + hi lo + lo hi with the weights from shared memory and commits to the group's mbarrier; every thread
+// then reads its own lane of the accumulator.  TMEM columns of group g at 256 g: accumulator [0,128), operand hi
+// [128,192), lo [192,256).  The weights, split and in operand layout, were packed once (block_pack_kernel) and arrive
+// by one bulk copy.  Pixels are addressed one by one (channel rows of any alignment, any image size, fp32 or bf16);
+// the values of the next tile are requested while the current one computes.
+//
+// What bounds it: bytes (PRE 3 C, POST 4 C channel planes), the MMAs (24 of 128x128x8 a tile for PRE, 72 of which 48 of
+// 128x64x8 for POST) and instruction issue (about 2400 and 4000 a warp and tile) are within 1.5 x of one another.
+// Every wait is bounded; after a time-out a thread stops working but keeps meeting the group's barriers.
+#include "../../include/converse_b200.h"
+#include "cvb_internal.h"
+#include "cvb_block.cuh"
+#include "cvb_tc.cuh"
+
+namespace cvb {
+
+// ---- packed weights: PRE | POST, each a multiple of 16 bytes
+constexpr int kW = kBlkC * kBlkM;                               // floats of one weight matrix
+constexpr int kPreFloats = 2 * kW + kBlkM;                      // W1 hi, lo; b1
+constexpr int kPostFloats = 6 * kW + 4 * kBlkC + kBlkM;         // W2, W3, W4 hi, lo; b2, a1, b4, a2; b3
+size_t block_pack_bytes() { return (size_t)(kPreFloats + kPostFloats) * sizeof(float); }
+
+// float index of element (n, k) of an operand with N rows (K-major core matrices, no swizzle)
+__host__ __device__ constexpr int pack_index(int N, int n, int k) {
+  return (n >> 3) * 32 + (n & 7) * 4 + (k & 3) + ((k >> 2) & 1) * (N / 8) * 32 + (k >> 3) * (N / 8) * 64;
+}
+
+struct PackParams {
+  const float *ln1_w, *ln1_b, *w1, *b1, *w2, *b2, *a1, *ln2_w, *ln2_b, *w3, *b3, *w4, *b4, *a2;
+  float* out;
+};
+
+// grid: 4 matrices x 16 slices.  The LayerNorm affine is folded into the weights that follow it.
+__global__ void __launch_bounds__(256) block_pack_kernel(const PackParams P) {
+  const int which = blockIdx.x >> 4, slice = blockIdx.x & 15;
+  float* post = P.out + kPreFloats;
+  const float* w = which == 0 ? P.w1 : which == 1 ? P.w2 : which == 2 ? P.w3 : P.w4;
+  const float* g = which == 0 ? P.ln1_w : which == 2 ? P.ln2_w : nullptr;
+  const int N = which == 0 || which == 2 ? kBlkM : kBlkC, K = kW / N;
+  float* hi = which == 0 ? P.out : post + (which - 1) * 2 * kW;
+  for (int i = slice * (kW / 16) + threadIdx.x; i < (slice + 1) * (kW / 16); i += 256) {
+    const int n = i / K, k = i - n * K;
+    float a, b;
+    tc::split_tf32(g ? w[i] * g[k] : w[i], a, b);
+    hi[pack_index(N, n, k)] = a;
+    hi[kW + pack_index(N, n, k)] = b;
+  }
+  if (slice != 0) return;
+  float* vec = post + 6 * kW;
+  const float* bias = which == 0 ? P.b1 : which == 1 ? P.b2 : which == 2 ? P.b3 : P.b4;
+  const float* beta = which == 0 ? P.ln1_b : which == 2 ? P.ln2_b : nullptr;
+  float* dst = which == 0 ? P.out + 2 * kW : which == 1 ? vec : which == 2 ? vec + 4 * kBlkC : vec + 2 * kBlkC;
+  for (int n = threadIdx.x; n < N; n += 256) {
+    float s = bias[n];
+    if (beta)
+      for (int k = 0; k < K; ++k) s = fmaf(w[n * K + k], beta[k], s);
+    dst[n] = s;
+    if (which == 1) vec[kBlkC + n] = P.a1 ? P.a1[n] : 1.0f;
+    if (which == 3) vec[3 * kBlkC + n] = P.a2 ? P.a2[n] : 1.0f;
+  }
+}
+
+int launch_block_pack(const float* ln1_w, const float* ln1_b, const float* w1, const float* b1, const float* w2,
+                      const float* b2, const float* a1, const float* ln2_w, const float* ln2_b, const float* w3,
+                      const float* b3, const float* w4, const float* b4, const float* a2, void* pack, cudaStream_t st) {
+  const PackParams P = {ln1_w, ln1_b, w1, b1, w2, b2, a1, ln2_w, ln2_b, w3, b3, w4, b4, a2, (float*)pack};
+  block_pack_kernel<<<64, 256, 0, st>>>(P);
+  CVB_CUDA(cudaGetLastError());
+  return CVB_OK;
+}
+
+struct MixParams {
+  const void* x;
+  const void* t;
+  void* out;
+  const float* pack;
+  float eps;
+  int HW;
+  long long npix;
+  int* status;
+};
+
+constexpr int kMixThreads = 256;
+constexpr uint32_t kOpHi = 128, kOpLo = 192;
+
+// sixteen consecutive columns of this thread's TMEM lane
+__device__ __forceinline__ void mix_st16(uint32_t taddr, const float (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+      "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
+      "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
+      "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
+      "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15]))
+      : "memory");
+}
+// 64 channel values -> operand columns
+__device__ __forceinline__ void mix_stage(uint32_t lane, const float (&v)[64]) {
+#pragma unroll
+  for (int c0 = 0; c0 < 64; c0 += 16) {
+    float hi[16], lo[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) tc::split_tf32(v[c0 + e], hi[e], lo[e]);
+    mix_st16(lane + kOpHi + (uint32_t)c0, hi);
+    mix_st16(lane + kOpLo + (uint32_t)c0, lo);
+  }
+  tc::tmem_wait_st();
+}
+// D (+)= A[64 channels in the operand columns] . B, B = N rows, K columns k0 .. k0 + 63 of a packed matrix
+template <int N>
+__device__ __forceinline__ void mix_mma(uint32_t tmem, const float* b_hi, int k0, bool accumulate) {
+  constexpr uint32_t idesc = tc::idesc_tf32(128, N, false, false);
+  constexpr int LBO = (N / 8) * 128, KSTEP = 2 * LBO;
+#pragma unroll
+  for (int ks = 0; ks < 8; ++ks) {
+    const uint64_t bh = tc::smem_desc((const char*)b_hi + (k0 / 8 + ks) * KSTEP, LBO, 128);
+    const uint64_t bl = tc::smem_desc((const char*)(b_hi + kW) + (k0 / 8 + ks) * KSTEP, LBO, 128);
+    tc::mma_tf32_ta(tmem, tmem + kOpHi + ks * 8, bh, idesc, (accumulate || ks > 0) ? 1u : 0u);
+    tc::mma_tf32_ta(tmem, tmem + kOpHi + ks * 8, bl, idesc, 1u);
+    tc::mma_tf32_ta(tmem, tmem + kOpLo + ks * 8, bh, idesc, 1u);
+  }
+}
+// centre and scale 64 values (the affine part is in the weights)
+__device__ __forceinline__ void mix_norm(float (&v)[64], float eps) {
+  float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+  for (int c = 0; c < 64; c += 4) { s0 += v[c]; s1 += v[c + 1]; s2 += v[c + 2]; s3 += v[c + 3]; }
+  const float mean = ((s0 + s1) + (s2 + s3)) * (1.0f / 64);
+  s0 = s1 = s2 = s3 = 0.f;
+#pragma unroll
+  for (int c = 0; c < 64; c += 4) {
+    v[c] -= mean; v[c + 1] -= mean; v[c + 2] -= mean; v[c + 3] -= mean;
+    s0 = fmaf(v[c], v[c], s0); s1 = fmaf(v[c + 1], v[c + 1], s1);
+    s2 = fmaf(v[c + 2], v[c + 2], s2); s3 = fmaf(v[c + 3], v[c + 3], s3);
+  }
+  const float rstd = 1.0f / sqrtf(((s0 + s1) + (s2 + s3)) * (1.0f / 64) + eps);
+#pragma unroll
+  for (int c = 0; c < 64; ++c) v[c] *= rstd;
+}
+template <typename IO>
+__device__ __forceinline__ void mix_load(float (&v)[64], const IO* p, int HW, bool valid) {
+#pragma unroll
+  for (int c = 0; c < 64; ++c) v[c] = valid ? ld_io<IO>(p, (size_t)c * HW) : 0.f;
+}
+__device__ __forceinline__ void mix_bar(int g) {
+  if (g == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
+  else asm volatile("bar.sync 2, 128;" ::: "memory");
+}
+
+template <bool POST, typename IO>
+__global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_constant__ MixParams P) {
+  extern __shared__ __align__(128) float msm[];
+  constexpr int kFloats = POST ? kPostFloats : kPreFloats;
+  float* wts = msm;
+  const float* vec = wts + (POST ? 6 : 2) * kW;    // PRE: b1.  POST: b2, a1, b4, a2, b3
+  uint64_t* bars = (uint64_t*)(msm + kFloats);      // MMA of group 0, 1; weights
+  uint32_t* holder = (uint32_t*)(bars + 3);
+  const int tid = threadIdx.x, warp = tid >> 5, g = tid >> 7, m = tid & 127;
+  if (tid == 0) {
+    for (int i = 0; i < 3; ++i) mbar_init(&bars[i], 1);
+    mbar_fence_init();
+    mbar_expect_tx(&bars[2], kFloats * 4);
+    bulk_g2s(wts, P.pack + (POST ? kPreFloats : 0), kFloats * 4, &bars[2]);
+  }
+  if (warp == 0) tc::tmem_alloc(holder, 512);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = *holder + 256u * (uint32_t)g;
+  const uint32_t lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  uint64_t* done = &bars[g];
+  uint32_t uses = 0;                                // commits of this group so far
+  bool ok = true;
+
+  const long long ntiles = (P.npix + 127) / 128, step = 2ll * gridDim.x;
+  const int HW = P.HW;
+  const int Cin = POST ? kBlkM : kBlkC, Cout = POST ? kBlkC : kBlkM;
+  // this thread's pixel of a tile: image, position
+  auto place = [&](long long tile, bool& valid, long long& img, int& pos) {
+    const long long pix = tile * 128 + m;
+    valid = pix < P.npix;
+    img = valid ? pix / HW : 0;
+    pos = valid ? (int)(pix - img * HW) : 0;
+  };
+  auto commit_wait = [&]() {                        // the group's last MMAs have finished
+    if (ok) ok = mbar_wait_bounded(done, uses & 1u, kWaitLimit);
+    uses += 1;
+    tc::fence_after_sync();
+  };
+  auto publish = [&]() {                            // operand columns written, accumulator read, by the whole group
+    tc::fence_before_sync();
+    mix_bar(g);
+    tc::fence_after_sync();
+  };
+
+  long long tile = blockIdx.x + (long long)g * gridDim.x;
+  bool valid = false;
+  long long img = 0;
+  int pos = 0;
+  float v[64];
+  if (tile < ntiles) {
+    place(tile, valid, img, pos);
+    mix_load<IO>(v, (const IO*)(POST ? P.t : P.x) + (size_t)img * Cin * HW + pos, HW, valid);
+  }
+  if (ok) ok = mbar_wait_bounded(&bars[2], 0, kWaitLimit);   // weights
+  for (; tile < ntiles; tile += step) {
+    const long long ntile = tile + step;
+    bool nvalid = false;
+    long long nimg = 0;
+    int npos = 0;
+    if (ntile < ntiles) place(ntile, nvalid, nimg, npos);
+    const IO* next = (const IO*)(POST ? P.t : P.x) + (size_t)nimg * Cin * HW + npos;
+    IO* op = (IO*)P.out + (size_t)img * Cout * HW + pos;
+    if constexpr (!POST) {
+      mix_norm(v, P.eps);
+      mix_stage(lane, v);
+      publish();
+      if (m == 0 && ok) { mix_mma<128>(tmem, wts, 0, false); tc::mma_commit(done); }
+      mix_load<IO>(v, next, HW, nvalid);
+      commit_wait();
+#pragma unroll 1
+      for (int c0 = 0; c0 < 128; c0 += 32) {
+        float a[32];
+        tc::tmem_ld32(lane + (uint32_t)c0, a);
+        if (valid && ok) {
+#ifdef __CUDA_ARCH__
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            const float2 b = *(const float2*)(vec + c0 + j);
+            const float2 o = gelu_erf2(a[j] + b.x, a[j + 1] + b.y);
+            st_io<IO>(op, (size_t)(c0 + j) * HW, o.x);
+            st_io<IO>(op, (size_t)(c0 + j + 1) * HW, o.y);
+          }
+#endif
+        }
+      }
+    } else {
+      const float *w2 = wts, *w3 = wts + 2 * kW, *w4 = wts + 4 * kW;
+      const IO* tp = (const IO*)P.t + (size_t)img * Cin * HW + pos;
+      // x1 = x + a1 (W2 . t + b2)
+      mix_stage(lane, v);
+      publish();
+      if (m == 0 && ok) { mix_mma<64>(tmem, w2, 0, false); tc::mma_commit(done); }
+      mix_load<IO>(v, tp + (size_t)64 * HW, HW, valid);
+      commit_wait();
+      mix_stage(lane, v);
+      publish();
+      if (m == 0 && ok) { mix_mma<64>(tmem, w2, 64, true); tc::mma_commit(done); }
+      float x1[64];
+      mix_load<IO>(x1, (const IO*)P.x + (size_t)img * kBlkC * HW + pos, HW, valid);
+      commit_wait();
+#pragma unroll
+      for (int c0 = 0; c0 < 64; c0 += 32) {
+        float a[32];
+        tc::tmem_ld32(lane + (uint32_t)c0, a);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) x1[c0 + j] = fmaf(vec[kBlkC + c0 + j], a[j] + vec[c0 + j], x1[c0 + j]);
+      }
+      // W3 . LN(x1)
+#pragma unroll
+      for (int c = 0; c < 64; ++c) v[c] = x1[c];
+      mix_norm(v, P.eps);
+      mix_stage(lane, v);
+      publish();
+      if (m == 0 && ok) { mix_mma<128>(tmem, w3, 0, false); tc::mma_commit(done); }
+      commit_wait();
+      // GELU, 64 hidden channels at a time -> W4; the accumulator's first half is free once they have been read
+#pragma unroll 1
+      for (int hf = 0; hf < 2; ++hf) {
+#pragma unroll
+        for (int c0 = 0; c0 < 64; c0 += 32) {
+          float a[32];
+          tc::tmem_ld32(lane + (uint32_t)(64 * hf + c0), a);
+#ifdef __CUDA_ARCH__
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            const float2 b = *(const float2*)(vec + 4 * kBlkC + 64 * hf + c0 + j);
+            const float2 o = gelu_erf2(a[j] + b.x, a[j + 1] + b.y);
+            v[c0 + j] = o.x; v[c0 + j + 1] = o.y;
+          }
+#endif
+        }
+        if (hf) commit_wait();                      // the first half's MMAs have read the operand columns
+        mix_stage(lane, v);
+        publish();
+        if (m == 0 && ok) { mix_mma<64>(tmem, w4, 64 * hf, hf != 0); tc::mma_commit(done); }
+      }
+      mix_load<IO>(v, next, HW, nvalid);
+      commit_wait();
+#pragma unroll
+      for (int c0 = 0; c0 < 64; c0 += 32) {
+        float a[32];
+        tc::tmem_ld32(lane + (uint32_t)c0, a);
+        if (valid && ok) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            st_io<IO>(op, (size_t)(c0 + j) * HW,
+                      fmaf(vec[3 * kBlkC + c0 + j], a[j] + vec[2 * kBlkC + c0 + j], x1[c0 + j]));
+        }
+      }
+    }
+    valid = nvalid; img = nimg; pos = npos;
+  }
+  if (!ok && P.status) atomicExch(P.status, 3);
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(*holder, 512);
+}
+
+template <bool POST, typename IO>
+static int launch_mix(const MixParams& P, int sms, cudaStream_t st) {
+  const size_t smem = (size_t)(POST ? kPostFloats : kPreFloats) * sizeof(float) + 3 * sizeof(uint64_t) + 16;
+  CVB_CUDA(cudaFuncSetAttribute(block_mix_kernel<POST, IO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const long long ntiles = (P.npix + 127) / 128;
+  const int grid = (int)(ntiles < sms ? ntiles : sms);     // one block per SM; tiles go round the blocks first
+  block_mix_kernel<POST, IO><<<grid, kMixThreads, smem, st>>>(P);
+  CVB_CUDA(cudaGetLastError());
+  return CVB_OK;
+}
+
+int launch_block_mix(bool post, const void* x, const void* t, void* out, const void* pack, float eps, int B, int HW,
+                     int io_dtype, int sms, int* status, cudaStream_t st) {
+  MixParams P;
+  P.x = x; P.t = t; P.out = out; P.pack = (const float*)pack; P.eps = eps;
+  P.HW = HW; P.npix = (long long)B * HW; P.status = status;
+  if (post) return io_dtype == CVB_F32 ? launch_mix<true, float>(P, sms, st) : launch_mix<true, __nv_bfloat16>(P, sms, st);
+  return io_dtype == CVB_F32 ? launch_mix<false, float>(P, sms, st) : launch_mix<false, __nv_bfloat16>(P, sms, st);
+}
+
+}  // namespace cvb

@@ -25,58 +25,13 @@ def build_transfer(weight, bias, scale, eps, h, w, x0_term=False):
     Plays the role of the reference's cached kernel spectrum
     (`converse2d.cpp:58-102`), but holds the complete weights-only multiplier.
     Returns a uint8 CUDA tensor owned by the caller."""
-    lib = _cabi.load()
-    if not weight.is_cuda:
-        raise RuntimeError("Converse2D parameters must live on a CUDA device")
-    if weight.dim() != 4 or weight.size(0) != 1:
-        raise RuntimeError("weight must be (1,C,kh,kw)")
-    C, k = weight.size(1), weight.size(2)
-    if weight.size(3) != k:
-        raise RuntimeError("only square kernels are supported")
-    if bias.dim() != 4 or bias.size(0) != 1 or bias.size(1) != C or bias.size(2) != 1 or bias.size(3) != 1:
-        raise RuntimeError("bias must be (1,C,1,1)")
-    if scale < 1:
-        raise RuntimeError("scale must be >= 1")
-    nbytes = lib.cvb_transfer_bytes(C, h, w)
-    if nbytes == 0:
-        raise RuntimeError("padded plane %dx%d is not supported by the FFT engine" % (h, w))
-    wf = weight.detach().reshape(C, k, k).to(torch.float32).contiguous()
-    bf = bias.detach().reshape(C).to(torch.float32).contiguous()
-    table = torch.empty(nbytes, dtype=torch.uint8, device=weight.device)
-    with torch.cuda.device(weight.device):
-        fn = lib.cvb_build_x0_table if x0_term else lib.cvb_build_transfer
-        rc = fn(wf.data_ptr(), bf.data_ptr(), C, k, int(scale), h, w, float(eps), table.data_ptr(),
-                _stream_ptr(weight.device))
-    _cabi.check(rc, "cvb_build_transfer")
-    return table, wf
+    return _cabi.host().build_transfer(weight, bias, int(scale), float(eps), int(h), int(w), bool(x0_term))
 
 
 def converse2d_forward(x, table, weight_f32, kernel_size, scale, padding, padding_mode, fuse_gelu=False,
                        out=None):
     """Fused pad -> solve -> crop (`models/util_converse.py:142-192`) on a CUDA tensor."""
-    lib = _cabi.load()
-    if not x.is_cuda:
-        raise RuntimeError("Converse2D needs a CUDA tensor; this build has no CPU path")
-    if x.dim() != 4:
-        raise RuntimeError("x must be (B,C,H,W)")
-    if padding_mode not in _cabi.PAD_MODES:
-        raise RuntimeError("unknown padding_mode %r" % (padding_mode,))
-    x = x.contiguous()
-    B, C, H, W = x.shape
-    io = _io_dtype(x)
-    s = int(scale)
-    if out is None:
-        out = torch.empty((B, C, H * s, W * s), dtype=x.dtype, device=x.device)
-    ws_bytes = lib.cvb_converse2d_workspace_bytes(B, C, H, W, s, int(padding), io)
-    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=x.device) if ws_bytes else None
-    with torch.cuda.device(x.device):
-        rc = lib.cvb_converse2d_fwd(x.data_ptr(), out.data_ptr(), table.data_ptr(), weight_f32.data_ptr(),
-                                    B, C, H, W, int(kernel_size), s, int(padding),
-                                    _cabi.PAD_MODES[padding_mode], io, 1 if fuse_gelu else 0,
-                                    ws.data_ptr() if ws is not None else None, ws_bytes,
-                                    _stream_ptr(x.device))
-    _cabi.check(rc, "cvb_converse2d_fwd")
-    return out
+    return _cabi.host().converse2d(x, table, weight_f32, kernel_size, scale, padding, padding_mode, fuse_gelu, out)
 
 
 def cross_spectrum_supported(h, w):
@@ -144,6 +99,12 @@ def tap_gradient(g_full, r, kernel_size, scale):
 
 def _f32(t):
     return t.detach().to(torch.float32).contiguous()
+
+
+def block_parameters(ln1, conv1, conv_out, alpha1, ln2, conv_up, conv_down, alpha2):
+    """The parameters of a ConverseBlock around its Converse2D, in the order `block_pack` takes them."""
+    return (ln1.weight, ln1.bias, conv1.weight, conv1.bias, conv_out.weight, conv_out.bias, alpha1, ln2.weight, ln2.bias,
+            conv_up.weight, conv_up.bias, conv_down.weight, conv_down.bias, alpha2)
 
 
 def ln_pw_gelu(x, ln, conv):

@@ -38,13 +38,16 @@ class ConvReverseDataNet(nn.Module):
         self.alpha = nn.Parameter(torch.zeros(1, 64, 1, 1))
         self.eps = eps
 
+    @property
+    def biaseps(self):
+        return torch.sigmoid(self.alpha.detach() - 9.0) + self.eps
+
     def forward(self, x, k, sf, padding=0, padding_mode="circular"):
         if not x.is_cuda:
             raise RuntimeError("ConvReverseDataNet needs CUDA tensors; this build has no CPU path")
         B, C, H, W = x.shape
         if k.dim() != 4 or k.size(0) != B or k.size(1) != C or k.size(2) != k.size(3):
             raise RuntimeError("k must be (B,C,kh,kh) matching x")
-        self.biaseps = torch.sigmoid(self.alpha.detach() - 9.0) + self.eps
         ks = k.size(2)
         h, w = H + 2 * padding, W + 2 * padding
         weight = k.reshape(1, B * C, ks, ks)

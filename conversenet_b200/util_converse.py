@@ -8,7 +8,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from . import functional as CF
+from . import _cabi, functional as CF
 
 
 # False: ConverseBlock runs its layers one by one (PyTorch LayerNorm / 1x1 / GELU around the native
@@ -105,47 +105,61 @@ class Converse2D(nn.Module):
         self.weight.data = F.softmax(self.weight.data.view(1, self.in_channels, -1), dim=-1).view(
             1, self.in_channels, self.kernel_size, self.kernel_size)
         self._tables = OrderedDict()
+        self._last_table = None      # the entry used last, looked at first
         self.fuse_gelu = False  # set by ConverseBlock: apply the following GELU inside the kernel
 
     # -- transfer-table cache: rebuilt when a parameter is modified in place or replaced
     def _table_for(self, h, w, device):
-        key = (h, w, device, self.weight.data_ptr(), self.bias.data_ptr(), self.weight._version,
-               self.bias._version, int(self.scale), float(self.eps))
+        weight, bias = self.weight, self.bias
+        key = (h, w, self.scale, self.eps, device.index, _cabi.host().state(weight, bias))
+        last = self._last_table
+        if last is not None and last[0] == key:
+            return last[1]
         hit = self._tables.get(key)
         if hit is not None:
             self._tables.move_to_end(key)
-            return hit
-        table, wf = CF.build_transfer(self.weight, self.bias, self.scale, self.eps, h, w)
-        self.biaseps = torch.sigmoid(self.bias.detach() - 9.0) + self.eps
-        self._tables[key] = (table, wf)
-        while len(self._tables) > self._TABLE_SLOTS:
-            self._tables.popitem(last=False)
-        return table, wf
+        else:
+            hit = CF.build_transfer(weight, bias, self.scale, self.eps, h, w)
+            self._tables[key] = hit
+            while len(self._tables) > self._TABLE_SLOTS:
+                self._tables.popitem(last=False)
+        self._last_table = (key, hit)
+        return hit
+
+    @property
+    def biaseps(self):
+        """lambda = sigmoid(bias - 9) + eps (`models/util_converse.py:147`)."""
+        return torch.sigmoid(self.bias.detach() - 9.0) + self.eps
 
     def clear_cache(self):
         self._tables.clear()
+        self._last_table = None
 
-    def forward(self, x):
+    def _check_backend(self):
         backend = (os.environ.get("CONVERSE2D_BACKEND", "") or self.backend).lower()
         if backend == "pytorch":
             raise RuntimeError("Converse2D backend='pytorch' is not available: this build only has the "
                                "native sm_100a path")
         if backend not in ("auto", "cuda"):
             raise ValueError(f"backend must be 'auto' | 'cuda' | 'pytorch', got: {backend}")
+
+    def forward(self, x):
+        self._check_backend()
         if not x.is_cuda:
             raise RuntimeError("Converse2D backend='cuda' but the input is not a CUDA tensor.")
-        if x.dim() != 4 or x.size(1) != self.in_channels:
+        shape = x.shape
+        if len(shape) != 4 or shape[1] != self.in_channels:
             raise RuntimeError("x must be (B,%d,H,W)" % self.in_channels)
-        h, w = x.size(2) + 2 * self.padding, x.size(3) + 2 * self.padding
-        table, wf = self._table_for(h, w, x.device)
+        p = self.padding
+        table, wf = self._table_for(shape[2] + 2 * p, shape[3] + 2 * p, x.device)
         if torch.is_grad_enabled() and (x.requires_grad or self.weight.requires_grad or self.bias.requires_grad):
             # differentiable route (the reference is differentiable through torch.fft, converse2d.cpp:223)
             from .autograd import Converse2DFunction
             out = Converse2DFunction.apply(x, self.weight, self.bias, table, wf, self.kernel_size, self.scale,
                                            self.padding, self.padding_mode, self.eps)
             return F.gelu(out) if self.fuse_gelu else out
-        return CF.converse2d_forward(x, table, wf, self.kernel_size, self.scale, self.padding,
-                                     self.padding_mode, fuse_gelu=self.fuse_gelu)
+        return _cabi.host().converse2d(x, table, wf, self.kernel_size, self.scale, p, self.padding_mode, self.fuse_gelu,
+                                       None)
 
 
 class ConverseBlock(nn.Module):
@@ -166,6 +180,7 @@ class ConverseBlock(nn.Module):
                                    nn.Conv2d(out_channels, 2 * out_channels, 1, 1, 0),
                                    nn.GELU(),
                                    nn.Conv2d(2 * out_channels, out_channels, 1, 1, 0))
+        self._pack, self._pack_state = None, None     # 1x1 weights laid out for the kernels
 
     def _branch1(self, x):
         c = self.conv1
@@ -179,19 +194,34 @@ class ConverseBlock(nn.Module):
         return c[5](t)
 
     def _fusable(self, x):
-        c1, c2 = self.conv1, self.conv2
         if torch.is_grad_enabled() and (x.requires_grad or any(q.requires_grad for q in self.parameters())):
             return False  # the fused block kernels are forward-only
-        return (x.is_cuda and x.dim() == 4 and x.size(1) == 64 and c1[1].out_channels == 128 and
-                c1[5].out_channels == 64 and c1[3].scale == 1 and x.dtype in (torch.float32, torch.bfloat16) and
-                c1[1].bias is not None and c1[5].bias is not None and c2[1].bias is not None and
-                c2[3].bias is not None and BLOCK_FUSION)
+        c1, c2 = self.conv1._modules, self.conv2._modules
+        return (x.is_cuda and x.dim() == 4 and x.size(1) == 64 and c1["1"].out_channels == 128 and
+                c1["5"].out_channels == 64 and c1["3"].scale == 1 and x.dtype in (torch.float32, torch.bfloat16) and
+                c1["1"].bias is not None and c1["5"].bias is not None and c2["1"].bias is not None and
+                c2["3"].bias is not None and BLOCK_FUSION)
 
     def _forward_fused(self, x, alpha1=None, alpha2=None):
-        # three kernels per block: LN+1x1+GELU, Converse2D(+GELU), 1x1+residual+LN+1x1+GELU+1x1+residual
+        # LN+1x1+GELU, Converse2D(+GELU), 1x1+residual+LN+1x1+GELU+1x1+residual: one host call
+        c1, c2 = self.conv1._modules, self.conv2._modules
+        conv = c1["3"]
+        params = CF.block_parameters(c1["0"], c1["1"], c1["5"], alpha1, c2["0"], c2["1"], c2["3"], alpha2)
+        host = _cabi.host()
+        state = host.state(*params)
+        if state != self._pack_state:      # weights in the kernels' operand layout, once per version of the parameters
+            self._pack, self._pack_state = host.block_pack(*params), state
+        if conv._forward_hooks or conv._forward_pre_hooks:
+            return self._forward_layers(x, conv, alpha1, alpha2)
+        conv._check_backend()
+        shape, p = x.shape, conv.padding
+        table, wf = conv._table_for(shape[2] + 2 * p, shape[3] + 2 * p, x.device)
+        return host.block(x, table, wf, self._pack, conv.kernel_size, p, conv.padding_mode, c1["0"].eps, c2["0"].eps)
+
+    def _forward_layers(self, x, conv, alpha1, alpha2):
+        # the same kernels with Converse2D called as a module (someone hooked it)
         c1, c2 = self.conv1, self.conv2
         t = CF.ln_pw_gelu(x, c1[0], c1[1])
-        conv = c1[3]
         conv.fuse_gelu = True
         try:
             t = conv(t)

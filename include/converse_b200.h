@@ -165,6 +165,24 @@ int cvb_pw_res_fwd(const void* t, const void* res, void* out, const float* w, co
                    const float* alpha, int B, int C, int HW, int io_dtype, void* stream);
 
 /*
+ * The two sides of ConverseBlock around Converse2D with the weights prepared once (tcgen05; any image size, any
+ * alignment, fp32 or bf16 tensors, C = 64):
+ *   cvb_block_pack     weights and vectors of the whole block (as the two functions above name them; alphas may be NULL)
+ *                      in the operand layout of the kernels, LayerNorm affines folded in: cvb_block_pack_bytes()
+ *                      device bytes at `pack`, 16-byte aligned
+ *   cvb_block_pre_fwd  out (B,2C,HW) = GELU( W1 . LayerNorm(x) + b1 )            (models/util_converse.py:278-280)
+ *   cvb_block_post_fwd x1 = x + alpha1 (W2 . t + b2);
+ *                      out = x1 + alpha2 (W4 . GELU( W3 . LayerNorm(x1) + b3 ) + b4)    (:283, :285-288, :291-292)
+ */
+size_t cvb_block_pack_bytes(void);
+int cvb_block_pack(const float* ln1_w, const float* ln1_b, const float* w1, const float* b1, const float* w2,
+                   const float* b2, const float* alpha1, const float* ln2_w, const float* ln2_b, const float* w3,
+                   const float* b3, const float* w4, const float* b4, const float* alpha2, void* pack, void* stream);
+int cvb_block_pre_fwd(const void* x, void* out, const void* pack, float ln_eps, int B, int HW, int io_dtype, void* stream);
+int cvb_block_post_fwd(const void* t, const void* x, void* out, const void* pack, float ln_eps, int B, int HW,
+                       int io_dtype, void* stream);
+
+/*
  * Converse2D forward for callers that cannot allocate device memory.
  *
  * Same arguments, result and error codes as cvb_converse2d_fwd, minus the workspace:
