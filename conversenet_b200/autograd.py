@@ -22,17 +22,17 @@ dL/dweight and dL/dbias.  The parameters act through the multiplier M (G or P, o
 tensor) and, at scale >= 2, through the taps of the epilogue's correlation:
     L = (1 / (h w)) Re sum_f M[f] D[f]  (+ terms without M),
     D[f] = sum_b FFT2(y_b)[f] conj(FFT2(q_b)[f]),   q = g_full (scale 1) or v (scale >= 2).
-D, the reduction over the batch, is one native kernel (`functional.cross_spectrum`); the chain rule
-from D to the k x k taps and lambda runs through `transfer_multiplier`, the closed form of M written
-with `torch.fft` on that single (C, s h, s w) tensor.  The direct tap term of scale >= 2,
-dK[a] = sum_m g_full[s m - a + c] r[m], needs r = IFFT2(P . FFT2(y)): the forward kernel at scale 1
-on the padded planes, followed by k^2 strided products.  Planes the cross-spectrum kernel does not
-take (two planes must fit shared memory) fall back to autograd through `spectral_forward`, the
-whole operator restated with `torch.fft` (library kernels).
+All of it runs in the kernels of `csrc/k_rp_bwd.cu` (one native call, eight launches): the row transforms
+of y and q meet in one kernel that sums D over the batch and sends q on through conj(M); the chain rule
+from D to the taps and lambda is closed form; the direct tap term of scale >= 2 uses the plane
+r = IFFT2(P . FFT2(y)) kept by the forward.  Planes without a two-stage transform plan (a prime factor
+times a remainder above the kernels' radices) take `grad_input_composed` and autograd through
+`spectral_forward`, the operator restated with `torch.fft` (library kernels).
 """
 import torch
 import torch.nn.functional as F
 
+from . import _cabi
 from . import functional as CF
 
 
@@ -119,19 +119,27 @@ class _Cotangent:
             self.v = F.conv2d(gp, wf.flip(-2, -1).reshape(C, 1, k, k), stride=s, groups=C).contiguous()
 
 
-def grad_input(g, weight, bias, scale, padding, padding_mode, eps, in_shape, table=None, cot=None):
+def grad_input(g, weight, bias, scale, padding, padding_mode, eps, in_shape, table=None):
     """dL/dx for g = dL/dout (B,C,sH,sW) through the native kernels.  `table`: the forward's
     transfer table for the padded size, if the caller has it."""
+    if table is None:
+        table, _ = CF.build_transfer(weight, bias, scale, eps, in_shape[2] + 2 * int(padding), in_shape[3] + 2 * int(padding))
+    out = _cabi.host().backward(None, g, None, table, weight, bias, tuple(in_shape), int(scale), int(padding), padding_mode,
+                                float(eps), True, False)
+    if out is not None:
+        return out[0].to(g.dtype)
+    return grad_input_composed(g, weight, bias, scale, padding, padding_mode, eps, in_shape, table)
+
+
+def grad_input_composed(g, weight, bias, scale, padding, padding_mode, eps, in_shape, table):
+    """The same through the forward kernels with the conjugated table and PyTorch tensor ops around them."""
     s, p = int(scale), int(padding)
     B, C, H, W = in_shape
     h, w = H + 2 * p, W + 2 * p
     k = weight.size(-1)
-    if table is None:
-        table, _ = CF.build_transfer(weight, bias, s, eps, h, w)
     wf = weight.detach().reshape(C, k, k).to(torch.float32).contiguous()
     ctab = _conjugated(table, C * h * w)
-    if cot is None:
-        cot = _Cotangent(g, wf, k, s, p)
+    cot = _Cotangent(g, wf, k, s, p)
     if s == 1:
         g_y = CF.converse2d_forward(cot.g_full, ctab, wf, k, 1, 0, "circular")
     else:
@@ -147,67 +155,68 @@ def grad_input(g, weight, bias, scale, padding, padding_mode, eps, in_shape, tab
     return torch.autograd.grad(padded, probe, g_y)[0]
 
 
-def grad_params(x, g, weight, bias, scale, padding, padding_mode, eps, table=None, cot=None):
-    """(dL/dweight, dL/dbias) in fp32 for g = dL/dout, batch reductions in the native kernels; None when
-    the cross-spectrum kernel does not take the padded plane (the caller then falls back)."""
+def grad_params(x, g, weight, bias, scale, padding, padding_mode, eps, table=None, r=None):
+    """(dL/dweight, dL/dbias) in fp32 for g = dL/dout; None when the native kernels do not take the padded plane (the
+    caller then falls back).  `r`: the plane the training forward kept (scale >= 2)."""
     s, p = int(scale), int(padding)
-    B, C, H, W = x.shape
-    h, w = H + 2 * p, W + 2 * p
-    if not CF.cross_spectrum_supported(h, w):
-        return None
     k = weight.size(-1)
     if table is None:
-        table, _ = CF.build_transfer(weight, bias, s, eps, h, w)
-    wf = weight.detach().reshape(C, k, k).to(torch.float32).contiguous()
-    xf = x.detach().float().contiguous()
-    if cot is None:
-        cot = _Cotangent(g, wf, k, s, p)
-    D = CF.cross_spectrum(xf, cot.g_full if s == 1 else cot.v, table, p, padding_mode)   # (C,h,w) complex
-    with torch.enable_grad():
-        w_ = weight.detach().float().requires_grad_(True)
-        b_ = bias.detach().float().requires_grad_(True)
-        M = transfer_multiplier(w_, b_, s, eps, h, w)[0]
-        proxy = (M * D).real.sum() / float(h * w)
-        gw, gb = torch.autograd.grad(proxy, (w_, b_))
-    if s > 1:
-        # direct dependence of corr(K, zero_insert(r)) on the taps; r = the forward at scale 1 on the padded planes
-        y = _pad(xf, p, padding_mode).contiguous()
-        r = CF.converse2d_forward(y, table, wf, k, 1, 0, "circular")
-        gw = gw + CF.tap_gradient(cot.g_full, r, k, s).reshape(1, C, k, k)
-    return gw, gb
+        table, _ = CF.build_transfer(weight, bias, s, eps, x.size(2) + 2 * p, x.size(3) + 2 * p)
+    if s > 1 and r is None:
+        wf = weight.detach().reshape(weight.size(1), k, k).to(torch.float32).contiguous()
+        kept = _cabi.host().train_forward(x.detach().float(), table, wf, k, s, p, padding_mode)
+        if kept is None:
+            return None
+        r = kept[1]
+    out = _cabi.host().backward(x, g, r, table, weight, bias, tuple(x.shape), s, p, padding_mode, float(eps), False, True)
+    return None if out is None else out[1:]
 
 
 class Converse2DFunction(torch.autograd.Function):
-    """Native forward; native dL/dx; parameter gradients from the native batch-summed cross spectrum
-    (`grad_params`), through `spectral_forward` for planes that kernel does not take."""
+    """Native forward and gradients; `grad_input_composed` and `spectral_forward` for planes the gradient kernels do
+    not take."""
 
     @staticmethod
     def forward(ctx, x, weight, bias, table, wf, kernel_size, scale, padding, padding_mode, eps):
         ctx.save_for_backward(x, weight, bias)
         ctx.table = table
+        ctx.r = None
         ctx.cfg = (int(kernel_size), int(scale), int(padding), padding_mode, float(eps))
+        if ctx.needs_input_grad[1] or ctx.needs_input_grad[2]:
+            kept = _cabi.host().train_forward(x, table, wf, kernel_size, scale, padding, padding_mode)
+            if kept is not None:
+                out, ctx.r = kept
+                return out
         return CF.converse2d_forward(x, table, wf, kernel_size, scale, padding, padding_mode)
 
     @staticmethod
     def backward(ctx, g):
         x, weight, bias = ctx.saved_tensors
         k, s, p, mode, eps = ctx.cfg
+        want_x = ctx.needs_input_grad[0]
+        want_p = ctx.needs_input_grad[1] or ctx.needs_input_grad[2]
         gx = gw = gb = None
-        C = weight.size(1)
-        cot = _Cotangent(g, weight.detach().reshape(C, k, k).to(torch.float32), k, s, p)
-        if ctx.needs_input_grad[0]:
-            gx = grad_input(g, weight, bias, s, p, mode, eps, x.shape, table=ctx.table, cot=cot)
-        if ctx.needs_input_grad[1] or ctx.needs_input_grad[2]:
-            native = (grad_params(x, g, weight, bias, s, p, mode, eps, table=ctx.table, cot=cot)
-                      if NATIVE_PARAM_GRADS else None)
-            if native is not None:
-                gw, gb = native
-            else:
-                with torch.enable_grad():
-                    w_ = weight.detach().float().requires_grad_(True)
-                    b_ = bias.detach().float().requires_grad_(True)
-                    out = spectral_forward(x.detach().float(), w_, b_, s, p, mode, eps)
-                    gw, gb = torch.autograd.grad(out, (w_, b_), g.float())
-            gw = gw.to(weight.dtype) if ctx.needs_input_grad[1] else None
-            gb = gb.to(bias.dtype) if ctx.needs_input_grad[2] else None
+        native_p = want_p and NATIVE_PARAM_GRADS and (s == 1 or ctx.r is not None)
+        out = None
+        if want_x or native_p:
+            out = _cabi.host().backward(x, g, ctx.r, ctx.table, weight, bias, tuple(x.shape), s, p, mode, eps, want_x,
+                                        native_p)
+            if out is None and native_p and want_x:      # perhaps dL/dx alone
+                native_p = False
+                out = _cabi.host().backward(None, g, None, ctx.table, weight, bias, tuple(x.shape), s, p, mode, eps, True,
+                                            False)
+        if out is not None:
+            gx, gw, gb = out
+        elif want_x:
+            gx = grad_input_composed(g, weight, bias, s, p, mode, eps, x.shape, ctx.table)
+        if want_p and gw is None:
+            with torch.enable_grad():
+                w_ = weight.detach().float().requires_grad_(True)
+                b_ = bias.detach().float().requires_grad_(True)
+                y = spectral_forward(x.detach().float(), w_, b_, s, p, mode, eps)
+                gw, gb = torch.autograd.grad(y, (w_, b_), g.float())
+        if gx is not None:
+            gx = gx.to(x.dtype)
+        gw = gw.to(weight.dtype) if gw is not None and ctx.needs_input_grad[1] else None
+        gb = gb.to(bias.dtype) if gb is not None and ctx.needs_input_grad[2] else None
         return gx, gw, gb, None, None, None, None, None, None, None

@@ -466,6 +466,48 @@ int cvb_pw_res_fwd(const void* t, const void* res, void* out, const float* w, co
                    : launch_pw_res_tc(P, sm_count(), status_ptr(), (cudaStream_t)stream);
 }
 
+int cvb_converse2d_fwd_train(const void* x, void* out, const void* table, const float* weight, float* r_keep, int B,
+                             int C, int H, int W, int k, int s, int p, int pad_mode, int io_dtype, void* workspace,
+                             size_t workspace_bytes, void* stream) {
+  if (!x || !out || !table || B < 1 || C < 1 || H < 1 || W < 1 || k < 1 || s < 1) return CVB_ERR_BAD_ARGUMENT;
+  if (s > 1 && !weight) return CVB_ERR_BAD_ARGUMENT;
+  if (io_dtype != CVB_F32 && io_dtype != CVB_BF16) return CVB_ERR_BAD_ARGUMENT;
+  if (k > kMaxTaps || k > s * (H + 2 * p) || k > s * (W + 2 * p)) return CVB_ERR_KERNEL_TOO_LARGE;
+  const int rc = check_padding(H, W, p, pad_mode);
+  if (rc != CVB_OK) return rc;
+  rp::Params Q;
+  if (!rp::fill_params(Q, table, B, C, H, W, k, s, p, pad_mode)) return CVB_ERR_UNSUPPORTED_SIZE;
+  Q.x = x; Q.out = out; Q.weight = weight; Q.rsave = s > 1 ? r_keep : nullptr;
+  const rp::Route r = rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0,
+                                std::max(kRpWorkspace, rp::ws_plane_bytes(Q.h, Q.w, s)));
+  return rp::run(Q, r, io_dtype, workspace, workspace_bytes, (cudaStream_t)stream);
+}
+
+size_t cvb_converse2d_train_workspace_bytes(int B, int C, int H, int W, int s, int p) {
+  if (B < 1 || C < 1 || H < 1 || W < 1 || p < 0 || s < 1 || !rp::supported(H + 2 * p, W + 2 * p)) return 0;
+  return rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0,
+                   std::max(kRpWorkspace, rp::ws_plane_bytes(H + 2 * p, W + 2 * p, s))).ws_bytes;
+}
+
+size_t cvb_converse2d_bwd_workspace_bytes(int B, int C, int H, int W, int k, int s, int p, int want_x, int want_params) {
+  if (B < 1 || C < 1 || H < 1 || W < 1 || k < 1 || k > kMaxTaps || p < 0 || s < 1) return 0;
+  if (!rp::supported(H + 2 * p, W + 2 * p)) return 0;
+  return rp::bwd_workspace(B, C, H, W, k, s, p, want_x != 0, want_params != 0, sm_count());
+}
+
+int cvb_converse2d_bwd(const float* x, const float* g, const float* r, const void* table, const float* weight,
+                       const float* bias, float* gx, float* gw, float* gb, int B, int C, int H, int W, int k, int s,
+                       int p, int pad_mode, float eps, void* workspace, size_t workspace_bytes, void* stream) {
+  if (!g || !table || !weight || B < 1 || C < 1 || H < 1 || W < 1 || k < 1 || s < 1) return CVB_ERR_BAD_ARGUMENT;
+  if ((gw == nullptr) != (gb == nullptr) || (!gx && !gw)) return CVB_ERR_BAD_ARGUMENT;
+  if (gw && (!x || !bias)) return CVB_ERR_BAD_ARGUMENT;
+  if (k > kMaxTaps || k > s * (H + 2 * p) || k > s * (W + 2 * p)) return CVB_ERR_KERNEL_TOO_LARGE;
+  const int rc = check_padding(H, W, p, pad_mode);
+  if (rc != CVB_OK) return rc;
+  return rp::run_bwd(x, g, r, table, weight, bias, gx, gw, gb, B, C, H, W, k, s, p, pad_mode, eps, workspace,
+                     workspace_bytes, sm_count(), (cudaStream_t)stream);
+}
+
 size_t cvb_block_pack_bytes(void) { return block_pack_bytes(); }
 
 int cvb_block_pack(const float* ln1_w, const float* ln1_b, const float* w1, const float* b1, const float* w2,

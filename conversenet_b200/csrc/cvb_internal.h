@@ -47,6 +47,13 @@ struct Route;
 size_t table_bytes(int C, int h, int w);
 int build_table(const float* weight, const float* bias, int C, int k, int s, int h, int w, float eps, int kind,
                 void* table, cudaStream_t st);
+int cols_fwd(Params& P, int planes, cudaStream_t st);
+int rows(Params& P, int planes, cudaStream_t st);
+int cols_inv(Params& P, int planes, cudaStream_t st);
+size_t bwd_workspace(int B, int C, int H, int W, int k, int s, int p, bool want_x, bool want_params, int sms);
+int run_bwd(const float* x, const float* g, const float* r, const void* table, const float* weight, const float* bias,
+            float* gx, float* gw, float* gb, int B, int C, int H, int W, int k, int s, int p, int pad_mode, float eps,
+            void* workspace, size_t ws_bytes, int sms, cudaStream_t st);
 int run(Params& P, const Route& r, int io_dtype, void* workspace, size_t ws_bytes, cudaStream_t st);
 }  // namespace rp
 

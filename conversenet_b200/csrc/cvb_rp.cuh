@@ -46,9 +46,11 @@ struct Params {
   int h, w, hh, wc, wp; // hh = h / 2 + 1 rows, wc column pairs, wp = 2 wc
   int conj;             // 1: multiply by the conjugated table (the adjoint)
   int plane0, nplane;   // planes of this launch (plane = b * C + c)
-  int vec;              // p and W even, pointers aligned: pairs of columns are loaded and stored at once
+  int po, OH, OW;       // the output is the solved plane cropped to rows po .. po + OH - 1, columns likewise
+  int vec, vec_out;     // pairs of columns are loaded (stored) at once: offset and width even, pointer aligned
   float2* ws;           // [nplane][hh][wp]
   float* r;             // scale >= 2: [nplane][h][wp]
+  float* rsave;         // scale >= 2: all planes' r kept for the backward ([B C][h][wp]), or null
   int pitch;            // rows kernel / plane kernel: odd row pitch (complex) of the shared-memory rows
   float inv_wc, inv_hh;
   Axis ay, ax;
@@ -261,14 +263,14 @@ __device__ __forceinline__ void load_rows(const Params& P, const ColumnPair<IO>&
 // store (column 2c, -column 2c+1) of padded row y: crop, GELU
 template <typename IO>
 __device__ __forceinline__ void store_crop(const Params& P, IO* op, int y, int c, float2 v) {
-  const int oy = y - P.p;
-  if ((unsigned)oy >= (unsigned)P.H) return;
-  const int ox = 2 * c - P.p;
+  const int oy = y - P.po;
+  if ((unsigned)oy >= (unsigned)P.OH) return;
+  const int ox = 2 * c - P.po;
   float a = v.x, b = -v.y;
   if (P.gelu) gelu_pair(a, b);
-  IO* o = op + (size_t)(oy * P.W + ox);
-  if (P.vec) {    // p and W even: both columns are inside or outside, and aligned
-    if ((unsigned)ox < (unsigned)P.W) {
+  IO* o = op + (size_t)(oy * P.OW + ox);
+  if (P.vec_out) {    // both columns are inside or outside, and aligned
+    if ((unsigned)ox < (unsigned)P.OW) {
       if constexpr (sizeof(IO) == 4) {
         *(float2*)o = make_float2(a, b);
       } else {
@@ -276,8 +278,8 @@ __device__ __forceinline__ void store_crop(const Params& P, IO* op, int y, int c
       }
     }
   } else {
-    if ((unsigned)ox < (unsigned)P.W) st_io<IO>(o, 0, a);
-    if ((unsigned)(ox + 1) < (unsigned)P.W) st_io<IO>(o, 1, b);
+    if ((unsigned)ox < (unsigned)P.OW) st_io<IO>(o, 0, a);
+    if ((unsigned)(ox + 1) < (unsigned)P.OW) st_io<IO>(o, 1, b);
   }
 }
 
@@ -627,7 +629,7 @@ __device__ __forceinline__ void cols_inv_body(const Params& P, float2* T) {
     }
   });
   __syncthreads();
-  IO* op = (IO*)P.out + (size_t)(P.plane0 + pl) * P.H * P.W;
+  IO* op = (IO*)P.out + (size_t)(P.plane0 + pl) * P.OH * P.OW;
   float2* rl = (float2*)P.r + (size_t)pl * P.h * P.wc + c;
   if constexpr (MP == 0) {
     if (!valid) return;
@@ -1058,6 +1060,10 @@ __device__ __forceinline__ void plane_body(const Params& P, float2* sm) {
       });
     if (P.s > 1) {
       __syncthreads();
+      if (P.rsave) {
+        float2* keep = (float2*)P.rsave + (size_t)plane * h * wc;
+        for (int i = tid; i < h * wc; i += nthr) keep[i] = T1[i];
+      }
       epilogue<IO>(P, (const float*)T1, 2 * wc, wk, xp, op, tid, nthr, 0, P.H);
     }
   }

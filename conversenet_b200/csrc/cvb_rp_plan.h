@@ -86,7 +86,7 @@ inline bool fill_params(Params& P, const void* table, int B, int C, int H, int W
   P.inv_wc = 1.0f / (float)P.wc; P.inv_hh = 1.0f / (float)P.hh;
   fill_axis(P.ay, h, r0y, r1y, t + bl.twy, t + bl.dmy);
   fill_axis(P.ax, w, r0x, r1x, t + bl.twx, t + bl.dmx);
-  P.gelu = 0; P.conj = 0; P.plane0 = 0; P.nplane = 0; P.vec = 0;
+  P.gelu = 0; P.conj = 0; P.plane0 = 0; P.nplane = 0; P.vec = 0; P.vec_out = 0; P.po = p; P.OH = H; P.OW = W; P.rsave = nullptr;
   P.ws = nullptr; P.r = nullptr; P.x = nullptr; P.out = nullptr; P.weight = nullptr;
   return true;
 }

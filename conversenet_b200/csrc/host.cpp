@@ -31,6 +31,10 @@ struct Api {
   decltype(&cvb_block_pack) block_pack = nullptr;
   decltype(&cvb_block_pre_fwd) block_pre = nullptr;
   decltype(&cvb_block_post_fwd) block_post = nullptr;
+  decltype(&cvb_converse2d_train_workspace_bytes) train_workspace_bytes = nullptr;
+  decltype(&cvb_converse2d_fwd_train) fwd_train = nullptr;
+  decltype(&cvb_converse2d_bwd_workspace_bytes) bwd_workspace_bytes = nullptr;
+  decltype(&cvb_converse2d_bwd) bwd = nullptr;
 } api;
 
 struct Failed : std::runtime_error { using std::runtime_error::runtime_error; };
@@ -221,17 +225,82 @@ PyObject* py_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+// train_forward(x, table, weight_f32, kernel_size, scale, padding, padding_mode) -> (out, r or None); None when the
+// gradient kernels have no plan for the padded plane
+PyObject* py_train_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    want(n, 7);
+    const at::Tensor& x0 = cuda_tensor(a[0], "x");
+    if (x0.dim() != 4) throw Failed("x must be (B,C,H,W)");
+    const c10::cuda::CUDAGuard dev(x0.device());
+    const at::Tensor x = x0.is_contiguous() ? x0 : x0.contiguous();
+    const int B = (int)x.size(0), C = (int)x.size(1), H = (int)x.size(2), W = (int)x.size(3), io = io_type(x);
+    const int k = (int)integer(a[3]), s = (int)integer(a[4]), p = (int)integer(a[5]), mode = pad_mode(a[6]);
+    at::Tensor out = at::empty({B, C, (int64_t)H * s, (int64_t)W * s}, x.options().requires_grad(false)), r, w;
+    if (s > 1) r = at::empty({B, C, H + 2 * p, (W + 2 * p + 1) / 2 * 2}, x.options().dtype(at::kFloat).requires_grad(false));
+    const size_t ws = api.train_workspace_bytes(B, C, H, W, s, p);
+    if (ws) w = bytes_like(x, ws);
+    const int rc = api.fwd_train(x.data_ptr(), out.data_ptr(), tensor(a[1], "table").data_ptr(),
+                                 (const float*)tensor(a[2], "weight").data_ptr(), s > 1 ? (float*)r.data_ptr() : nullptr, B, C,
+                                 H, W, k, s, p, mode, io, ws ? w.data_ptr() : nullptr, ws, stream(x));
+    if (rc == CVB_ERR_UNSUPPORTED_SIZE) Py_RETURN_NONE;
+    check(rc, "cvb_converse2d_fwd_train");
+    PyObject* rr = Py_None;
+    if (s > 1) rr = THPVariable_Wrap(r);
+    else Py_INCREF(rr);
+    return Py_BuildValue("(NN)", THPVariable_Wrap(out), rr);
+  });
+}
+
+// backward(x or None, g, r or None, table, weight, bias, (B,C,H,W) of x, scale, padding, padding_mode, eps, want_x,
+// want_params) -> (gx, gw, gb), unwanted ones None; None when the kernels do not take the shape
+PyObject* py_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    want(n, 13);
+    const at::Tensor g = f32(cuda_tensor(a[1], "g").detach());
+    const c10::cuda::CUDAGuard dev(g.device());
+    const at::Tensor &w0 = tensor(a[4], "weight"), &b0 = tensor(a[5], "bias");
+    int d[4];
+    for (int i = 0; i < 4; ++i) d[i] = (int)integer(PyTuple_GetItem(a[6], i));
+    const int B = d[0], C = d[1], H = d[2], W = d[3], k = (int)w0.size(-1);
+    const int s = (int)integer(a[7]), p = (int)integer(a[8]), mode = pad_mode(a[9]);
+    const bool wx = PyObject_IsTrue(a[11]), wp = PyObject_IsTrue(a[12]);
+    const size_t ws = api.bwd_workspace_bytes(B, C, H, W, k, s, p, wx, wp);
+    if (!ws) Py_RETURN_NONE;
+    const at::Tensor wf = f32(w0.detach()), bf = f32(b0.detach());
+    at::Tensor x, r, gx, gw, gb;
+    if (wp) x = f32(cuda_tensor(a[0], "x").detach());
+    if (a[2] != Py_None) r = tensor(a[2], "r");
+    const auto opt = g.options().requires_grad(false);
+    if (wx) gx = at::empty({B, C, H, W}, opt);
+    if (wp) {
+      gw = at::empty(w0.sizes(), opt);
+      gb = at::empty(b0.sizes(), opt);
+    }
+    at::Tensor work = bytes_like(g, ws);
+    auto ptr = [](const at::Tensor& t) { return t.defined() ? (float*)t.data_ptr() : nullptr; };
+    check(api.bwd(ptr(x), ptr(g), ptr(r), tensor(a[3], "table").data_ptr(), ptr(wf), ptr(bf), ptr(gx), ptr(gw), ptr(gb), B, C,
+                  H, W, k, s, p, mode, (float)real(a[10]), work.data_ptr(), ws, stream(g)),
+          "cvb_converse2d_bwd");
+    auto wrap = [](const at::Tensor& t) -> PyObject* {
+      if (t.defined()) return THPVariable_Wrap(t);
+      Py_RETURN_NONE;
+    };
+    return Py_BuildValue("(NNN)", wrap(gx), wrap(gw), wrap(gb));
+  });
+}
+
 // init(address of each C ABI function in the order of `names`)
 PyObject* py_init(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    want(n, 11);
-    void* p[11];
-    for (int i = 0; i < 11; ++i) p[i] = PyLong_AsVoidPtr(a[i]);
+    want(n, 15);
+    void* p[15];
+    for (int i = 0; i < 15; ++i) p[i] = PyLong_AsVoidPtr(a[i]);
     int i = 0;
     auto set = [&](auto& f) { f = (std::decay_t<decltype(f)>)p[i++]; };
     set(api.strerror_); set(api.last_cuda_error); set(api.transfer_bytes); set(api.build_transfer); set(api.build_x0_table);
     set(api.workspace_bytes); set(api.converse2d_fwd); set(api.block_pack_bytes); set(api.block_pack); set(api.block_pre);
-    set(api.block_post);
+    set(api.block_post); set(api.train_workspace_bytes); set(api.fwd_train); set(api.bwd_workspace_bytes); set(api.bwd);
     Py_RETURN_NONE;
   });
 }
@@ -242,6 +311,8 @@ PyMethodDef methods[] = {
     {"build_transfer", (PyCFunction)(void (*)(void))py_build_transfer, METH_FASTCALL, nullptr},
     {"state", (PyCFunction)(void (*)(void))py_state, METH_FASTCALL, nullptr},
     {"block_pack", (PyCFunction)(void (*)(void))py_block_pack, METH_FASTCALL, nullptr},
+    {"train_forward", (PyCFunction)(void (*)(void))py_train_forward, METH_FASTCALL, nullptr},
+    {"backward", (PyCFunction)(void (*)(void))py_backward, METH_FASTCALL, nullptr},
     {"block", (PyCFunction)(void (*)(void))py_block, METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
@@ -251,10 +322,11 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, null
 PyMODINIT_FUNC PyInit__host(void) {
   PyObject* m = PyModule_Create(&module);
   if (!m) return nullptr;
-  PyObject* names = Py_BuildValue("(sssssssssss)", "cvb_strerror", "cvb_last_cuda_error", "cvb_transfer_bytes",
+  PyObject* names = Py_BuildValue("(sssssssssssssss)", "cvb_strerror", "cvb_last_cuda_error", "cvb_transfer_bytes",
                                   "cvb_build_transfer", "cvb_build_x0_table", "cvb_converse2d_workspace_bytes",
                                   "cvb_converse2d_fwd", "cvb_block_pack_bytes", "cvb_block_pack", "cvb_block_pre_fwd",
-                                  "cvb_block_post_fwd");
+                                  "cvb_block_post_fwd", "cvb_converse2d_train_workspace_bytes",
+                                  "cvb_converse2d_fwd_train", "cvb_converse2d_bwd_workspace_bytes", "cvb_converse2d_bwd");
   if (!names || PyModule_AddObject(m, "names", names) < 0) return nullptr;
   return m;
 }

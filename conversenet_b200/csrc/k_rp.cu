@@ -206,10 +206,31 @@ int build_table(const float* weight, const float* bias, int C, int k, int s, int
 }
 
 // ------------------------------------------------------------------ forward
+static void set_vec(Params& P, bool f32) {
+  P.vec = P.p % 2 == 0 && P.W % 2 == 0 && ((size_t)P.x) % (f32 ? 8 : 4) == 0;
+  P.vec_out = P.po % 2 == 0 && P.OW % 2 == 0 && ((size_t)P.out) % (f32 ? 8 : 4) == 0;
+}
+
+// one launch of each strip kernel over planes 0 .. planes - 1 (fp32 tensors)
+static int strip(Params& P, int planes, int which, cudaStream_t st) {
+  set_vec(P, true);
+  P.plane0 = 0; P.nplane = planes;
+  const int gc = (planes * P.wc + kLines - 1) / kLines, gr = (planes * P.hh + kLines - 1) / kLines;
+  if (which == 1)
+    return P.ax.mp ? matrix_entry(P.ax.mp).rows(P, CVB_F32, gr, rows_smem(P), st)
+                   : launch_rows(P, small_axis(P.ax), gr, rows_smem(P), st);
+  if (P.ay.mp)
+    return (which == 0 ? matrix_entry(P.ay.mp).cols_fwd : matrix_entry(P.ay.mp).cols_inv)(P, CVB_F32, gc, cols_smem(P), st);
+  return (which == 0 ? launch_cols_fwd_f32 : launch_cols_inv_f32)(P, small_axis(P.ay), gc, cols_smem(P), st);
+}
+int cols_fwd(Params& P, int planes, cudaStream_t st) { return strip(P, planes, 0, st); }
+int rows(Params& P, int planes, cudaStream_t st) { return strip(P, planes, 1, st); }
+int cols_inv(Params& P, int planes, cudaStream_t st) { return strip(P, planes, 2, st); }
+
 int run(Params& P, const Route& r, int io_dtype, void* workspace, size_t ws_bytes, cudaStream_t st) {
   const bool f32 = io_dtype == CVB_F32;
   const int planes = P.B * P.C;
-  P.vec = P.p % 2 == 0 && P.W % 2 == 0 && (((size_t)P.out) | ((size_t)P.x)) % (f32 ? 8 : 4) == 0;
+  set_vec(P, f32);
   if (r.one_block) {
     P.plane0 = 0; P.nplane = planes;
     const size_t smem = plane_smem(P.h, P.w, P.k);
@@ -225,7 +246,9 @@ int run(Params& P, const Route& r, int io_dtype, void* workspace, size_t ws_byte
   for (int p0 = 0; p0 < planes; p0 += r.chunk) {
     P.plane0 = p0;
     P.nplane = planes - p0 < r.chunk ? planes - p0 : r.chunk;
-    if (P.s > 1) P.r = (float*)((char*)workspace + (size_t)P.nplane * P.hh * P.wp * sizeof(float2));
+    if (P.s > 1)
+      P.r = P.rsave ? P.rsave + (size_t)p0 * P.h * P.wp
+                    : (float*)((char*)workspace + (size_t)P.nplane * P.hh * P.wp * sizeof(float2));
     const int gc = (P.nplane * P.wc + kLines - 1) / kLines, gr = (P.nplane * P.hh + kLines - 1) / kLines;
     int rc = P.ay.mp ? matrix_entry(P.ay.mp).cols_fwd(P, io_dtype, gc, smem_c, st)
              : f32   ? launch_cols_fwd_f32(P, sy, gc, smem_c, st)

@@ -2,7 +2,7 @@
 // once per width with -DCVB_MP=..; 128 threads, as many blocks on an SM as the pairs held in registers allow.
 #include "../../include/converse_b200.h"
 #include "cvb_internal.h"
-#include "cvb_rp.cuh"
+#include "cvb_rp_bwd.cuh"
 
 #define CVB_CAT_(a, b) a##_##b
 #define CVB_CAT(a, b) CVB_CAT_(a, b)
@@ -27,6 +27,12 @@ __global__ void __launch_bounds__(128, CVB_RP_BLOCKS) matrix_cols_inv_kernel(con
   cols_inv_body<IO, kMatrixR1, MP>(P, smem);
 }
 
+template <int MP>
+__global__ void __launch_bounds__(128, 3) matrix_rows_bwd_kernel(const __grid_constant__ BwdParams Q) {
+  extern __shared__ float2 smem[];
+  rows_bwd_body<kMatrixR1, MP>(Q, smem);
+}
+
 template <typename K>
 static int go(K kernel, const Params& P, int grid, size_t smem, cudaStream_t st) {
   CVB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -44,6 +50,13 @@ int CVB_CAT(launch_matrix_rows, CVB_MP)(const Params& P, int, int grid, size_t s
 int CVB_CAT(launch_matrix_cols_inv, CVB_MP)(const Params& P, int io_dtype, int grid, size_t smem, cudaStream_t st) {
   return io_dtype == CVB_F32 ? go(matrix_cols_inv_kernel<float, CVB_MP>, P, grid, smem, st)
                              : go(matrix_cols_inv_kernel<__nv_bfloat16, CVB_MP>, P, grid, smem, st);
+}
+
+int CVB_CAT(launch_matrix_rows_bwd, CVB_MP)(const BwdParams& Q, dim3 grid, size_t smem, cudaStream_t st) {
+  CVB_CUDA(cudaFuncSetAttribute(matrix_rows_bwd_kernel<CVB_MP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  matrix_rows_bwd_kernel<CVB_MP><<<grid, 128, smem, st>>>(Q);
+  CVB_CUDA(cudaGetLastError());
+  return CVB_OK;
 }
 
 }  // namespace rp

@@ -215,6 +215,29 @@ int cvb_converse2d_fwd_static_scratch(const void* x, void* out, const void* tabl
                                       int io_dtype, int fuse_gelu, void* stream);
 
 /*
+ * Training form of cvb_converse2d_fwd (no fused GELU): at scale >= 2, r_keep (B,C,h,wp) fp32 with wp = w rounded up to
+ * even receives the plane r = IFFT2(P . FFT2(pad(x))) that the gradient of the taps needs.  CVB_ERR_UNSUPPORTED_SIZE
+ * (workspace query 0 does not tell: it is also 0 for planes that need none) when a padded length has no two-stage plan.
+ */
+int cvb_converse2d_fwd_train(const void* x, void* out, const void* table, const float* weight, float* r_keep, int B,
+                             int C, int H, int W, int k, int s, int p, int pad_mode, int io_dtype, void* workspace,
+                             size_t workspace_bytes, void* stream);
+size_t cvb_converse2d_train_workspace_bytes(int B, int C, int H, int W, int s, int p);
+
+/*
+ * Gradients of Converse2D (the reference: autograd through torch.fft, converse2d.cpp:223), fp32:
+ *   gx (B,C,H,W) = dL/dx and / or gw (C,k,k), gb (C) = dL/dweight, dL/dbias (both or neither; unwanted ones NULL)
+ *   for g (B,C,sH,sW) = dL/dout.  x (B,C,H,W) is read for gw / gb only, r (from cvb_converse2d_fwd_train) for gw / gb at
+ *   scale >= 2.  `table`: cvb_build_transfer's for the padded size.
+ * The workspace query answers 0 for shapes these kernels do not take (no two-stage plan, scale > 4 with parameter
+ * gradients, rows too long for shared memory).
+ */
+size_t cvb_converse2d_bwd_workspace_bytes(int B, int C, int H, int W, int k, int s, int p, int want_x, int want_params);
+int cvb_converse2d_bwd(const float* x, const float* g, const float* r, const void* table, const float* weight,
+                       const float* bias, float* gx, float* gw, float* gb, int B, int C, int H, int W, int k, int s,
+                       int p, int pad_mode, float eps, void* workspace, size_t workspace_bytes, void* stream);
+
+/*
  * Batch-summed cross spectrum for the parameter gradients.  The reference obtains dL/dweight and
  * dL/dbias from autograd through torch.fft (CompositeImplicitAutograd registration,
  * Converse2D/torch_converse2d/csrc/converse2d.cpp:223); here the batch reduction they need runs in
