@@ -109,11 +109,10 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
 }
 
-// a = hi + lo, hi representable in TF32
+// a = hi + lo, hi = a rounded to the nearest TF32 (half away from zero: the rounding of cvt.rna.tf32, on the integer
+// units, which have four times that conversion's rate)
 __device__ __forceinline__ void split_tf32(float a, float& hi, float& lo) {
-  uint32_t h;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(a));
-  hi = __uint_as_float(h);
+  hi = __uint_as_float((__float_as_uint(a) + 0x1000u) & 0xffffe000u);
   lo = a - hi;
 }
 

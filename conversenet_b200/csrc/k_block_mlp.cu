@@ -246,56 +246,57 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
       }
     } else {
       const float *w2 = wts, *w3 = wts + 2 * kW, *w4 = wts + 4 * kW;
-      const IO* tp = (const IO*)P.t + (size_t)img * Cin * HW + pos;
-      // x1 = x + a1 (W2 . t + b2)
-      mix_stage(lane, v);
-      publish();
-      if (m == 0 && ok) { mix_mma<64>(tmem, w2, 0, false); tc::mma_commit(done); }
-      mix_load<IO>(v, tp + (size_t)64 * HW, HW, valid);
-      commit_wait();
-      mix_stage(lane, v);
-      publish();
-      if (m == 0 && ok) { mix_mma<64>(tmem, w2, 64, true); tc::mma_commit(done); }
       float x1[64];
       mix_load<IO>(x1, (const IO*)P.x + (size_t)img * kBlkC * HW + pos, HW, valid);
-      commit_wait();
-#pragma unroll
-      for (int c0 = 0; c0 < 64; c0 += 32) {
-        float a[32];
-        tc::tmem_ld32(lane + (uint32_t)c0, a);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) x1[c0 + j] = fmaf(vec[kBlkC + c0 + j], a[j] + vec[c0 + j], x1[c0 + j]);
-      }
-      // W3 . LN(x1)
-#pragma unroll
-      for (int c = 0; c < 64; ++c) v[c] = x1[c];
-      mix_norm(v, P.eps);
-      mix_stage(lane, v);
-      publish();
-      if (m == 0 && ok) { mix_mma<128>(tmem, w3, 0, false); tc::mma_commit(done); }
-      commit_wait();
-      // GELU, 64 hidden channels at a time -> W4; the accumulator's first half is free once they have been read
+      // five operands of 64 channels: t (two halves), LN(x1), GELU (two halves).  One copy of the staging code: the whole
+      // kernel has to stay in the instruction cache.
 #pragma unroll 1
-      for (int hf = 0; hf < 2; ++hf) {
+      for (int ph = 0; ph < 5; ++ph) {
+        if (ph == 1) {
+          commit_wait();
+        } else if (ph == 2) {                       // x1 = x + a1 (W2 . t + b2)
+          commit_wait();
 #pragma unroll
-        for (int c0 = 0; c0 < 64; c0 += 32) {
-          float a[32];
-          tc::tmem_ld32(lane + (uint32_t)(64 * hf + c0), a);
+          for (int c0 = 0; c0 < 64; c0 += 32) {
+            float a[32];
+            tc::tmem_ld32(lane + (uint32_t)c0, a);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              x1[c0 + j] = fmaf(vec[kBlkC + c0 + j], a[j] + vec[c0 + j], x1[c0 + j]);
+              v[c0 + j] = x1[c0 + j];
+            }
+          }
+          mix_norm(v, P.eps);
+        } else if (ph >= 3) {                       // GELU of 64 hidden channels
+          const int h0 = 64 * (ph - 3);
+          if (ph == 3) commit_wait();
+#pragma unroll
+          for (int c0 = 0; c0 < 64; c0 += 32) {
+            float a[32];
+            tc::tmem_ld32(lane + (uint32_t)(h0 + c0), a);
 #ifdef __CUDA_ARCH__
 #pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const float2 b = *(const float2*)(vec + 4 * kBlkC + 64 * hf + c0 + j);
-            const float2 o = gelu_erf2(a[j] + b.x, a[j + 1] + b.y);
-            v[c0 + j] = o.x; v[c0 + j + 1] = o.y;
-          }
+            for (int j = 0; j < 32; j += 2) {
+              const float2 b = *(const float2*)(vec + 4 * kBlkC + h0 + c0 + j);
+              const float2 o = gelu_erf2(a[j] + b.x, a[j + 1] + b.y);
+              v[c0 + j] = o.x; v[c0 + j + 1] = o.y;
+            }
 #endif
+          }
+          if (ph == 4) commit_wait();               // the MMAs of the first half have read the operand columns
         }
-        if (hf) commit_wait();                      // the first half's MMAs have read the operand columns
         mix_stage(lane, v);
-        publish();
-        if (m == 0 && ok) { mix_mma<64>(tmem, w4, 64 * hf, hf != 0); tc::mma_commit(done); }
+        publish();                                  // (the accumulator's first 64 columns have been read by ph = 3)
+        if (m == 0 && ok) {
+          if (ph == 2) mix_mma<128>(tmem, w3, 0, false);
+          else mix_mma<64>(tmem, ph < 2 ? w2 : w4, (ph & 1) ? (ph == 1 ? 64 : 0) : (ph == 4 ? 64 : 0), ph == 1 || ph == 4);
+          tc::mma_commit(done);
+        }
+        if (ph == 0 || ph == 4) {                   // the second half of t; the next tile
+          const IO* q = ph == 0 ? (const IO*)P.t + ((size_t)img * Cin + 64) * HW + pos : next;
+          mix_load<IO>(v, q, HW, ph == 0 ? valid : nvalid);
+        }
       }
-      mix_load<IO>(v, next, HW, nvalid);
       commit_wait();
 #pragma unroll
       for (int c0 = 0; c0 < 64; c0 += 32) {
