@@ -148,6 +148,15 @@ constexpr size_t kRpWorkspace = (size_t)64 << 20;
 // planes: 0.21 ms against 0.25).
 static bool dual_tables(int h, int w) { return gemm_axis(h) && gemm_axis(w) && rp::supported(h, w) && !gemm_disabled(); }
 static size_t dual_offset(int C, int h, int w) { return (rp::table_bytes(C, h, w) + 255) / 256 * 256; }
+// Compile-time-plan kernels on pairs of planes that share their taps (k_static.cu), for the sizes that have one: with
+// full pairs they beat the run-time plans (136 x 136, 4 x 128 planes: 53 us against 76; 68 x 68 upsampled by 2, 16 x 64
+// planes: 37 against 42).  An odd batch leaves one pair half empty, which pays from five images on.
+static bool takes_static_pairs(int B, int h, int w) {
+  if (B < 2 || (B % 2 && B < 5) || option(CVB_OPT_RUNTIME_PLAN) || option(CVB_OPT_MULTIPASS)) return false;
+  for (const StaticEntry& e : kStatic)
+    if (e.ry0 * e.ry1 == h && e.rx0 * e.rx1 == w) return rp::supported(h, w);
+  return false;
+}
 static bool takes_tensor_cores(int B, int h, int w) { return B >= 2 && dual_tables(h, w); }
 
 static int check_padding(int H, int W, int p, int pad_mode) {
@@ -289,6 +298,7 @@ size_t cvb_converse2d_workspace_bytes(int B, int C, int H, int W, int s, int p, 
   (void)io_dtype;
   if (B < 1 || C < 1 || H < 1 || W < 1 || p < 0 || s < 1) return 0;
   const int h = H + 2 * p, w = W + 2 * p;
+  if (takes_static_pairs(B, h, w)) return 0;
   if (rp::supported(h, w) && !takes_tensor_cores(B, h, w))
     return rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0, std::max(kRpWorkspace, rp::ws_plane_bytes(h, w, s))).ws_bytes;
   Plan1D py, px;
@@ -310,9 +320,10 @@ int cvb_converse2d_fwd(const void* x, void* out, const void* table, const float*
   if (H + 2 * p < 2 || W + 2 * p < 2) return CVB_ERR_BAD_ARGUMENT;
   if (k > s * (H + 2 * p) || k > s * (W + 2 * p)) return CVB_ERR_KERNEL_TOO_LARGE;
   rp::Params Q;
+  const bool pairs = takes_static_pairs(B, H + 2 * p, W + 2 * p);
   if (takes_tensor_cores(B, H + 2 * p, W + 2 * p)) {
     table = (const char*)table + dual_offset(C, H + 2 * p, W + 2 * p);
-  } else if (rp::fill_params(Q, table, B, C, H, W, k, s, p, pad_mode)) {
+  } else if (!pairs && rp::fill_params(Q, table, B, C, H, W, k, s, p, pad_mode)) {
     Q.x = x; Q.out = out; Q.weight = weight; Q.gelu = fuse_gelu ? 1 : 0;
     const rp::Route r = rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0,
                                   std::max(kRpWorkspace, rp::ws_plane_bytes(H + 2 * p, W + 2 * p, s)));
@@ -323,6 +334,7 @@ int cvb_converse2d_fwd(const void* x, void* out, const void* table, const float*
   P.B = B; P.C = C; P.H = H; P.W = W; P.k = k; P.s = s; P.p = p; P.pad_mode = pad_mode;
   P.fuse_gelu = fuse_gelu ? 1 : 0;
   P.h = H + 2 * p; P.w = W + 2 * p; P.pitch = P.w | 1;
+  P.hh = pairs ? P.h / 2 + 1 : 0;
   P.skip_mask = CVB_TUNE("CVB_SKIP", 0);
   P.status = status_ptr();
   P.ystash = CVB_TUNE("CVB_NO_YSTASH", 0) ? 0 : choose_ystash(P.h, P.w, k, s);

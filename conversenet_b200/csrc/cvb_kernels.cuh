@@ -59,6 +59,8 @@ struct FwdParams {
   int ystash;     // 1: shared memory also keeps the padded input (x0 of the s > 1 epilogue)
   int* status;    // device word set non-zero when a bounded wait gives up; may be null
   Plan1D py, px;
+  int hh = 0;     // 0: `table` is [C][w][h] in digit-reversed order; h / 2 + 1: the table of the real-plane kernels
+                  // (cvb_rp.cuh), [C][w][hh] in natural order and half as large, the other rows being its conjugates
 };
 
 struct PassArgs {
@@ -87,6 +89,9 @@ struct IoArgs {
   int wes, wls;       //   its element stride along the transform axis / stride between lines
   int xoff;           // plane column of line 0 (PASS_DST_GLOBAL of a column strip)
   int yoff;           // ycopy - plane, in float2 units
+  int hh = 0;         // FwdParams::hh, with the column plan that turns a position into a frequency
+  int ry0 = 0, ry1 = 0;
+  float inv_ry1 = 0.f;
 };
 
 // ---------------------------------------------------------------- helpers
@@ -221,6 +226,23 @@ CVB_HD void mid_table_load(const PassArgs& a, const IoArgs& io, int wi, float2 (
     line = wi - t * CNL;
   } else {
     divmod_small(wi, a.nlines, a.inv_nlines, t, line);
+  }
+  if constexpr (CN != 0) {
+    if (io.hh) {
+      // lanes are consecutive positions: RY1 runs of consecutive frequencies, so natural order stays coalesced
+      int k0, j;
+      divmod_small(line, io.ry1, io.inv_ry1, k0, j);
+      const int u = k0 + io.ry0 * j;
+      const bool mir = 2 * u > io.h;
+      const float2* tp = io.tab + (mir ? io.h - u : u);
+#pragma unroll
+      for (int p = 0; p < R; ++p) {
+        const int v = t + (CN / R) * p;
+        const float2 z = tp[(size_t)(mir && v ? CN - v : v) * io.hh];
+        g[p] = make_float2(2.f * z.x, mir ? -2.f * z.y : 2.f * z.y);   // the stored multiplier carries a factor 1 / 2
+      }
+      return;
+    }
   }
   const int tes = a.tab ? a.tab_es : io.h;
   const float2* tp = a.tab ? a.tab + (t * R) * a.tab_es + line * a.tab_ls
@@ -745,7 +767,7 @@ CVB_HD SmemLayout smem_layout(int h, int w, int pitch, int k, int ystash) {
 
 CVB_HD void load_tables(int tid, int nthr, const FwdParams& P, int c, float2* twy, float2* twx, float* wk,
                         int* maps) {
-  const float2* gtw = P.table + (size_t)P.C * P.h * P.w;
+  const float2* gtw = P.table + (size_t)P.C * (P.hh ? P.hh : P.h) * P.w;
   for (int i = tid; i < P.h; i += nthr) {
     twy[i] = gtw[i];
     const int ry = pad_index(i - P.p, P.H, P.pad_mode);
@@ -777,7 +799,12 @@ CVB_HD IoArgs make_io(const FwdParams& P, int c, int pa, int pb) {
   io.ob = pb >= 0 ? (void*)((IO*)P.out + (size_t)pb * out_plane) : nullptr;
   io.H = P.H; io.W = P.W; io.p = P.p; io.pad_mode = P.pad_mode; io.gelu = P.fuse_gelu;
   io.h = P.h; io.w = P.w;
-  io.tab = P.table + (size_t)c * P.h * P.w;
+  io.tab = P.table + (size_t)c * (P.hh ? P.hh : P.h) * P.w;
+  io.hh = P.hh;
+  if (P.hh) {
+    io.ry0 = P.py.radix[0]; io.ry1 = P.py.radix[1];
+    io.inv_ry1 = 1.0f / (float)io.ry1;
+  }
   io.rmap = nullptr;
   io.cmap = nullptr;
   io.ycopy = nullptr;

@@ -67,6 +67,10 @@ inline size_t rows_smem(const Params& P) {
 // kernels built for small radices serve an axis whose two radices are small
 inline bool small_axis(const Axis& a) { return a.mp == 0 && a.r0 <= kSmallRadix && a.r1 <= kSmallRadix; }
 
+// Block size of the strip kernels with up to 128 registers a thread: four blocks of 128 threads on an SM while four
+// tiles fit its memory, else two of 256 (264 x 264: 324 us against 362 with 256; 520 x 520: 1600 against 1451).
+inline int strip_threads(size_t smem) { return 4 * (smem + 1024) <= kSmemLimit + 1024 ? 128 : 256; }
+
 inline size_t plane_smem(int h, int w, int k) {
   const int wc = (w + 1) / 2, hh = h / 2 + 1;
   return ((size_t)h * wc + (size_t)hh * (w | 1) + (k * k + 1) / 2) * sizeof(float2) + (size_t)h * sizeof(int);
@@ -98,14 +102,16 @@ inline size_t ws_plane_bytes(int h, int w, int s) {
   return s > 1 ? spec + ((size_t)h * wp * sizeof(float) + 15) / 16 * 16 : spec;
 }
 
+constexpr size_t kPlaneWide = 150 * 1024;
+
 struct Route {
   bool one_block;       // plane_body, no workspace
   int threads;          //   its block size
   int chunk;            // multi-launch form: planes per chunk
   size_t ws_bytes;
 };
-// One block per plane while three of them share an SM's memory (or the planes are too few and small for launches of
-// strips to pay), else the multi-launch form over chunks of at most ws_cap bytes of workspace.
+// One block per plane while three of them share an SM's memory, or while there are no more planes than SMs and one
+// fits (blocks of up to 512 threads then); else the multi-launch form over chunks of at most ws_cap bytes of workspace.
 inline Route route(int B, int C, int H, int W, int s, int p, int sms, bool force_multi, size_t ws_cap) {
   const int h = H + 2 * p, w = W + 2 * p, planes = B * C;
   Route r;
@@ -113,24 +119,25 @@ inline Route route(int B, int C, int H, int W, int s, int p, int sms, bool force
   int a, b, c, d;
   axis_plan(h, a, b);
   axis_plan(w, c, d);
-  r.one_block = !force_multi && register_radix(a) && register_radix(c) && (sm <= 75 * 1024 && (planes >= sms || sm <= 24 * 1024));
+  r.one_block = !force_multi && register_radix(a) && register_radix(c) && (planes <= sms ? sm <= kPlaneWide : sm <= 75 * 1024);
   r.threads = 256;
   const size_t per = ws_plane_bytes(h, w, s);
   size_t n = ws_cap / per;
   if (n > (size_t)planes) n = planes;
+  if (n > 0) n = (planes + (planes + n - 1) / n - 1) / ((planes + n - 1) / n);   // chunks of equal size
   r.chunk = (int)n;
   r.ws_bytes = r.one_block ? 0 : n * per;
   return r;
 }
 
 // block size of plane_body: the count that wastes the fewest thread slots over its stages
-inline int plane_threads(const Params& P) {
+inline int plane_threads(const Params& P, int most) {
   const Axis &y = P.ay, &x = P.ax;
   const int items[4] = {y.r1 * P.wc, (y.r0 / 2 + 1) * P.wc, x.r1 * P.hh, x.r0 * P.hh};
   const int cost[4] = {y.r0, 2 * y.r1, x.r0, x.r1};
   double best = 1e30;
   int bt = 64;
-  for (int t = 64; t <= 256; t += 32) {
+  for (int t = 64; t <= most; t += 32) {
     double c = 0;
     for (int i = 0; i < 4; ++i) c += (double)((items[i] + t - 1) / t) * t * (cost[i] + 2);
     c *= 1.0 + 8.0 / t;      // fewer warps hide less latency

@@ -7,13 +7,13 @@ namespace cvb {
 namespace rp {
 
 // generated launchers: register plans (k_rp_cols.cu, k_rp_rows.cu), matrix stages by width (k_rp_matrix.cu)
-int launch_cols_fwd_f32(const Params&, bool, int, size_t, cudaStream_t);
-int launch_cols_fwd_bf16(const Params&, bool, int, size_t, cudaStream_t);
-int launch_cols_inv_f32(const Params&, bool, int, size_t, cudaStream_t);
-int launch_cols_inv_bf16(const Params&, bool, int, size_t, cudaStream_t);
+int launch_cols_fwd_f32(const Params&, bool, int, int, size_t, cudaStream_t);
+int launch_cols_fwd_bf16(const Params&, bool, int, int, size_t, cudaStream_t);
+int launch_cols_inv_f32(const Params&, bool, int, int, size_t, cudaStream_t);
+int launch_cols_inv_bf16(const Params&, bool, int, int, size_t, cudaStream_t);
 int launch_epilogue_f32(const Params&, cudaStream_t);
 int launch_epilogue_bf16(const Params&, cudaStream_t);
-int launch_rows(const Params&, bool, int, size_t, cudaStream_t);
+int launch_rows(const Params&, bool, int, int, size_t, cudaStream_t);
 int launch_plane_f32(const Params&, bool, int, size_t, cudaStream_t);
 int launch_plane_bf16(const Params&, bool, int, size_t, cudaStream_t);
 typedef int (*MatrixLauncher)(const Params&, int, int, size_t, cudaStream_t);   // (.., tensor type, grid, ..)
@@ -218,10 +218,10 @@ static int strip(Params& P, int planes, int which, cudaStream_t st) {
   const int gc = (planes * P.wc + kLines - 1) / kLines, gr = (planes * P.hh + kLines - 1) / kLines;
   if (which == 1)
     return P.ax.mp ? matrix_entry(P.ax.mp).rows(P, CVB_F32, gr, rows_smem(P), st)
-                   : launch_rows(P, small_axis(P.ax), gr, rows_smem(P), st);
+                   : launch_rows(P, small_axis(P.ax), strip_threads(rows_smem(P)), gr, rows_smem(P), st);
   if (P.ay.mp)
     return (which == 0 ? matrix_entry(P.ay.mp).cols_fwd : matrix_entry(P.ay.mp).cols_inv)(P, CVB_F32, gc, cols_smem(P), st);
-  return (which == 0 ? launch_cols_fwd_f32 : launch_cols_inv_f32)(P, small_axis(P.ay), gc, cols_smem(P), st);
+  return (which == 0 ? launch_cols_fwd_f32 : launch_cols_inv_f32)(P, small_axis(P.ay), strip_threads(cols_smem(P)), gc, cols_smem(P), st);
 }
 int cols_fwd(Params& P, int planes, cudaStream_t st) { return strip(P, planes, 0, st); }
 int rows(Params& P, int planes, cudaStream_t st) { return strip(P, planes, 1, st); }
@@ -234,14 +234,18 @@ int run(Params& P, const Route& r, int io_dtype, void* workspace, size_t ws_byte
   if (r.one_block) {
     P.plane0 = 0; P.nplane = planes;
     const size_t smem = plane_smem(P.h, P.w, P.k);
-    const bool small = small_axis(P.ay) && small_axis(P.ax);
-    return f32 ? launch_plane_f32(P, small, plane_threads(P), smem, st) : launch_plane_bf16(P, small, plane_threads(P), smem, st);
+    // planes that leave SMs idle take the wide block (up to 512 threads, 128 registers)
+    const bool wide = planes <= sm_count();
+    const bool small = !wide && small_axis(P.ay) && small_axis(P.ax);
+    const int threads = plane_threads(P, wide ? 512 : 256);
+    return f32 ? launch_plane_f32(P, small, threads, smem, st) : launch_plane_bf16(P, small, threads, smem, st);
   }
   if (r.chunk < 1) return CVB_ERR_TOO_LARGE;
   if (!workspace || ws_bytes < r.ws_bytes) return CVB_ERR_WORKSPACE;
   const size_t smem_c = cols_smem(P), smem_r = rows_smem(P);
   if (smem_c > kSmemLimit || smem_r > kSmemLimit) return CVB_ERR_UNSUPPORTED_SIZE;
   const bool sy = small_axis(P.ay), sx = small_axis(P.ax);
+  const int tc = strip_threads(smem_c);
   P.ws = (float2*)workspace;
   for (int p0 = 0; p0 < planes; p0 += r.chunk) {
     P.plane0 = p0;
@@ -251,14 +255,14 @@ int run(Params& P, const Route& r, int io_dtype, void* workspace, size_t ws_byte
                     : (float*)((char*)workspace + (size_t)P.nplane * P.hh * P.wp * sizeof(float2));
     const int gc = (P.nplane * P.wc + kLines - 1) / kLines, gr = (P.nplane * P.hh + kLines - 1) / kLines;
     int rc = P.ay.mp ? matrix_entry(P.ay.mp).cols_fwd(P, io_dtype, gc, smem_c, st)
-             : f32   ? launch_cols_fwd_f32(P, sy, gc, smem_c, st)
-                     : launch_cols_fwd_bf16(P, sy, gc, smem_c, st);
+             : f32   ? launch_cols_fwd_f32(P, sy, tc, gc, smem_c, st)
+                     : launch_cols_fwd_bf16(P, sy, tc, gc, smem_c, st);
     if (rc == CVB_OK)
-      rc = P.ax.mp ? matrix_entry(P.ax.mp).rows(P, io_dtype, gr, smem_r, st) : launch_rows(P, sx, gr, smem_r, st);
+      rc = P.ax.mp ? matrix_entry(P.ax.mp).rows(P, io_dtype, gr, smem_r, st) : launch_rows(P, sx, strip_threads(smem_r), gr, smem_r, st);
     if (rc == CVB_OK)
       rc = P.ay.mp ? matrix_entry(P.ay.mp).cols_inv(P, io_dtype, gc, smem_c, st)
-           : f32   ? launch_cols_inv_f32(P, sy, gc, smem_c, st)
-                   : launch_cols_inv_bf16(P, sy, gc, smem_c, st);
+           : f32   ? launch_cols_inv_f32(P, sy, tc, gc, smem_c, st)
+                   : launch_cols_inv_bf16(P, sy, tc, gc, smem_c, st);
     if (rc == CVB_OK && P.s > 1) rc = f32 ? launch_epilogue_f32(P, st) : launch_epilogue_bf16(P, st);
     if (rc != CVB_OK) return rc;
   }

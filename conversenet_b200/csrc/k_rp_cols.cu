@@ -22,12 +22,12 @@ __global__ void __launch_bounds__(128, 6) cols_inv_small_kernel(const __grid_con
   cols_inv_body<IO, kSmallRadix, 0>(P, smem);
 }
 template <typename IO>
-__global__ void __launch_bounds__(128, 4) cols_fwd_kernel(const __grid_constant__ Params P) {
+__global__ void __launch_bounds__(256, 2) cols_fwd_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
   cols_fwd_body<IO, kAnyRadix, 0>(P, smem);
 }
 template <typename IO>
-__global__ void __launch_bounds__(128, 4) cols_inv_kernel(const __grid_constant__ Params P) {
+__global__ void __launch_bounds__(256, 2) cols_inv_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
   cols_inv_body<IO, kAnyRadix, 0>(P, smem);
 }
@@ -43,13 +43,13 @@ static int go(K kernel, const Params& P, int grid, int threads, size_t smem, cud
   CVB_CUDA(cudaGetLastError());
   return CVB_OK;
 }
-int CVB_CAT(launch_cols_fwd, CVB_IO_NAME)(const Params& P, bool small, int grid, size_t smem, cudaStream_t st) {
+int CVB_CAT(launch_cols_fwd, CVB_IO_NAME)(const Params& P, bool small, int threads, int grid, size_t smem, cudaStream_t st) {
   if (small) return go(cols_fwd_small_kernel<CVB_IO>, P, grid, 128, smem, st);
-  return go(cols_fwd_kernel<CVB_IO>, P, grid, 128, smem, st);
+  return go(cols_fwd_kernel<CVB_IO>, P, grid, threads, smem, st);
 }
-int CVB_CAT(launch_cols_inv, CVB_IO_NAME)(const Params& P, bool small, int grid, size_t smem, cudaStream_t st) {
+int CVB_CAT(launch_cols_inv, CVB_IO_NAME)(const Params& P, bool small, int threads, int grid, size_t smem, cudaStream_t st) {
   if (small) return go(cols_inv_small_kernel<CVB_IO>, P, grid, 128, smem, st);
-  return go(cols_inv_kernel<CVB_IO>, P, grid, 128, smem, st);
+  return go(cols_inv_kernel<CVB_IO>, P, grid, threads, smem, st);
 }
 int CVB_CAT(launch_epilogue, CVB_IO_NAME)(const Params& P, cudaStream_t st) {
   epilogue_kernel<CVB_IO><<<dim3((P.H + kEpiRows - 1) / kEpiRows, P.nplane), 128, 0, st>>>(P);

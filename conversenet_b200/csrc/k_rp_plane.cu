@@ -16,7 +16,7 @@ __global__ void __launch_bounds__(256, 3) plane_small_kernel(const __grid_consta
   plane_body<IO, kSmallRadix>(P, smem);
 }
 template <typename IO>
-__global__ void __launch_bounds__(256, 2) plane_kernel(const __grid_constant__ Params P) {
+__global__ void __launch_bounds__(512, 1) plane_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
   plane_body<IO, kAnyRadix>(P, smem);
 }

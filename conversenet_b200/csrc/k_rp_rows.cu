@@ -10,7 +10,7 @@ __global__ void __launch_bounds__(128, 6) rows_small_kernel(const __grid_constan
   extern __shared__ float2 smem[];
   rows_body<kSmallRadix, 0>(P, smem);
 }
-__global__ void __launch_bounds__(128, 4) rows_kernel(const __grid_constant__ Params P) {
+__global__ void __launch_bounds__(256, 2) rows_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
   rows_body<kAnyRadix, 0>(P, smem);
 }
@@ -22,9 +22,9 @@ static int go(K kernel, const Params& P, int grid, int threads, size_t smem, cud
   CVB_CUDA(cudaGetLastError());
   return CVB_OK;
 }
-int launch_rows(const Params& P, bool small, int grid, size_t smem, cudaStream_t st) {
+int launch_rows(const Params& P, bool small, int threads, int grid, size_t smem, cudaStream_t st) {
   if (small) return go(rows_small_kernel, P, grid, 128, smem, st);
-  return go(rows_kernel, P, grid, 128, smem, st);
+  return go(rows_kernel, P, grid, threads, smem, st);
 }
 
 }  // namespace rp
