@@ -234,12 +234,15 @@ CVB_HD void mid_table_load(const PassArgs& a, const IoArgs& io, int wi, float2 (
       divmod_small(line, io.ry1, io.inv_ry1, k0, j);
       const int u = k0 + io.ry0 * j;
       const bool mir = 2 * u > io.h;
-      const float2* tp = io.tab + (mir ? io.h - u : u);
+      const int step = (CN / R) * io.hh;
+      const float2* tp = io.tab + (mir ? (CN - t) * io.hh + (io.h - u) : t * io.hh + u);
+      const float sy = mir ? -2.f : 2.f;       // the stored multiplier carries a factor 1 / 2
 #pragma unroll
       for (int p = 0; p < R; ++p) {
-        const int v = t + (CN / R) * p;
-        const float2 z = tp[(size_t)(mir && v ? CN - v : v) * io.hh];
-        g[p] = make_float2(2.f * z.x, mir ? -2.f * z.y : 2.f * z.y);   // the stored multiplier carries a factor 1 / 2
+        // frequency t + (CN / R) p, mirrored CN - that; frequency 0 is its own mirror
+        const float2* q = mir ? tp - p * step : tp + p * step;
+        const float2 z = *(p == 0 && mir && t == 0 ? q - CN * io.hh : q);
+        g[p] = make_float2(2.f * z.x, sy * z.y);
       }
       return;
     }

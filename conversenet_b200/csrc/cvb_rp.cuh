@@ -71,6 +71,15 @@ __host__ __device__ constexpr int matrix_width(int r0) {
   return -1;
 }
 
+// The smallest R0 / 2 that width M serves
+__host__ __device__ constexpr int matrix_least(int m) {
+  int least = 1;
+#define CVB_RP_X(M) if (M < m) least = M + 1;
+  CVB_RP_EACH_WIDTH(CVB_RP_X)
+#undef CVB_RP_X
+  return least;
+}
+
 // Builds of every kernel: both radices up to kSmallRadix (80 registers a thread); up to kAnyRadix; a matrix stage of a
 // given width with R1 up to kMatrixR1.
 constexpr int kSmallRadix = 20, kAnyRadix = 32, kMatrixR1 = 16;
@@ -123,44 +132,6 @@ __device__ __forceinline__ void twiddle(float (&re)[R], float (&im)[R], const fl
 // vector in registers and runs over the k: two FMAs per (k, q), the cosines four at a time from shared memory.  Element
 // k then holds a_k and element R - k holds b_k (matrix_value puts them together), so that the two threads of a vector
 // never have to meet.  FMA-bound by construction: about R FMAs per point.
-// The MP values of one thread, neighbours packed: one fma .f32x2 multiplies two q by their two cosines, which a 16-byte
-// read of the matrix row delivers as register pairs.  (The packed form has the same FMA rate as the scalar one and half
-// its issue slots.)
-template <int MP>
-struct MatrixRow {
-#ifdef __CUDA_ARCH__
-  p2 xs[MP / 2], ys[MP / 2];
-  __device__ __forceinline__ void set(int i, float2 a, float2 b) {
-    xs[i] = p2_pack(a.x, b.x);
-    ys[i] = p2_pack(a.y, b.y);
-  }
-  __device__ __forceinline__ float2 dot(const float* row) const {
-    const ulonglong2* c = (const ulonglong2*)row;
-    p2 r0 = 0, r1 = 0, i0 = 0, i1 = 0;
-#pragma unroll
-    for (int q = 0; q < MP / 4; ++q) {
-      const ulonglong2 v = c[q];
-      r0 = p2_fma(v.x, xs[2 * q], r0);
-      i0 = p2_fma(v.x, ys[2 * q], i0);
-      r1 = p2_fma(v.y, xs[2 * q + 1], r1);
-      i1 = p2_fma(v.y, ys[2 * q + 1], i1);
-    }
-    float a, b, d, e;
-    p2_unpack(p2_add(r0, r1), a, b);
-    p2_unpack(p2_add(i0, i1), d, e);
-    return make_float2(a + b, d + e);
-  }
-#else
-  float2 v[MP];
-  void set(int i, float2 a, float2 b) { v[2 * i] = a; v[2 * i + 1] = b; }
-  float2 dot(const float* row) const {
-    float2 s = make_float2(0.f, 0.f);
-    for (int q = 0; q < MP; ++q) { s.x = fmaf(row[q], v[q].x, s.x); s.y = fmaf(row[q], v[q].y, s.y); }
-    return s;
-  }
-#endif
-};
-
 template <int MP, class Base>
 __device__ __forceinline__ void matrix_stage(int R, int nvec, int stride, const float* mats, Base base) {
   const int tid = threadIdx.x, half = blockDim.x >> 1;
@@ -174,28 +145,47 @@ __device__ __forceinline__ void matrix_stage(int R, int nvec, int stride, const 
   for (int v0 = 0; v0 < nvec; v0 += nvr) {
     const bool act = v0 + vl < nvec && kg < ng;
     float2* x = base(act ? v0 + vl : 0);
-    MatrixRow<MP> p;
+    float2 p[MP];
     const float2 x0 = side ? make_float2(0.f, 0.f) : x[0];
-    auto element = [&](int q) {
-      float2 r = make_float2(0.f, 0.f);
-      if (q <= QH) {
-        const float2 u = x[q * stride], w = x[(R - q) * stride];
-        r = side ? make_float2(u.x - w.x, u.y - w.y) : make_float2(u.x + w.x, u.y + w.y);
-      } else if (q == KH) {                        // even R: the middle element, cosines only
-        if (!side) r = x[q * stride];
-      }
-      return r;
-    };
+    const float sg = side ? -1.f : 1.f;
+    const float2 *up = x + stride, *dn = x + (R - 1) * stride;
 #pragma unroll
-    for (int q = 0; q < MP; q += 2) p.set(q / 2, element(q + 1), element(q + 2));
+    for (int q = 1; q <= MP; ++q, up += stride, dn -= stride) {
+      if (q < matrix_least(MP) || q <= QH) {
+        const float2 u = *up, w = *dn;
+        p[q - 1] = make_float2(fmaf(sg, w.x, u.x), fmaf(sg, w.y, u.y));
+      } else {
+        p[q - 1] = make_float2(0.f, 0.f);
+        if (q == KH && !side) p[q - 1] = *up;      // even R: the middle element, cosines only
+      }
+    }
     __syncthreads();
     if (act) {
       const int k0 = kg * kper > side ? kg * kper : side, k1 = (kg + 1) * kper < KH + 1 ? (kg + 1) * kper : KH + 1;
       const int kend = side && k1 > QH + 1 ? QH + 1 : k1;
-#pragma unroll 2
-      for (int k = k0; k < kend; ++k) {
-        const float2 s = p.dot(mat + k * MP);
-        x[(side ? R - k : k) * stride] = make_float2(x0.x + s.x, x0.y + s.y);
+      // two rows at a time: four independent sums, and one row's cosines arrive while the other's are used
+      float2* o = x + (side ? R - k0 : k0) * stride;
+      const int ostep = side ? -stride : stride;
+#pragma unroll 1
+      for (int k = k0; k < kend; k += 2, o += 2 * ostep) {
+        const bool two = k + 1 < kend;
+        const float4* c4 = (const float4*)(mat + k * MP);
+        const float4* d4 = two ? c4 + MP / 4 : c4;
+        float r0 = x0.x, i0 = x0.y, r1 = x0.x, i1 = x0.y;
+#pragma unroll
+        for (int q = 0; q < MP; q += 4) {
+          const float4 c = c4[q >> 2], d = d4[q >> 2];
+          r0 = fmaf(c.x, p[q].x, r0);     i0 = fmaf(c.x, p[q].y, i0);
+          r1 = fmaf(d.x, p[q].x, r1);     i1 = fmaf(d.x, p[q].y, i1);
+          r0 = fmaf(c.y, p[q + 1].x, r0); i0 = fmaf(c.y, p[q + 1].y, i0);
+          r1 = fmaf(d.y, p[q + 1].x, r1); i1 = fmaf(d.y, p[q + 1].y, i1);
+          r0 = fmaf(c.z, p[q + 2].x, r0); i0 = fmaf(c.z, p[q + 2].y, i0);
+          r1 = fmaf(d.z, p[q + 2].x, r1); i1 = fmaf(d.z, p[q + 2].y, i1);
+          r0 = fmaf(c.w, p[q + 3].x, r0); i0 = fmaf(c.w, p[q + 3].y, i0);
+          r1 = fmaf(d.w, p[q + 3].x, r1); i1 = fmaf(d.w, p[q + 3].y, i1);
+        }
+        o[0] = make_float2(r0, i0);
+        if (two) o[ostep] = make_float2(r1, i1);
       }
     }
   }

@@ -6,7 +6,7 @@
 
 #define CVB_CAT_(a, b) a##_##b
 #define CVB_CAT(a, b) CVB_CAT_(a, b)
-#define CVB_RP_BLOCKS (CVB_MP <= 36 ? 5 : CVB_MP <= 44 ? 4 : 3)
+#define CVB_RP_BLOCKS (CVB_MP <= 24 ? 5 : CVB_MP <= 44 ? 4 : 3)
 
 namespace cvb {
 namespace rp {
