@@ -5,14 +5,16 @@
 // residuals and the operands of all three contractions of POST stay inside one thread and its lane of tensor memory,
 // so the 128-channel hidden tensor and x1 never leave the SM.
 //
-// A block is two groups of 128 threads; each works on a 128-pixel tile of its own, so that one group's arithmetic
-// covers the other's MMAs.  Per contraction: the thread splits its values into TF32 hi + lo and writes them to its
-// lane of the group's operand columns (tcgen05.st, 64 channels at a time); after a barrier of the group one thread
-// issues hi hi + hi lo + lo hi with the weights from shared memory and commits to the group's mbarrier; every thread
-// then reads its own lane of the accumulator.  TMEM columns of group g at 256 g: accumulator [0,128), operand hi
-// [128,192), lo [192,256).  The weights, split and in operand layout, were packed once (block_pack_kernel) and arrive
-// by one bulk copy.  Pixels are addressed one by one (channel rows of any alignment, any image size, fp32 or bf16);
-// the values of the next tile are requested while the current one computes.
+// A block is two groups of 256 threads; each works on a 128-pixel tile of its own, so that one group's arithmetic
+// covers the other's MMAs.  Two threads share a pixel, 32 channels each (sixteen warps on an SM: with one thread per
+// pixel and eight warps POST took 239 us instead of N us); they meet only in LayerNorm, whose halves' means and
+// squared deviations go through shared memory.  Per contraction: the thread splits its values into TF32 hi + lo and
+// writes them to its lane of the group's operand columns (tcgen05.st, 64 channels at a time); after a barrier of the
+// group one thread issues hi hi + hi lo + lo hi with the weights from shared memory and commits to the group's mbarrier;
+// every thread then reads its half of its lane of the accumulator.  TMEM columns of group g at 256 g: accumulator
+// [0,128), operand hi [128,192), lo [192,256).  The weights, split and in operand layout, were packed once
+// (block_pack_kernel) and arrive by one bulk copy.  Pixels are addressed one by one (channel rows of any alignment, any
+// image size, fp32 or bf16); the values of the next tile are requested while the current one computes.
 //
 // What bounds it: bytes (PRE 3 C, POST 4 C channel planes), the MMAs (24 of 128x128x8 a tile for PRE, 72 of which 48 of
 // 128x64x8 for POST) and instruction issue (about 2400 and 4000 a warp and tile) are within 1.5 x of one another.
@@ -90,7 +92,7 @@ struct MixParams {
   int* status;
 };
 
-constexpr int kMixThreads = 256;
+constexpr int kMixThreads = 512;
 constexpr uint32_t kOpHi = 128, kOpLo = 192;
 
 // sixteen consecutive columns of this thread's TMEM lane
@@ -104,10 +106,10 @@ __device__ __forceinline__ void mix_st16(uint32_t taddr, const float (&v)[16]) {
       "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15]))
       : "memory");
 }
-// 64 channel values -> operand columns
-__device__ __forceinline__ void mix_stage(uint32_t lane, const float (&v)[64]) {
+// this thread's 32 of 64 channel values -> operand columns (lane: its half's first column of the accumulator)
+__device__ __forceinline__ void mix_stage(uint32_t lane, const float (&v)[32]) {
 #pragma unroll
-  for (int c0 = 0; c0 < 64; c0 += 16) {
+  for (int c0 = 0; c0 < 32; c0 += 16) {
     float hi[16], lo[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) tc::split_tf32(v[c0 + e], hi[e], lo[e]);
@@ -130,31 +132,36 @@ __device__ __forceinline__ void mix_mma(uint32_t tmem, const float* b_hi, int k0
     tc::mma_tf32_ta(tmem, tmem + kOpLo + ks * 8, bh, idesc, 1u);
   }
 }
-// centre and scale 64 values (the affine part is in the weights)
-__device__ __forceinline__ void mix_norm(float (&v)[64], float eps) {
-  float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-#pragma unroll
-  for (int c = 0; c < 64; c += 4) { s0 += v[c]; s1 += v[c + 1]; s2 += v[c + 2]; s3 += v[c + 3]; }
-  const float mean = ((s0 + s1) + (s2 + s3)) * (1.0f / 64);
-  s0 = s1 = s2 = s3 = 0.f;
-#pragma unroll
-  for (int c = 0; c < 64; c += 4) {
-    v[c] -= mean; v[c + 1] -= mean; v[c + 2] -= mean; v[c + 3] -= mean;
-    s0 = fmaf(v[c], v[c], s0); s1 = fmaf(v[c + 1], v[c + 1], s1);
-    s2 = fmaf(v[c + 2], v[c + 2], s2); s3 = fmaf(v[c + 3], v[c + 3], s3);
-  }
-  const float rstd = 1.0f / sqrtf(((s0 + s1) + (s2 + s3)) * (1.0f / 64) + eps);
-#pragma unroll
-  for (int c = 0; c < 64; ++c) v[c] *= rstd;
-}
 template <typename IO>
-__device__ __forceinline__ void mix_load(float (&v)[64], const IO* p, int HW, bool valid) {
+__device__ __forceinline__ void mix_load(float (&v)[32], const IO* p, int HW, bool valid) {
 #pragma unroll
-  for (int c = 0; c < 64; ++c) v[c] = valid ? ld_io<IO>(p, (size_t)c * HW) : 0.f;
+  for (int c = 0; c < 32; ++c) v[c] = valid ? ld_io<IO>(p, (size_t)c * HW) : 0.f;
 }
 __device__ __forceinline__ void mix_bar(int g) {
-  if (g == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
-  else asm volatile("bar.sync 2, 128;" ::: "memory");
+  if (g == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
+  else asm volatile("bar.sync 2, 256;" ::: "memory");
+}
+// centre and scale a pixel's 64 values, 32 of them here (the affine part is in the weights).  `mine`, `other`: this and
+// the partner thread's cell for (mean, sum of squared deviations) of a half; the two combine to the whole's.
+__device__ __forceinline__ void mix_norm(float (&v)[32], float eps, float2* mine, const float2* other, int g) {
+  float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+  for (int c = 0; c < 32; c += 4) { s0 += v[c]; s1 += v[c + 1]; s2 += v[c + 2]; s3 += v[c + 3]; }
+  const float m0 = ((s0 + s1) + (s2 + s3)) * (1.0f / 32);
+  s0 = s1 = s2 = s3 = 0.f;
+#pragma unroll
+  for (int c = 0; c < 32; c += 4) {
+    const float a = v[c] - m0, b = v[c + 1] - m0, d = v[c + 2] - m0, e = v[c + 3] - m0;
+    s0 = fmaf(a, a, s0); s1 = fmaf(b, b, s1); s2 = fmaf(d, d, s2); s3 = fmaf(e, e, s3);
+  }
+  const float q0 = (s0 + s1) + (s2 + s3);
+  *mine = make_float2(m0, q0);
+  mix_bar(g);
+  const float2 o = *other;
+  const float d = m0 - o.x, mean = 0.5f * (m0 + o.x);
+  const float rstd = 1.0f / sqrtf(fmaf(16.f * d, d, q0 + o.y) * (1.0f / 64) + eps);
+#pragma unroll
+  for (int c = 0; c < 32; ++c) v[c] = (v[c] - mean) * rstd;
 }
 
 template <bool POST, typename IO>
@@ -165,7 +172,11 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
   const float* vec = wts + (POST ? 6 : 2) * kW;    // PRE: b1.  POST: b2, a1, b4, a2, b3
   uint64_t* bars = (uint64_t*)(msm + kFloats);      // MMA of group 0, 1; weights
   uint32_t* holder = (uint32_t*)(bars + 3);
-  const int tid = threadIdx.x, warp = tid >> 5, g = tid >> 7, m = tid & 127;
+  float2* halves = (float2*)(holder + 2);           // [group][half][pixel]
+  const int tid = threadIdx.x, warp = tid >> 5, g = tid >> 8, m = tid & 127, hf = (tid >> 7) & 1;
+  const bool lead = (tid & 255) == 0;
+  float2* mine = halves + (g * 2 + hf) * 128 + m;
+  const float2* other = halves + (g * 2 + (hf ^ 1)) * 128 + m;
   if (tid == 0) {
     for (int i = 0; i < 3; ++i) mbar_init(&bars[i], 1);
     mbar_fence_init();
@@ -177,7 +188,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = *holder + 256u * (uint32_t)g;
-  const uint32_t lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  const uint32_t lane = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 32u * (uint32_t)hf;   // 32 columns a thread
   uint64_t* done = &bars[g];
   uint32_t uses = 0;                                // commits of this group so far
   bool ok = true;
@@ -207,10 +218,11 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
   bool valid = false;
   long long img = 0;
   int pos = 0;
-  float v[64];
+  const size_t half_off = (size_t)(32 * hf) * HW;
+  float v[32];
   if (tile < ntiles) {
     place(tile, valid, img, pos);
-    mix_load<IO>(v, (const IO*)(POST ? P.t : P.x) + (size_t)img * Cin * HW + pos, HW, valid);
+    mix_load<IO>(v, (const IO*)(POST ? P.t : P.x) + (size_t)img * Cin * HW + pos + half_off, HW, valid);
   }
   if (ok) ok = mbar_wait_bounded(&bars[2], 0, kWaitLimit);   // weights
   for (; tile < ntiles; tile += step) {
@@ -219,24 +231,24 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
     long long nimg = 0;
     int npos = 0;
     if (ntile < ntiles) place(ntile, nvalid, nimg, npos);
-    const IO* next = (const IO*)(POST ? P.t : P.x) + (size_t)nimg * Cin * HW + npos;
-    IO* op = (IO*)P.out + (size_t)img * Cout * HW + pos;
+    const IO* next = (const IO*)(POST ? P.t : P.x) + (size_t)nimg * Cin * HW + npos + half_off;
+    IO* op = (IO*)P.out + (size_t)img * Cout * HW + pos + (POST ? half_off : 2 * half_off);
     if constexpr (!POST) {
-      mix_norm(v, P.eps);
+      mix_norm(v, P.eps, mine, other, g);
       mix_stage(lane, v);
       publish();
-      if (m == 0 && ok) { mix_mma<128>(tmem, wts, 0, false); tc::mma_commit(done); }
+      if (lead && ok) { mix_mma<128>(tmem, wts, 0, false); tc::mma_commit(done); }
       mix_load<IO>(v, next, HW, nvalid);
       commit_wait();
 #pragma unroll 1
-      for (int c0 = 0; c0 < 128; c0 += 32) {
+      for (int c0 = 0; c0 < 64; c0 += 32) {         // 64 of the 128 output channels
         float a[32];
-        tc::tmem_ld32(lane + (uint32_t)c0, a);
+        tc::tmem_ld32(lane + (uint32_t)(32 * hf + c0), a);
         if (valid && ok) {
 #ifdef __CUDA_ARCH__
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
-            const float2 b = *(const float2*)(vec + c0 + j);
+            const float2 b = *(const float2*)(vec + 64 * hf + c0 + j);
             const float2 o = gelu_erf2(a[j] + b.x, a[j + 1] + b.y);
             st_io<IO>(op, (size_t)(c0 + j) * HW, o.x);
             st_io<IO>(op, (size_t)(c0 + j + 1) * HW, o.y);
@@ -246,8 +258,9 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
       }
     } else {
       const float *w2 = wts, *w3 = wts + 2 * kW, *w4 = wts + 4 * kW;
-      float x1[64];
-      mix_load<IO>(x1, (const IO*)P.x + (size_t)img * kBlkC * HW + pos, HW, valid);
+      const float* vh = vec + 32 * hf;              // this thread's channels of b2, a1, b4, a2
+      float x1[32];
+      mix_load<IO>(x1, (const IO*)P.x + (size_t)img * kBlkC * HW + pos + half_off, HW, valid);
       // five operands of 64 channels: t (two halves), LN(x1), GELU (two halves).  One copy of the staging code: the whole
       // kernel has to stay in the instruction cache.
 #pragma unroll 1
@@ -256,58 +269,48 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
           commit_wait();
         } else if (ph == 2) {                       // x1 = x + a1 (W2 . t + b2)
           commit_wait();
+          float a[32];
+          tc::tmem_ld32(lane, a);
 #pragma unroll
-          for (int c0 = 0; c0 < 64; c0 += 32) {
-            float a[32];
-            tc::tmem_ld32(lane + (uint32_t)c0, a);
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              x1[c0 + j] = fmaf(vec[kBlkC + c0 + j], a[j] + vec[c0 + j], x1[c0 + j]);
-              v[c0 + j] = x1[c0 + j];
-            }
+          for (int j = 0; j < 32; ++j) {
+            x1[j] = fmaf(vh[kBlkC + j], a[j] + vh[j], x1[j]);
+            v[j] = x1[j];
           }
-          mix_norm(v, P.eps);
-        } else if (ph >= 3) {                       // GELU of 64 hidden channels
+          mix_norm(v, P.eps, mine, other, g);
+        } else if (ph >= 3) {                       // GELU of 32 of 64 hidden channels
           const int h0 = 64 * (ph - 3);
           if (ph == 3) commit_wait();
-#pragma unroll
-          for (int c0 = 0; c0 < 64; c0 += 32) {
-            float a[32];
-            tc::tmem_ld32(lane + (uint32_t)(h0 + c0), a);
+          float a[32];
+          tc::tmem_ld32(lane + (uint32_t)h0, a);
 #ifdef __CUDA_ARCH__
 #pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              const float2 b = *(const float2*)(vec + 4 * kBlkC + h0 + c0 + j);
-              const float2 o = gelu_erf2(a[j] + b.x, a[j + 1] + b.y);
-              v[c0 + j] = o.x; v[c0 + j + 1] = o.y;
-            }
-#endif
+          for (int j = 0; j < 32; j += 2) {
+            const float2 b = *(const float2*)(vh + 4 * kBlkC + h0 + j);
+            const float2 o = gelu_erf2(a[j] + b.x, a[j + 1] + b.y);
+            v[j] = o.x; v[j + 1] = o.y;
           }
+#endif
           if (ph == 4) commit_wait();               // the MMAs of the first half have read the operand columns
         }
         mix_stage(lane, v);
         publish();                                  // (the accumulator's first 64 columns have been read by ph = 3)
-        if (m == 0 && ok) {
+        if (lead && ok) {
           if (ph == 2) mix_mma<128>(tmem, w3, 0, false);
-          else mix_mma<64>(tmem, ph < 2 ? w2 : w4, (ph & 1) ? (ph == 1 ? 64 : 0) : (ph == 4 ? 64 : 0), ph == 1 || ph == 4);
+          else mix_mma<64>(tmem, ph < 2 ? w2 : w4, ph == 1 || ph == 4 ? 64 : 0, ph == 1 || ph == 4);
           tc::mma_commit(done);
         }
         if (ph == 0 || ph == 4) {                   // the second half of t; the next tile
-          const IO* q = ph == 0 ? (const IO*)P.t + ((size_t)img * Cin + 64) * HW + pos : next;
+          const IO* q = ph == 0 ? (const IO*)P.t + ((size_t)img * Cin + 64) * HW + pos + half_off : next;
           mix_load<IO>(v, q, HW, ph == 0 ? valid : nvalid);
         }
       }
       commit_wait();
+      float a[32];
+      tc::tmem_ld32(lane, a);
+      if (valid && ok) {
 #pragma unroll
-      for (int c0 = 0; c0 < 64; c0 += 32) {
-        float a[32];
-        tc::tmem_ld32(lane + (uint32_t)c0, a);
-        if (valid && ok) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            st_io<IO>(op, (size_t)(c0 + j) * HW,
-                      fmaf(vec[3 * kBlkC + c0 + j], a[j] + vec[2 * kBlkC + c0 + j], x1[c0 + j]));
-        }
+        for (int j = 0; j < 32; ++j)
+          st_io<IO>(op, (size_t)j * HW, fmaf(vh[3 * kBlkC + j], a[j] + vh[2 * kBlkC + j], x1[j]));
       }
     }
     valid = nvalid; img = nimg; pos = npos;
@@ -320,7 +323,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
 
 template <bool POST, typename IO>
 static int launch_mix(const MixParams& P, int sms, cudaStream_t st) {
-  const size_t smem = (size_t)(POST ? kPostFloats : kPreFloats) * sizeof(float) + 3 * sizeof(uint64_t) + 16;
+  const size_t smem = (size_t)(POST ? kPostFloats : kPreFloats) * sizeof(float) + 3 * sizeof(uint64_t) + 8 + 512 * sizeof(float2) + 16;
   CVB_CUDA(cudaFuncSetAttribute(block_mix_kernel<POST, IO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const long long ntiles = (P.npix + 127) / 128;
   const int grid = (int)(ntiles < sms ? ntiles : sms);     // one block per SM; tiles go round the blocks first
