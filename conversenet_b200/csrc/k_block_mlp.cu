@@ -7,7 +7,7 @@
 //
 // A block is two groups of 256 threads; each works on a 128-pixel tile of its own, so that one group's arithmetic
 // covers the other's MMAs.  Two threads share a pixel, 32 channels each (sixteen warps on an SM: with one thread per
-// pixel and eight warps POST took 239 us instead of N us); they meet only in LayerNorm, whose halves' means and
+// pixel and eight warps 8 x 256 x 256 pixels of POST took 239 us); they meet only in LayerNorm, whose halves' means and
 // squared deviations go through shared memory.  Per contraction: the thread splits its values into TF32 hi + lo and
 // writes them to its lane of the group's operand columns (tcgen05.st, 64 channels at a time); after a barrier of the
 // group one thread issues hi hi + hi lo + lo hi with the weights from shared memory and commits to the group's mbarrier;
@@ -21,21 +21,14 @@
 // Every wait is bounded; after a time-out a thread stops working but keeps meeting the group's barriers.
 #include "../../include/converse_b200.h"
 #include "cvb_internal.h"
-#include "cvb_block.cuh"
-#include "cvb_tc.cuh"
+#include "cvb_mix.cuh"
 
 namespace cvb {
 
 // ---- packed weights: PRE | POST, each a multiple of 16 bytes
-constexpr int kW = kBlkC * kBlkM;                               // floats of one weight matrix
 constexpr int kPreFloats = 2 * kW + kBlkM;                      // W1 hi, lo; b1
 constexpr int kPostFloats = 6 * kW + 4 * kBlkC + kBlkM;         // W2, W3, W4 hi, lo; b2, a1, b4, a2; b3
 size_t block_pack_bytes() { return (size_t)(kPreFloats + kPostFloats) * sizeof(float); }
-
-// float index of element (n, k) of an operand with N rows (K-major core matrices, no swizzle)
-__host__ __device__ constexpr int pack_index(int N, int n, int k) {
-  return (n >> 3) * 32 + (n & 7) * 4 + (k & 3) + ((k >> 2) & 1) * (N / 8) * 32 + (k >> 3) * (N / 8) * 64;
-}
 
 struct PackParams {
   const float *ln1_w, *ln1_b, *w1, *b1, *w2, *b2, *a1, *ln2_w, *ln2_b, *w3, *b3, *w4, *b4, *a2;
@@ -90,81 +83,12 @@ struct MixParams {
   int HW;
   long long npix;
   int* status;
+  float *z, *x1;        // TRAIN: (B,128,HW), (B,64,HW)
 };
 
-constexpr int kMixThreads = 512;
-constexpr uint32_t kOpHi = 128, kOpLo = 192;
-
-// sixteen consecutive columns of this thread's TMEM lane
-__device__ __forceinline__ void mix_st16(uint32_t taddr, const float (&v)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-      "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
-      "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
-      "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
-      "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15]))
-      : "memory");
-}
-// this thread's 32 of 64 channel values -> operand columns (lane: its half's first column of the accumulator)
-__device__ __forceinline__ void mix_stage(uint32_t lane, const float (&v)[32]) {
-#pragma unroll
-  for (int c0 = 0; c0 < 32; c0 += 16) {
-    float hi[16], lo[16];
-#pragma unroll
-    for (int e = 0; e < 16; ++e) tc::split_tf32(v[c0 + e], hi[e], lo[e]);
-    mix_st16(lane + kOpHi + (uint32_t)c0, hi);
-    mix_st16(lane + kOpLo + (uint32_t)c0, lo);
-  }
-  tc::tmem_wait_st();
-}
-// D (+)= A[64 channels in the operand columns] . B, B = N rows, K columns k0 .. k0 + 63 of a packed matrix
-template <int N>
-__device__ __forceinline__ void mix_mma(uint32_t tmem, const float* b_hi, int k0, bool accumulate) {
-  constexpr uint32_t idesc = tc::idesc_tf32(128, N, false, false);
-  constexpr int LBO = (N / 8) * 128, KSTEP = 2 * LBO;
-#pragma unroll
-  for (int ks = 0; ks < 8; ++ks) {
-    const uint64_t bh = tc::smem_desc((const char*)b_hi + (k0 / 8 + ks) * KSTEP, LBO, 128);
-    const uint64_t bl = tc::smem_desc((const char*)(b_hi + kW) + (k0 / 8 + ks) * KSTEP, LBO, 128);
-    tc::mma_tf32_ta(tmem, tmem + kOpHi + ks * 8, bh, idesc, (accumulate || ks > 0) ? 1u : 0u);
-    tc::mma_tf32_ta(tmem, tmem + kOpHi + ks * 8, bl, idesc, 1u);
-    tc::mma_tf32_ta(tmem, tmem + kOpLo + ks * 8, bh, idesc, 1u);
-  }
-}
-template <typename IO>
-__device__ __forceinline__ void mix_load(float (&v)[32], const IO* p, int HW, bool valid) {
-#pragma unroll
-  for (int c = 0; c < 32; ++c) v[c] = valid ? ld_io<IO>(p, (size_t)c * HW) : 0.f;
-}
-__device__ __forceinline__ void mix_bar(int g) {
-  if (g == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
-  else asm volatile("bar.sync 2, 256;" ::: "memory");
-}
-// centre and scale a pixel's 64 values, 32 of them here (the affine part is in the weights).  `mine`, `other`: this and
-// the partner thread's cell for (mean, sum of squared deviations) of a half; the two combine to the whole's.
-__device__ __forceinline__ void mix_norm(float (&v)[32], float eps, float2* mine, const float2* other, int g) {
-  float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-#pragma unroll
-  for (int c = 0; c < 32; c += 4) { s0 += v[c]; s1 += v[c + 1]; s2 += v[c + 2]; s3 += v[c + 3]; }
-  const float m0 = ((s0 + s1) + (s2 + s3)) * (1.0f / 32);
-  s0 = s1 = s2 = s3 = 0.f;
-#pragma unroll
-  for (int c = 0; c < 32; c += 4) {
-    const float a = v[c] - m0, b = v[c + 1] - m0, d = v[c + 2] - m0, e = v[c + 3] - m0;
-    s0 = fmaf(a, a, s0); s1 = fmaf(b, b, s1); s2 = fmaf(d, d, s2); s3 = fmaf(e, e, s3);
-  }
-  const float q0 = (s0 + s1) + (s2 + s3);
-  *mine = make_float2(m0, q0);
-  mix_bar(g);
-  const float2 o = *other;
-  const float d = m0 - o.x, mean = 0.5f * (m0 + o.x);
-  const float rstd = 1.0f / sqrtf(fmaf(16.f * d, d, q0 + o.y) * (1.0f / 64) + eps);
-#pragma unroll
-  for (int c = 0; c < 32; ++c) v[c] = (v[c] - mean) * rstd;
-}
-
-template <bool POST, typename IO>
+// TRAIN (fp32): also keeps what the gradients need -- PRE the hidden layer before its GELU (z), POST x1 and the hidden
+// layer before its GELU -- and POST takes t before ITS GELU.
+template <bool POST, typename IO, bool TRAIN>
 __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_constant__ MixParams P) {
   extern __shared__ __align__(128) float msm[];
   constexpr int kFloats = POST ? kPostFloats : kPreFloats;
@@ -249,7 +173,13 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
             const float2 b = *(const float2*)(vec + 64 * hf + c0 + j);
-            const float2 o = gelu_erf2(a[j] + b.x, a[j + 1] + b.y);
+            const float za = a[j] + b.x, zb = a[j + 1] + b.y;
+            const float2 o = gelu_erf2(za, zb);
+            if (TRAIN) {
+              float* zp = P.z + (op - (IO*)P.out);
+              zp[(size_t)(c0 + j) * HW] = za;
+              zp[(size_t)(c0 + j + 1) * HW] = zb;
+            }
             st_io<IO>(op, (size_t)(c0 + j) * HW, o.x);
             st_io<IO>(op, (size_t)(c0 + j + 1) * HW, o.y);
           }
@@ -275,6 +205,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
           for (int j = 0; j < 32; ++j) {
             x1[j] = fmaf(vh[kBlkC + j], a[j] + vh[j], x1[j]);
             v[j] = x1[j];
+            if (TRAIN && valid) P.x1[(op - (IO*)P.out) + (size_t)j * HW] = x1[j];
           }
           mix_norm(v, P.eps, mine, other, g);
         } else if (ph >= 3) {                       // GELU of 32 of 64 hidden channels
@@ -286,12 +217,27 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
             const float2 b = *(const float2*)(vh + 4 * kBlkC + h0 + j);
-            const float2 o = gelu_erf2(a[j] + b.x, a[j + 1] + b.y);
+            const float za = a[j] + b.x, zb = a[j + 1] + b.y;
+            const float2 o = gelu_erf2(za, zb);
+            if (TRAIN && valid) {
+              float* zp = P.z + ((size_t)img * kBlkM + h0) * HW + pos + half_off;
+              zp[(size_t)j * HW] = za;
+              zp[(size_t)(j + 1) * HW] = zb;
+            }
             v[j] = o.x; v[j + 1] = o.y;
           }
 #endif
           if (ph == 4) commit_wait();               // the MMAs of the first half have read the operand columns
         }
+#ifdef __CUDA_ARCH__
+        if (TRAIN && ph < 2) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            const float2 o = gelu_erf2(v[j], v[j + 1]);
+            v[j] = o.x; v[j + 1] = o.y;
+          }
+        }
+#endif
         mix_stage(lane, v);
         publish();                                  // (the accumulator's first 64 columns have been read by ph = 3)
         if (lead && ok) {
@@ -321,13 +267,13 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
   if (warp == 0) tc::tmem_dealloc(*holder, 512);
 }
 
-template <bool POST, typename IO>
+template <bool POST, typename IO, bool TRAIN = false>
 static int launch_mix(const MixParams& P, int sms, cudaStream_t st) {
   const size_t smem = (size_t)(POST ? kPostFloats : kPreFloats) * sizeof(float) + 3 * sizeof(uint64_t) + 8 + 512 * sizeof(float2) + 16;
-  CVB_CUDA(cudaFuncSetAttribute(block_mix_kernel<POST, IO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CVB_CUDA(cudaFuncSetAttribute(block_mix_kernel<POST, IO, TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const long long ntiles = (P.npix + 127) / 128;
   const int grid = (int)(ntiles < sms ? ntiles : sms);     // one block per SM; tiles go round the blocks first
-  block_mix_kernel<POST, IO><<<grid, kMixThreads, smem, st>>>(P);
+  block_mix_kernel<POST, IO, TRAIN><<<grid, kMixThreads, smem, st>>>(P);
   CVB_CUDA(cudaGetLastError());
   return CVB_OK;
 }
@@ -336,9 +282,17 @@ int launch_block_mix(bool post, const void* x, const void* t, void* out, const v
                      int io_dtype, int sms, int* status, cudaStream_t st) {
   MixParams P;
   P.x = x; P.t = t; P.out = out; P.pack = (const float*)pack; P.eps = eps;
-  P.HW = HW; P.npix = (long long)B * HW; P.status = status;
+  P.HW = HW; P.npix = (long long)B * HW; P.status = status; P.z = nullptr; P.x1 = nullptr;
   if (post) return io_dtype == CVB_F32 ? launch_mix<true, float>(P, sms, st) : launch_mix<true, __nv_bfloat16>(P, sms, st);
   return io_dtype == CVB_F32 ? launch_mix<false, float>(P, sms, st) : launch_mix<false, __nv_bfloat16>(P, sms, st);
+}
+
+int launch_block_mix_train(bool post, const float* x, const float* t, float* out, float* z, float* x1, const void* pack,
+                           float eps, int B, int HW, int sms, int* status, cudaStream_t st) {
+  MixParams P;
+  P.x = x; P.t = t; P.out = out; P.pack = (const float*)pack; P.eps = eps;
+  P.HW = HW; P.npix = (long long)B * HW; P.status = status; P.z = z; P.x1 = x1;
+  return post ? launch_mix<true, float, true>(P, sms, st) : launch_mix<false, float, true>(P, sms, st);
 }
 
 }  // namespace cvb
