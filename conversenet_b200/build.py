@@ -8,6 +8,7 @@ next to this file.  Nothing here needs a GPU.
 """
 import hashlib
 import os
+import re
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
@@ -105,12 +106,21 @@ def _units():
     return units
 
 
-def _stamp(defs):
+def _sources(path, seen):
+    """`path` and everything it includes by a quoted name, recursively."""
+    path = os.path.normpath(path)
+    if path in seen or not os.path.exists(path):
+        return seen
+    seen.add(path)
+    for name in re.findall(r'^\s*#\s*include\s+"([^"]+)"', open(path).read(), re.M):
+        _sources(os.path.join(os.path.dirname(path), name), seen)
+    return seen
+
+
+def _stamp(src, defs):
     h = hashlib.sha1()
-    for name in sorted(os.listdir(CSRC)):
-        if name.endswith((".cu", ".cuh", ".h", ".inc")):
-            h.update(open(os.path.join(CSRC, name), "rb").read())
-    h.update(open(os.path.join(HERE, "..", "include", "converse_b200.h"), "rb").read())
+    for path in sorted(_sources(os.path.join(CSRC, src), set())):
+        h.update(open(path, "rb").read())
     h.update(" ".join(NVCC_FLAGS + defs).encode())
     return h.hexdigest()
 
@@ -151,7 +161,7 @@ def build(force=False, ptxas_v=False, verbose=True):
     for name, src, defs in units:
         obj = os.path.join(OBJ, name + ".o")
         stamp_path = obj + ".stamp"
-        stamp = _stamp(defs)
+        stamp = _stamp(src, defs)
         fresh = (not force and os.path.exists(obj) and os.path.exists(stamp_path)
                  and open(stamp_path).read() == stamp)
         if not fresh:
