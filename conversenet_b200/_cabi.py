@@ -44,6 +44,11 @@ SIGNATURES = {
     "cvb_converse2d_train_workspace_bytes": (_c.c_size_t, [_c.c_int] * 6),
     "cvb_converse2d_bwd_workspace_bytes": (_c.c_size_t, [_c.c_int] * 9),
     "cvb_converse2d_bwd": (_c.c_int, [_c.c_void_p] * 9 + [_c.c_int] * 8 + [_c.c_float, _c.c_void_p, _c.c_size_t, _c.c_void_p]),
+    "cvb_block_pre_train": (_c.c_int, [_c.c_void_p] * 4 + [_c.c_float, _c.c_int, _c.c_int, _c.c_void_p]),
+    "cvb_block_post_train": (_c.c_int, [_c.c_void_p] * 6 + [_c.c_float, _c.c_int, _c.c_int, _c.c_void_p]),
+    "cvb_block_grad_floats": (_c.c_size_t, []),
+    "cvb_block_bwd_workspace_bytes": (_c.c_size_t, [_c.c_int] * 5),
+    "cvb_block_bwd": (_c.c_int, [_c.c_void_p]),
     "cvb_plan_radices": (_c.c_int, [_c.c_int, _c.POINTER(_c.c_int), _c.c_int]),
     "cvb_fits_shared": (_c.c_int, [_c.c_int, _c.c_int]),
     "cvb_cross_spectrum": (_c.c_int, [_c.c_void_p] * 4 + [_c.c_int] * 7 + [_c.c_void_p]),

@@ -220,3 +220,28 @@ class Converse2DFunction(torch.autograd.Function):
         gw = gw.to(weight.dtype) if gw is not None and ctx.needs_input_grad[1] else None
         gb = gb.to(bias.dtype) if gb is not None and ctx.needs_input_grad[2] else None
         return gx, gw, gb, None, None, None, None, None, None, None
+
+
+class ConverseBlockFunction(torch.autograd.Function):
+    """A whole ConverseBlock (64 channels, scale 1, fp32) under autograd: the fused forward keeping the layers before the
+    GELUs, the gradients in one native call (`csrc/k_block_train.cu`).  `params`: the fourteen parameters around Converse2D
+    in the order of `functional.block_parameters`, None for absent alphas."""
+
+    @staticmethod
+    def forward(ctx, kept, x, conv_w, conv_b, table, cfg, *params):
+        ctx.save_for_backward(x, conv_w, conv_b, *params)
+        ctx.kept = kept[1:]
+        ctx.table = table
+        ctx.cfg = cfg
+        return kept[0]
+
+    @staticmethod
+    def backward(ctx, g):
+        x, conv_w, conv_b, *params = ctx.saved_tensors
+        eps1, eps2, conv_eps, p, mode = ctx.cfg
+        grads = _cabi.host().block_backward(x, *ctx.kept, g, ctx.table, conv_w, conv_b, tuple(params), eps1, eps2, conv_eps,
+                                            p, mode)
+        need = ctx.needs_input_grad
+        gx, gcw, gcb, *gp = grads
+        return (None, gx if need[1] else None, gcw if need[2] else None, gcb if need[3] else None, None, None,
+                *[q if n else None for q, n in zip(gp, need[6:])])

@@ -520,6 +520,47 @@ int cvb_converse2d_bwd(const float* x, const float* g, const float* r, const voi
                      workspace_bytes, sm_count(), (cudaStream_t)stream);
 }
 
+int cvb_block_pre_train(const float* x, float* out, float* z1, const void* pack, float ln_eps, int B, int HW,
+                        void* stream) {
+  if (!x || !out || !z1 || !pack || ((size_t)pack) % 16 || B < 1 || HW < 1) return CVB_ERR_BAD_ARGUMENT;
+  return launch_block_mix_train(false, x, nullptr, out, z1, nullptr, pack, ln_eps, B, HW, sm_count(), status_ptr(),
+                                (cudaStream_t)stream);
+}
+
+int cvb_block_post_train(const float* u, const float* x, float* out, float* x1, float* z3, const void* pack, float ln_eps,
+                         int B, int HW, void* stream) {
+  if (!u || !x || !out || !x1 || !z3 || !pack || ((size_t)pack) % 16 || B < 1 || HW < 1) return CVB_ERR_BAD_ARGUMENT;
+  return launch_block_mix_train(true, x, u, out, z3, x1, pack, ln_eps, B, HW, sm_count(), status_ptr(),
+                                (cudaStream_t)stream);
+}
+
+size_t cvb_block_grad_floats(void) { return block_grad_floats(); }
+
+size_t cvb_block_bwd_workspace_bytes(int B, int H, int W, int k, int p) {
+  const size_t conv = cvb_converse2d_bwd_workspace_bytes(B, kBlkM, H, W, k, 1, p, 1, 1);
+  return conv ? block_grad_workspace(B, H * W, conv, sm_count()) : 0;
+}
+
+int cvb_block_bwd(const cvb_block_bwd_args* args) {
+  if (!args) return CVB_ERR_BAD_ARGUMENT;
+  const cvb_block_bwd_args& A = *args;
+  const void* need[] = {A.x, A.t1, A.z1, A.u, A.x1, A.z3, A.g, A.table, A.conv_w, A.conv_b, A.ln1_w, A.ln1_b, A.w1, A.b1,
+                        A.w2, A.b2, A.ln2_w, A.ln2_b, A.w3, A.b3, A.w4, A.b4, A.gx, A.gconv_w, A.gconv_b, A.gparams};
+  for (const void* q : need)
+    if (!q) return CVB_ERR_BAD_ARGUMENT;
+  if (A.B < 1 || A.H < 1 || A.W < 1) return CVB_ERR_BAD_ARGUMENT;
+  const int rc = check_padding(A.H, A.W, A.p, A.pad_mode);
+  if (rc != CVB_OK) return rc;
+  const size_t conv = cvb_converse2d_bwd_workspace_bytes(A.B, kBlkM, A.H, A.W, A.k, 1, A.p, 1, 1);
+  if (!conv) return CVB_ERR_UNSUPPORTED_SIZE;
+  return run_block_grad(A, conv, sm_count(), status_ptr(), (cudaStream_t)A.stream,
+                        [](const cvb_block_bwd_args& a, const float* gu, float* gt, void* ws, size_t bytes) {
+                          return rp::run_bwd(a.t1, gu, nullptr, a.table, a.conv_w, a.conv_b, gt, a.gconv_w, a.gconv_b, a.B,
+                                             kBlkM, a.H, a.W, a.k, 1, a.p, a.pad_mode, a.conv_eps, ws, bytes, sm_count(),
+                                             (cudaStream_t)a.stream);
+                        });
+}
+
 size_t cvb_block_pack_bytes(void) { return block_pack_bytes(); }
 
 int cvb_block_pack(const float* ln1_w, const float* ln1_b, const float* w1, const float* b1, const float* w2,

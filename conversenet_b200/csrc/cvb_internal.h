@@ -79,6 +79,14 @@ int launch_block_pack(const float* ln1_w, const float* ln1_b, const float* w1, c
 int launch_block_mix(bool post, const void* x, const void* t, void* out, const void* pack, float eps, int B, int HW,
                      int io_dtype, int sms, int* status, cudaStream_t st);
 
+int launch_block_mix_train(bool post, const float* x, const float* t, float* out, float* z, float* x1, const void* pack,
+                           float eps, int B, int HW, int sms, int* status, cudaStream_t st);
+// gradients of the block (k_block_train.cu); `conv`: the gradient of its Converse2D
+size_t block_grad_floats();
+size_t block_grad_workspace(int B, int HW, size_t conv_ws, int sms);
+int run_block_grad(const cvb_block_bwd_args& A, size_t conv_ws, int sms, int* status, cudaStream_t st,
+                   int (*conv)(const cvb_block_bwd_args&, const float* gu, float* gt, void* ws, size_t bytes));
+
 // Multi-pass kernels with a compile-time axis plan (k_strip2.cu, one object per registry line).
 struct StripParams;
 typedef int (*Strip2Launcher)(const StripParams& SP, int io_dtype, cudaStream_t st);

@@ -35,6 +35,11 @@ struct Api {
   decltype(&cvb_converse2d_fwd_train) fwd_train = nullptr;
   decltype(&cvb_converse2d_bwd_workspace_bytes) bwd_workspace_bytes = nullptr;
   decltype(&cvb_converse2d_bwd) bwd = nullptr;
+  decltype(&cvb_block_pre_train) block_pre_train = nullptr;
+  decltype(&cvb_block_post_train) block_post_train = nullptr;
+  decltype(&cvb_block_grad_floats) block_grad_floats = nullptr;
+  decltype(&cvb_block_bwd_workspace_bytes) block_bwd_workspace = nullptr;
+  decltype(&cvb_block_bwd) block_bwd = nullptr;
 } api;
 
 struct Failed : std::runtime_error { using std::runtime_error::runtime_error; };
@@ -290,17 +295,105 @@ PyObject* py_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+// block_train(x, table, weight_f32, pack, kernel_size, padding, padding_mode, eps1, eps2) -> (out, t1, z1, u, x1, z3), the
+// last five for block_backward; None when the gradient kernels do not take the shape
+PyObject* py_block_train(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    want(n, 9);
+    const at::Tensor x = f32(cuda_tensor(a[0], "x").detach());
+    const c10::cuda::CUDAGuard dev(x.device());
+    const at::Tensor &table = tensor(a[1], "table"), &wf = tensor(a[2], "weight"), &pack = tensor(a[3], "pack");
+    const int B = (int)x.size(0), C = (int)x.size(1), H = (int)x.size(2), W = (int)x.size(3);
+    const int k = (int)integer(a[4]), p = (int)integer(a[5]), mode = pad_mode(a[6]);
+    if (!api.block_bwd_workspace(B, H, W, k, p)) Py_RETURN_NONE;
+    const auto opt = x.options().requires_grad(false);
+    void* st = stream(x);
+    at::Tensor t1 = at::empty({B, 2 * C, H, W}, opt), z1 = at::empty({B, 2 * C, H, W}, opt), u = at::empty({B, 2 * C, H, W}, opt);
+    at::Tensor x1 = at::empty({B, C, H, W}, opt), z3 = at::empty({B, 2 * C, H, W}, opt), out = at::empty({B, C, H, W}, opt);
+    check(api.block_pre_train((const float*)x.data_ptr(), (float*)t1.data_ptr(), (float*)z1.data_ptr(), pack.data_ptr(),
+                              (float)real(a[7]), B, H * W, st), "cvb_block_pre_train");
+    forward(t1, table, wf, k, 1, p, mode, 0, u);
+    check(api.block_post_train((const float*)u.data_ptr(), (const float*)x.data_ptr(), (float*)out.data_ptr(),
+                               (float*)x1.data_ptr(), (float*)z3.data_ptr(), pack.data_ptr(), (float)real(a[8]), B, H * W, st),
+          "cvb_block_post_train");
+    return Py_BuildValue("(NNNNNN)", THPVariable_Wrap(out), THPVariable_Wrap(t1), THPVariable_Wrap(z1), THPVariable_Wrap(u),
+                         THPVariable_Wrap(x1), THPVariable_Wrap(z3));
+  });
+}
+
+// block_backward(x, t1, z1, u, x1, z3, g, table, conv_weight, conv_bias, params (14 tensors or None), eps1, eps2, conv_eps,
+// padding, padding_mode) -> [gx, gconv_w, gconv_b, the 14 parameter gradients (None for an absent alpha)]
+PyObject* py_block_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    want(n, 16);
+    at::Tensor in[7];
+    const float* ip[7];
+    for (int i = 0; i < 7; ++i) {
+      in[i] = f32(cuda_tensor(a[i], "tensor").detach());
+      ip[i] = (const float*)in[i].data_ptr();
+    }
+    const c10::cuda::CUDAGuard dev(in[0].device());
+    at::Tensor par[14];
+    const float* pp[14];
+    for (int i = 0; i < 14; ++i) {
+      PyObject* o = PyTuple_GetItem(a[10], i);
+      if (!o) throw std::invalid_argument("params");
+      pp[i] = nullptr;
+      if (o == Py_None) continue;
+      par[i] = f32(tensor(o, "parameter").detach());
+      pp[i] = (const float*)par[i].data_ptr();
+    }
+    const at::Tensor &cw = tensor(a[8], "weight"), &cb = tensor(a[9], "bias");
+    const at::Tensor cwf = f32(cw.detach()), cbf = f32(cb.detach());
+    const auto opt = in[0].options().requires_grad(false);
+    cvb_block_bwd_args A;
+    std::memset(&A, 0, sizeof(A));
+    A.x = ip[0]; A.t1 = ip[1]; A.z1 = ip[2]; A.u = ip[3]; A.x1 = ip[4]; A.z3 = ip[5]; A.g = ip[6];
+    A.table = tensor(a[7], "table").data_ptr();
+    A.conv_w = (const float*)cwf.data_ptr(); A.conv_b = (const float*)cbf.data_ptr();
+    A.ln1_w = pp[0]; A.ln1_b = pp[1]; A.w1 = pp[2]; A.b1 = pp[3]; A.w2 = pp[4]; A.b2 = pp[5]; A.alpha1 = pp[6];
+    A.ln2_w = pp[7]; A.ln2_b = pp[8]; A.w3 = pp[9]; A.b3 = pp[10]; A.w4 = pp[11]; A.b4 = pp[12]; A.alpha2 = pp[13];
+    A.eps1 = (float)real(a[11]); A.eps2 = (float)real(a[12]); A.conv_eps = (float)real(a[13]);
+    A.B = (int)in[0].size(0); A.H = (int)in[0].size(2); A.W = (int)in[0].size(3);
+    A.k = (int)cw.size(-1); A.p = (int)integer(a[14]); A.pad_mode = pad_mode(a[15]);
+    at::Tensor gx = at::empty(in[0].sizes(), opt), gcw = at::empty(cw.sizes(), opt), gcb = at::empty(cb.sizes(), opt);
+    at::Tensor gp = at::empty({(int64_t)api.block_grad_floats()}, opt);
+    const size_t ws = api.block_bwd_workspace(A.B, A.H, A.W, A.k, A.p);
+    at::Tensor work = bytes_like(in[0], ws ? ws : 1);
+    A.gx = (float*)gx.data_ptr(); A.gconv_w = (float*)gcw.data_ptr(); A.gconv_b = (float*)gcb.data_ptr();
+    A.gparams = (float*)gp.data_ptr();
+    A.workspace = work.data_ptr(); A.workspace_bytes = ws; A.stream = stream(in[0]);
+    check(api.block_bwd(&A), "cvb_block_bwd");
+    PyObject* out = PyList_New(17);
+    PyList_SET_ITEM(out, 0, THPVariable_Wrap(gx));
+    PyList_SET_ITEM(out, 1, THPVariable_Wrap(gcw));
+    PyList_SET_ITEM(out, 2, THPVariable_Wrap(gcb));
+    static const int64_t size[7] = {64, 64, 8192, 128, 8192, 64, 64};
+    int64_t off = 0;
+    for (int i = 0; i < 14; ++i) {
+      PyObject* o = Py_None;
+      if (pp[i]) o = THPVariable_Wrap(gp.narrow(0, off, size[i % 7]).view(par[i].sizes()));
+      else Py_INCREF(o);
+      PyList_SET_ITEM(out, 3 + i, o);
+      off += size[i % 7];
+    }
+    return out;
+  });
+}
+
 // init(address of each C ABI function in the order of `names`)
 PyObject* py_init(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    want(n, 15);
-    void* p[15];
-    for (int i = 0; i < 15; ++i) p[i] = PyLong_AsVoidPtr(a[i]);
+    want(n, 20);
+    void* p[20];
+    for (int i = 0; i < 20; ++i) p[i] = PyLong_AsVoidPtr(a[i]);
     int i = 0;
     auto set = [&](auto& f) { f = (std::decay_t<decltype(f)>)p[i++]; };
     set(api.strerror_); set(api.last_cuda_error); set(api.transfer_bytes); set(api.build_transfer); set(api.build_x0_table);
     set(api.workspace_bytes); set(api.converse2d_fwd); set(api.block_pack_bytes); set(api.block_pack); set(api.block_pre);
     set(api.block_post); set(api.train_workspace_bytes); set(api.fwd_train); set(api.bwd_workspace_bytes); set(api.bwd);
+    set(api.block_pre_train); set(api.block_post_train); set(api.block_grad_floats); set(api.block_bwd_workspace);
+    set(api.block_bwd);
     Py_RETURN_NONE;
   });
 }
@@ -313,6 +406,8 @@ PyMethodDef methods[] = {
     {"block_pack", (PyCFunction)(void (*)(void))py_block_pack, METH_FASTCALL, nullptr},
     {"train_forward", (PyCFunction)(void (*)(void))py_train_forward, METH_FASTCALL, nullptr},
     {"backward", (PyCFunction)(void (*)(void))py_backward, METH_FASTCALL, nullptr},
+    {"block_train", (PyCFunction)(void (*)(void))py_block_train, METH_FASTCALL, nullptr},
+    {"block_backward", (PyCFunction)(void (*)(void))py_block_backward, METH_FASTCALL, nullptr},
     {"block", (PyCFunction)(void (*)(void))py_block, METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
@@ -322,11 +417,13 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, null
 PyMODINIT_FUNC PyInit__host(void) {
   PyObject* m = PyModule_Create(&module);
   if (!m) return nullptr;
-  PyObject* names = Py_BuildValue("(sssssssssssssss)", "cvb_strerror", "cvb_last_cuda_error", "cvb_transfer_bytes",
+  PyObject* names = Py_BuildValue("(ssssssssssssssssssss)", "cvb_strerror", "cvb_last_cuda_error", "cvb_transfer_bytes",
                                   "cvb_build_transfer", "cvb_build_x0_table", "cvb_converse2d_workspace_bytes",
                                   "cvb_converse2d_fwd", "cvb_block_pack_bytes", "cvb_block_pack", "cvb_block_pre_fwd",
                                   "cvb_block_post_fwd", "cvb_converse2d_train_workspace_bytes",
-                                  "cvb_converse2d_fwd_train", "cvb_converse2d_bwd_workspace_bytes", "cvb_converse2d_bwd");
+                                  "cvb_converse2d_fwd_train", "cvb_converse2d_bwd_workspace_bytes", "cvb_converse2d_bwd",
+                                  "cvb_block_pre_train", "cvb_block_post_train", "cvb_block_grad_floats",
+                                  "cvb_block_bwd_workspace_bytes", "cvb_block_bwd");
   if (!names || PyModule_AddObject(m, "names", names) < 0) return nullptr;
   return m;
 }

@@ -193,6 +193,37 @@ class ConverseBlock(nn.Module):
             conv.fuse_gelu = False
         return c[5](t)
 
+    def _forward_trainable(self, x, alpha1=None, alpha2=None):
+        """The block under autograd through the native kernels; None where they do not apply (other widths, dtypes or
+        scales, hooked children, autocast, planes without a gradient kernel)."""
+        c1, c2 = self.conv1._modules, self.conv2._modules
+        conv = c1["3"]
+        if not (BLOCK_FUSION and torch.is_grad_enabled() and x.is_cuda and x.dim() == 4 and x.size(1) == 64 and
+                x.dtype == torch.float32 and c1["1"].out_channels == 128 and c1["5"].out_channels == 64 and
+                conv.scale == 1 and not torch.is_autocast_enabled()):
+            return None
+        params = CF.block_parameters(c1["0"], c1["1"], c1["5"], alpha1, c2["0"], c2["1"], c2["3"], alpha2)
+        given = [q for i, q in enumerate(params) if i not in (6, 13)] + [conv.weight, conv.bias]
+        if any(q is None or q.dtype != torch.float32 or not q.is_cuda for q in given):
+            return None
+        for m in (self.conv1, self.conv2, *c1.values(), *c2.values()):
+            if m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks:
+                return None
+        conv._check_backend()
+        host = _cabi.host()
+        state = host.state(*params)
+        if state != self._pack_state:
+            self._pack, self._pack_state = host.block_pack(*params), state
+        p, eps1, eps2 = conv.padding, c1["0"].eps, c2["0"].eps
+        table, wf = conv._table_for(x.shape[2] + 2 * p, x.shape[3] + 2 * p, x.device)
+        x = x.contiguous()
+        kept = host.block_train(x, table, wf, self._pack, conv.kernel_size, p, conv.padding_mode, eps1, eps2)
+        if kept is None:
+            return None
+        from .autograd import ConverseBlockFunction
+        return ConverseBlockFunction.apply(kept, x, conv.weight, conv.bias, table,
+                                           (eps1, eps2, conv.eps, p, conv.padding_mode), *params)
+
     def _fusable(self, x):
         if torch.is_grad_enabled() and (x.requires_grad or any(q.requires_grad for q in self.parameters())):
             return False  # the fused block kernels are forward-only
@@ -232,6 +263,9 @@ class ConverseBlock(nn.Module):
     def forward(self, x):
         if self._fusable(x):
             return self._forward_fused(x)
+        out = self._forward_trainable(x)
+        if out is not None:
+            return out
         with _exact_fp32():
             x = self._branch1(x) + x
             x = self.conv2(x) + x
@@ -250,6 +284,9 @@ class ConverseBlockAlphaVariant(ConverseBlock):
     def forward(self, x):
         if self._fusable(x):
             return self._forward_fused(x, self.alpha1, self.alpha2)
+        out = self._forward_trainable(x, self.alpha1, self.alpha2)
+        if out is not None:
+            return out
         with _exact_fp32():
             x = self.alpha1 * self._branch1(x) + x
             x = self.alpha2 * self.conv2(x) + x

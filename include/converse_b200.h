@@ -183,6 +183,34 @@ int cvb_block_post_fwd(const void* t, const void* x, void* out, const void* pack
                        int io_dtype, void* stream);
 
 /*
+ * Training forms of the two (fp32) and the gradients of the whole block, scale 1:
+ *   cvb_block_pre_train   out = GELU(z1), z1 (B,2C,HW) kept
+ *   cvb_block_post_train  takes u, the Converse2D output BEFORE its GELU; keeps x1 (B,C,HW) and z3 (B,2C,HW), the hidden
+ *                         layer of conv2 before its GELU
+ *   cvb_block_bwd         dL/dx and all parameter gradients from g = dL/dout (the reference: autograd).  gparams receives,
+ *                         one after the other: ln1_w ln1_b w1 b1 w2 b2 alpha1, ln2_w ln2_b w3 b3 w4 b4 alpha2 (alphas
+ *                         also when there are none).  Workspace query 0: shape not taken.
+ */
+int cvb_block_pre_train(const float* x, float* out, float* z1, const void* pack, float ln_eps, int B, int HW, void* stream);
+int cvb_block_post_train(const float* u, const float* x, float* out, float* x1, float* z3, const void* pack, float ln_eps,
+                         int B, int HW, void* stream);
+typedef struct {
+  const float *x, *t1, *z1, *u, *x1, *z3, *g;            /* t1 = GELU(z1), the input of Converse2D */
+  const void* table;                                     /* Converse2D's, for the padded size */
+  const float *conv_w, *conv_b;                          /* (2C,k,k), (2C) */
+  const float *ln1_w, *ln1_b, *w1, *b1, *w2, *b2, *alpha1, *ln2_w, *ln2_b, *w3, *b3, *w4, *b4, *alpha2;
+  float eps1, eps2, conv_eps;
+  int B, H, W, k, p, pad_mode;
+  float *gx, *gconv_w, *gconv_b, *gparams;
+  void* workspace;
+  size_t workspace_bytes;
+  void* stream;
+} cvb_block_bwd_args;
+size_t cvb_block_grad_floats(void);                      /* floats at gparams */
+size_t cvb_block_bwd_workspace_bytes(int B, int H, int W, int k, int p);
+int cvb_block_bwd(const cvb_block_bwd_args* args);
+
+/*
  * Converse2D forward for callers that cannot allocate device memory.
  *
  * Same arguments, result and error codes as cvb_converse2d_fwd, minus the workspace:
