@@ -33,7 +33,8 @@ __global__ void __launch_bounds__(256, 2) cols_inv_kernel(const __grid_constant_
 }
 template <typename IO>
 __global__ void __launch_bounds__(128) epilogue_kernel(const __grid_constant__ Params P) {
-  epilogue_body<IO>(P);
+  __shared__ __align__(16) unsigned char band[kEpiBand];
+  epilogue_body<IO>(P, band);
 }
 
 template <typename K>
