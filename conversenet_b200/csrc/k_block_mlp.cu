@@ -157,6 +157,20 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
     if (ntile < ntiles) place(ntile, nvalid, nimg, npos);
     const IO* next = (const IO*)(POST ? P.t : P.x) + (size_t)nimg * Cin * HW + npos + half_off;
     IO* op = (IO*)P.out + (size_t)img * Cout * HW + pos + (POST ? half_off : 2 * half_off);
+    {
+      // the tile after: rows of its first pixel in this warp
+      const long long npix0 = ntile * 128 + (m & ~31);
+      if (npix0 < P.npix) {
+        const long long i0 = npix0 / HW;
+        const size_t p0 = (size_t)(npix0 - i0 * HW) + half_off;
+        const IO* q = (const IO*)(POST ? P.t : P.x) + (size_t)i0 * Cin * HW + p0;
+        mix_prefetch<IO>(q, HW);
+        if (POST) {
+          mix_prefetch<IO>(q + (size_t)64 * HW, HW);
+          mix_prefetch<IO>((const IO*)P.x + (size_t)i0 * kBlkC * HW + p0, HW);
+        }
+      }
+    }
     if constexpr (!POST) {
       mix_norm(v, P.eps, mine, other, g);
       mix_stage(lane, v);
