@@ -142,11 +142,15 @@ static bool needs_strip(int h, int w, int k, bool big) {
 // chunk workspace of the multi-launch real-plane kernels
 constexpr size_t kRpWorkspace = (size_t)64 << 20;
 
-// Planes whose two lengths are in the tensor-core registry keep the tables of both kernel families: the tensor-core
-// kernels pack two planes that share their taps (two images of a batch) into one complex plane and win when there are
-// two (268 x 268, 8 x 128 planes: 1.01 ms against 1.55), the real-plane kernels when every pair would hold one (1 x 128
-// planes: 0.21 ms against 0.25).
-static bool dual_tables(int h, int w) { return gemm_axis(h) && gemm_axis(w) && rp::supported(h, w) && !gemm_disabled(); }
+// Planes whose two lengths have a compile-time multi-pass plan that beats the run-time ones on FULL pairs of planes (two
+// images of a batch share their taps and travel as one complex plane) keep the tables of both kernel families:
+//   tensor-core plans   268 x 268, 8 x 128 planes: 1.01 ms against 1.26;  1 x 128 planes: 0.25 against 0.16
+//   264 and 520         4 x 128 planes of 264 x 264: 280 us against 309, of 520 x 520: 1256 against 1463
+// At scale >= 2 the run-time kernels' epilogue wins (260 x 260 by 2, 4 x 64 planes: 270 us against 596).
+static bool strip_axis(int n) { return n == 264 || n == 520; }
+static bool dual_tables(int h, int w) {
+  return rp::supported(h, w) && ((gemm_axis(h) && gemm_axis(w) && !gemm_disabled()) || (strip_axis(h) && strip_axis(w)));
+}
 static size_t dual_offset(int C, int h, int w) { return (rp::table_bytes(C, h, w) + 255) / 256 * 256; }
 // Compile-time-plan kernels on pairs of planes that share their taps (k_static.cu), for the sizes that have one: with
 // full pairs they beat the run-time plans (136 x 136, 4 x 128 planes: 53 us against 76; 68 x 68 upsampled by 2, 16 x 64
@@ -157,7 +161,9 @@ static bool takes_static_pairs(int B, int h, int w) {
     if (e.ry0 * e.ry1 == h && e.rx0 * e.rx1 == w) return rp::supported(h, w);
   return false;
 }
-static bool takes_tensor_cores(int B, int h, int w) { return B >= 2 && dual_tables(h, w); }
+static bool takes_multipass_pairs(int B, int h, int w, int s) {
+  return s == 1 && B >= 2 && (B % 2 == 0 || B >= 5) && dual_tables(h, w);
+}
 
 static int check_padding(int H, int W, int p, int pad_mode) {
   if (p < 0) return CVB_ERR_BAD_ARGUMENT;
@@ -299,7 +305,7 @@ size_t cvb_converse2d_workspace_bytes(int B, int C, int H, int W, int s, int p, 
   if (B < 1 || C < 1 || H < 1 || W < 1 || p < 0 || s < 1) return 0;
   const int h = H + 2 * p, w = W + 2 * p;
   if (takes_static_pairs(B, h, w)) return 0;
-  if (rp::supported(h, w) && !takes_tensor_cores(B, h, w))
+  if (rp::supported(h, w) && !takes_multipass_pairs(B, h, w, s))
     return rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0, std::max(kRpWorkspace, rp::ws_plane_bytes(h, w, s))).ws_bytes;
   Plan1D py, px;
   bool big = false;
@@ -321,7 +327,7 @@ int cvb_converse2d_fwd(const void* x, void* out, const void* table, const float*
   if (k > s * (H + 2 * p) || k > s * (W + 2 * p)) return CVB_ERR_KERNEL_TOO_LARGE;
   rp::Params Q;
   const bool pairs = takes_static_pairs(B, H + 2 * p, W + 2 * p);
-  if (takes_tensor_cores(B, H + 2 * p, W + 2 * p)) {
+  if (takes_multipass_pairs(B, H + 2 * p, W + 2 * p, s)) {
     table = (const char*)table + dual_offset(C, H + 2 * p, W + 2 * p);
   } else if (!pairs && rp::fill_params(Q, table, B, C, H, W, k, s, p, pad_mode)) {
     Q.x = x; Q.out = out; Q.weight = weight; Q.gelu = fuse_gelu ? 1 : 0;
@@ -487,9 +493,23 @@ int cvb_converse2d_fwd_train(const void* x, void* out, const void* table, const 
   if (k > kMaxTaps || k > s * (H + 2 * p) || k > s * (W + 2 * p)) return CVB_ERR_KERNEL_TOO_LARGE;
   const int rc = check_padding(H, W, p, pad_mode);
   if (rc != CVB_OK) return rc;
+  if (H + 2 * p < 2 || W + 2 * p < 2 || !rp::supported(H + 2 * p, W + 2 * p)) return CVB_ERR_UNSUPPORTED_SIZE;
+  if (s == 1)    // nothing to keep
+    return cvb_converse2d_fwd(x, out, table, weight, B, C, H, W, k, s, p, pad_mode, io_dtype, 0, workspace, workspace_bytes,
+                              stream);
   rp::Params Q;
-  if (!rp::fill_params(Q, table, B, C, H, W, k, s, p, pad_mode)) return CVB_ERR_UNSUPPORTED_SIZE;
-  Q.x = x; Q.out = out; Q.weight = weight; Q.rsave = s > 1 ? r_keep : nullptr;
+  rp::fill_params(Q, table, B, C, H, W, k, s, p, pad_mode);
+  if (takes_static_pairs(B, Q.h, Q.w)) {
+    FwdParams P;
+    if (!make_axis_plans(Q.h, Q.w, P.py, P.px)) return CVB_ERR_UNSUPPORTED_SIZE;
+    P.x = x; P.out = out; P.table = (const float2*)table; P.weight = weight;
+    P.B = B; P.C = C; P.H = H; P.W = W; P.k = k; P.s = s; P.p = p; P.pad_mode = pad_mode; P.fuse_gelu = 0;
+    P.h = Q.h; P.w = Q.w; P.pitch = P.w | 1; P.hh = Q.hh; P.skip_mask = 0; P.status = status_ptr();
+    P.ystash = choose_ystash(P.h, P.w, k, s);
+    P.rsave = r_keep;
+    return dispatch_smem(P, io_dtype, (cudaStream_t)stream);
+  }
+  Q.x = x; Q.out = out; Q.weight = weight; Q.rsave = r_keep;
   const rp::Route r = rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0,
                                 std::max(kRpWorkspace, rp::ws_plane_bytes(Q.h, Q.w, s)));
   return rp::run(Q, r, io_dtype, workspace, workspace_bytes, (cudaStream_t)stream);
@@ -497,6 +517,8 @@ int cvb_converse2d_fwd_train(const void* x, void* out, const void* table, const 
 
 size_t cvb_converse2d_train_workspace_bytes(int B, int C, int H, int W, int s, int p) {
   if (B < 1 || C < 1 || H < 1 || W < 1 || p < 0 || s < 1 || !rp::supported(H + 2 * p, W + 2 * p)) return 0;
+  if (s == 1) return cvb_converse2d_workspace_bytes(B, C, H, W, s, p, CVB_F32);
+  if (takes_static_pairs(B, H + 2 * p, W + 2 * p)) return 0;
   return rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0,
                    std::max(kRpWorkspace, rp::ws_plane_bytes(H + 2 * p, W + 2 * p, s))).ws_bytes;
 }

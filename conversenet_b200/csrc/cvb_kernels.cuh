@@ -61,6 +61,7 @@ struct FwdParams {
   Plan1D py, px;
   int hh = 0;     // 0: `table` is [C][w][h] in digit-reversed order; h / 2 + 1: the table of the real-plane kernels
                   // (cvb_rp.cuh), [C][w][hh] in natural order and half as large, the other rows being its conjugates
+  float* rsave = nullptr;   // scale >= 2, compile-time plans: r of every plane kept for the gradients, [B C][h][w even]
 };
 
 struct PassArgs {
@@ -1083,6 +1084,21 @@ CVB_HD void static_stages(const FwdParams& P, const IoArgs& io, float2* plane, c
     } else {
       CVB_PHASE_CT((fft_pass<RY0, IO, h, h, RY1, w, PASS_PRE | PASS_CONJ_OUT>(tid, nthr, ay0, io, 0)));
     }
+  }
+  if (P.s != 1 && P.rsave) {
+    // io.oa / ob are the planes' outputs: their numbers place the copies of r
+    constexpr int wp = (w + 1) / 2 * 2;
+    const size_t out_plane = (size_t)P.H * P.W * P.s * P.s;
+    const size_t na = (size_t)((const IO*)io.oa - (const IO*)P.out) / out_plane;
+    const size_t nb = io.ob ? (size_t)((const IO*)io.ob - (const IO*)P.out) / out_plane : na;
+    CVB_PHASE_CT(([&] {
+      for (int i = tid; i < h * w; i += nthr) {
+        const int row = i / w, col = i - row * w;
+        const float2 v = plane[row * pitch + col];
+        P.rsave[(na * h + row) * wp + col] = v.x;
+        if (io.ob) P.rsave[(nb * h + row) * wp + col] = v.y;
+      }
+    }()));
   }
   if (P.s != 1 && !(sk & 256)) CVB_PHASE_CT(run_epilogue<IO>(tid, nthr, plane, wk, P, io));
 }

@@ -227,6 +227,9 @@ __device__ __forceinline__ void adjoint_epilogue_body(const AdjointParams& A, fl
   for (int i = 0; i < K * K; ++i) { kw[i] = A.weight[(size_t)ch * K * K + i]; acc[i] = 0.f; }
   const int pairs = (A.w + 1) / 2, total = A.h * pairs;
   const float inv = 1.0f / (float)pairs;
+  // the window of a pair of cells starts (c - K + 1) mod 4 past a multiple of four columns: three 16-byte loads a row
+  constexpr int SHIFT = ((c - K + 1) % 4 + 4) % 4, NV = (SHIFT + NW + 3) / 4;
+  const bool quads = S % 2 == 0 && off % 4 == 0 && sW % 4 == 0 && ((size_t)A.g) % 16 == 0;
   for (int it = tid; it < total; it += nthr) {
     int my, px;
     divmod_small(it, pairs, inv, my, px);
@@ -247,6 +250,8 @@ __device__ __forceinline__ void adjoint_epilogue_body(const AdjointParams& A, fl
       x -= off;
       gx[i] = (unsigned)x < (unsigned)sW ? x : -1;
     }
+    const int lo = S * mx + c - K + 1 - off - SHIFT;    // first loaded column of the fast path
+    const bool fast = quads && lo >= 0 && lo + 4 * NV <= sW;
     float v0 = 0.f, v1 = 0.f;
 #pragma unroll
     for (int a = 0; a < K; ++a) {
@@ -255,9 +260,20 @@ __device__ __forceinline__ void adjoint_epilogue_body(const AdjointParams& A, fl
       y -= off;
       if ((unsigned)y >= (unsigned)sH) continue;
       const float* row = g + (size_t)y * sW;
-      float win[NW];
+      float win[NW];                                    // win[i]: column S mx + S + c - i
+      if (fast) {
+        float q[4 * NV];
 #pragma unroll
-      for (int i = 0; i < NW; ++i) win[i] = gx[i] >= 0 ? row[gx[i]] : 0.f;
+        for (int i = 0; i < NV; ++i) {
+          const float4 t = __ldg((const float4*)(row + lo) + i);
+          q[4 * i] = t.x; q[4 * i + 1] = t.y; q[4 * i + 2] = t.z; q[4 * i + 3] = t.w;
+        }
+#pragma unroll
+        for (int i = 0; i < NW; ++i) win[i] = q[SHIFT + NW - 1 - i];
+      } else {
+#pragma unroll
+        for (int i = 0; i < NW; ++i) win[i] = gx[i] >= 0 ? row[gx[i]] : 0.f;
+      }
 #pragma unroll
       for (int b = 0; b < K; ++b) {
         v0 = fmaf(kw[a * K + b], win[S + b], v0);
@@ -347,32 +363,56 @@ __device__ __forceinline__ Preimage preimage(int i, int n, int p, int mode) {
   }
   return r;
 }
+__device__ __forceinline__ float pad_adjoint_at(const PadAdjointParams& A, const float* f, int y, int x) {
+  // away from the margins' images a source sample has one padded copy
+  if (y > A.p && y < A.H - 1 - A.p && x > A.p && x < A.W - 1 - A.p) return f[(size_t)(y + A.p) * A.w + x + A.p];
+  const Preimage py = preimage(y, A.H, A.p, A.pad_mode), px = preimage(x, A.W, A.p, A.pad_mode);
+  auto row = [&](int yy) {
+    const float* q = f + (size_t)yy * A.w;
+    float t = 0.f;
+    for (int xx = px.first; xx <= px.last; ++xx) t += q[xx];
+    if (px.e0 >= 0) t += q[px.e0];
+    if (px.e1 >= 0) t += q[px.e1];
+    return t;
+  };
+  float v = 0.f;
+  for (int yy = py.first; yy <= py.last; ++yy) v += row(yy);
+  if (py.e0 >= 0) v += row(py.e0);
+  if (py.e1 >= 0) v += row(py.e1);
+  return v;
+}
 __device__ __forceinline__ void pad_adjoint_body(const PadAdjointParams& A) {
   const int plane = blockIdx.y;
   const float* f = A.f + (size_t)plane * A.h * A.w;
+  float* out = A.gx + (size_t)plane * A.H * A.W;
+  const int start = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  if (A.g && A.s == 2 && A.W % 2 == 0 && ((size_t)A.g) % 16 == 0 && ((size_t)A.gx) % 8 == 0) {
+    // two samples at a time: their eight values of g are two 16-byte loads
+    const int half = A.W / 2;
+    const float inv = 1.0f / (float)half;
+    const float* g = A.g + (size_t)plane * 4 * A.H * A.W;
+    for (int i = start; i < A.H * half; i += step) {
+      int y, xh;
+      divmod_small(i, half, inv, y, xh);
+      const float4 a = __ldg((const float4*)(g + (size_t)(2 * y) * 2 * A.W) + xh);
+      const float4 b = __ldg((const float4*)(g + (size_t)(2 * y + 1) * 2 * A.W) + xh);
+      const float v0 = pad_adjoint_at(A, f, y, 2 * xh) + ((a.x + a.y) + (b.x + b.y));
+      const float v1 = pad_adjoint_at(A, f, y, 2 * xh + 1) + ((a.z + a.w) + (b.z + b.w));
+      ((float2*)out)[i] = make_float2(v0, v1);
+    }
+    return;
+  }
   const float invW = 1.0f / (float)A.W;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.H * A.W; i += gridDim.x * blockDim.x) {
+  for (int i = start; i < A.H * A.W; i += step) {
     int y, x;
     divmod_small(i, A.W, invW, y, x);
-    const Preimage py = preimage(y, A.H, A.p, A.pad_mode), px = preimage(x, A.W, A.p, A.pad_mode);
-    auto row = [&](int yy) {
-      const float* q = f + (size_t)yy * A.w;
-      float t = 0.f;
-      for (int xx = px.first; xx <= px.last; ++xx) t += q[xx];
-      if (px.e0 >= 0) t += q[px.e0];
-      if (px.e1 >= 0) t += q[px.e1];
-      return t;
-    };
-    float v = 0.f;
-    for (int yy = py.first; yy <= py.last; ++yy) v += row(yy);
-    if (py.e0 >= 0) v += row(py.e0);
-    if (py.e1 >= 0) v += row(py.e1);
+    float v = pad_adjoint_at(A, f, y, x);
     if (A.g) {
       const float* g = A.g + ((size_t)plane * A.s * A.H + (size_t)A.s * y) * A.s * A.W + A.s * x;
       for (int a = 0; a < A.s; ++a)
         for (int b = 0; b < A.s; ++b) v += g[(size_t)a * A.s * A.W + b];
     }
-    A.gx[(size_t)plane * A.H * A.W + i] = v;
+    out[i] = v;
   }
 }
 
