@@ -234,8 +234,7 @@ int cvb_fits_shared(int h, int w) {
   return needs_strip(h, w, kMaxTaps, big) ? 0 : 1;
 }
 
-size_t cvb_transfer_bytes(int C, int h, int w) {
-  if (C < 1 || h < 2 || w < 2) return 0;
+static size_t pair_table_bytes(int C, int h, int w) {
   Plan1D py, px;
   // sized for the register-FFT plans (with their Rader tables) where they exist, so that the size
   // does not depend on which multi-pass kernels serve the plane
@@ -244,12 +243,22 @@ size_t cvb_transfer_bytes(int C, int h, int w) {
   }
   RaderInfo ry, rx;
   rader_both(py, px, ry, rx);
-  const size_t n = ((size_t)C * h * w + h + w + rader_blob_float2(ry) + rader_blob_float2(rx)) * sizeof(float2);
-  return dual_tables(h, w) ? n + dual_offset(C, h, w) : std::max(n, rp::table_bytes(C, h, w));
+  return ((size_t)C * h * w + h + w + rader_blob_float2(ry) + rader_blob_float2(rx)) * sizeof(float2);
 }
 
+size_t cvb_transfer_bytes(int C, int h, int w) {
+  if (C < 1 || h < 2 || w < 2) return 0;
+  const size_t n = pair_table_bytes(C, h, w);
+  return n == 0 ? 0 : dual_tables(h, w) ? n + dual_offset(C, h, w) : std::max(n, rp::table_bytes(C, h, w));
+}
+size_t cvb_pair_transfer_bytes(int C, int h, int w) { return C < 1 || h < 2 || w < 2 ? 0 : pair_table_bytes(C, h, w); }
+
 static int build_table(const float* weight, const float* bias, int C, int k, int s, int h, int w, float eps,
-                       int kind, void* table, void* stream);
+                       int kind, void* table, void* stream, bool pair_only = false);
+int cvb_build_pair_transfer(const float* weight, const float* bias, int C, int k, int s, int h, int w, float eps,
+                            void* table, void* stream) {
+  return build_table(weight, bias, C, k, s, h, w, eps, 0, table, stream, true);
+}
 
 int cvb_build_transfer(const float* weight, const float* bias, int C, int k, int s, int h, int w,
                        float eps, void* table, void* stream) {
@@ -262,11 +271,11 @@ int cvb_build_x0_table(const float* weight, const float* bias, int C, int k, int
 }
 
 static int build_table(const float* weight, const float* bias, int C, int k, int s, int h, int w, float eps,
-                       int kind, void* table, void* stream) {
+                       int kind, void* table, void* stream, bool pair_only) {
   if (!weight || !bias || !table || C < 1 || k < 1 || s < 1 || h < 2 || w < 2) return CVB_ERR_BAD_ARGUMENT;
   // the tiled build keeps k-long arrays of kMaxTaps entries per thread and per block
   if (k > kMaxTaps || k > s * h || k > s * w) return CVB_ERR_KERNEL_TOO_LARGE;
-  if (rp::supported(h, w)) {
+  if (!pair_only && rp::supported(h, w)) {
     const int rc = rp::build_table(weight, bias, C, k, s, h, w, eps, kind, table, (cudaStream_t)stream);
     if (rc != CVB_OK || !dual_tables(h, w)) return rc;
     table = (char*)table + dual_offset(C, h, w);
@@ -300,13 +309,7 @@ static int build_table(const float* weight, const float* bias, int C, int k, int
   return CVB_OK;
 }
 
-size_t cvb_converse2d_workspace_bytes(int B, int C, int H, int W, int s, int p, int io_dtype) {
-  (void)io_dtype;
-  if (B < 1 || C < 1 || H < 1 || W < 1 || p < 0 || s < 1) return 0;
-  const int h = H + 2 * p, w = W + 2 * p;
-  if (takes_static_pairs(B, h, w)) return 0;
-  if (rp::supported(h, w) && !takes_multipass_pairs(B, h, w, s))
-    return rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0, std::max(kRpWorkspace, rp::ws_plane_bytes(h, w, s))).ws_bytes;
+static size_t pair_workspace(int B, int C, int h, int w, int s) {
   Plan1D py, px;
   bool big = false;
   if (h < 2 || w < 2 || !make_axis_plans(h, w, py, px, &big)) return 0;
@@ -314,47 +317,83 @@ size_t cvb_converse2d_workspace_bytes(int B, int C, int H, int W, int s, int p, 
   return strip_geometry(h, w, kMaxTaps, s, C * ((B + 1) / 2)).ws_bytes;
 }
 
-int cvb_converse2d_fwd(const void* x, void* out, const void* table, const float* weight, int B,
-                       int C, int H, int W, int k, int s, int p, int pad_mode, int io_dtype,
-                       int fuse_gelu, void* workspace, size_t workspace_bytes, void* stream) {
-  if (!x || !out || !table || B < 1 || C < 1 || H < 1 || W < 1 || k < 1 || s < 1) return CVB_ERR_BAD_ARGUMENT;
-  if (s > 1 && !weight) return CVB_ERR_BAD_ARGUMENT;
-  if (io_dtype != CVB_F32 && io_dtype != CVB_BF16) return CVB_ERR_BAD_ARGUMENT;
-  if (k > kMaxTaps) return CVB_ERR_KERNEL_TOO_LARGE;
-  int rc = check_padding(H, W, p, pad_mode);
-  if (rc != CVB_OK) return rc;
-  if (H + 2 * p < 2 || W + 2 * p < 2) return CVB_ERR_BAD_ARGUMENT;
-  if (k > s * (H + 2 * p) || k > s * (W + 2 * p)) return CVB_ERR_KERNEL_TOO_LARGE;
-  rp::Params Q;
-  const bool pairs = takes_static_pairs(B, H + 2 * p, W + 2 * p);
-  if (takes_multipass_pairs(B, H + 2 * p, W + 2 * p, s)) {
-    table = (const char*)table + dual_offset(C, H + 2 * p, W + 2 * p);
-  } else if (!pairs && rp::fill_params(Q, table, B, C, H, W, k, s, p, pad_mode)) {
-    Q.x = x; Q.out = out; Q.weight = weight; Q.gelu = fuse_gelu ? 1 : 0;
-    const rp::Route r = rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0,
-                                  std::max(kRpWorkspace, rp::ws_plane_bytes(H + 2 * p, W + 2 * p, s)));
-    return rp::run(Q, r, io_dtype, workspace, workspace_bytes, (cudaStream_t)stream);
-  }
+// The kernels that carry two planes with the same taps as one complex plane.  hh: the table's form (FwdParams::hh).
+static int pair_forward(const void* x, void* out, const void* table, const float* weight, int B, int C, int H, int W, int k,
+                        int s, int p, int pad_mode, int io_dtype, int fuse_gelu, int hh, void* workspace,
+                        size_t workspace_bytes, cudaStream_t st) {
   FwdParams P;
   P.x = x; P.out = out; P.table = (const float2*)table; P.weight = weight;
   P.B = B; P.C = C; P.H = H; P.W = W; P.k = k; P.s = s; P.p = p; P.pad_mode = pad_mode;
   P.fuse_gelu = fuse_gelu ? 1 : 0;
   P.h = H + 2 * p; P.w = W + 2 * p; P.pitch = P.w | 1;
-  P.hh = pairs ? P.h / 2 + 1 : 0;
+  P.hh = hh;
   P.skip_mask = CVB_TUNE("CVB_SKIP", 0);
   P.status = status_ptr();
   P.ystash = CVB_TUNE("CVB_NO_YSTASH", 0) ? 0 : choose_ystash(P.h, P.w, k, s);
-  if (P.h < 2 || P.w < 2) return CVB_ERR_BAD_ARGUMENT;
-  if (k > s * P.h || k > s * P.w) return CVB_ERR_KERNEL_TOO_LARGE;
   bool big = false;
   if (!make_axis_plans(P.h, P.w, P.py, P.px, &big)) return CVB_ERR_UNSUPPORTED_SIZE;
-  cudaStream_t st = (cudaStream_t)stream;
   // workspace need is computed with the largest tap count so that it does not depend on k
   if (needs_strip(P.h, P.w, kMaxTaps, big)) {
     P.ystash = 0;
     return launch_strip(P, io_dtype, workspace, workspace_bytes, st);
   }
   return dispatch_smem(P, io_dtype, st);
+}
+
+static int check_forward(const void* x, void* out, const void* table, const float* weight, int B, int C, int H, int W, int k,
+                         int s, int p, int pad_mode, int io_dtype) {
+  if (!x || !out || !table || B < 1 || C < 1 || H < 1 || W < 1 || k < 1 || s < 1) return CVB_ERR_BAD_ARGUMENT;
+  if (s > 1 && !weight) return CVB_ERR_BAD_ARGUMENT;
+  if (io_dtype != CVB_F32 && io_dtype != CVB_BF16) return CVB_ERR_BAD_ARGUMENT;
+  if (k > kMaxTaps) return CVB_ERR_KERNEL_TOO_LARGE;
+  const int rc = check_padding(H, W, p, pad_mode);
+  if (rc != CVB_OK) return rc;
+  if (H + 2 * p < 2 || W + 2 * p < 2) return CVB_ERR_BAD_ARGUMENT;
+  return k > s * (H + 2 * p) || k > s * (W + 2 * p) ? CVB_ERR_KERNEL_TOO_LARGE : CVB_OK;
+}
+
+int cvb_pair_fwd(const void* x, void* out, const void* table, const float* weight, int B, int C, int H, int W, int k, int s,
+                 int p, int pad_mode, int io_dtype, int fuse_gelu, void* workspace, size_t workspace_bytes, void* stream) {
+  const int rc = check_forward(x, out, table, weight, B, C, H, W, k, s, p, pad_mode, io_dtype);
+  if (rc != CVB_OK) return rc;
+  return pair_forward(x, out, table, weight, B, C, H, W, k, s, p, pad_mode, io_dtype, fuse_gelu, 0, workspace,
+                      workspace_bytes, (cudaStream_t)stream);
+}
+
+size_t cvb_converse2d_workspace_bytes(int B, int C, int H, int W, int s, int p, int io_dtype) {
+  (void)io_dtype;
+  if (B < 1 || C < 1 || H < 1 || W < 1 || p < 0 || s < 1) return 0;
+  const int h = H + 2 * p, w = W + 2 * p;
+  if (takes_static_pairs(B, h, w)) return 0;
+  if (rp::supported(h, w) && !takes_multipass_pairs(B, h, w, s))
+    return rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0, std::max(kRpWorkspace, rp::ws_plane_bytes(h, w, s))).ws_bytes;
+  return pair_workspace(B, C, h, w, s);
+}
+size_t cvb_pair_workspace_bytes(int B, int C, int H, int W, int s, int p) {
+  if (B < 1 || C < 1 || H < 1 || W < 1 || p < 0 || s < 1) return 0;
+  return pair_workspace(B, C, H + 2 * p, W + 2 * p, s);
+}
+
+int cvb_converse2d_fwd(const void* x, void* out, const void* table, const float* weight, int B,
+                       int C, int H, int W, int k, int s, int p, int pad_mode, int io_dtype,
+                       int fuse_gelu, void* workspace, size_t workspace_bytes, void* stream) {
+  const int rc = check_forward(x, out, table, weight, B, C, H, W, k, s, p, pad_mode, io_dtype);
+  if (rc != CVB_OK) return rc;
+  const int h = H + 2 * p, w = W + 2 * p;
+  int hh = 0;
+  rp::Params Q;
+  if (takes_multipass_pairs(B, h, w, s)) {
+    table = (const char*)table + dual_offset(C, h, w);
+  } else if (takes_static_pairs(B, h, w)) {
+    hh = h / 2 + 1;
+  } else if (rp::fill_params(Q, table, B, C, H, W, k, s, p, pad_mode)) {
+    Q.x = x; Q.out = out; Q.weight = weight; Q.gelu = fuse_gelu ? 1 : 0;
+    const rp::Route r = rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0,
+                                  std::max(kRpWorkspace, rp::ws_plane_bytes(h, w, s)));
+    return rp::run(Q, r, io_dtype, workspace, workspace_bytes, (cudaStream_t)stream);
+  }
+  return pair_forward(x, out, table, weight, B, C, H, W, k, s, p, pad_mode, io_dtype, fuse_gelu, hh, workspace,
+                      workspace_bytes, (cudaStream_t)stream);
 }
 
 int cvb_cross_spectrum_supported(int h, int w) {

@@ -138,10 +138,34 @@ CVB_HD float gelu_erf(float v) {
 }
 
 #ifdef __CUDA_ARCH__
-// Two GELUs at once, polynomial and exponent on packed pairs (fma .f32x2).  The same polynomial in u = |v| (the factor
+// Two GELUs at once: the polynomial, the product with t and the final product run on packed pairs
+// (fma / mul .f32x2); |v|, the clamp, the two exp2 and the sign select stay per value.  Same polynomial
+// and the same result as gelu_erf up to the rounding of the fused steps.
+__device__ __forceinline__ float2 gelu_erf2(float vx, float vy) {
+  const float tx = fminf(fabsf(vx) * 0.70710678118654752440f, 4.4f);
+  const float ty = fminf(fabsf(vy) * 0.70710678118654752440f, 4.4f);
+  const p2 t = p2_pack(tx, ty);
+  p2 q = p2_pack(3.7796224119226001e-05f, 3.7796224119226001e-05f);
+  q = p2_fma(q, t, p2_pack(-3.8324893763594527e-04f, -3.8324893763594527e-04f));
+  q = p2_fma(q, t, p2_pack(1.2864194185710442e-03f, 1.2864194185710442e-03f));
+  q = p2_fma(q, t, p2_pack(1.1106310484120274e-03f, 1.1106310484120274e-03f));
+  q = p2_fma(q, t, p2_pack(-2.8553848453755075e-02f, -2.8553848453755075e-02f));
+  q = p2_fma(q, t, p2_pack(1.4862335641232380e-01f, 1.4862335641232380e-01f));
+  q = p2_fma(q, t, p2_pack(9.1838461344425293e-01f, 9.1838461344425293e-01f));
+  q = p2_fma(q, t, p2_pack(1.6279110826289691e+00f, 1.6279110826289691e+00f));
+  float ex, ey;
+  p2_unpack(p2_mul(q, p2_mul(t, p2_pack(-1.0f, -1.0f))), ex, ey);   // -q t
+  const float hx = 0.5f * exp2f(ex), hy = 0.5f * exp2f(ey);         // erfc / 2
+  const p2 phi = p2_pack(vx >= 0.f ? 1.0f - hx : hx, vy >= 0.f ? 1.0f - hy : hy);
+  float ox, oy;
+  p2_unpack(p2_mul(p2_pack(vx, vy), phi), ox, oy);
+  return make_float2(ox, oy);
+}
+
+// The newer kernels' form: polynomial and exponent on packed pairs (fma .f32x2).  The same polynomial in u = |v| (the factor
 // 1 / sqrt(2) is in the coefficients) gives erfc / 2 = 2^(-u q(u) - 1), and GELU = max(v, 0) - |v| erfc / 2 needs no
 // select: about eight instructions a value.  The exponent lies in [-29, -1], so ex2 needs no denormal scaling.
-__device__ __forceinline__ float2 gelu_erf2(float vx, float vy) {
+__device__ __forceinline__ float2 gelu_fast2(float vx, float vy) {
   const float ux = fminf(fabsf(vx), 6.2225397f), uy = fminf(fabsf(vy), 6.2225397f);
   const p2 u = p2_pack(ux, uy);
   p2 q = p2_pack(-2.3622640075e-06f, -2.3622640075e-06f);
@@ -159,6 +183,15 @@ __device__ __forceinline__ float2 gelu_erf2(float vx, float vy) {
   return make_float2(fmaf(-fabsf(vx), hx, fmaxf(vx, 0.f)), fmaf(-fabsf(vy), hy, fmaxf(vy, 0.f)));
 }
 #endif
+
+CVB_HD void gelu_fast_pair(float& a, float& b) {
+#ifdef __CUDA_ARCH__
+  const float2 g = gelu_fast2(a, b);
+  a = g.x; b = g.y;
+#else
+  a = gelu_erf(a); b = gelu_erf(b);
+#endif
+}
 
 // GELU of the two planes' values of one output position
 CVB_HD void gelu_pair(float& a, float& b) {

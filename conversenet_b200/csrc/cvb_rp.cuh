@@ -289,7 +289,7 @@ __device__ __forceinline__ void store_crop(const Params& P, IO* op, int y, int c
   if ((unsigned)oy >= (unsigned)P.OH) return;
   const int ox = 2 * c - P.po;
   float a = v.x, b = -v.y;
-  if (P.gelu) gelu_pair(a, b);
+  if (P.gelu) gelu_fast_pair(a, b);
   IO* o = op + (size_t)(oy * P.OW + ox);
   if (P.vec_out) {    // both columns are inside or outside, and aligned
     if ((unsigned)ox < (unsigned)P.OW) {
@@ -775,7 +775,7 @@ __device__ __forceinline__ void epi_rows(const Params& P, const float* r, int rp
       if (P.gelu) {
 #pragma unroll
         for (int i = 0; i < NO; i += 2) {
-          if (i + 1 < NO) gelu_pair(oa[i], oa[i + 1]);
+          if (i + 1 < NO) gelu_fast_pair(oa[i], oa[i + 1]);
           else oa[i] = gelu_erf(oa[i]);
         }
       }

@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
           for (int j = 0; j < 32; j += 2) {
             const float2 b = *(const float2*)(vec + 64 * hf + c0 + j);
             const float za = a[j] + b.x, zb = a[j + 1] + b.y;
-            const float2 o = gelu_erf2(za, zb);
+            const float2 o = gelu_fast2(za, zb);
             if (TRAIN) {
               float* zp = P.z + (op - (IO*)P.out);
               zp[(size_t)(c0 + j) * HW] = za;
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
           for (int j = 0; j < 32; j += 2) {
             const float2 b = *(const float2*)(vh + 4 * kBlkC + h0 + j);
             const float za = a[j] + b.x, zb = a[j + 1] + b.y;
-            const float2 o = gelu_erf2(za, zb);
+            const float2 o = gelu_fast2(za, zb);
             if (TRAIN && valid) {
               float* zp = P.z + ((size_t)img * kBlkM + h0) * HW + pos + half_off;
               zp[(size_t)j * HW] = za;
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
         if (TRAIN && ph < 2) {
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
-            const float2 o = gelu_erf2(v[j], v[j + 1]);
+            const float2 o = gelu_fast2(v[j], v[j + 1]);
             v[j] = o.x; v[j + 1] = o.y;
           }
         }

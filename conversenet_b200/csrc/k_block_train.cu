@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(256) block_grad_pack_kernel(const GradPackPara
   }
 }
 
-// gelu'(v) = Phi(v) + v phi(v), Phi by the erfc polynomial of gelu_erf2
+// gelu'(v) = Phi(v) + v phi(v), Phi by the erfc polynomial of gelu_fast2
 __device__ __forceinline__ float gelu_grad(float v) {
   const float u = fminf(fabsf(v), 6.2225397f);
   float q = -2.3622640075e-06f;

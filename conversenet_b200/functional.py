@@ -34,6 +34,39 @@ def converse2d_forward(x, table, weight_f32, kernel_size, scale, padding, paddin
     return _cabi.host().converse2d(x, table, weight_f32, kernel_size, scale, padding, padding_mode, fuse_gelu, out)
 
 
+def build_pair_transfer(weight, bias, eps, h, w):
+    """Scale-1 table of the pair kernels (`cvb_build_pair_transfer`) and the weight as contiguous fp32."""
+    lib = _cabi.load()
+    C, k = weight.size(1), weight.size(2)
+    nbytes = lib.cvb_pair_transfer_bytes(C, h, w)
+    if nbytes == 0:
+        raise RuntimeError("padded plane %dx%d is not supported by the FFT engine" % (h, w))
+    wf, bf = _f32(weight).reshape(C, k, k), _f32(bias).reshape(C)
+    table = torch.empty(nbytes, dtype=torch.uint8, device=weight.device)
+    with torch.cuda.device(weight.device):
+        rc = lib.cvb_build_pair_transfer(wf.data_ptr(), bf.data_ptr(), C, k, 1, h, w, float(eps), table.data_ptr(),
+                                         _stream_ptr(weight.device))
+    _cabi.check(rc, "cvb_build_pair_transfer")
+    return table, wf
+
+
+def pair_forward(x, table, weight_f32, kernel_size, padding, padding_mode, fuse_gelu=False):
+    """Scale-1 forward through the pair kernels, whatever the size (`cvb_pair_fwd`)."""
+    lib = _cabi.load()
+    x = x.contiguous()
+    B, C, H, W = x.shape
+    out = torch.empty_like(x)
+    ws_bytes = lib.cvb_pair_workspace_bytes(B, C, H, W, 1, int(padding))
+    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=x.device) if ws_bytes else None
+    with torch.cuda.device(x.device):
+        rc = lib.cvb_pair_fwd(x.data_ptr(), out.data_ptr(), table.data_ptr(), weight_f32.data_ptr(), B, C, H, W,
+                              int(kernel_size), 1, int(padding), _cabi.PAD_MODES[padding_mode], _io_dtype(x),
+                              1 if fuse_gelu else 0, ws.data_ptr() if ws is not None else None, ws_bytes,
+                              _stream_ptr(x.device))
+    _cabi.check(rc, "cvb_pair_fwd")
+    return out
+
+
 def cross_spectrum_supported(h, w):
     """True when `cross_spectrum` has a kernel for the padded plane h x w."""
     return _cabi.load().cvb_cross_spectrum_supported(int(h), int(w)) in (1, 2)

@@ -1,4 +1,5 @@
 """Converse-DnCNN (`models/converse_dncnn.py:11-35`)."""
+import torch
 import torch.nn as nn
 
 from ..util_converse import ConverseBlock
@@ -29,6 +30,16 @@ class ConverseDnCNN(nn.Module):
                                       for _ in range(20)])
         self.m_tail = nn.Sequential(nn.Conv2d(num_features, in_channels, 1, 1, 0))
         self.activation_dtype = None
+
+    @property
+    def activation_dtype(self):
+        return self._activation_dtype
+
+    @activation_dtype.setter
+    def activation_dtype(self, dtype):
+        self._activation_dtype = dtype
+        for block in self.m_body:      # twenty blocks of bf16 rounding: see ConverseBlock.fixed_order
+            block.fixed_order = dtype == torch.bfloat16
 
     def forward(self, x):
         if self.activation_dtype is None:

@@ -181,6 +181,11 @@ class ConverseBlock(nn.Module):
                                    nn.GELU(),
                                    nn.Conv2d(2 * out_channels, out_channels, 1, 1, 0))
         self._pack, self._pack_state = None, None     # 1x1 weights laid out for the kernels
+        # True: bf16 tensors keep one order of sums.  A network that rounds every activation to bf16 amplifies the last bit
+        # of a value (ConverseDnCNN with random weights: one pixel scaled by 1.0001 moves the output by 3 %), so only a
+        # fixed order reproduces its outputs; set by the networks that round between their blocks.
+        self.fixed_order = False
+        self._pair_table = None
 
     def _branch1(self, x):
         c = self.conv1
@@ -244,10 +249,24 @@ class ConverseBlock(nn.Module):
             self._pack, self._pack_state = host.block_pack(*params), state
         if conv._forward_hooks or conv._forward_pre_hooks:
             return self._forward_layers(x, conv, alpha1, alpha2)
+        if self.fixed_order and x.dtype == torch.bfloat16:
+            return self._forward_fixed_order(x, conv, alpha1, alpha2)
         conv._check_backend()
         shape, p = x.shape, conv.padding
         table, wf = conv._table_for(shape[2] + 2 * p, shape[3] + 2 * p, x.device)
         return host.block(x, table, wf, self._pack, conv.kernel_size, p, conv.padding_mode, c1["0"].eps, c2["0"].eps)
+
+    def _forward_fixed_order(self, x, conv, alpha1, alpha2):
+        # one order of sums for every size and batch (see `fixed_order`)
+        c1, c2 = self.conv1, self.conv2
+        h, w = x.size(2) + 2 * conv.padding, x.size(3) + 2 * conv.padding
+        key = (h, w, conv.eps, x.device.index, _cabi.host().state(conv.weight, conv.bias))
+        if self._pair_table is None or self._pair_table[0] != key:
+            self._pair_table = (key, CF.build_pair_transfer(conv.weight, conv.bias, conv.eps, h, w))
+        table, wf = self._pair_table[1]
+        t = CF.ln_pw_gelu(x, c1[0], c1[1])
+        t = CF.pair_forward(t, table, wf, conv.kernel_size, conv.padding, conv.padding_mode, fuse_gelu=True)
+        return CF.pw_res_mlp(t, x, c1[5], c2[0], c2[1], c2[3], alpha1, alpha2)
 
     def _forward_layers(self, x, conv, alpha1, alpha2):
         # the same kernels with Converse2D called as a module (someone hooked it)

@@ -134,6 +134,19 @@ int cvb_converse2d_fwd(const void* x, void* out, const void* table, const float*
                        int fuse_gelu, void* workspace, size_t workspace_bytes, void* stream);
 
 /*
+ * The same operator on the kernels that carry two planes with the same taps (two images of a batch) as one complex plane,
+ * whatever the size and batch, with a table of their own.  cvb_converse2d_fwd takes them where they are the faster ones;
+ * called directly they give one fixed order of sums, which a deep network with bf16 activations needs to be reproducible
+ * (its rounding amplifies the last bit of any value).
+ */
+size_t cvb_pair_transfer_bytes(int C, int h, int w);
+int cvb_build_pair_transfer(const float* weight, const float* bias, int C, int k, int s, int h, int w, float eps,
+                            void* table, void* stream);
+size_t cvb_pair_workspace_bytes(int B, int C, int H, int W, int s, int p);
+int cvb_pair_fwd(const void* x, void* out, const void* table, const float* weight, int B, int C, int H, int W, int k, int s,
+                 int p, int pad_mode, int io_dtype, int fuse_gelu, void* workspace, size_t workspace_bytes, void* stream);
+
+/*
  * ConverseBlock, first fused kernel: out = GELU( W . LayerNorm(x) + b ), C -> 2C channels,
  * i.e. conv1[0..2] of the block: channels_first LayerNorm (models/util_converse.py:60-68),
  * 1x1 Conv2d (:279), GELU (:280).  x (B,C,HW), out (B,2C,HW) contiguous, io_dtype;
