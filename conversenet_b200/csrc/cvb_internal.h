@@ -13,6 +13,30 @@ int cuda_fail(cudaError_t e);
     if (e__ != cudaSuccess) return ::cvb::cuda_fail(e__); \
   } while (0)
 
+#ifdef __CUDACC__
+// Launch with programmatic dependent launch: the kernel (it calls pdl_start() first) may be placed on SMs that the kernel
+// before it has left, which hides the launch gap of back-to-back kernels (N us a launch on B200).
+template <typename... P, typename... A>
+int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  CVB_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+  return CVB_OK;
+}
+// dynamic shared memory beyond 48 KB has to be allowed
+template <typename... P>
+int allow_smem(void (*kernel)(P...), size_t smem) {
+  return smem <= 48 * 1024 ? CVB_OK : [&]() -> int {
+    CVB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    return CVB_OK;
+  }();
+}
+#endif
+
 // Tuning aids read the environment only in tuning builds (-DCVB_TUNING); a shipped library ignores them.
 #ifdef CVB_TUNING
 int env_int(const char* name, int dflt);

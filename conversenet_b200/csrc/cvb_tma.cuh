@@ -13,6 +13,13 @@
 namespace cvb {
 
 #ifdef __CUDA_ARCH__
+// Programmatic dependent launch: `pdl_start` at the top of a kernel lets the next one be placed while this one still runs
+// and waits until the one before has finished and its writes are visible.  No effect in a kernel launched without the
+// attribute (launch_chained).
+__device__ __forceinline__ void pdl_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
@@ -55,6 +62,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return false;
 }
 #else
+inline void pdl_start() {}
 inline uint32_t smem_u32(const void*) { return 0; }
 inline void mbar_init(uint64_t*, int) {}
 inline void mbar_fence_init() {}

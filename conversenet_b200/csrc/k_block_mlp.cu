@@ -91,6 +91,7 @@ struct MixParams {
 template <bool POST, typename IO, bool TRAIN>
 __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_constant__ MixParams P) {
   extern __shared__ __align__(128) float msm[];
+  pdl_start();
   constexpr int kFloats = POST ? kPostFloats : kPreFloats;
   float* wts = msm;
   const float* vec = wts + (POST ? 6 : 2) * kW;    // PRE: b1.  POST: b2, a1, b4, a2, b3
@@ -284,12 +285,11 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
 template <bool POST, typename IO, bool TRAIN = false>
 static int launch_mix(const MixParams& P, int sms, cudaStream_t st) {
   const size_t smem = (size_t)(POST ? kPostFloats : kPreFloats) * sizeof(float) + 3 * sizeof(uint64_t) + 8 + 512 * sizeof(float2) + 16;
-  CVB_CUDA(cudaFuncSetAttribute(block_mix_kernel<POST, IO, TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int rc = allow_smem(block_mix_kernel<POST, IO, TRAIN>, smem);
+  if (rc != CVB_OK) return rc;
   const long long ntiles = (P.npix + 127) / 128;
   const int grid = (int)(ntiles < sms ? ntiles : sms);     // one block per SM; tiles go round the blocks first
-  block_mix_kernel<POST, IO, TRAIN><<<grid, kMixThreads, smem, st>>>(P);
-  CVB_CUDA(cudaGetLastError());
-  return CVB_OK;
+  return launch_chained(block_mix_kernel<POST, IO, TRAIN>, dim3(grid), kMixThreads, smem, st, P);
 }
 
 int launch_block_mix(bool post, const void* x, const void* t, void* out, const void* pack, float eps, int B, int HW,

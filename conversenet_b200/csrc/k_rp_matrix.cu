@@ -14,31 +14,33 @@ namespace rp {
 template <typename IO, int MP>
 __global__ void __launch_bounds__(128, CVB_RP_BLOCKS) matrix_cols_fwd_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
+  pdl_start();
   cols_fwd_body<IO, kMatrixR1, MP>(P, smem);
 }
 template <int MP>
 __global__ void __launch_bounds__(128, CVB_RP_BLOCKS) matrix_rows_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
+  pdl_start();
   rows_body<kMatrixR1, MP>(P, smem);
 }
 template <typename IO, int MP>
 __global__ void __launch_bounds__(128, CVB_RP_BLOCKS) matrix_cols_inv_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
+  pdl_start();
   cols_inv_body<IO, kMatrixR1, MP>(P, smem);
 }
 
 template <int MP>
 __global__ void __launch_bounds__(128, 3) matrix_rows_bwd_kernel(const __grid_constant__ BwdParams Q) {
   extern __shared__ float2 smem[];
+  pdl_start();
   rows_bwd_body<kMatrixR1, MP>(Q, smem);
 }
 
 template <typename K>
 static int go(K kernel, const Params& P, int grid, size_t smem, cudaStream_t st) {
-  CVB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kernel<<<grid, 128, smem, st>>>(P);
-  CVB_CUDA(cudaGetLastError());
-  return CVB_OK;
+  const int rc = allow_smem(kernel, smem);
+  return rc != CVB_OK ? rc : launch_chained(kernel, dim3(grid), 128, smem, st, P);
 }
 int CVB_CAT(launch_matrix_cols_fwd, CVB_MP)(const Params& P, int io_dtype, int grid, size_t smem, cudaStream_t st) {
   return io_dtype == CVB_F32 ? go(matrix_cols_fwd_kernel<float, CVB_MP>, P, grid, smem, st)

@@ -13,20 +13,20 @@ namespace rp {
 template <typename IO>
 __global__ void __launch_bounds__(256, 3) plane_small_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
+  pdl_start();
   plane_body<IO, kSmallRadix>(P, smem);
 }
 template <typename IO>
 __global__ void __launch_bounds__(512, 1) plane_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
+  pdl_start();
   plane_body<IO, kAnyRadix>(P, smem);
 }
 
 template <typename K>
 static int go(K kernel, const Params& P, int threads, size_t smem, cudaStream_t st) {
-  CVB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kernel<<<P.nplane, threads, smem, st>>>(P);
-  CVB_CUDA(cudaGetLastError());
-  return CVB_OK;
+  const int rc = allow_smem(kernel, smem);
+  return rc != CVB_OK ? rc : launch_chained(kernel, dim3(P.nplane), threads, smem, st, P);
 }
 int CVB_CAT(launch_plane, CVB_IO_NAME)(const Params& P, bool small, int threads, size_t smem, cudaStream_t st) {
   return small ? go(plane_small_kernel<CVB_IO>, P, threads, smem, st) : go(plane_kernel<CVB_IO>, P, threads, smem, st);

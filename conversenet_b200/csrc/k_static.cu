@@ -17,6 +17,7 @@ namespace cvb {
 template <typename IO, int RY0, int RY1, int RX0, int RX1, int NT, int MB>
 __global__ void __launch_bounds__(NT, MB) smem_static_kernel(const FwdParams P) {
   extern __shared__ float2 smem[];
+  pdl_start();
   smem_block_static<IO, RY0, RY1, RX0, RX1, NT>(P, blockIdx.x, smem);
 }
 
@@ -30,10 +31,9 @@ namespace {
 template <typename IO>
 int launch_t(const FwdParams& P, size_t smem, cudaStream_t st) {
   auto kernel = smem_static_kernel<IO, CVB_RY0, CVB_RY1, CVB_RX0, CVB_RX1, CVB_NT, CVB_MB>;
-  CVB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kernel<<<num_pairs(P), CVB_NT, smem, st>>>(P);  // the block size is baked into the index arithmetic
-  CVB_CUDA(cudaGetLastError());
-  return CVB_OK;
+  const int rc = allow_smem(kernel, smem);
+  // (the block size is baked into the index arithmetic)
+  return rc != CVB_OK ? rc : launch_chained(kernel, dim3(num_pairs(P)), CVB_NT, smem, st, P);
 }
 
 template <typename IO>
