@@ -67,9 +67,12 @@ inline size_t rows_smem(const Params& P) {
 // kernels built for small radices serve an axis whose two radices are small
 inline bool small_axis(const Axis& a) { return a.mp == 0 && a.r0 <= kSmallRadix && a.r1 <= kSmallRadix; }
 
-// Block size of the strip kernels with up to 128 registers a thread: four blocks of 128 threads on an SM while four
-// tiles fit its memory, else two of 256 (264 x 264: 324 us against 362 with 256; 520 x 520: 1600 against 1451).
-inline int strip_threads(size_t smem) { return 4 * (smem + 1024) <= kSmemLimit + 1024 ? 128 : 256; }
+// Block size of the strip kernels: 256 threads where the blocks leave SMs idle (they then take half the passes over their
+// tile: 64 planes of 132 x 132) or where four tiles do not fit an SM's memory (520 x 520: 1451 us with 256 threads, 1600
+// with 128), else 128 (264 x 264: 324 us against 362).
+inline int strip_threads(size_t smem, int grid, int sms) {
+  return grid <= 2 * sms || 4 * (smem + 1024) > kSmemLimit + 1024 ? 256 : 128;
+}
 
 inline size_t plane_smem(int h, int w, int k) {
   const int wc = (w + 1) / 2, hh = h / 2 + 1;

@@ -16,12 +16,12 @@ int launch_epilogue_bf16(const Params&, cudaStream_t);
 int launch_rows(const Params&, bool, int, int, size_t, cudaStream_t);
 int launch_plane_f32(const Params&, bool, int, size_t, cudaStream_t);
 int launch_plane_bf16(const Params&, bool, int, size_t, cudaStream_t);
-typedef int (*MatrixLauncher)(const Params&, int, int, size_t, cudaStream_t);   // (.., tensor type, grid, ..)
+typedef int (*MatrixLauncher)(const Params&, int, int, int, size_t, cudaStream_t);   // (.., tensor type, threads, grid, ..)
 struct MatrixEntry { int width; MatrixLauncher cols_fwd, rows, cols_inv; };
 #define CVB_RP_X(M)                                                            \
-  int launch_matrix_cols_fwd_##M(const Params&, int, int, size_t, cudaStream_t); \
-  int launch_matrix_rows_##M(const Params&, int, int, size_t, cudaStream_t);     \
-  int launch_matrix_cols_inv_##M(const Params&, int, int, size_t, cudaStream_t);
+  int launch_matrix_cols_fwd_##M(const Params&, int, int, int, size_t, cudaStream_t); \
+  int launch_matrix_rows_##M(const Params&, int, int, int, size_t, cudaStream_t);     \
+  int launch_matrix_cols_inv_##M(const Params&, int, int, int, size_t, cudaStream_t);
 CVB_RP_EACH_WIDTH(CVB_RP_X)
 #undef CVB_RP_X
 static const MatrixEntry kMatrix[] = {
@@ -216,12 +216,13 @@ static int strip(Params& P, int planes, int which, cudaStream_t st) {
   set_vec(P, true);
   P.plane0 = 0; P.nplane = planes;
   const int gc = (planes * P.wc + kLines - 1) / kLines, gr = (planes * P.hh + kLines - 1) / kLines;
+  const int tc = strip_threads(cols_smem(P), gc, sm_count()), tr = strip_threads(rows_smem(P), gr, sm_count());
   if (which == 1)
-    return P.ax.mp ? matrix_entry(P.ax.mp).rows(P, CVB_F32, gr, rows_smem(P), st)
-                   : launch_rows(P, small_axis(P.ax), strip_threads(rows_smem(P)), gr, rows_smem(P), st);
+    return P.ax.mp ? matrix_entry(P.ax.mp).rows(P, CVB_F32, tr, gr, rows_smem(P), st)
+                   : launch_rows(P, small_axis(P.ax), tr, gr, rows_smem(P), st);
   if (P.ay.mp)
-    return (which == 0 ? matrix_entry(P.ay.mp).cols_fwd : matrix_entry(P.ay.mp).cols_inv)(P, CVB_F32, gc, cols_smem(P), st);
-  return (which == 0 ? launch_cols_fwd_f32 : launch_cols_inv_f32)(P, small_axis(P.ay), strip_threads(cols_smem(P)), gc, cols_smem(P), st);
+    return (which == 0 ? matrix_entry(P.ay.mp).cols_fwd : matrix_entry(P.ay.mp).cols_inv)(P, CVB_F32, tc, gc, cols_smem(P), st);
+  return (which == 0 ? launch_cols_fwd_f32 : launch_cols_inv_f32)(P, small_axis(P.ay), tc, gc, cols_smem(P), st);
 }
 int cols_fwd(Params& P, int planes, cudaStream_t st) { return strip(P, planes, 0, st); }
 int rows(Params& P, int planes, cudaStream_t st) { return strip(P, planes, 1, st); }
@@ -245,7 +246,6 @@ int run(Params& P, const Route& r, int io_dtype, void* workspace, size_t ws_byte
   const size_t smem_c = cols_smem(P), smem_r = rows_smem(P);
   if (smem_c > kSmemLimit || smem_r > kSmemLimit) return CVB_ERR_UNSUPPORTED_SIZE;
   const bool sy = small_axis(P.ay), sx = small_axis(P.ax);
-  const int tc = strip_threads(smem_c);
   P.ws = (float2*)workspace;
   for (int p0 = 0; p0 < planes; p0 += r.chunk) {
     P.plane0 = p0;
@@ -254,13 +254,14 @@ int run(Params& P, const Route& r, int io_dtype, void* workspace, size_t ws_byte
       P.r = P.rsave ? P.rsave + (size_t)p0 * P.h * P.wp
                     : (float*)((char*)workspace + (size_t)P.nplane * P.hh * P.wp * sizeof(float2));
     const int gc = (P.nplane * P.wc + kLines - 1) / kLines, gr = (P.nplane * P.hh + kLines - 1) / kLines;
-    int rc = P.ay.mp ? matrix_entry(P.ay.mp).cols_fwd(P, io_dtype, gc, smem_c, st)
+    const int tc = strip_threads(smem_c, gc, sm_count()), tr = strip_threads(smem_r, gr, sm_count());
+    int rc = P.ay.mp ? matrix_entry(P.ay.mp).cols_fwd(P, io_dtype, tc, gc, smem_c, st)
              : f32   ? launch_cols_fwd_f32(P, sy, tc, gc, smem_c, st)
                      : launch_cols_fwd_bf16(P, sy, tc, gc, smem_c, st);
     if (rc == CVB_OK)
-      rc = P.ax.mp ? matrix_entry(P.ax.mp).rows(P, io_dtype, gr, smem_r, st) : launch_rows(P, sx, strip_threads(smem_r), gr, smem_r, st);
+      rc = P.ax.mp ? matrix_entry(P.ax.mp).rows(P, io_dtype, tr, gr, smem_r, st) : launch_rows(P, sx, tr, gr, smem_r, st);
     if (rc == CVB_OK)
-      rc = P.ay.mp ? matrix_entry(P.ay.mp).cols_inv(P, io_dtype, gc, smem_c, st)
+      rc = P.ay.mp ? matrix_entry(P.ay.mp).cols_inv(P, io_dtype, tc, gc, smem_c, st)
            : f32   ? launch_cols_inv_f32(P, sy, tc, gc, smem_c, st)
                    : launch_cols_inv_bf16(P, sy, tc, gc, smem_c, st);
     if (rc == CVB_OK && P.s > 1) rc = f32 ? launch_epilogue_f32(P, st) : launch_epilogue_bf16(P, st);

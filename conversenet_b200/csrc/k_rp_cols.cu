@@ -10,15 +10,15 @@
 namespace cvb {
 namespace rp {
 
-// Small radices: 16-line blocks of 128 threads, six of them on an SM (80 registers); any radix: 128 registers.
+// Small radices: 24 warps on an SM (80 registers); any radix: 128 registers.
 template <typename IO>
-__global__ void __launch_bounds__(128, 6) cols_fwd_small_kernel(const __grid_constant__ Params P) {
+__global__ void __launch_bounds__(256, 3) cols_fwd_small_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
   pdl_start();
   cols_fwd_body<IO, kSmallRadix, 0>(P, smem);
 }
 template <typename IO>
-__global__ void __launch_bounds__(128, 6) cols_inv_small_kernel(const __grid_constant__ Params P) {
+__global__ void __launch_bounds__(256, 3) cols_inv_small_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
   pdl_start();
   cols_inv_body<IO, kSmallRadix, 0>(P, smem);
@@ -48,11 +48,11 @@ static int go(K kernel, const Params& P, int grid, int threads, size_t smem, cud
   return rc != CVB_OK ? rc : launch_chained(kernel, dim3(grid), threads, smem, st, P);
 }
 int CVB_CAT(launch_cols_fwd, CVB_IO_NAME)(const Params& P, bool small, int threads, int grid, size_t smem, cudaStream_t st) {
-  if (small) return go(cols_fwd_small_kernel<CVB_IO>, P, grid, 128, smem, st);
+  if (small) return go(cols_fwd_small_kernel<CVB_IO>, P, grid, threads, smem, st);
   return go(cols_fwd_kernel<CVB_IO>, P, grid, threads, smem, st);
 }
 int CVB_CAT(launch_cols_inv, CVB_IO_NAME)(const Params& P, bool small, int threads, int grid, size_t smem, cudaStream_t st) {
-  if (small) return go(cols_inv_small_kernel<CVB_IO>, P, grid, 128, smem, st);
+  if (small) return go(cols_inv_small_kernel<CVB_IO>, P, grid, threads, smem, st);
   return go(cols_inv_kernel<CVB_IO>, P, grid, threads, smem, st);
 }
 int CVB_CAT(launch_epilogue, CVB_IO_NAME)(const Params& P, cudaStream_t st) {

@@ -6,7 +6,7 @@
 namespace cvb {
 namespace rp {
 
-__global__ void __launch_bounds__(128, 6) rows_small_kernel(const __grid_constant__ Params P) {
+__global__ void __launch_bounds__(256, 3) rows_small_kernel(const __grid_constant__ Params P) {
   extern __shared__ float2 smem[];
   pdl_start();
   rows_body<kSmallRadix, 0>(P, smem);
@@ -23,7 +23,7 @@ static int go(K kernel, const Params& P, int grid, int threads, size_t smem, cud
   return rc != CVB_OK ? rc : launch_chained(kernel, dim3(grid), threads, smem, st, P);
 }
 int launch_rows(const Params& P, bool small, int threads, int grid, size_t smem, cudaStream_t st) {
-  if (small) return go(rows_small_kernel, P, grid, 128, smem, st);
+  if (small) return go(rows_small_kernel, P, grid, threads, smem, st);
   return go(rows_kernel, P, grid, threads, smem, st);
 }
 
