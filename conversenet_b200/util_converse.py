@@ -181,9 +181,10 @@ class ConverseBlock(nn.Module):
                                    nn.GELU(),
                                    nn.Conv2d(2 * out_channels, out_channels, 1, 1, 0))
         self._pack, self._pack_state = None, None     # 1x1 weights laid out for the kernels
-        # True: bf16 tensors keep one order of sums.  A network that rounds every activation to bf16 amplifies the last bit
-        # of a value (ConverseDnCNN with random weights: one pixel scaled by 1.0001 moves the output by 3 %), so only a
-        # fixed order reproduces its outputs; set by the networks that round between their blocks.
+        # True: bf16 tensors stay on the pair kernels and the layer-wise 1x1 kernels.  A network that rounds every
+        # activation to bf16 amplifies the last bit of a value (ConverseDnCNN with random weights: one pixel scaled by
+        # 1.0001 moves the output by 3 %, as far as bf16 itself is from fp32), so its outputs stay what they were only while
+        # the order of every sum does.  Set by the networks that round between their blocks; a block alone does not need it.
         self.fixed_order = False
         self._pair_table = None
 
@@ -257,7 +258,7 @@ class ConverseBlock(nn.Module):
         return host.block(x, table, wf, self._pack, conv.kernel_size, p, conv.padding_mode, c1["0"].eps, c2["0"].eps)
 
     def _forward_fixed_order(self, x, conv, alpha1, alpha2):
-        # one order of sums for every size and batch (see `fixed_order`)
+        # (see `fixed_order`)
         c1, c2 = self.conv1, self.conv2
         h, w = x.size(2) + 2 * conv.padding, x.size(3) + 2 * conv.padding
         key = (h, w, conv.eps, x.device.index, _cabi.host().state(conv.weight, conv.bias))

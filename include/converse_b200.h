@@ -136,7 +136,7 @@ int cvb_converse2d_fwd(const void* x, void* out, const void* table, const float*
 /*
  * The same operator on the kernels that carry two planes with the same taps (two images of a batch) as one complex plane,
  * whatever the size and batch, with a table of their own.  cvb_converse2d_fwd takes them where they are the faster ones;
- * called directly they give one fixed order of sums, which a deep network with bf16 activations needs to be reproducible
+ * called directly they keep their order of sums, on which the outputs of a deep network with bf16 activations depend
  * (its rounding amplifies the last bit of any value).
  */
 size_t cvb_pair_transfer_bytes(int C, int h, int w);

@@ -1,0 +1,173 @@
+"""The real-plane kernels (`csrc/cvb_rp.cuh`: run-time two-stage plans, one plane at a time), their gradients and the
+block kernels around them, at the sizes where they can go wrong: every width of the dense large-prime stage at its
+smallest and largest length, one-stage axes, odd and even lengths, strips and bands with remainders."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import converse2d_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(a, r):
+    return float((a.detach().double() - r.double()).norm() / r.double().norm())
+
+
+CASES = [
+    # B, C, H, W, k, s, p, mode, dtype
+    (1, 1, 2, 3, 1, 1, 0, "circular", "fp32"),            # the smallest axes
+    (1, 3, 29, 32, 3, 1, 0, "circular", "fp32"),          # largest register radices, one stage
+    (1, 2, 37, 41, 3, 1, 0, "replicate", "fp32"),         # dense stage, width 20: both ends
+    (1, 2, 43, 47, 5, 1, 0, "reflect", "fp32"),           # width 24
+    (3, 2, 53, 61, 3, 1, 0, "constant", "fp32"),          # width 32
+    (1, 2, 67, 73, 7, 1, 0, "circular", "fp32"),          # width 36
+    (1, 2, 79, 89, 3, 1, 0, "circular", "fp32"),          # width 44
+    (1, 2, 97, 113, 3, 1, 0, "circular", "fp32"),         # widths 56 and 64
+    (1, 2, 127, 254, 3, 1, 0, "circular", "fp32"),
+    (2, 3, 131 * 2 - 2, 53 * 12 - 2, 3, 1, 1, "replicate", "fp32"),   # 262 is refused below; 636 = 53 * 12
+    (1, 130, 20, 26, 3, 1, 2, "constant", "bf16"),        # one block a plane, constant margins
+    (2, 5, 26 * 26 - 4, 40, 3, 1, 2, "circular", "fp32"),   # 676 = 26 * 26
+    (1, 3, 77, 118, 3, 3, 1, "reflect", "bf16"),          # epilogue through a band, ragged rows
+    (2, 70, 19, 23, 5, 3, 2, "replicate", "fp32"),
+    (1, 2, 33, 301, 3, 4, 1, "constant", "bf16"),         # bands shorter than a row segment
+    (1, 2, 21, 18, 4, 2, 2, "circular", "fp32"),          # tap count without a compile-time epilogue
+    (1, 2, 24, 27, 3, 5, 1, "circular", "fp32"),          # scale without one
+    (3, 4, 128, 128, 5, 2, 4, "circular", "fp32"),        # odd batch at a size with pair kernels
+]
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_forward_matches_oracle(case):
+    from conversenet_b200 import Converse2D
+    B, C, H, W, k, s, p, mode, dt = case
+    rng = np.random.default_rng(H * 1000 + W)
+    w, b = orc.init_weight(C, k, rng)
+    b = b + rng.standard_normal(b.shape).astype(np.float32)
+    dtype = torch.float32 if dt == "fp32" else torch.bfloat16
+    x = torch.from_numpy(rng.standard_normal((B, C, H, W)).astype(np.float32)).to(dtype)
+    m = Converse2D(C, C, k, scale=s, padding=p, padding_mode=mode).cuda().eval()
+    with torch.no_grad():
+        m.weight.copy_(torch.from_numpy(w))
+        m.bias.copy_(torch.from_numpy(b))
+        if (H + 2 * p) % 131 == 0:
+            with pytest.raises(RuntimeError):      # a prime factor above 127
+                m(x.cuda())
+            return
+        y = m(x.cuda()).float().cpu().numpy()
+    ref = orc.converse2d_forward(x.float().numpy(), w, b, s, p, mode, 1e-5, dtype=np.float64)
+    assert orc.rel_l2(y, ref) <= (2e-6 if dt == "fp32" else 3e-3)
+
+
+def test_chunks_of_the_workspace_agree_with_single_planes():
+    # 320 planes of 300 x 260 need several chunks; one plane alone needs one
+    from conversenet_b200 import Converse2D
+    torch.manual_seed(1)
+    m = Converse2D(160, 160, 3, padding=0).cuda().eval()
+    x = torch.randn(2, 160, 300, 260, device="cuda")
+    with torch.no_grad():
+        y = m(x)
+        one = Converse2D(1, 1, 3, padding=0).cuda().eval()
+        for c in (0, 77, 159):
+            one.weight.copy_(m.weight[:, c:c + 1])
+            one.bias.copy_(m.bias[:, c:c + 1])
+            assert _rel(y[1:, c:c + 1], one(x[1:, c:c + 1].contiguous())) <= 1e-6
+
+
+@pytest.mark.parametrize("case", [
+    (2, 3, 24, 31, 3, 1, 3, "replicate"),
+    (3, 2, 33, 41, 5, 1, 2, "reflect"),        # 37 x 45: dense stage along y
+    (2, 2, 30, 49, 3, 2, 2, "circular"),       # 34 x 53: dense stage along x
+    (1, 2, 60, 63, 7, 1, 2, "constant"),       # 64 x 67
+    (2, 2, 16, 18, 5, 3, 2, "circular"),       # odd scale
+    (2, 2, 15, 14, 4, 4, 1, "replicate"),      # run-time taps and scale
+    (4, 3, 64, 64, 5, 2, 2, "reflect"),        # r kept by the pair kernels
+    (2, 2, 12, 12, 3, 5, 1, "circular"),       # scale without native parameter gradients
+    (2, 2, 12, 9, 3, 1, 8, "circular"),        # margins almost as wide as the plane
+])
+def test_gradients_match_fp64_autograd(case):
+    from conversenet_b200 import Converse2D
+    from conversenet_b200.autograd import spectral_forward
+    B, C, H, W, k, s, p, mode = case
+    torch.manual_seed(H + W)
+    m = Converse2D(C, C, k, scale=s, padding=p, padding_mode=mode).cuda()
+    with torch.no_grad():
+        m.bias.add_(torch.randn_like(m.bias) + 4.0)
+    x = torch.randn(B, C, H, W, device="cuda", requires_grad=True)
+    y = m(x)
+    g = torch.randn_like(y)
+    got = torch.autograd.grad(y, (x, m.weight, m.bias), g)
+    a = [t.detach().double().requires_grad_(True) for t in (x, m.weight, m.bias)]
+    ref = torch.autograd.grad(spectral_forward(*a, s, p, mode, 1e-5), a, g.double())
+    for q, r in zip(got, ref):
+        assert _rel(q, r) <= 2e-5
+
+
+@pytest.mark.parametrize("B,H,W", [(1, 4, 5), (3, 24, 31), (2, 16, 16), (1, 37, 64)])
+@pytest.mark.parametrize("alphas", [False, True])
+def test_block_and_its_gradients_match_the_layer_by_layer_block(monkeypatch, B, H, W, alphas):
+    """Pixel counts that are no multiple of a 128-pixel tile, of a 32-pixel tile, fewer than one tile."""
+    from conversenet_b200 import ConverseBlock, ConverseBlockAlphaVariant
+    from conversenet_b200 import util_converse as uc
+    torch.backends.cuda.matmul.allow_tf32 = False
+    torch.manual_seed(H)
+    blk = (ConverseBlockAlphaVariant if alphas else ConverseBlock)(64, 64, 3, 1, 2, "circular").cuda()
+    with torch.no_grad():
+        for q in blk.parameters():
+            if q.dim() == 1 or q.shape[-1] == 1 and q.shape[0] == 1:
+                q.add_(0.2 * torch.randn_like(q))
+    x = torch.randn(B, 64, H, W, device="cuda", requires_grad=True)
+    g = torch.randn_like(x)
+
+    def step():
+        y = blk(x)
+        return [y] + list(torch.autograd.grad(y, [x] + list(blk.parameters()), g))
+
+    with torch.no_grad():
+        inference = blk(x)
+    fused = step()
+    monkeypatch.setattr(uc, "BLOCK_FUSION", False)
+    plain = step()
+    assert _rel(inference, plain[0]) <= 2e-6
+    for a, r in zip(fused, plain):
+        assert float((a - r).norm()) <= 2e-5 * float(r.norm()) + 1e-6
+    from conversenet_b200 import _cabi
+    assert _cabi.load().cvb_last_device_status(1) == 0
+
+
+def test_block_follows_its_parameters():
+    from conversenet_b200 import ConverseBlock
+    torch.manual_seed(3)
+    blk = ConverseBlock(64, 64, 3, 1, 2, "circular").cuda().eval()
+    x = torch.randn(1, 64, 24, 20, device="cuda")
+    with torch.no_grad():
+        a = blk(x)
+        blk.conv2[3].bias.add_(1.0)
+        b = blk(x)
+    assert _rel(b - a, torch.ones_like(a)) <= 1e-5
+
+
+def test_bf16_network_keeps_the_pair_kernels():
+    from conversenet_b200 import functional as CF
+    from conversenet_b200.models import ConverseDnCNN
+    torch.manual_seed(4)
+    net = ConverseDnCNN().cuda().eval()
+    net.activation_dtype = torch.bfloat16
+    assert all(b.fixed_order for b in net.m_body)
+    blk = net.m_body[0]
+    conv = blk.conv1[3]
+    x = torch.randn(3, 64, 40, 37, device="cuda").bfloat16()       # 52 x 49, an unpaired plane
+    with torch.no_grad():
+        y = blk(x)
+        t = CF.ln_pw_gelu(x, blk.conv1[0], blk.conv1[1])
+        table, wf = CF.build_pair_transfer(conv.weight, conv.bias, conv.eps, 52, 49)
+        u = CF.pair_forward(t, table, wf, 7, 6, "circular", fuse_gelu=True)
+        z = CF.pw_res_mlp(u, x, blk.conv1[5], blk.conv2[0], blk.conv2[1], blk.conv2[3])
+    assert torch.equal(y, z)
+    conv.fuse_gelu = True
+    with torch.no_grad():
+        ref = conv(t.float())
+    conv.fuse_gelu = False
+    assert _rel(u, ref) <= 3e-3
+    net.activation_dtype = None
+    assert not any(b.fixed_order for b in net.m_body)
