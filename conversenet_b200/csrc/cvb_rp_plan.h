@@ -133,8 +133,9 @@ inline Route route(int B, int C, int H, int W, int s, int p, int sms, bool force
   return r;
 }
 
-// block size of plane_body: the count that wastes the fewest thread slots over its stages
-inline int plane_threads(const Params& P, int most) {
+// Block size of plane_body.  Planes enough to fill the SMs: the count that wastes the fewest thread slots over the
+// stages.  Fewer: the count with the shortest chain of stage passes.
+inline int plane_threads(const Params& P, int most, bool fills) {
   const Axis &y = P.ay, &x = P.ax;
   const int items[4] = {y.r1 * P.wc, (y.r0 / 2 + 1) * P.wc, x.r1 * P.hh, x.r0 * P.hh};
   const int cost[4] = {y.r0, 2 * y.r1, x.r0, x.r1};
@@ -142,8 +143,8 @@ inline int plane_threads(const Params& P, int most) {
   int bt = 64;
   for (int t = 64; t <= most; t += 32) {
     double c = 0;
-    for (int i = 0; i < 4; ++i) c += (double)((items[i] + t - 1) / t) * t * (cost[i] + 2);
-    c *= 1.0 + 8.0 / t;      // fewer warps hide less latency
+    for (int i = 0; i < 4; ++i) c += (double)((items[i] + t - 1) / t) * (cost[i] + (fills ? 2 : 8));
+    c *= fills ? t * (1.0 + 8.0 / t) : 1.0 + t / 4096.0;      // (fewer warps hide less latency; more wait longer)
     if (c < best - 1e-9) { best = c; bt = t; }
   }
   return bt;

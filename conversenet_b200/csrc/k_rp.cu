@@ -238,7 +238,7 @@ int run(Params& P, const Route& r, int io_dtype, void* workspace, size_t ws_byte
     // planes that leave SMs idle take the wide block (up to 512 threads, 128 registers)
     const bool wide = planes <= sm_count();
     const bool small = !wide && small_axis(P.ay) && small_axis(P.ax);
-    const int threads = plane_threads(P, wide ? 512 : 256);
+    const int threads = plane_threads(P, wide ? 512 : 256, planes > 2 * sm_count());
     return f32 ? launch_plane_f32(P, small, threads, smem, st) : launch_plane_bf16(P, small, threads, smem, st);
   }
   if (r.chunk < 1) return CVB_ERR_TOO_LARGE;

@@ -109,7 +109,8 @@ def test_block_and_its_gradients_match_the_layer_by_layer_block(monkeypatch, B, 
     """Pixel counts that are no multiple of a 128-pixel tile, of a 32-pixel tile, fewer than one tile."""
     from conversenet_b200 import ConverseBlock, ConverseBlockAlphaVariant
     from conversenet_b200 import util_converse as uc
-    torch.backends.cuda.matmul.allow_tf32 = False
+    monkeypatch.setattr(torch.backends.cudnn, "allow_tf32", False)      # the library convolutions' gradients
+    monkeypatch.setattr(torch.backends.cuda.matmul, "allow_tf32", False)
     torch.manual_seed(H)
     blk = (ConverseBlockAlphaVariant if alphas else ConverseBlock)(64, 64, 3, 1, 2, "circular").cuda()
     with torch.no_grad():
