@@ -863,7 +863,7 @@ __device__ __forceinline__ void epilogue(const Params& P, const float* r, int rp
     const bool aligned = P.W % CW == 0 && (oW * (int)sizeof(IO)) % 16 == 0 &&                           \
                          (CW * S_ * (int)sizeof(IO)) % 16 == 0 && ((size_t)op) % 16 == 0;               \
     int per = aligned ? 0 : (band - 16) / (S_ * oW * (int)sizeof(IO));   /* low rows of a band */       \
-    const bool direct = per < 1;                                                                        \
+    const bool direct = per < 8 && per < my1 - my0;   /* bands of a few rows leave threads idle */      \
     if (direct) per = my1 - my0;                                                                        \
     for (int m0 = my0; m0 < my1; m0 += per) {                                                           \
       const int m1 = m0 + per < my1 ? m0 + per : my1, rows = m1 - m0;                                   \
