@@ -862,6 +862,15 @@ __device__ __forceinline__ void epilogue(const Params& P, const float* r, int rp
     const int spr = (P.W + CW - 1) / CW;                                                                \
     const bool aligned = P.W % CW == 0 && (oW * (int)sizeof(IO)) % 16 == 0 &&                           \
                          (CW * S_ * (int)sizeof(IO)) % 16 == 0 && ((size_t)op) % 16 == 0;               \
+    if (sizeof(IO) == 4 && S_ == 3 && !aligned) {   /* one cell a lane: neighbouring lanes write neighbouring runs */ \
+      const int nseg = items / P.W < 1 ? 1 : items / P.W > my1 - my0 ? my1 - my0 : items / P.W;         \
+      const int rps = (my1 - my0 + nseg - 1) / nseg;                                                    \
+      for (int i = t; i < P.W * nseg; i += items) {                                                     \
+        const int seg = i / P.W, b0 = my0 + seg * rps, b1 = b0 + rps < my1 ? b0 + rps : my1;            \
+        if (b0 < b1) epi_rows<S_, K_, S_ == 3 ? 1 : CW, IO>(P, r, rp, wk, xp, op, i - seg * P.W, b0, b1, 0, true); \
+      }                                                                                                 \
+      break;                                                                                            \
+    }                                                                                                   \
     int per = aligned ? 0 : (band - 16) / (S_ * oW * (int)sizeof(IO));   /* low rows of a band */       \
     const bool direct = per < 8 && per < my1 - my0;   /* bands of a few rows leave threads idle */      \
     if (direct) per = my1 - my0;                                                                        \
