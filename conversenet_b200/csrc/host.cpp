@@ -167,9 +167,13 @@ PyObject* py_build_transfer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
-// state(t, ...) -> bytes: storage addresses and version counters; equal bytes = unmodified tensors (None allowed)
+// state(t, ...) -> bytes: storage addresses and version counters; equal bytes = unmodified tensors (None allowed).  None
+// when a tensor was made in inference mode: it counts no versions, so a change in place could not be seen and nothing
+// derived from it may be kept.
 PyObject* py_state(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
+    for (Py_ssize_t i = 0; i < n; ++i)
+      if (a[i] != Py_None && THPVariable_Check(a[i]) && THPVariable_Unpack(a[i]).is_inference()) Py_RETURN_NONE;
     PyObject* o = PyBytes_FromStringAndSize(nullptr, n * 16);
     if (!o) return nullptr;
     char* d = PyBytes_AS_STRING(o);
@@ -178,7 +182,7 @@ PyObject* py_state(PyObject*, PyObject* const* a, Py_ssize_t n) {
       if (a[i] != Py_None && THPVariable_Check(a[i])) {
         const at::Tensor& t = THPVariable_Unpack(a[i]);
         v[0] = (int64_t)t.data_ptr();
-        v[1] = t.is_inference() ? 0 : (int64_t)t._version();
+        v[1] = (int64_t)t._version();
       }
       std::memcpy(d + 16 * i, v, 16);
     }

@@ -111,7 +111,10 @@ class Converse2D(nn.Module):
     # -- transfer-table cache: rebuilt when a parameter is modified in place or replaced
     def _table_for(self, h, w, device):
         weight, bias = self.weight, self.bias
-        key = (h, w, self.scale, self.eps, device.index, _cabi.host().state(weight, bias))
+        state = _cabi.host().state(weight, bias)
+        if state is None:            # inference tensors: nothing says when they change
+            return CF.build_transfer(weight, bias, self.scale, self.eps, h, w)
+        key = (h, w, self.scale, self.eps, device.index, state)
         last = self._last_table
         if last is not None and last[0] == key:
             return last[1]
@@ -199,6 +202,14 @@ class ConverseBlock(nn.Module):
             conv.fuse_gelu = False
         return c[5](t)
 
+    def _packed(self, params):
+        """The 1x1 weights in the kernels' operand layout, laid out once per version of the parameters."""
+        host = _cabi.host()
+        state = host.state(*params)
+        if state is None or state != self._pack_state:
+            self._pack, self._pack_state = host.block_pack(*params), state
+        return self._pack
+
     def _forward_trainable(self, x, alpha1=None, alpha2=None):
         """The block under autograd through the native kernels; None where they do not apply (other widths, dtypes or
         scales, hooked children, autocast, planes without a gradient kernel)."""
@@ -216,14 +227,11 @@ class ConverseBlock(nn.Module):
             if m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks:
                 return None
         conv._check_backend()
-        host = _cabi.host()
-        state = host.state(*params)
-        if state != self._pack_state:
-            self._pack, self._pack_state = host.block_pack(*params), state
+        pack = self._packed(params)
         p, eps1, eps2 = conv.padding, c1["0"].eps, c2["0"].eps
         table, wf = conv._table_for(x.shape[2] + 2 * p, x.shape[3] + 2 * p, x.device)
         x = x.contiguous()
-        kept = host.block_train(x, table, wf, self._pack, conv.kernel_size, p, conv.padding_mode, eps1, eps2)
+        kept = _cabi.host().block_train(x, table, wf, pack, conv.kernel_size, p, conv.padding_mode, eps1, eps2)
         if kept is None:
             return None
         from .autograd import ConverseBlockFunction
@@ -244,10 +252,7 @@ class ConverseBlock(nn.Module):
         c1, c2 = self.conv1._modules, self.conv2._modules
         conv = c1["3"]
         params = CF.block_parameters(c1["0"], c1["1"], c1["5"], alpha1, c2["0"], c2["1"], c2["3"], alpha2)
-        host = _cabi.host()
-        state = host.state(*params)
-        if state != self._pack_state:      # weights in the kernels' operand layout, once per version of the parameters
-            self._pack, self._pack_state = host.block_pack(*params), state
+        pack = self._packed(params)
         if conv._forward_hooks or conv._forward_pre_hooks:
             return self._forward_layers(x, conv, alpha1, alpha2)
         if self.fixed_order and x.dtype == torch.bfloat16:
@@ -255,14 +260,15 @@ class ConverseBlock(nn.Module):
         conv._check_backend()
         shape, p = x.shape, conv.padding
         table, wf = conv._table_for(shape[2] + 2 * p, shape[3] + 2 * p, x.device)
-        return host.block(x, table, wf, self._pack, conv.kernel_size, p, conv.padding_mode, c1["0"].eps, c2["0"].eps)
+        return _cabi.host().block(x, table, wf, pack, conv.kernel_size, p, conv.padding_mode, c1["0"].eps, c2["0"].eps)
 
     def _forward_fixed_order(self, x, conv, alpha1, alpha2):
         # (see `fixed_order`)
         c1, c2 = self.conv1, self.conv2
         h, w = x.size(2) + 2 * conv.padding, x.size(3) + 2 * conv.padding
-        key = (h, w, conv.eps, x.device.index, _cabi.host().state(conv.weight, conv.bias))
-        if self._pair_table is None or self._pair_table[0] != key:
+        state = _cabi.host().state(conv.weight, conv.bias)
+        key = (h, w, conv.eps, x.device.index, state)
+        if self._pair_table is None or self._pair_table[0] != key or state is None:
             self._pair_table = (key, CF.build_pair_transfer(conv.weight, conv.bias, conv.eps, h, w))
         table, wf = self._pair_table[1]
         t = CF.ln_pw_gelu(x, c1[0], c1[1])
