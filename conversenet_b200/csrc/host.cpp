@@ -7,6 +7,7 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <ATen/ATen.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -167,26 +168,79 @@ PyObject* py_build_transfer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
-// state(t, ...) -> bytes: storage addresses and version counters; equal bytes = unmodified tensors (None allowed).  None
+// state(t, ...) -> bytes: storage addresses and version counters, equal bytes = unmodified tensors (None allowed), then
+// (eight bytes) the current stream of the first CUDA tensor's device.  None
 // when a tensor was made in inference mode: it counts no versions, so a change in place could not be seen and nothing
 // derived from it may be kept.
 PyObject* py_state(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     for (Py_ssize_t i = 0; i < n; ++i)
       if (a[i] != Py_None && THPVariable_Check(a[i]) && THPVariable_Unpack(a[i]).is_inference()) Py_RETURN_NONE;
-    PyObject* o = PyBytes_FromStringAndSize(nullptr, n * 16);
+    PyObject* o = PyBytes_FromStringAndSize(nullptr, n * 16 + 8);
     if (!o) return nullptr;
     char* d = PyBytes_AS_STRING(o);
+    void* st = nullptr;
+    bool found = false;
     for (Py_ssize_t i = 0; i < n; ++i) {
       int64_t v[2] = {0, 0};
       if (a[i] != Py_None && THPVariable_Check(a[i])) {
         const at::Tensor& t = THPVariable_Unpack(a[i]);
         v[0] = (int64_t)t.data_ptr();
         v[1] = (int64_t)t._version();
+        if (!found && t.is_cuda()) st = stream(t), found = true;
       }
       std::memcpy(d + 16 * i, v, 16);
     }
+    std::memcpy(d + 16 * n, &st, 8);
     return o;
+  });
+}
+
+void cuda(cudaError_t e, const char* what) {
+  if (e == cudaSuccess) return;
+  (void)cudaGetLastError();
+  throw Failed(std::string(what) + " failed: " + cudaGetErrorString(e));
+}
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  cuda(cudaStreamIsCapturing(st, &s), "cudaStreamIsCapturing");
+  return s != cudaStreamCaptureStatusNone;
+}
+
+// ready(t) -> an event behind the work on the current stream of t's device so far; None during a capture
+PyObject* py_ready(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    want(n, 1);
+    const at::Tensor& t = cuda_tensor(a[0], "tensor");
+    const c10::cuda::CUDAGuard dev(t.device());
+    const cudaStream_t st = (cudaStream_t)stream(t);
+    if (capturing(st)) Py_RETURN_NONE;
+    cudaEvent_t e = nullptr;
+    cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+    const cudaError_t rc = cudaEventRecord(e, st);
+    if (rc != cudaSuccess) cudaEventDestroy(e);
+    cuda(rc, "cudaEventRecord");
+    PyObject* o = PyCapsule_New(e, "cvb.event", [](PyObject* c) { cudaEventDestroy((cudaEvent_t)PyCapsule_GetPointer(c, "cvb.event")); });
+    if (!o) cudaEventDestroy(e);
+    return o;
+  });
+}
+
+// join(event, t, ...): the current stream waits for the event, and the allocator learns that it uses the tensors.  False,
+// and nothing done, during a capture.
+PyObject* py_join(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    if (n < 2) throw Failed("wrong number of arguments");
+    cudaEvent_t e = (cudaEvent_t)PyCapsule_GetPointer(a[0], "cvb.event");
+    if (!e) throw std::invalid_argument("event");
+    const at::Tensor& t = cuda_tensor(a[1], "tensor");
+    const c10::cuda::CUDAGuard dev(t.device());
+    const c10::cuda::CUDAStream st = c10::cuda::getCurrentCUDAStream(t.device().index());
+    if (capturing(st.stream())) Py_RETURN_FALSE;
+    cuda(cudaStreamWaitEvent(st.stream(), e, 0), "cudaStreamWaitEvent");
+    for (Py_ssize_t i = 1; i < n; ++i)
+      c10::cuda::CUDACachingAllocator::recordStream(cuda_tensor(a[i], "tensor").storage().data_ptr(), st);
+    Py_RETURN_TRUE;
   });
 }
 
@@ -407,6 +461,8 @@ PyMethodDef methods[] = {
     {"converse2d", (PyCFunction)(void (*)(void))py_converse2d, METH_FASTCALL, nullptr},
     {"build_transfer", (PyCFunction)(void (*)(void))py_build_transfer, METH_FASTCALL, nullptr},
     {"state", (PyCFunction)(void (*)(void))py_state, METH_FASTCALL, nullptr},
+    {"ready", (PyCFunction)(void (*)(void))py_ready, METH_FASTCALL, nullptr},
+    {"join", (PyCFunction)(void (*)(void))py_join, METH_FASTCALL, nullptr},
     {"block_pack", (PyCFunction)(void (*)(void))py_block_pack, METH_FASTCALL, nullptr},
     {"train_forward", (PyCFunction)(void (*)(void))py_train_forward, METH_FASTCALL, nullptr},
     {"backward", (PyCFunction)(void (*)(void))py_backward, METH_FASTCALL, nullptr},

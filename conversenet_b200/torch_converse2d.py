@@ -20,15 +20,14 @@ device comparison (a synchronisation) per forward call unless the two are the sa
 Do not import this module in a process that also loads the reference's own extension:
 a schema can be defined once.
 """
-from collections import OrderedDict
-
 import torch
 import torch.nn.functional as F
 
-from . import functional as CF
+from . import _cabi, functional as CF
+from ._kept import Kept
 
 _CACHE_SLOTS = 64  # as the reference's FB cache (`converse2d.cpp:52`)
-_cache = OrderedDict()
+_cache = Kept(_CACHE_SLOTS)
 
 _lib = torch.library.Library("converse2d", "DEF")
 _lib.define("forward(Tensor x, Tensor x0, Tensor weight, Tensor bias, int scale, float eps=1e-5) -> Tensor")
@@ -60,17 +59,8 @@ def _forward(x, x0, weight, bias, scale, eps=1e-5):
         ref = x if scale == 1 else F.interpolate(x, scale_factor=scale, mode="nearest")
         if not torch.equal(x0, ref):
             d = (x0 - ref).float()
-    key = (x.device, weight.data_ptr(), weight._version, bias.data_ptr(), bias._version, C, h, w, int(scale),
-           float(eps))
-    hit = _cache.get(key)
-    if hit is None:
-        hit = CF.build_transfer(weight, bias, int(scale), float(eps), h, w)
-        _cache[key] = hit
-        while len(_cache) > _CACHE_SLOTS:
-            _cache.popitem(last=False)
-    else:
-        _cache.move_to_end(key)
-    table, wf = hit
+    key = (C, h, w, int(scale), float(eps), _cabi.host().state(weight, bias))
+    table, wf = _cache.get(key, (weight, bias), lambda: CF.build_transfer(weight, bias, int(scale), float(eps), h, w))
     # padding 0: the solve on the plane as given, nothing cropped
     out = CF.converse2d_forward(x, table, wf, weight.size(2), int(scale), 0, "circular")
     if d is not None:
@@ -82,11 +72,8 @@ def _x0_term(d, weight, bias, wf, s, eps, h, w):
     """T(d) for d = x0 - nearest(x), (B,C,s*h,s*w) fp32."""
     C, k = wf.size(0), wf.size(1)
     c = k // 2
-    key = ("x0", d.device, weight.data_ptr(), weight._version, bias.data_ptr(), bias._version, C, h, w, s, eps)
-    tab = _cache.get(key)
-    if tab is None:
-        tab = CF.build_transfer(weight, bias, s, eps, h, w, x0_term=True)[0]
-        _cache[key] = tab
+    key = ("x0", C, h, w, s, eps, _cabi.host().state(weight, bias))
+    tab = _cache.get(key, (weight, bias), lambda: CF.build_transfer(weight, bias, s, eps, h, w, x0_term=True)[0])
     # e[m] = (K * d)[s m] = sum_a K[a] d[s m - a + c], circular
     dp = F.pad(d, (k - 1 - c, c, k - 1 - c, c), mode="circular")
     e = F.conv2d(dp, wf.flip(-2, -1).reshape(C, 1, k, k), stride=s, groups=C).contiguous()

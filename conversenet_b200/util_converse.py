@@ -9,6 +9,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import _cabi, functional as CF
+from ._kept import Kept
 
 
 # False: ConverseBlock runs its layers one by one (PyTorch LayerNorm / 1x1 / GELU around the native
@@ -104,30 +105,22 @@ class Converse2D(nn.Module):
         self.bias = nn.Parameter(torch.zeros(1, self.in_channels, 1, 1))
         self.weight.data = F.softmax(self.weight.data.view(1, self.in_channels, -1), dim=-1).view(
             1, self.in_channels, self.kernel_size, self.kernel_size)
-        self._tables = OrderedDict()
-        self._last_table = None      # the entry used last, looked at first
+        self._tables = Kept(self._TABLE_SLOTS)
         self.fuse_gelu = False  # set by ConverseBlock: apply the following GELU inside the kernel
+
+    def __setstate__(self, state):
+        super().__setstate__(state)
+        self._tables = Kept(self._TABLE_SLOTS)      # (also for modules pickled by earlier versions)
 
     # -- transfer-table cache: rebuilt when a parameter is modified in place or replaced
     def _table_for(self, h, w, device):
         weight, bias = self.weight, self.bias
         state = _cabi.host().state(weight, bias)
-        if state is None:            # inference tensors: nothing says when they change
-            return CF.build_transfer(weight, bias, self.scale, self.eps, h, w)
         key = (h, w, self.scale, self.eps, device.index, state)
-        last = self._last_table
+        last = self._tables.last
         if last is not None and last[0] == key:
             return last[1]
-        hit = self._tables.get(key)
-        if hit is not None:
-            self._tables.move_to_end(key)
-        else:
-            hit = CF.build_transfer(weight, bias, self.scale, self.eps, h, w)
-            self._tables[key] = hit
-            while len(self._tables) > self._TABLE_SLOTS:
-                self._tables.popitem(last=False)
-        self._last_table = (key, hit)
-        return hit
+        return self._tables.get(key, (weight, bias), lambda: CF.build_transfer(weight, bias, self.scale, self.eps, h, w))
 
     @property
     def biaseps(self):
@@ -136,7 +129,6 @@ class Converse2D(nn.Module):
 
     def clear_cache(self):
         self._tables.clear()
-        self._last_table = None
 
     def _check_backend(self):
         backend = (os.environ.get("CONVERSE2D_BACKEND", "") or self.backend).lower()
@@ -183,13 +175,18 @@ class ConverseBlock(nn.Module):
                                    nn.Conv2d(out_channels, 2 * out_channels, 1, 1, 0),
                                    nn.GELU(),
                                    nn.Conv2d(2 * out_channels, out_channels, 1, 1, 0))
-        self._pack, self._pack_state = None, None     # 1x1 weights laid out for the kernels
+        self._pack = Kept()          # 1x1 weights laid out for the kernels
         # True: bf16 tensors stay on the pair kernels and the layer-wise 1x1 kernels.  A network that rounds every
         # activation to bf16 amplifies the last bit of a value (ConverseDnCNN with random weights: one pixel scaled by
         # 1.0001 moves the output by 3 %, as far as bf16 itself is from fp32), so its outputs stay what they were only while
         # the order of every sum does.  Set by the networks that round between their blocks; a block alone does not need it.
         self.fixed_order = False
-        self._pair_table = None
+        self._pair_table = Kept()
+
+    def __setstate__(self, state):
+        super().__setstate__(state)
+        self._pack, self._pair_table = Kept(), Kept()
+        self.__dict__.setdefault("fixed_order", False)
 
     def _branch1(self, x):
         c = self.conv1
@@ -205,10 +202,11 @@ class ConverseBlock(nn.Module):
     def _packed(self, params):
         """The 1x1 weights in the kernels' operand layout, laid out once per version of the parameters."""
         host = _cabi.host()
-        state = host.state(*params)
-        if state is None or state != self._pack_state:
-            self._pack, self._pack_state = host.block_pack(*params), state
-        return self._pack
+        key = (host.state(*params),)
+        last = self._pack.last
+        if last is not None and last[0] == key:
+            return last[1]
+        return self._pack.get(key, params, lambda: host.block_pack(*params))
 
     def _forward_trainable(self, x, alpha1=None, alpha2=None):
         """The block under autograd through the native kernels; None where they do not apply (other widths, dtypes or
@@ -266,11 +264,9 @@ class ConverseBlock(nn.Module):
         # (see `fixed_order`)
         c1, c2 = self.conv1, self.conv2
         h, w = x.size(2) + 2 * conv.padding, x.size(3) + 2 * conv.padding
-        state = _cabi.host().state(conv.weight, conv.bias)
-        key = (h, w, conv.eps, x.device.index, state)
-        if self._pair_table is None or self._pair_table[0] != key or state is None:
-            self._pair_table = (key, CF.build_pair_transfer(conv.weight, conv.bias, conv.eps, h, w))
-        table, wf = self._pair_table[1]
+        key = (h, w, conv.eps, x.device.index, _cabi.host().state(conv.weight, conv.bias))
+        table, wf = self._pair_table.get(key, (conv.weight, conv.bias), lambda: CF.build_pair_transfer(
+            conv.weight, conv.bias, conv.eps, h, w))
         t = CF.ln_pw_gelu(x, c1[0], c1[1])
         t = CF.pair_forward(t, table, wf, conv.kernel_size, conv.padding, conv.padding_mode, fuse_gelu=True)
         return CF.pw_res_mlp(t, x, c1[5], c2[0], c2[1], c2[3], alpha1, alpha2)

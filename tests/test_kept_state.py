@@ -41,3 +41,145 @@ def test_modules_made_in_inference_mode_follow_their_parameters(dtype):
                 change(ordinary)
                 assert torch.equal(second, ordinary(x))
             assert _rel(second, first) > 1e-3
+
+
+def _block_step(blk, x):
+    with torch.no_grad():
+        return blk(x)
+
+
+def test_copies_and_pickles_start_without_kept_values():
+    import copy
+    import pickle
+    from conversenet_b200 import ConverseBlock
+    blk = ConverseBlock(64, 64, 3, 1, 1)
+    for kept in (blk._pack, blk._pair_table, blk.conv1[3]._tables):
+        kept.last = ("key", "value", None)
+        kept.entries["key"] = "value"
+    for c in (copy.deepcopy(blk), pickle.loads(pickle.dumps(blk))):
+        for kept in (c._pack, c._pair_table, c.conv1[3]._tables):
+            assert kept.last is None and not kept.entries
+    old = blk.__dict__.copy()          # a module pickled before these attributes existed
+    for name in ("_pack", "_pair_table", "fixed_order"):
+        del old[name]
+    c = ConverseBlock.__new__(ConverseBlock)
+    c.__setstate__(old)
+    assert c._pack.last is None and c.fixed_order is False
+
+
+class _FakeHost:
+    """Stands in for the native module: streams are numbers, joins are recorded."""
+
+    def __init__(self, capturing=False):
+        self.capturing, self.joined = capturing, []
+
+    def ready(self, t):
+        return None if self.capturing else "event"
+
+    def join(self, event, *tensors):
+        if self.capturing:
+            return False
+        self.joined.append(event)
+        return True
+
+
+def _state(stream, version=0):
+    return version.to_bytes(16, "little") + stream.to_bytes(8, "little")
+
+
+def test_other_streams_wait_for_a_kept_value_once(monkeypatch):
+    from conversenet_b200 import _cabi
+    from conversenet_b200._kept import Kept
+    host = _FakeHost()
+    monkeypatch.setattr(_cabi, "host", lambda: host)
+    made = []
+
+    def build():
+        made.append(torch.zeros(2))
+        return made[-1]
+
+    kept, q = Kept(2), torch.zeros(1)
+    for stream in (1, 2, 1, 2, 3):
+        assert kept.get(("k", _state(stream)), (q,), build) is made[0]
+    assert len(made) == 1 and host.joined == ["event"] * 2
+    # the parameter's storage stays taken while the entry lives
+    e = kept.last[2]
+    assert e.pins[0].data_ptr() == q.data_ptr()
+    # bounded; the oldest goes first
+    kept.get(("k", _state(1, version=1)), (q,), build)
+    kept.get(("k", _state(1, version=2)), (q,), build)
+    assert len(kept.entries) == 2 and len(made) == 3
+    kept.get(("k", _state(1)), (q,), build)
+    assert len(made) == 4
+
+
+def test_nothing_is_kept_while_capturing(monkeypatch):
+    from conversenet_b200 import _cabi
+    from conversenet_b200._kept import Kept
+    host = _FakeHost(capturing=True)
+    monkeypatch.setattr(_cabi, "host", lambda: host)
+    kept, q = Kept(2), torch.zeros(1)
+    kept.get(("k", _state(1)), (q,), lambda: torch.zeros(2))
+    assert kept.last is None and not kept.entries
+    host.capturing = False
+    value = kept.get(("k", _state(1)), (q,), lambda: torch.zeros(2))
+    host.capturing = True
+    assert kept.get(("k", _state(2)), (q,), lambda: torch.zeros(2)) is value
+    host.capturing = False
+    kept.get(("k", _state(2)), (q,), lambda: torch.zeros(2))
+    assert host.joined == ["event"]      # the eager call on that stream waits
+
+
+@pytest.mark.gpu
+def test_tables_and_packed_weights_across_streams_and_threads():
+    """Tables and packed weights are made behind a long queue of work on one stream; calls on another stream, from
+    another thread, may not read them before."""
+    import threading
+    from conversenet_b200 import Converse2D, ConverseBlock
+    torch.manual_seed(11)
+    for make, C in ((lambda: Converse2D(128, 128, 5, padding=2), 128), (lambda: ConverseBlock(64, 64, 3, 1, 1), 64)):
+        m, twin = make().cuda().eval(), make().cuda().eval()
+        twin.load_state_dict(m.state_dict())
+        x = torch.randn(2, C, 40, 36, device="cuda")
+        busy = torch.randn(4096, 4096, device="cuda")
+        with torch.no_grad():
+            ref = twin(x)
+        for _ in range(3):
+            a, b = torch.cuda.Stream(), torch.cuda.Stream()
+            with torch.no_grad():
+                for q in m.parameters():
+                    q.add_(0.0)               # a new version: tables and weights are laid out again
+            torch.cuda.synchronize()
+            with torch.cuda.stream(a), torch.no_grad():
+                for _ in range(20):
+                    busy @ busy
+                first = m(x)
+            got = []
+
+            def other():
+                with torch.cuda.stream(b), torch.no_grad():
+                    got.append(m(x))
+
+            t = threading.Thread(target=other)
+            t.start()
+            t.join()
+            torch.cuda.synchronize()
+            assert torch.equal(first, ref) and torch.equal(got[0], ref)
+
+
+@pytest.mark.gpu
+def test_capture_without_warm_up_and_eager_calls_after_it():
+    from conversenet_b200 import ConverseBlock
+    torch.manual_seed(12)
+    blk, twin = ConverseBlock(64, 64, 3, 1, 1).cuda().eval(), ConverseBlock(64, 64, 3, 1, 1).cuda().eval()
+    twin.load_state_dict(blk.state_dict())
+    x = torch.randn(1, 64, 24, 20, device="cuda")
+    ref = _block_step(twin, x)
+    g = torch.cuda.CUDAGraph()
+    with torch.no_grad(), torch.cuda.graph(g):
+        y = blk(x)
+    assert torch.equal(_block_step(blk, x), ref)      # before any replay
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, ref)
+    assert torch.equal(_block_step(blk, x), ref)
