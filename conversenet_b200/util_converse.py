@@ -106,7 +106,7 @@ class Converse2D(nn.Module):
         self.weight.data = F.softmax(self.weight.data.view(1, self.in_channels, -1), dim=-1).view(
             1, self.in_channels, self.kernel_size, self.kernel_size)
         self._tables = Kept(self._TABLE_SLOTS)
-        self.fuse_gelu = False  # set by ConverseBlock: apply the following GELU inside the kernel
+        self.fuse_gelu = False  # True: apply a GELU that follows inside the kernel
 
     def __setstate__(self, state):
         super().__setstate__(state)
@@ -138,7 +138,10 @@ class Converse2D(nn.Module):
         if backend not in ("auto", "cuda"):
             raise ValueError(f"backend must be 'auto' | 'cuda' | 'pytorch', got: {backend}")
 
-    def forward(self, x):
+    def forward(self, x, fuse_gelu=None):
+        """`fuse_gelu`: apply the GELU that follows inside the kernel, for this call (None: the attribute decides)."""
+        if fuse_gelu is None:
+            fuse_gelu = self.fuse_gelu
         self._check_backend()
         if not x.is_cuda:
             raise RuntimeError("Converse2D backend='cuda' but the input is not a CUDA tensor.")
@@ -152,9 +155,21 @@ class Converse2D(nn.Module):
             from .autograd import Converse2DFunction
             out = Converse2DFunction.apply(x, self.weight, self.bias, table, wf, self.kernel_size, self.scale,
                                            self.padding, self.padding_mode, self.eps)
-            return F.gelu(out) if self.fuse_gelu else out
-        return _cabi.host().converse2d(x, table, wf, self.kernel_size, self.scale, p, self.padding_mode, self.fuse_gelu,
-                                       None)
+            return F.gelu(out) if fuse_gelu else out
+        return _cabi.host().converse2d(x, table, wf, self.kernel_size, self.scale, p, self.padding_mode, fuse_gelu, None)
+
+
+def _with_gelu(conv, x):
+    """conv(x) followed by the block's GELU, in one kernel.  Told by the call and not by the module's attribute, which
+    another thread (or a hook that runs the block again) would see and reset; modules put in Converse2D's place that
+    know only the attribute still get it."""
+    if type(conv).forward is Converse2D.forward:
+        return conv(x, fuse_gelu=True)
+    conv.fuse_gelu = True
+    try:
+        return conv(x)
+    finally:
+        conv.fuse_gelu = False
 
 
 class ConverseBlock(nn.Module):
@@ -191,13 +206,7 @@ class ConverseBlock(nn.Module):
     def _branch1(self, x):
         c = self.conv1
         t = c[2](c[1](c[0](x)))
-        conv = c[3]
-        conv.fuse_gelu = True  # c[4] runs inside the Converse2D kernel
-        try:
-            t = conv(t)
-        finally:
-            conv.fuse_gelu = False
-        return c[5](t)
+        return c[5](_with_gelu(c[3], t))     # c[4] runs inside the Converse2D kernel
 
     def _packed(self, params):
         """The 1x1 weights in the kernels' operand layout, laid out once per version of the parameters."""
@@ -275,11 +284,7 @@ class ConverseBlock(nn.Module):
         # the same kernels with Converse2D called as a module (someone hooked it)
         c1, c2 = self.conv1, self.conv2
         t = CF.ln_pw_gelu(x, c1[0], c1[1])
-        conv.fuse_gelu = True
-        try:
-            t = conv(t)
-        finally:
-            conv.fuse_gelu = False
+        t = _with_gelu(conv, t)
         return CF.pw_res_mlp(t, x, c1[5], c2[0], c2[1], c2[3], alpha1, alpha2)
 
     def forward(self, x):

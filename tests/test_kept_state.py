@@ -183,3 +183,26 @@ def test_capture_without_warm_up_and_eager_calls_after_it():
     torch.cuda.synchronize()
     assert torch.equal(y, ref)
     assert torch.equal(_block_step(blk, x), ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("C", [64, 16])      # the hooked route and the layer-by-layer route
+def test_block_keeps_its_gelu_when_another_call_runs_inside(C):
+    """Another thread's call of the same block may begin and end while this one is between its layers; a hook that runs
+    the block again puts it there."""
+    from conversenet_b200 import ConverseBlock
+    torch.manual_seed(13)
+    blk, twin = ConverseBlock(C, C, 3, 1, 1).cuda().eval(), ConverseBlock(C, C, 3, 1, 1).cuda().eval()
+    twin.load_state_dict(blk.state_dict())
+    x = torch.randn(1, C, 12, 10, device="cuda")
+    depth = [0]
+
+    def again(module, args):
+        if depth[0] == 0:
+            depth[0] = 1
+            _block_step(blk, x)
+            depth[0] = 0
+
+    blk.conv1[3].register_forward_pre_hook(again)
+    twin.conv1[3].register_forward_pre_hook(lambda module, args: None)
+    assert torch.equal(_block_step(blk, x), _block_step(twin, x))
