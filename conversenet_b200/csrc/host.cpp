@@ -110,6 +110,13 @@ at::Tensor forward(const at::Tensor& x, const at::Tensor& table, const at::Tenso
   return out;
 }
 
+// The calling thread without the interpreter's lock: allocations and launches may wait (a full launch queue, an allocator
+// that has to synchronise), and other Python threads go on meanwhile.  Arguments are read before, results wrapped after.
+struct Unlocked {
+  PyThreadState* state = PyEval_SaveThread();
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
+
 template <class F>
 PyObject* guarded(F f) {
   try {
@@ -134,11 +141,16 @@ PyObject* py_converse2d(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor& x0 = cuda_tensor(a[0], "x");
     if (x0.dim() != 4) throw Failed("x must be (B,C,H,W)");
     const c10::cuda::CUDAGuard dev(x0.device());
-    const at::Tensor x = x0.is_contiguous() ? x0 : x0.contiguous();
+    const at::Tensor &table = tensor(a[1], "table"), &wf = tensor(a[2], "weight");
+    const int k = (int)integer(a[3]), s = (int)integer(a[4]), p = (int)integer(a[5]), mode = pad_mode(a[6]);
+    const int gelu = PyObject_IsTrue(a[7]);
     at::Tensor out;
     if (a[8] != Py_None) out = tensor(a[8], "out");
-    return THPVariable_Wrap(forward(x, tensor(a[1], "table"), tensor(a[2], "weight"), (int)integer(a[3]), (int)integer(a[4]),
-                                    (int)integer(a[5]), pad_mode(a[6]), PyObject_IsTrue(a[7]), std::move(out)));
+    {
+      const Unlocked unlocked;
+      out = forward(x0.is_contiguous() ? x0 : x0.contiguous(), table, wf, k, s, p, mode, gelu, std::move(out));
+    }
+    return THPVariable_Wrap(std::move(out));
   });
 }
 
@@ -158,12 +170,18 @@ PyObject* py_build_transfer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const size_t bytes = api.transfer_bytes(C, (int)h, (int)wd);
     if (!bytes) throw Failed("padded plane " + std::to_string(h) + "x" + std::to_string(wd) + " is not supported by the FFT engine");
     const c10::cuda::CUDAGuard dev(w.device());
-    const at::Tensor wf = f32(w.detach()).view({C, k, k}), bf = f32(b.detach());
-    at::Tensor table = bytes_like(w, bytes);
     auto fn = PyObject_IsTrue(a[6]) ? api.build_x0_table : api.build_transfer;
-    check(fn((const float*)wf.data_ptr(), (const float*)bf.data_ptr(), C, k, (int)s, (int)h, (int)wd, (float)real(a[3]),
-             table.data_ptr(), stream(w)),
-          "cvb_build_transfer");
+    const float eps = (float)real(a[3]);
+    at::Tensor table, wf;
+    {
+      const Unlocked unlocked;
+      wf = f32(w.detach()).view({C, k, k});
+      const at::Tensor bf = f32(b.detach());
+      table = bytes_like(w, bytes);
+      check(fn((const float*)wf.data_ptr(), (const float*)bf.data_ptr(), C, k, (int)s, (int)h, (int)wd, eps,
+               table.data_ptr(), stream(w)),
+            "cvb_build_transfer");
+    }
     return Py_BuildValue("(NN)", THPVariable_Wrap(table), THPVariable_Wrap(wf));
   });
 }
@@ -248,20 +266,23 @@ PyObject* py_join(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_block_pack(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     want(n, 14);
-    at::Tensor t[14];
+    at::Tensor t[14], pack;
     const float* q[14];
-    for (int i = 0; i < 14; ++i) {
-      q[i] = nullptr;
-      if (a[i] == Py_None) continue;
-      t[i] = f32(cuda_tensor(a[i], "parameter"));
-      q[i] = (const float*)t[i].data_ptr();
-    }
+    for (int i = 0; i < 14; ++i)
+      if (a[i] != Py_None) t[i] = cuda_tensor(a[i], "parameter");
     const c10::cuda::CUDAGuard dev(t[2].device());
-    at::Tensor pack = bytes_like(t[2], api.block_pack_bytes());
-    check(api.block_pack(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7], q[8], q[9], q[10], q[11], q[12], q[13],
-                         pack.data_ptr(), stream(pack)),
-          "cvb_block_pack");
-    return THPVariable_Wrap(pack);
+    {
+      const Unlocked unlocked;
+      for (int i = 0; i < 14; ++i) {
+        if (t[i].defined()) t[i] = f32(t[i]);
+        q[i] = t[i].defined() ? (const float*)t[i].data_ptr() : nullptr;
+      }
+      pack = bytes_like(t[2], api.block_pack_bytes());
+      check(api.block_pack(q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7], q[8], q[9], q[10], q[11], q[12], q[13],
+                           pack.data_ptr(), stream(pack)),
+            "cvb_block_pack");
+    }
+    return THPVariable_Wrap(std::move(pack));
   });
 }
 
@@ -272,19 +293,24 @@ PyObject* py_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor& x0 = cuda_tensor(a[0], "x");
     if (x0.dim() != 4) throw Failed("x must be (B,C,H,W)");
     const c10::cuda::CUDAGuard dev(x0.device());
-    const at::Tensor x = x0.is_contiguous() ? x0 : x0.contiguous();
-    const at::Tensor& pack = tensor(a[3], "pack");
-    const int B = (int)x.size(0), C = (int)x.size(1), H = (int)x.size(2), W = (int)x.size(3), io = io_type(x);
-    const auto opt = x.options().requires_grad(false);
-    void* st = stream(x);
-    at::Tensor t = at::empty({B, 2 * C, H, W}, opt);
-    check(api.block_pre(x.data_ptr(), t.data_ptr(), pack.data_ptr(), (float)real(a[7]), B, H * W, io, st), "cvb_block_pre_fwd");
-    t = forward(t, tensor(a[1], "table"), tensor(a[2], "weight"), (int)integer(a[4]), 1, (int)integer(a[5]), pad_mode(a[6]), 1,
-                at::Tensor());
-    at::Tensor out = at::empty({B, C, H, W}, opt);
-    check(api.block_post(t.data_ptr(), x.data_ptr(), out.data_ptr(), pack.data_ptr(), (float)real(a[8]), B, H * W, io, st),
-          "cvb_block_post_fwd");
-    return THPVariable_Wrap(out);
+    const at::Tensor &table = tensor(a[1], "table"), &wf = tensor(a[2], "weight"), &pack = tensor(a[3], "pack");
+    const int B = (int)x0.size(0), C = (int)x0.size(1), H = (int)x0.size(2), W = (int)x0.size(3), io = io_type(x0);
+    const int k = (int)integer(a[4]), p = (int)integer(a[5]), mode = pad_mode(a[6]);
+    const float eps1 = (float)real(a[7]), eps2 = (float)real(a[8]);
+    at::Tensor out;
+    {
+      const Unlocked unlocked;
+      const at::Tensor x = x0.is_contiguous() ? x0 : x0.contiguous();
+      const auto opt = x.options().requires_grad(false);
+      void* st = stream(x);
+      at::Tensor t = at::empty({B, 2 * C, H, W}, opt);
+      check(api.block_pre(x.data_ptr(), t.data_ptr(), pack.data_ptr(), eps1, B, H * W, io, st), "cvb_block_pre_fwd");
+      t = forward(t, table, wf, k, 1, p, mode, 1, at::Tensor());
+      out = at::empty({B, C, H, W}, opt);
+      check(api.block_post(t.data_ptr(), x.data_ptr(), out.data_ptr(), pack.data_ptr(), eps2, B, H * W, io, st),
+            "cvb_block_post_fwd");
+    }
+    return THPVariable_Wrap(std::move(out));
   });
 }
 
@@ -296,18 +322,25 @@ PyObject* py_train_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor& x0 = cuda_tensor(a[0], "x");
     if (x0.dim() != 4) throw Failed("x must be (B,C,H,W)");
     const c10::cuda::CUDAGuard dev(x0.device());
-    const at::Tensor x = x0.is_contiguous() ? x0 : x0.contiguous();
-    const int B = (int)x.size(0), C = (int)x.size(1), H = (int)x.size(2), W = (int)x.size(3), io = io_type(x);
+    const at::Tensor &table = tensor(a[1], "table"), &wf = tensor(a[2], "weight");
+    const int B = (int)x0.size(0), C = (int)x0.size(1), H = (int)x0.size(2), W = (int)x0.size(3), io = io_type(x0);
     const int k = (int)integer(a[3]), s = (int)integer(a[4]), p = (int)integer(a[5]), mode = pad_mode(a[6]);
-    at::Tensor out = at::empty({B, C, (int64_t)H * s, (int64_t)W * s}, x.options().requires_grad(false)), r, w;
-    if (s > 1) r = at::empty({B, C, H + 2 * p, (W + 2 * p + 1) / 2 * 2}, x.options().dtype(at::kFloat).requires_grad(false));
-    const size_t ws = api.train_workspace_bytes(B, C, H, W, s, p);
-    if (ws) w = bytes_like(x, ws);
-    const int rc = api.fwd_train(x.data_ptr(), out.data_ptr(), tensor(a[1], "table").data_ptr(),
-                                 (const float*)tensor(a[2], "weight").data_ptr(), s > 1 ? (float*)r.data_ptr() : nullptr, B, C,
-                                 H, W, k, s, p, mode, io, ws ? w.data_ptr() : nullptr, ws, stream(x));
+    at::Tensor out, r;
+    int rc;
+    {
+      const Unlocked unlocked;
+      const at::Tensor x = x0.is_contiguous() ? x0 : x0.contiguous();
+      at::Tensor w;
+      out = at::empty({B, C, (int64_t)H * s, (int64_t)W * s}, x.options().requires_grad(false));
+      if (s > 1) r = at::empty({B, C, H + 2 * p, (W + 2 * p + 1) / 2 * 2}, x.options().dtype(at::kFloat).requires_grad(false));
+      const size_t ws = api.train_workspace_bytes(B, C, H, W, s, p);
+      if (ws) w = bytes_like(x, ws);
+      rc = api.fwd_train(x.data_ptr(), out.data_ptr(), table.data_ptr(), (const float*)wf.data_ptr(),
+                         s > 1 ? (float*)r.data_ptr() : nullptr, B, C, H, W, k, s, p, mode, io, ws ? w.data_ptr() : nullptr, ws,
+                         stream(x));
+      if (rc != CVB_ERR_UNSUPPORTED_SIZE) check(rc, "cvb_converse2d_fwd_train");
+    }
     if (rc == CVB_ERR_UNSUPPORTED_SIZE) Py_RETURN_NONE;
-    check(rc, "cvb_converse2d_fwd_train");
     PyObject* rr = Py_None;
     if (s > 1) rr = THPVariable_Wrap(r);
     else Py_INCREF(rr);
@@ -320,31 +353,36 @@ PyObject* py_train_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     want(n, 13);
-    const at::Tensor g = f32(cuda_tensor(a[1], "g").detach());
-    const c10::cuda::CUDAGuard dev(g.device());
-    const at::Tensor &w0 = tensor(a[4], "weight"), &b0 = tensor(a[5], "bias");
+    const at::Tensor &g0 = cuda_tensor(a[1], "g"), &w0 = tensor(a[4], "weight"), &b0 = tensor(a[5], "bias");
+    const c10::cuda::CUDAGuard dev(g0.device());
     int d[4];
     for (int i = 0; i < 4; ++i) d[i] = (int)integer(PyTuple_GetItem(a[6], i));
     const int B = d[0], C = d[1], H = d[2], W = d[3], k = (int)w0.size(-1);
     const int s = (int)integer(a[7]), p = (int)integer(a[8]), mode = pad_mode(a[9]);
+    const float eps = (float)real(a[10]);
     const bool wx = PyObject_IsTrue(a[11]), wp = PyObject_IsTrue(a[12]);
     const size_t ws = api.bwd_workspace_bytes(B, C, H, W, k, s, p, wx, wp);
     if (!ws) Py_RETURN_NONE;
-    const at::Tensor wf = f32(w0.detach()), bf = f32(b0.detach());
+    const at::Tensor& table = tensor(a[3], "table");
     at::Tensor x, r, gx, gw, gb;
-    if (wp) x = f32(cuda_tensor(a[0], "x").detach());
+    if (wp) x = cuda_tensor(a[0], "x").detach();
     if (a[2] != Py_None) r = tensor(a[2], "r");
-    const auto opt = g.options().requires_grad(false);
-    if (wx) gx = at::empty({B, C, H, W}, opt);
-    if (wp) {
-      gw = at::empty(w0.sizes(), opt);
-      gb = at::empty(b0.sizes(), opt);
+    {
+      const Unlocked unlocked;
+      const at::Tensor g = f32(g0.detach()), wf = f32(w0.detach()), bf = f32(b0.detach());
+      if (wp) x = f32(x);
+      const auto opt = g.options().requires_grad(false);
+      if (wx) gx = at::empty({B, C, H, W}, opt);
+      if (wp) {
+        gw = at::empty(w0.sizes(), opt);
+        gb = at::empty(b0.sizes(), opt);
+      }
+      at::Tensor work = bytes_like(g, ws);
+      auto ptr = [](const at::Tensor& t) { return t.defined() ? (float*)t.data_ptr() : nullptr; };
+      check(api.bwd(ptr(x), ptr(g), ptr(r), table.data_ptr(), ptr(wf), ptr(bf), ptr(gx), ptr(gw), ptr(gb), B, C, H, W, k, s, p,
+                    mode, eps, work.data_ptr(), ws, stream(g)),
+            "cvb_converse2d_bwd");
     }
-    at::Tensor work = bytes_like(g, ws);
-    auto ptr = [](const at::Tensor& t) { return t.defined() ? (float*)t.data_ptr() : nullptr; };
-    check(api.bwd(ptr(x), ptr(g), ptr(r), tensor(a[3], "table").data_ptr(), ptr(wf), ptr(bf), ptr(gx), ptr(gw), ptr(gb), B, C,
-                  H, W, k, s, p, mode, (float)real(a[10]), work.data_ptr(), ws, stream(g)),
-          "cvb_converse2d_bwd");
     auto wrap = [](const at::Tensor& t) -> PyObject* {
       if (t.defined()) return THPVariable_Wrap(t);
       Py_RETURN_NONE;
@@ -358,22 +396,28 @@ PyObject* py_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_block_train(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     want(n, 9);
-    const at::Tensor x = f32(cuda_tensor(a[0], "x").detach());
-    const c10::cuda::CUDAGuard dev(x.device());
+    const at::Tensor& x0 = cuda_tensor(a[0], "x");
+    const c10::cuda::CUDAGuard dev(x0.device());
     const at::Tensor &table = tensor(a[1], "table"), &wf = tensor(a[2], "weight"), &pack = tensor(a[3], "pack");
-    const int B = (int)x.size(0), C = (int)x.size(1), H = (int)x.size(2), W = (int)x.size(3);
+    const int B = (int)x0.size(0), C = (int)x0.size(1), H = (int)x0.size(2), W = (int)x0.size(3);
     const int k = (int)integer(a[4]), p = (int)integer(a[5]), mode = pad_mode(a[6]);
+    const float eps1 = (float)real(a[7]), eps2 = (float)real(a[8]);
     if (!api.block_bwd_workspace(B, H, W, k, p)) Py_RETURN_NONE;
-    const auto opt = x.options().requires_grad(false);
-    void* st = stream(x);
-    at::Tensor t1 = at::empty({B, 2 * C, H, W}, opt), z1 = at::empty({B, 2 * C, H, W}, opt), u = at::empty({B, 2 * C, H, W}, opt);
-    at::Tensor x1 = at::empty({B, C, H, W}, opt), z3 = at::empty({B, 2 * C, H, W}, opt), out = at::empty({B, C, H, W}, opt);
-    check(api.block_pre_train((const float*)x.data_ptr(), (float*)t1.data_ptr(), (float*)z1.data_ptr(), pack.data_ptr(),
-                              (float)real(a[7]), B, H * W, st), "cvb_block_pre_train");
-    forward(t1, table, wf, k, 1, p, mode, 0, u);
-    check(api.block_post_train((const float*)u.data_ptr(), (const float*)x.data_ptr(), (float*)out.data_ptr(),
-                               (float*)x1.data_ptr(), (float*)z3.data_ptr(), pack.data_ptr(), (float)real(a[8]), B, H * W, st),
-          "cvb_block_post_train");
+    at::Tensor t1, z1, u, x1, z3, out;
+    {
+      const Unlocked unlocked;
+      const at::Tensor x = f32(x0.detach());
+      const auto opt = x.options().requires_grad(false);
+      void* st = stream(x);
+      t1 = at::empty({B, 2 * C, H, W}, opt), z1 = at::empty({B, 2 * C, H, W}, opt), u = at::empty({B, 2 * C, H, W}, opt);
+      x1 = at::empty({B, C, H, W}, opt), z3 = at::empty({B, 2 * C, H, W}, opt), out = at::empty({B, C, H, W}, opt);
+      check(api.block_pre_train((const float*)x.data_ptr(), (float*)t1.data_ptr(), (float*)z1.data_ptr(), pack.data_ptr(), eps1,
+                                B, H * W, st), "cvb_block_pre_train");
+      forward(t1, table, wf, k, 1, p, mode, 0, u);
+      check(api.block_post_train((const float*)u.data_ptr(), (const float*)x.data_ptr(), (float*)out.data_ptr(),
+                                 (float*)x1.data_ptr(), (float*)z3.data_ptr(), pack.data_ptr(), eps2, B, H * W, st),
+            "cvb_block_post_train");
+    }
     return Py_BuildValue("(NNNNNN)", THPVariable_Wrap(out), THPVariable_Wrap(t1), THPVariable_Wrap(z1), THPVariable_Wrap(u),
                          THPVariable_Wrap(x1), THPVariable_Wrap(z3));
   });
@@ -384,44 +428,49 @@ PyObject* py_block_train(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_block_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     want(n, 16);
-    at::Tensor in[7];
-    const float* ip[7];
-    for (int i = 0; i < 7; ++i) {
-      in[i] = f32(cuda_tensor(a[i], "tensor").detach());
-      ip[i] = (const float*)in[i].data_ptr();
-    }
-    const c10::cuda::CUDAGuard dev(in[0].device());
-    at::Tensor par[14];
+    at::Tensor in[7], par[14];
     const float* pp[14];
+    for (int i = 0; i < 7; ++i) in[i] = cuda_tensor(a[i], "tensor").detach();
+    const c10::cuda::CUDAGuard dev(in[0].device());
     for (int i = 0; i < 14; ++i) {
       PyObject* o = PyTuple_GetItem(a[10], i);
       if (!o) throw std::invalid_argument("params");
-      pp[i] = nullptr;
-      if (o == Py_None) continue;
-      par[i] = f32(tensor(o, "parameter").detach());
-      pp[i] = (const float*)par[i].data_ptr();
+      if (o != Py_None) par[i] = tensor(o, "parameter").detach();
     }
-    const at::Tensor &cw = tensor(a[8], "weight"), &cb = tensor(a[9], "bias");
-    const at::Tensor cwf = f32(cw.detach()), cbf = f32(cb.detach());
-    const auto opt = in[0].options().requires_grad(false);
+    const at::Tensor &table = tensor(a[7], "table"), &cw = tensor(a[8], "weight"), &cb = tensor(a[9], "bias");
     cvb_block_bwd_args A;
     std::memset(&A, 0, sizeof(A));
-    A.x = ip[0]; A.t1 = ip[1]; A.z1 = ip[2]; A.u = ip[3]; A.x1 = ip[4]; A.z3 = ip[5]; A.g = ip[6];
-    A.table = tensor(a[7], "table").data_ptr();
-    A.conv_w = (const float*)cwf.data_ptr(); A.conv_b = (const float*)cbf.data_ptr();
-    A.ln1_w = pp[0]; A.ln1_b = pp[1]; A.w1 = pp[2]; A.b1 = pp[3]; A.w2 = pp[4]; A.b2 = pp[5]; A.alpha1 = pp[6];
-    A.ln2_w = pp[7]; A.ln2_b = pp[8]; A.w3 = pp[9]; A.b3 = pp[10]; A.w4 = pp[11]; A.b4 = pp[12]; A.alpha2 = pp[13];
     A.eps1 = (float)real(a[11]); A.eps2 = (float)real(a[12]); A.conv_eps = (float)real(a[13]);
-    A.B = (int)in[0].size(0); A.H = (int)in[0].size(2); A.W = (int)in[0].size(3);
     A.k = (int)cw.size(-1); A.p = (int)integer(a[14]); A.pad_mode = pad_mode(a[15]);
-    at::Tensor gx = at::empty(in[0].sizes(), opt), gcw = at::empty(cw.sizes(), opt), gcb = at::empty(cb.sizes(), opt);
-    at::Tensor gp = at::empty({(int64_t)api.block_grad_floats()}, opt);
-    const size_t ws = api.block_bwd_workspace(A.B, A.H, A.W, A.k, A.p);
-    at::Tensor work = bytes_like(in[0], ws ? ws : 1);
-    A.gx = (float*)gx.data_ptr(); A.gconv_w = (float*)gcw.data_ptr(); A.gconv_b = (float*)gcb.data_ptr();
-    A.gparams = (float*)gp.data_ptr();
-    A.workspace = work.data_ptr(); A.workspace_bytes = ws; A.stream = stream(in[0]);
-    check(api.block_bwd(&A), "cvb_block_bwd");
+    at::Tensor gx, gcw, gcb, gp;
+    {
+      const Unlocked unlocked;
+      const float* ip[7];
+      for (int i = 0; i < 7; ++i) {
+        in[i] = f32(in[i]);
+        ip[i] = (const float*)in[i].data_ptr();
+      }
+      for (int i = 0; i < 14; ++i) {
+        if (par[i].defined()) par[i] = f32(par[i]);
+        pp[i] = par[i].defined() ? (const float*)par[i].data_ptr() : nullptr;
+      }
+      const at::Tensor cwf = f32(cw.detach()), cbf = f32(cb.detach());
+      const auto opt = in[0].options().requires_grad(false);
+      A.x = ip[0]; A.t1 = ip[1]; A.z1 = ip[2]; A.u = ip[3]; A.x1 = ip[4]; A.z3 = ip[5]; A.g = ip[6];
+      A.table = table.data_ptr();
+      A.conv_w = (const float*)cwf.data_ptr(); A.conv_b = (const float*)cbf.data_ptr();
+      A.ln1_w = pp[0]; A.ln1_b = pp[1]; A.w1 = pp[2]; A.b1 = pp[3]; A.w2 = pp[4]; A.b2 = pp[5]; A.alpha1 = pp[6];
+      A.ln2_w = pp[7]; A.ln2_b = pp[8]; A.w3 = pp[9]; A.b3 = pp[10]; A.w4 = pp[11]; A.b4 = pp[12]; A.alpha2 = pp[13];
+      A.B = (int)in[0].size(0); A.H = (int)in[0].size(2); A.W = (int)in[0].size(3);
+      gx = at::empty(in[0].sizes(), opt), gcw = at::empty(cw.sizes(), opt), gcb = at::empty(cb.sizes(), opt);
+      gp = at::empty({(int64_t)api.block_grad_floats()}, opt);
+      const size_t ws = api.block_bwd_workspace(A.B, A.H, A.W, A.k, A.p);
+      at::Tensor work = bytes_like(in[0], ws ? ws : 1);
+      A.gx = (float*)gx.data_ptr(); A.gconv_w = (float*)gcw.data_ptr(); A.gconv_b = (float*)gcb.data_ptr();
+      A.gparams = (float*)gp.data_ptr();
+      A.workspace = work.data_ptr(); A.workspace_bytes = ws; A.stream = stream(in[0]);
+      check(api.block_bwd(&A), "cvb_block_bwd");
+    }
     PyObject* out = PyList_New(17);
     PyList_SET_ITEM(out, 0, THPVariable_Wrap(gx));
     PyList_SET_ITEM(out, 1, THPVariable_Wrap(gcw));

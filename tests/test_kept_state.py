@@ -206,3 +206,37 @@ def test_block_keeps_its_gelu_when_another_call_runs_inside(C):
     blk.conv1[3].register_forward_pre_hook(again)
     twin.conv1[3].register_forward_pre_hook(lambda module, args: None)
     assert torch.equal(_block_step(blk, x), _block_step(twin, x))
+
+
+@pytest.mark.gpu
+def test_a_call_that_waits_for_the_launch_queue_lets_other_threads_run():
+    import threading
+    import time
+    from conversenet_b200 import Converse2D
+    m = Converse2D(8, 8, 3, padding=1).cuda().eval()
+    x = torch.randn(1, 8, 16, 16, device="cuda")
+    with torch.no_grad():
+        m(x)
+        torch.cuda.synchronize()
+        gaps, stop = [], threading.Event()
+
+        def tick():
+            last = time.perf_counter()
+            while not stop.is_set():
+                time.sleep(0.001)
+                now = time.perf_counter()
+                gaps.append(now - last)
+                last = now
+
+        t = threading.Thread(target=tick)
+        t.start()
+        torch.cuda._sleep(1_500_000_000)      # about 0.8 s of the GPU's time; the calls behind it fill the launch queue
+        t0 = time.perf_counter()
+        for _ in range(4000):
+            m(x)
+        waited = time.perf_counter() - t0
+        stop.set()
+        t.join()
+        torch.cuda.synchronize()
+    assert waited > 0.4                       # the queue did fill
+    assert max(gaps) < 0.3 * waited
