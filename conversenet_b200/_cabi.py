@@ -104,6 +104,11 @@ def host():
     return _host
 
 
+def loaded_host():
+    """The host module if a call has loaded it, else None."""
+    return _host
+
+
 def check(status, what):
     if status != 0:
         lib = load()

@@ -131,7 +131,9 @@ class Converse2D(nn.Module):
         self._tables.clear()
 
     def _check_backend(self):
-        backend = (os.environ.get("CONVERSE2D_BACKEND", "") or self.backend).lower()
+        host = _cabi.loaded_host()
+        chosen = os.environ.get("CONVERSE2D_BACKEND") if host is None else host.backend()
+        backend = (chosen or self.backend).lower()
         if backend == "pytorch":
             raise RuntimeError("Converse2D backend='pytorch' is not available: this build only has the "
                                "native sm_100a path")

@@ -240,3 +240,20 @@ def test_a_call_that_waits_for_the_launch_queue_lets_other_threads_run():
         torch.cuda.synchronize()
     assert waited > 0.4                       # the queue did fill
     assert max(gaps) < 0.3 * waited
+
+
+def test_backend_variable_is_read_at_every_call(monkeypatch):
+    from conversenet_b200 import Converse2D, _cabi
+    m = Converse2D(2, 2, 3)
+    for load in (False, True):
+        monkeypatch.setattr(_cabi, "_host", _cabi.host() if load else None)
+        for value, error in (("pytorch", RuntimeError), ("nope", ValueError), ("", None), ("CUDA", None), (None, None)):
+            if value is None:
+                monkeypatch.delenv("CONVERSE2D_BACKEND", raising=False)
+            else:
+                monkeypatch.setenv("CONVERSE2D_BACKEND", value)
+            if error is None:
+                m._check_backend()
+            else:
+                with pytest.raises(error):
+                    m._check_backend()
