@@ -8,7 +8,10 @@ _LOCK = threading.Lock()      # guards the slow path of every cache: a look-up t
 
 
 class _Entry:
-    __slots__ = ("value", "tensors", "pins", "ready", "streams")
+    __slots__ = ("value", "tensors", "ready", "streams")
+
+    def __init__(self, value, tensors, ready, streams):
+        self.value, self.tensors, self.ready, self.streams = value, tensors, ready, streams
 
 
 class Kept:
@@ -48,13 +51,11 @@ class Kept:
             e = self.entries.get(own)
             if e is None:
                 value = build()
-                e = _Entry()
-                e.value, e.tensors = value, value if isinstance(value, tuple) else (value,)
-                e.ready = host.ready(e.tensors[0])
-                if e.ready is None:      # capturing
+                tensors = value if isinstance(value, tuple) else (value,)
+                ready = host.ready(tensors[0], *params)
+                if ready is None:        # capturing
                     return value
-                e.pins, e.streams = [q.detach() for q in params if q is not None], {stream}
-                self.entries[own] = e
+                self.entries[own] = e = _Entry(value, tensors, ready, {stream})
                 while len(self.entries) > self.slots:
                     self.entries.popitem(last=False)
             else:

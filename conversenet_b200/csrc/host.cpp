@@ -14,8 +14,10 @@
 
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <stdexcept>
 #include <string>
+#include <vector>
 
 #include "../../include/converse_b200.h"
 
@@ -234,37 +236,47 @@ bool capturing(cudaStream_t st) {
   return s != cudaStreamCaptureStatusNone;
 }
 
-// ready(t) -> an event behind the work on the current stream of t's device so far; None during a capture
+// What a kept value needs beside itself: an event behind the work that makes it, and the storages whose addresses name it
+struct Ready {
+  cudaEvent_t event = nullptr;
+  std::vector<c10::Storage> pins;
+  ~Ready() {
+    if (event) cudaEventDestroy(event);
+  }
+};
+
+// ready(t, param, ...) -> a Ready behind the work on the current stream of t's device so far, holding the parameters'
+// storages; None during a capture
 PyObject* py_ready(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    want(n, 1);
+    if (n < 1) throw Failed("wrong number of arguments");
     const at::Tensor& t = cuda_tensor(a[0], "tensor");
     const c10::cuda::CUDAGuard dev(t.device());
     const cudaStream_t st = (cudaStream_t)stream(t);
     if (capturing(st)) Py_RETURN_NONE;
-    cudaEvent_t e = nullptr;
-    cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
-    const cudaError_t rc = cudaEventRecord(e, st);
-    if (rc != cudaSuccess) cudaEventDestroy(e);
-    cuda(rc, "cudaEventRecord");
-    PyObject* o = PyCapsule_New(e, "cvb.event", [](PyObject* c) { cudaEventDestroy((cudaEvent_t)PyCapsule_GetPointer(c, "cvb.event")); });
-    if (!o) cudaEventDestroy(e);
+    auto r = std::make_unique<Ready>();
+    for (Py_ssize_t i = 1; i < n; ++i)
+      if (a[i] != Py_None) r->pins.push_back(tensor(a[i], "parameter").storage());
+    cuda(cudaEventCreateWithFlags(&r->event, cudaEventDisableTiming), "cudaEventCreate");
+    cuda(cudaEventRecord(r->event, st), "cudaEventRecord");
+    PyObject* o = PyCapsule_New(r.get(), "cvb.ready", [](PyObject* c) { delete (Ready*)PyCapsule_GetPointer(c, "cvb.ready"); });
+    if (o) r.release();
     return o;
   });
 }
 
-// join(event, t, ...): the current stream waits for the event, and the allocator learns that it uses the tensors.  False,
+// join(ready, t, ...): the current stream waits for its event, and the allocator learns that it uses the tensors.  False,
 // and nothing done, during a capture.
 PyObject* py_join(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     if (n < 2) throw Failed("wrong number of arguments");
-    cudaEvent_t e = (cudaEvent_t)PyCapsule_GetPointer(a[0], "cvb.event");
-    if (!e) throw std::invalid_argument("event");
+    const Ready* r = (const Ready*)PyCapsule_GetPointer(a[0], "cvb.ready");
+    if (!r) throw std::invalid_argument("ready");
     const at::Tensor& t = cuda_tensor(a[1], "tensor");
     const c10::cuda::CUDAGuard dev(t.device());
     const c10::cuda::CUDAStream st = c10::cuda::getCurrentCUDAStream(t.device().index());
     if (capturing(st.stream())) Py_RETURN_FALSE;
-    cuda(cudaStreamWaitEvent(st.stream(), e, 0), "cudaStreamWaitEvent");
+    cuda(cudaStreamWaitEvent(st.stream(), r->event, 0), "cudaStreamWaitEvent");
     for (Py_ssize_t i = 1; i < n; ++i)
       c10::cuda::CUDACachingAllocator::recordStream(cuda_tensor(a[i], "tensor").storage().data_ptr(), st);
     Py_RETURN_TRUE;

@@ -73,7 +73,8 @@ class _FakeHost:
     def __init__(self, capturing=False):
         self.capturing, self.joined = capturing, []
 
-    def ready(self, t):
+    def ready(self, t, *params):
+        self.pinned = params
         return None if self.capturing else "event"
 
     def join(self, event, *tensors):
@@ -102,9 +103,7 @@ def test_other_streams_wait_for_a_kept_value_once(monkeypatch):
     for stream in (1, 2, 1, 2, 3):
         assert kept.get(("k", _state(stream)), (q,), build) is made[0]
     assert len(made) == 1 and host.joined == ["event"] * 2
-    # the parameter's storage stays taken while the entry lives
-    e = kept.last[2]
-    assert e.pins[0].data_ptr() == q.data_ptr()
+    assert host.pinned == (q,)           # the parameter's storage stays taken while the entry lives
     # bounded; the oldest goes first
     kept.get(("k", _state(1, version=1)), (q,), build)
     kept.get(("k", _state(1, version=2)), (q,), build)
