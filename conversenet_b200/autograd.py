@@ -31,6 +31,7 @@ times a remainder above the kernels' radices) take `grad_input_composed` and aut
 """
 import torch
 import torch.nn.functional as F
+from torch.autograd.function import once_differentiable
 
 from . import _cabi
 from . import functional as CF
@@ -174,41 +175,43 @@ def grad_params(x, g, weight, bias, scale, padding, padding_mode, eps, table=Non
 
 class Converse2DFunction(torch.autograd.Function):
     """Native forward and gradients; `grad_input_composed` and `spectral_forward` for planes the gradient kernels do
-    not take."""
+    not take.  Everything the backward reads is a saved tensor: released by it, and seen by saved-tensor hooks and
+    checkpointing."""
 
     @staticmethod
     def forward(ctx, x, weight, bias, table, wf, kernel_size, scale, padding, padding_mode, eps):
-        ctx.save_for_backward(x, weight, bias)
-        ctx.table = table
-        ctx.r = None
         ctx.cfg = (int(kernel_size), int(scale), int(padding), padding_mode, float(eps))
+        kept = r = None
         if ctx.needs_input_grad[1] or ctx.needs_input_grad[2]:
             kept = _cabi.host().train_forward(x, table, wf, kernel_size, scale, padding, padding_mode)
-            if kept is not None:
-                out, ctx.r = kept
-                return out
-        return CF.converse2d_forward(x, table, wf, kernel_size, scale, padding, padding_mode)
+        if kept is None:
+            out = CF.converse2d_forward(x, table, wf, kernel_size, scale, padding, padding_mode)
+        else:
+            out, r = kept
+        ctx.save_for_backward(x, weight, bias, table, r)
+        return out
 
     @staticmethod
+    @once_differentiable
     def backward(ctx, g):
-        x, weight, bias = ctx.saved_tensors
+        x, weight, bias, table, r = ctx.saved_tensors
         k, s, p, mode, eps = ctx.cfg
         want_x = ctx.needs_input_grad[0]
         want_p = ctx.needs_input_grad[1] or ctx.needs_input_grad[2]
         gx = gw = gb = None
-        native_p = want_p and NATIVE_PARAM_GRADS and (s == 1 or ctx.r is not None)
+        native_p = want_p and NATIVE_PARAM_GRADS and (s == 1 or r is not None)
         out = None
         if want_x or native_p:
-            out = _cabi.host().backward(x, g, ctx.r, ctx.table, weight, bias, tuple(x.shape), s, p, mode, eps, want_x,
+            out = _cabi.host().backward(x, g, r, table, weight, bias, tuple(x.shape), s, p, mode, eps, want_x,
                                         native_p)
             if out is None and native_p and want_x:      # perhaps dL/dx alone
                 native_p = False
-                out = _cabi.host().backward(None, g, None, ctx.table, weight, bias, tuple(x.shape), s, p, mode, eps, True,
+                out = _cabi.host().backward(None, g, None, table, weight, bias, tuple(x.shape), s, p, mode, eps, True,
                                             False)
         if out is not None:
             gx, gw, gb = out
         elif want_x:
-            gx = grad_input_composed(g, weight, bias, s, p, mode, eps, x.shape, ctx.table)
+            gx = grad_input_composed(g, weight, bias, s, p, mode, eps, x.shape, table)
         if want_p and gw is None:
             with torch.enable_grad():
                 w_ = weight.detach().float().requires_grad_(True)
@@ -225,21 +228,21 @@ class Converse2DFunction(torch.autograd.Function):
 class ConverseBlockFunction(torch.autograd.Function):
     """A whole ConverseBlock (64 channels, scale 1, fp32) under autograd: the fused forward keeping the layers before the
     GELUs, the gradients in one native call (`csrc/k_block_train.cu`).  `params`: the fourteen parameters around Converse2D
-    in the order of `functional.block_parameters`, None for absent alphas."""
+    in the order of `functional.block_parameters`, None for absent alphas; `kept`: what `host.block_train` returned."""
 
     @staticmethod
     def forward(ctx, kept, x, conv_w, conv_b, table, cfg, *params):
-        ctx.save_for_backward(x, conv_w, conv_b, *params)
-        ctx.kept = kept[1:]
-        ctx.table = table
+        out, *layers = kept
+        ctx.save_for_backward(x, *layers, table, conv_w, conv_b, *params)
         ctx.cfg = cfg
-        return kept[0]
+        return out
 
     @staticmethod
+    @once_differentiable
     def backward(ctx, g):
-        x, conv_w, conv_b, *params = ctx.saved_tensors
+        x, t1, z1, u, x1, z3, table, conv_w, conv_b, *params = ctx.saved_tensors
         eps1, eps2, conv_eps, p, mode = ctx.cfg
-        grads = _cabi.host().block_backward(x, *ctx.kept, g, ctx.table, conv_w, conv_b, tuple(params), eps1, eps2, conv_eps,
+        grads = _cabi.host().block_backward(x, t1, z1, u, x1, z3, g, table, conv_w, conv_b, tuple(params), eps1, eps2, conv_eps,
                                             p, mode)
         need = ctx.needs_input_grad
         gx, gcw, gcb, *gp = grads

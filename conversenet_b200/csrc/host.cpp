@@ -336,7 +336,7 @@ PyObject* py_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // train_forward(x, table, weight_f32, kernel_size, scale, padding, padding_mode) -> (out, r or None); None when the
-// gradient kernels have no plan for the padded plane
+// gradient kernels give no parameter gradients for the shape (nothing would read r)
 PyObject* py_train_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     want(n, 7);
@@ -346,6 +346,7 @@ PyObject* py_train_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor &table = tensor(a[1], "table"), &wf = tensor(a[2], "weight");
     const int B = (int)x0.size(0), C = (int)x0.size(1), H = (int)x0.size(2), W = (int)x0.size(3), io = io_type(x0);
     const int k = (int)integer(a[3]), s = (int)integer(a[4]), p = (int)integer(a[5]), mode = pad_mode(a[6]);
+    if (!api.bwd_workspace_bytes(B, C, H, W, k, s, p, 0, 1)) Py_RETURN_NONE;
     at::Tensor out, r;
     int rc;
     {
