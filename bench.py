@@ -452,10 +452,12 @@ def time_layer(R, cfg, dtype, K, W, target_ms, use_graph=True, check=False):
     outs = [torch.empty((cfg["B"], cfg["C"], cfg["H"] * cfg["s"], cfg["W"] * cfg["s"]), dtype=tdtype, device=dev)
             for _ in range(nbuf)]
     h, w = cfg["H"] + 2 * cfg["p"], cfg["W"] + 2 * cfg["p"]
-    table, wf = mod._table_for(h, w, dev)
+    pairs = CF.takes_pairs(cfg["B"], h, w, cfg["s"])
+    table, wf = CF.build_transfer(mod.weight, mod.bias, cfg["s"], cfg["eps"], h, w, batch=cfg["B"])
 
     def step(i):
-        CF.converse2d_forward(xs[i % nbuf], table, wf, cfg["k"], cfg["s"], cfg["p"], cfg["mode"], out=outs[i % nbuf])
+        CF.converse2d_forward(xs[i % nbuf], table, wf, cfg["k"], cfg["s"], cfg["p"], cfg["mode"], out=outs[i % nbuf],
+                              pairs=pairs)
 
     for i in range(max(W, 3)):
         step(i)

@@ -52,6 +52,10 @@ SIGNATURES = {
     "cvb_pair_transfer_bytes": (_c.c_size_t, [_c.c_int] * 3),
     "cvb_build_pair_transfer": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_int, _c.c_int, _c.c_int, _c.c_int,
                                            _c.c_int, _c.c_float, _c.c_void_p, _c.c_void_p]),
+    "cvb_takes_pairs": (_c.c_int, [_c.c_int] * 4),
+    "cvb_plane_transfer_bytes": (_c.c_size_t, [_c.c_int] * 3),
+    "cvb_build_plane_transfer": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_int, _c.c_int, _c.c_int, _c.c_int,
+                                            _c.c_int, _c.c_float, _c.c_void_p, _c.c_void_p]),
     "cvb_pair_workspace_bytes": (_c.c_size_t, [_c.c_int] * 6),
     "cvb_pair_fwd": (_c.c_int, [_c.c_void_p] * 4 + [_c.c_int] * 10 + [_c.c_void_p, _c.c_size_t, _c.c_void_p]),
     "cvb_plan_radices": (_c.c_int, [_c.c_int, _c.POINTER(_c.c_int), _c.c_int]),

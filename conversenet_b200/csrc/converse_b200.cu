@@ -149,21 +149,22 @@ constexpr size_t kRpWorkspace = (size_t)64 << 20;
 // At scale >= 2 the run-time kernels' epilogue wins (260 x 260 by 2, 4 x 64 planes: 270 us against 596).
 static bool strip_axis(int n) { return n == 264 || n == 520; }
 static bool dual_tables(int h, int w) {
-  return rp::supported(h, w) && ((gemm_axis(h) && gemm_axis(w) && !gemm_disabled()) || (strip_axis(h) && strip_axis(w)));
+  return ((gemm_axis(h) && gemm_axis(w) && !gemm_disabled()) || (strip_axis(h) && strip_axis(w))) && rp::supported(h, w);
 }
 static size_t dual_offset(int C, int h, int w) { return (rp::table_bytes(C, h, w) + 255) / 256 * 256; }
 // Compile-time-plan kernels on pairs of planes that share their taps (k_static.cu), for the sizes that have one: with
 // full pairs they beat the run-time plans (136 x 136, 4 x 128 planes: 53 us against 76; 68 x 68 upsampled by 2, 16 x 64
 // planes: 37 against 42).  An odd batch leaves one pair half empty, which pays from five images on.
-static bool takes_static_pairs(int B, int h, int w) {
-  if (B < 2 || (B % 2 && B < 5) || option(CVB_OPT_RUNTIME_PLAN) || option(CVB_OPT_MULTIPASS)) return false;
+static bool static_plan(int h, int w) {
   for (const StaticEntry& e : kStatic)
-    if (e.ry0 * e.ry1 == h && e.rx0 * e.rx1 == w) return rp::supported(h, w);
+    if (e.ry0 * e.ry1 == h && e.rx0 * e.rx1 == w) return true;
   return false;
 }
-static bool takes_multipass_pairs(int B, int h, int w, int s) {
-  return s == 1 && B >= 2 && (B % 2 == 0 || B >= 5) && dual_tables(h, w);
+static bool full_pairs(int B) { return B >= 2 && (B % 2 == 0 || B >= 5); }
+static bool takes_static_pairs(int B, int h, int w) {
+  return full_pairs(B) && !option(CVB_OPT_RUNTIME_PLAN) && !option(CVB_OPT_MULTIPASS) && static_plan(h, w) && rp::supported(h, w);
 }
+static bool takes_multipass_pairs(int B, int h, int w, int s) { return s == 1 && full_pairs(B) && dual_tables(h, w); }
 
 static int check_padding(int H, int W, int p, int pad_mode) {
   if (p < 0) return CVB_ERR_BAD_ARGUMENT;
@@ -246,18 +247,33 @@ static size_t pair_table_bytes(int C, int h, int w) {
   return ((size_t)C * h * w + h + w + rader_blob_float2(ry) + rader_blob_float2(rx)) * sizeof(float2);
 }
 
+// The real-plane table alone, the pair table alone (lengths without a two-stage plan), or one behind the other (sizes with
+// dual_tables).  Sizes of k_static.cu read the real-plane table in a blob that keeps the pair table's size, which callers
+// have allocated since before there were two.
 size_t cvb_transfer_bytes(int C, int h, int w) {
   if (C < 1 || h < 2 || w < 2) return 0;
+  const size_t plane = rp::table_bytes(C, h, w);
+  if (plane && !dual_tables(h, w) && !static_plan(h, w)) return plane;
   const size_t n = pair_table_bytes(C, h, w);
-  return n == 0 ? 0 : dual_tables(h, w) ? n + dual_offset(C, h, w) : std::max(n, rp::table_bytes(C, h, w));
+  return n == 0 ? 0 : plane && dual_tables(h, w) ? n + dual_offset(C, h, w) : std::max(n, plane);
 }
 size_t cvb_pair_transfer_bytes(int C, int h, int w) { return C < 1 || h < 2 || w < 2 ? 0 : pair_table_bytes(C, h, w); }
+size_t cvb_plane_transfer_bytes(int C, int h, int w) { return C < 1 || h < 2 || w < 2 ? 0 : rp::table_bytes(C, h, w); }
 
+int cvb_takes_pairs(int B, int h, int w, int s) {
+  return takes_multipass_pairs(B, h, w, s) ? 2 : takes_static_pairs(B, h, w) ? 1 : 0;
+}
+
+enum Tables { kAnyBatch, kPairTable, kPlaneTable };
 static int build_table(const float* weight, const float* bias, int C, int k, int s, int h, int w, float eps,
-                       int kind, void* table, void* stream, bool pair_only = false);
+                       int kind, void* table, void* stream, Tables which = kAnyBatch);
 int cvb_build_pair_transfer(const float* weight, const float* bias, int C, int k, int s, int h, int w, float eps,
                             void* table, void* stream) {
-  return build_table(weight, bias, C, k, s, h, w, eps, 0, table, stream, true);
+  return build_table(weight, bias, C, k, s, h, w, eps, 0, table, stream, kPairTable);
+}
+int cvb_build_plane_transfer(const float* weight, const float* bias, int C, int k, int s, int h, int w, float eps,
+                             void* table, void* stream) {
+  return build_table(weight, bias, C, k, s, h, w, eps, 0, table, stream, kPlaneTable);
 }
 
 int cvb_build_transfer(const float* weight, const float* bias, int C, int k, int s, int h, int w,
@@ -271,15 +287,16 @@ int cvb_build_x0_table(const float* weight, const float* bias, int C, int k, int
 }
 
 static int build_table(const float* weight, const float* bias, int C, int k, int s, int h, int w, float eps,
-                       int kind, void* table, void* stream, bool pair_only) {
+                       int kind, void* table, void* stream, Tables which) {
   if (!weight || !bias || !table || C < 1 || k < 1 || s < 1 || h < 2 || w < 2) return CVB_ERR_BAD_ARGUMENT;
   // the tiled build keeps k-long arrays of kMaxTaps entries per thread and per block
   if (k > kMaxTaps || k > s * h || k > s * w) return CVB_ERR_KERNEL_TOO_LARGE;
-  if (!pair_only && rp::supported(h, w)) {
+  if (which != kPairTable && rp::supported(h, w)) {
     const int rc = rp::build_table(weight, bias, C, k, s, h, w, eps, kind, table, (cudaStream_t)stream);
-    if (rc != CVB_OK || !dual_tables(h, w)) return rc;
+    if (rc != CVB_OK || which == kPlaneTable || !dual_tables(h, w)) return rc;
     table = (char*)table + dual_offset(C, h, w);
   }
+  if (which == kPlaneTable) return CVB_ERR_UNSUPPORTED_SIZE;
   TransferParams T;
   if (!make_axis_plans(h, w, T.py, T.px)) return CVB_ERR_UNSUPPORTED_SIZE;
   T.weight = weight; T.bias = bias; T.table = (float2*)table;
@@ -312,7 +329,7 @@ static int build_table(const float* weight, const float* bias, int C, int k, int
 static size_t pair_workspace(int B, int C, int h, int w, int s) {
   Plan1D py, px;
   bool big = false;
-  if (h < 2 || w < 2 || !make_axis_plans(h, w, py, px, &big)) return 0;
+  if (h < 2 || w < 2 || (static_plan(h, w) && !option(CVB_OPT_MULTIPASS)) || !make_axis_plans(h, w, py, px, &big)) return 0;
   if (!needs_strip(h, w, kMaxTaps, big)) return 0;
   return strip_geometry(h, w, kMaxTaps, s, C * ((B + 1) / 2)).ws_bytes;
 }

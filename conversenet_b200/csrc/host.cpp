@@ -44,6 +44,13 @@ struct Api {
   decltype(&cvb_block_grad_floats) block_grad_floats = nullptr;
   decltype(&cvb_block_bwd_workspace_bytes) block_bwd_workspace = nullptr;
   decltype(&cvb_block_bwd) block_bwd = nullptr;
+  decltype(&cvb_takes_pairs) takes_pairs = nullptr;
+  decltype(&cvb_plane_transfer_bytes) plane_bytes = nullptr;
+  decltype(&cvb_build_plane_transfer) build_plane = nullptr;
+  decltype(&cvb_pair_transfer_bytes) pair_bytes = nullptr;
+  decltype(&cvb_build_pair_transfer) build_pair = nullptr;
+  decltype(&cvb_pair_workspace_bytes) pair_workspace_bytes = nullptr;
+  decltype(&cvb_pair_fwd) pair_fwd = nullptr;
 } api;
 
 struct Failed : std::runtime_error { using std::runtime_error::runtime_error; };
@@ -100,15 +107,20 @@ at::Tensor f32(const at::Tensor& t) {
   return t.detach().to(at::kFloat).contiguous();
 }
 
+// `pairs`: `table` is the pair table and the pair kernels run; else the table of build_transfer for any batch, or the
+// real-plane one
 at::Tensor forward(const at::Tensor& x, const at::Tensor& table, const at::Tensor& wf, int k, int s, int p, int mode,
-                   int gelu, at::Tensor out) {
+                   int gelu, at::Tensor out, bool pairs) {
   const int B = (int)x.size(0), C = (int)x.size(1), H = (int)x.size(2), W = (int)x.size(3), io = io_type(x);
   if (!out.defined()) out = at::empty({B, C, (int64_t)H * s, (int64_t)W * s}, x.options().requires_grad(false));
-  const size_t ws = api.workspace_bytes(B, C, H, W, s, p, io);
+  const size_t full = sizeof(float) * 2 * (size_t)C * (H + 2 * p) * (W + 2 * p);   // below that: no pair table in it
+  if ((size_t)table.numel() < full && (pairs || api.takes_pairs(B, H + 2 * p, W + 2 * p, s) == 2))
+    throw Failed("the transfer table was built for another batch size");
+  const size_t ws = pairs ? api.pair_workspace_bytes(B, C, H, W, s, p) : api.workspace_bytes(B, C, H, W, s, p, io);
   at::Tensor w;
   if (ws) w = bytes_like(x, ws);
-  check(api.converse2d_fwd(x.data_ptr(), out.data_ptr(), table.data_ptr(), (const float*)wf.data_ptr(), B, C, H, W, k, s,
-                           p, mode, io, gelu, ws ? w.data_ptr() : nullptr, ws, stream(x)),
+  check((pairs ? api.pair_fwd : api.converse2d_fwd)(x.data_ptr(), out.data_ptr(), table.data_ptr(), (const float*)wf.data_ptr(), B, C,
+                                                    H, W, k, s, p, mode, io, gelu, ws ? w.data_ptr() : nullptr, ws, stream(x)),
         "cvb_converse2d_fwd");
   return out;
 }
@@ -137,30 +149,40 @@ void want(Py_ssize_t n, Py_ssize_t m) {
   if (n != m) throw Failed("wrong number of arguments");
 }
 
-// converse2d(x, table, weight_f32, kernel_size, scale, padding, padding_mode, fuse_gelu, out or None)
+// converse2d(x, table, weight_f32, kernel_size, scale, padding, padding_mode, fuse_gelu, out or None, pairs)
 PyObject* py_converse2d(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    want(n, 9);
+    want(n, 10);
     const at::Tensor& x0 = cuda_tensor(a[0], "x");
     if (x0.dim() != 4) throw Failed("x must be (B,C,H,W)");
     const c10::cuda::CUDAGuard dev(x0.device());
     const at::Tensor &table = tensor(a[1], "table"), &wf = tensor(a[2], "weight");
+    const bool pairs = PyObject_IsTrue(a[9]);
     const int k = (int)integer(a[3]), s = (int)integer(a[4]), p = (int)integer(a[5]), mode = pad_mode(a[6]);
     const int gelu = PyObject_IsTrue(a[7]);
     at::Tensor out;
     if (a[8] != Py_None) out = tensor(a[8], "out");
     {
       const Unlocked unlocked;
-      out = forward(x0.is_contiguous() ? x0 : x0.contiguous(), table, wf, k, s, p, mode, gelu, std::move(out));
+      out = forward(x0.is_contiguous() ? x0 : x0.contiguous(), table, wf, k, s, p, mode, gelu, std::move(out), pairs);
     }
     return THPVariable_Wrap(std::move(out));
   });
 }
 
-// build_transfer(weight, bias, scale, eps, h, w, x0_term) -> (table, weight as contiguous fp32 (C,k,k))
+// takes_pairs(B, h, w, scale) -> cvb_takes_pairs
+PyObject* py_takes_pairs(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    want(n, 4);
+    return PyLong_FromLong(api.takes_pairs((int)integer(a[0]), (int)integer(a[1]), (int)integer(a[2]), (int)integer(a[3])));
+  });
+}
+
+// build_transfer(weight, bias, scale, eps, h, w, x0_term, which) -> (table, weight as contiguous fp32 (C,k,k))
+// which: 0 tables for every batch, 1 the pair table, 2 the real-plane table (where there is one; else the pair table)
 PyObject* py_build_transfer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    want(n, 7);
+    want(n, 8);
     const at::Tensor &w = tensor(a[0], "weight"), &b = tensor(a[1], "bias");
     const long s = integer(a[2]), h = integer(a[4]), wd = integer(a[5]);
     if (!w.is_cuda()) throw Failed("Converse2D parameters must live on a CUDA device");
@@ -170,10 +192,18 @@ PyObject* py_build_transfer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (b.dim() != 4 || b.size(0) != 1 || b.size(1) != C || b.size(2) != 1 || b.size(3) != 1)
       throw Failed("bias must be (1,C,1,1)");
     if (s < 1) throw Failed("scale must be >= 1");
-    const size_t bytes = api.transfer_bytes(C, (int)h, (int)wd);
+    const bool x0 = PyObject_IsTrue(a[6]);
+    const long which = integer(a[7]);
+    const size_t plane = api.plane_bytes(C, (int)h, (int)wd);
+    size_t bytes = which == 1 ? api.pair_bytes(C, (int)h, (int)wd) : api.transfer_bytes(C, (int)h, (int)wd);
+    auto fn = which == 1 ? api.build_pair : x0 ? api.build_x0_table : api.build_transfer;
+    // every batch: the real-plane table alone serves the sizes whose blob is no larger than the pair table
+    if (plane && !x0 && which != 1 && (which == 2 || bytes <= api.pair_bytes(C, (int)h, (int)wd))) {
+      bytes = plane;
+      fn = api.build_plane;
+    }
     if (!bytes) throw Failed("padded plane " + std::to_string(h) + "x" + std::to_string(wd) + " is not supported by the FFT engine");
     const c10::cuda::CUDAGuard dev(w.device());
-    auto fn = PyObject_IsTrue(a[6]) ? api.build_x0_table : api.build_transfer;
     const float eps = (float)real(a[3]);
     at::Tensor table, wf;
     {
@@ -307,10 +337,10 @@ PyObject* py_block_pack(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
-// block(x, table, weight_f32, pack, kernel_size, padding, padding_mode, eps1, eps2) -> ConverseBlock.forward(x)
+// block(x, table, weight_f32, pack, kernel_size, padding, padding_mode, eps1, eps2, pairs) -> ConverseBlock.forward(x)
 PyObject* py_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    want(n, 9);
+    want(n, 10);
     const at::Tensor& x0 = cuda_tensor(a[0], "x");
     if (x0.dim() != 4) throw Failed("x must be (B,C,H,W)");
     const c10::cuda::CUDAGuard dev(x0.device());
@@ -318,6 +348,7 @@ PyObject* py_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int B = (int)x0.size(0), C = (int)x0.size(1), H = (int)x0.size(2), W = (int)x0.size(3), io = io_type(x0);
     const int k = (int)integer(a[4]), p = (int)integer(a[5]), mode = pad_mode(a[6]);
     const float eps1 = (float)real(a[7]), eps2 = (float)real(a[8]);
+    const bool pairs = PyObject_IsTrue(a[9]);
     at::Tensor out;
     {
       const Unlocked unlocked;
@@ -326,7 +357,7 @@ PyObject* py_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
       void* st = stream(x);
       at::Tensor t = at::empty({B, 2 * C, H, W}, opt);
       check(api.block_pre(x.data_ptr(), t.data_ptr(), pack.data_ptr(), eps1, B, H * W, io, st), "cvb_block_pre_fwd");
-      t = forward(t, table, wf, k, 1, p, mode, 1, at::Tensor());
+      t = forward(t, table, wf, k, 1, p, mode, 1, at::Tensor(), pairs);
       out = at::empty({B, C, H, W}, opt);
       check(api.block_post(t.data_ptr(), x.data_ptr(), out.data_ptr(), pack.data_ptr(), eps2, B, H * W, io, st),
             "cvb_block_post_fwd");
@@ -435,7 +466,7 @@ PyObject* py_block_train(PyObject*, PyObject* const* a, Py_ssize_t n) {
       x1 = at::empty({B, C, H, W}, opt), z3 = at::empty({B, 2 * C, H, W}, opt), out = at::empty({B, C, H, W}, opt);
       check(api.block_pre_train((const float*)x.data_ptr(), (float*)t1.data_ptr(), (float*)z1.data_ptr(), pack.data_ptr(), eps1,
                                 B, H * W, st), "cvb_block_pre_train");
-      forward(t1, table, wf, k, 1, p, mode, 0, u);
+      forward(t1, table, wf, k, 1, p, mode, 0, u, false);
       check(api.block_post_train((const float*)u.data_ptr(), (const float*)x.data_ptr(), (float*)out.data_ptr(),
                                  (float*)x1.data_ptr(), (float*)z3.data_ptr(), pack.data_ptr(), eps2, B, H * W, st),
             "cvb_block_post_train");
@@ -513,16 +544,17 @@ PyObject* py_block_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // init(address of each C ABI function in the order of `names`)
 PyObject* py_init(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    want(n, 20);
-    void* p[20];
-    for (int i = 0; i < 20; ++i) p[i] = PyLong_AsVoidPtr(a[i]);
+    want(n, 27);
+    void* p[27];
+    for (int i = 0; i < 27; ++i) p[i] = PyLong_AsVoidPtr(a[i]);
     int i = 0;
     auto set = [&](auto& f) { f = (std::decay_t<decltype(f)>)p[i++]; };
     set(api.strerror_); set(api.last_cuda_error); set(api.transfer_bytes); set(api.build_transfer); set(api.build_x0_table);
     set(api.workspace_bytes); set(api.converse2d_fwd); set(api.block_pack_bytes); set(api.block_pack); set(api.block_pre);
     set(api.block_post); set(api.train_workspace_bytes); set(api.fwd_train); set(api.bwd_workspace_bytes); set(api.bwd);
     set(api.block_pre_train); set(api.block_post_train); set(api.block_grad_floats); set(api.block_bwd_workspace);
-    set(api.block_bwd);
+    set(api.block_bwd); set(api.takes_pairs); set(api.plane_bytes); set(api.build_plane); set(api.pair_bytes);
+    set(api.build_pair); set(api.pair_workspace_bytes); set(api.pair_fwd);
     Py_RETURN_NONE;
   });
 }
@@ -530,6 +562,7 @@ PyObject* py_init(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyMethodDef methods[] = {
     {"init", (PyCFunction)(void (*)(void))py_init, METH_FASTCALL, nullptr},
     {"converse2d", (PyCFunction)(void (*)(void))py_converse2d, METH_FASTCALL, nullptr},
+    {"takes_pairs", (PyCFunction)(void (*)(void))py_takes_pairs, METH_FASTCALL, nullptr},
     {"build_transfer", (PyCFunction)(void (*)(void))py_build_transfer, METH_FASTCALL, nullptr},
     {"state", (PyCFunction)(void (*)(void))py_state, METH_FASTCALL, nullptr},
     {"backend", (PyCFunction)(void (*)(void))py_backend, METH_FASTCALL, nullptr},
@@ -549,13 +582,15 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, null
 PyMODINIT_FUNC PyInit__host(void) {
   PyObject* m = PyModule_Create(&module);
   if (!m) return nullptr;
-  PyObject* names = Py_BuildValue("(ssssssssssssssssssss)", "cvb_strerror", "cvb_last_cuda_error", "cvb_transfer_bytes",
+  PyObject* names = Py_BuildValue("(sssssssssssssssssssssssssss)", "cvb_strerror", "cvb_last_cuda_error", "cvb_transfer_bytes",
                                   "cvb_build_transfer", "cvb_build_x0_table", "cvb_converse2d_workspace_bytes",
                                   "cvb_converse2d_fwd", "cvb_block_pack_bytes", "cvb_block_pack", "cvb_block_pre_fwd",
                                   "cvb_block_post_fwd", "cvb_converse2d_train_workspace_bytes",
                                   "cvb_converse2d_fwd_train", "cvb_converse2d_bwd_workspace_bytes", "cvb_converse2d_bwd",
                                   "cvb_block_pre_train", "cvb_block_post_train", "cvb_block_grad_floats",
-                                  "cvb_block_bwd_workspace_bytes", "cvb_block_bwd");
+                                  "cvb_block_bwd_workspace_bytes", "cvb_block_bwd", "cvb_takes_pairs",
+                                  "cvb_plane_transfer_bytes", "cvb_build_plane_transfer", "cvb_pair_transfer_bytes",
+                                  "cvb_build_pair_transfer", "cvb_pair_workspace_bytes", "cvb_pair_fwd");
   if (!names || PyModule_AddObject(m, "names", names) < 0) return nullptr;
   return m;
 }

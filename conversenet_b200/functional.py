@@ -17,21 +17,29 @@ def _io_dtype(t):
     raise RuntimeError("Converse2D supports float32 and bfloat16 tensors, got %s" % t.dtype)
 
 
-def build_transfer(weight, bias, scale, eps, h, w, x0_term=False):
-    """Transfer table for `weight` (1,C,k,k) / `bias` (1,C,1,1) at padded size h x w.
+def takes_pairs(B, h, w, scale):
+    """True when a batch of B runs on the kernels that carry two planes with the same taps as one (`cvb_takes_pairs`)."""
+    return _cabi.host().takes_pairs(int(B), int(h), int(w), int(scale)) != 0
+
+
+def build_transfer(weight, bias, scale, eps, h, w, x0_term=False, batch=None):
+    """Transfer table for `weight` (1,C,k,k) / `bias` (1,C,1,1) at padded size h x w, for every batch size; with `batch`
+    only the table that a batch of that size reads, which `converse2d_forward` is told by `pairs=takes_pairs(batch, ...)`.
     `x0_term`: the real table 1 / (alias mean of |FK|^2 + lambda) that the term of an
     arbitrary `x0` needs (`cvb_build_x0_table`) instead of the operator's multiplier.
 
     Plays the role of the reference's cached kernel spectrum
     (`converse2d.cpp:58-102`), but holds the complete weights-only multiplier.
     Returns a uint8 CUDA tensor owned by the caller."""
-    return _cabi.host().build_transfer(weight, bias, int(scale), float(eps), int(h), int(w), bool(x0_term))
+    which = 0 if batch is None else 1 if takes_pairs(batch, h, w, scale) else 2
+    return _cabi.host().build_transfer(weight, bias, int(scale), float(eps), int(h), int(w), bool(x0_term), which)
 
 
 def converse2d_forward(x, table, weight_f32, kernel_size, scale, padding, padding_mode, fuse_gelu=False,
-                       out=None):
-    """Fused pad -> solve -> crop (`models/util_converse.py:142-192`) on a CUDA tensor."""
-    return _cabi.host().converse2d(x, table, weight_f32, kernel_size, scale, padding, padding_mode, fuse_gelu, out)
+                       out=None, pairs=False):
+    """Fused pad -> solve -> crop (`models/util_converse.py:142-192`) on a CUDA tensor.  `pairs`: `table` is the pair
+    table alone (see `build_transfer`)."""
+    return _cabi.host().converse2d(x, table, weight_f32, kernel_size, scale, padding, padding_mode, fuse_gelu, out, pairs)
 
 
 def build_pair_transfer(weight, bias, eps, h, w):

@@ -52,7 +52,7 @@ class ConvReverseDataNet(nn.Module):
         h, w = H + 2 * padding, W + 2 * padding
         weight = k.reshape(1, B * C, ks, ks)
         bias = self.alpha.expand(B, C, 1, 1).reshape(1, B * C, 1, 1)
-        table, wf = CF.build_transfer(weight, bias, int(sf), self.eps, h, w)
+        table, wf = CF.build_transfer(weight, bias, int(sf), self.eps, h, w, batch=1)
         planes = x.reshape(1, B * C, H, W)
         if torch.is_grad_enabled() and (x.requires_grad or k.requires_grad or self.alpha.requires_grad):
             # differentiable in x, the kernels and alpha, as the reference's torch.fft data step is

@@ -59,10 +59,12 @@ def _forward(x, x0, weight, bias, scale, eps=1e-5):
         ref = x if scale == 1 else F.interpolate(x, scale_factor=scale, mode="nearest")
         if not torch.equal(x0, ref):
             d = (x0 - ref).float()
-    key = (C, h, w, int(scale), float(eps), _cabi.host().state(weight, bias))
-    table, wf = _cache.get(key, (weight, bias), lambda: CF.build_transfer(weight, bias, int(scale), float(eps), h, w))
+    pairs = CF.takes_pairs(B, h, w, scale)
+    key = (C, h, w, int(scale), float(eps), pairs, _cabi.host().state(weight, bias))
+    table, wf = _cache.get(key, (weight, bias), lambda: CF.build_transfer(weight, bias, int(scale), float(eps), h, w,
+                                                                          batch=B))
     # padding 0: the solve on the plane as given, nothing cropped
-    out = CF.converse2d_forward(x, table, wf, weight.size(2), int(scale), 0, "circular")
+    out = CF.converse2d_forward(x, table, wf, weight.size(2), int(scale), 0, "circular", pairs=pairs)
     if d is not None:
         out = out + _x0_term(d, weight, bias, wf, int(scale), float(eps), h, w).to(out.dtype)
     return out

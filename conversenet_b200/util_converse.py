@@ -113,14 +113,17 @@ class Converse2D(nn.Module):
         self._tables = Kept(self._TABLE_SLOTS)      # (also for modules pickled by earlier versions)
 
     # -- transfer-table cache: rebuilt when a parameter is modified in place or replaced
-    def _table_for(self, h, w, device):
+    def _table_for(self, h, w, device, which=0):
+        """(table, weight as fp32) for padded planes h x w: 0 for every batch size; 1 the pair table and 2 the real-plane
+        table alone, built when the first call that reads them comes (where both exist each is 0.5 to 1 times 8 C h w
+        bytes, and a call reads one)."""
         weight, bias = self.weight, self.bias
-        state = _cabi.host().state(weight, bias)
-        key = (h, w, self.scale, self.eps, device.index, state)
+        key = (h, w, self.scale, self.eps, which, _cabi.host().state(weight, bias))
         last = self._tables.last
         if last is not None and last[0] == key:
             return last[1]
-        return self._tables.get(key, (weight, bias), lambda: CF.build_transfer(weight, bias, self.scale, self.eps, h, w))
+        return self._tables.get(key, (weight, bias), lambda: _cabi.host().build_transfer(
+            weight, bias, self.scale, self.eps, h, w, False, which))
 
     @property
     def biaseps(self):
@@ -150,15 +153,19 @@ class Converse2D(nn.Module):
         shape = x.shape
         if len(shape) != 4 or shape[1] != self.in_channels:
             raise RuntimeError("x must be (B,%d,H,W)" % self.in_channels)
-        p = self.padding
-        table, wf = self._table_for(shape[2] + 2 * p, shape[3] + 2 * p, x.device)
+        p, host = self.padding, _cabi.host()
+        h, w = shape[2] + 2 * p, shape[3] + 2 * p
+        pairs = host.takes_pairs(shape[0], h, w, self.scale)
         if torch.is_grad_enabled() and (x.requires_grad or self.weight.requires_grad or self.bias.requires_grad):
             # differentiable route (the reference is differentiable through torch.fft, converse2d.cpp:223)
+            # its gradients read the real-plane table; so does the forward, but for the multi-pass pair kernels
             from .autograd import Converse2DFunction
+            table, wf = self._table_for(h, w, x.device, 0 if pairs == 2 else 2)
             out = Converse2DFunction.apply(x, self.weight, self.bias, table, wf, self.kernel_size, self.scale,
                                            self.padding, self.padding_mode, self.eps)
             return F.gelu(out) if fuse_gelu else out
-        return _cabi.host().converse2d(x, table, wf, self.kernel_size, self.scale, p, self.padding_mode, fuse_gelu, None)
+        table, wf = self._table_for(h, w, x.device, 1 if pairs else 2)
+        return host.converse2d(x, table, wf, self.kernel_size, self.scale, p, self.padding_mode, fuse_gelu, None, pairs)
 
 
 def _with_gelu(conv, x):
@@ -237,10 +244,11 @@ class ConverseBlock(nn.Module):
                 return None
         conv._check_backend()
         pack = self._packed(params)
-        p, eps1, eps2 = conv.padding, c1["0"].eps, c2["0"].eps
-        table, wf = conv._table_for(x.shape[2] + 2 * p, x.shape[3] + 2 * p, x.device)
+        p, eps1, eps2, host = conv.padding, c1["0"].eps, c2["0"].eps, _cabi.host()
+        h, w = x.shape[2] + 2 * p, x.shape[3] + 2 * p
+        table, wf = conv._table_for(h, w, x.device, 0 if host.takes_pairs(x.shape[0], h, w, 1) == 2 else 2)
         x = x.contiguous()
-        kept = _cabi.host().block_train(x, table, wf, pack, conv.kernel_size, p, conv.padding_mode, eps1, eps2)
+        kept = host.block_train(x, table, wf, pack, conv.kernel_size, p, conv.padding_mode, eps1, eps2)
         if kept is None:
             return None
         from .autograd import ConverseBlockFunction
@@ -267,9 +275,11 @@ class ConverseBlock(nn.Module):
         if self.fixed_order and x.dtype == torch.bfloat16:
             return self._forward_fixed_order(x, conv, alpha1, alpha2)
         conv._check_backend()
-        shape, p = x.shape, conv.padding
-        table, wf = conv._table_for(shape[2] + 2 * p, shape[3] + 2 * p, x.device)
-        return _cabi.host().block(x, table, wf, pack, conv.kernel_size, p, conv.padding_mode, c1["0"].eps, c2["0"].eps)
+        shape, p, host = x.shape, conv.padding, _cabi.host()
+        h, w = shape[2] + 2 * p, shape[3] + 2 * p
+        pairs = host.takes_pairs(shape[0], h, w, 1)
+        table, wf = conv._table_for(h, w, x.device, 1 if pairs else 2)
+        return host.block(x, table, wf, pack, conv.kernel_size, p, conv.padding_mode, c1["0"].eps, c2["0"].eps, pairs)
 
     def _forward_fixed_order(self, x, conv, alpha1, alpha2):
         # (see `fixed_order`)

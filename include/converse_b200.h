@@ -138,13 +138,30 @@ int cvb_converse2d_fwd(const void* x, void* out, const void* table, const float*
  * whatever the size and batch, with a table of their own.  cvb_converse2d_fwd takes them where they are the faster ones;
  * called directly they keep their order of sums, on which the outputs of a deep network with bf16 activations depend
  * (its rounding amplifies the last bit of any value).
+ *
+ * cvb_takes_pairs: whether cvb_converse2d_fwd takes them for a batch of B on padded planes h x w at scale s: 0 no; 1 yes,
+ * reading the real-plane table of cvb_build_transfer (cvb_pair_fwd with the pair table is 1.5 to 2 us faster: the table is
+ * in the kernel's own order); 2 yes, reading the pair table that cvb_build_transfer puts behind the real-plane one.
+ * A caller that knows its batch can therefore keep one table where cvb_build_transfer makes two, or the faster one: the
+ * pair table for cvb_pair_fwd where the answer is not 0, else the real-plane table (cvb_plane_*, below) for
+ * cvb_converse2d_fwd.
  */
+int cvb_takes_pairs(int B, int h, int w, int s);
 size_t cvb_pair_transfer_bytes(int C, int h, int w);
 int cvb_build_pair_transfer(const float* weight, const float* bias, int C, int k, int s, int h, int w, float eps,
                             void* table, void* stream);
 size_t cvb_pair_workspace_bytes(int B, int C, int H, int W, int s, int p);
 int cvb_pair_fwd(const void* x, void* out, const void* table, const float* weight, int B, int C, int H, int W, int k, int s,
                  int p, int pad_mode, int io_dtype, int fuse_gelu, void* workspace, size_t workspace_bytes, void* stream);
+
+/*
+ * The real-plane table alone: what cvb_converse2d_fwd reads where cvb_takes_pairs answers 0 or 1, and what the gradients
+ * read.  0 bytes / CVB_ERR_UNSUPPORTED_SIZE when a padded length has no two-stage plan (cvb_build_transfer then makes the
+ * pair table).
+ */
+size_t cvb_plane_transfer_bytes(int C, int h, int w);
+int cvb_build_plane_transfer(const float* weight, const float* bias, int C, int k, int s, int h, int w, float eps,
+                             void* table, void* stream);
 
 /*
  * ConverseBlock, first fused kernel: out = GELU( W . LayerNorm(x) + b ), C -> 2C channels,

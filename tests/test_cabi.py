@@ -76,6 +76,25 @@ def test_argument_validation_without_device(lib):
     assert lib.cvb_transfer_bytes(0, 68, 68) == 0
 
 
+def test_table_sizes(lib):
+    """A blob holds no more than its readers need: the real-plane table (rows 0 .. h/2) alone; the pair table alone where a
+    length has no two-stage plan; both where either may be read."""
+    pair, plane, every = lib.cvb_pair_transfer_bytes, lib.cvb_plane_transfer_bytes, lib.cvb_transfer_bytes
+    for h, w in ((333, 493), (132, 100), (260, 260), (120, 160), (264, 268), (2, 3), (1024, 1024)):
+        assert plane(128, h, w) == every(128, h, w) > 0
+        assert plane(128, h, w) <= 8 * (128 * w * (h // 2 + 1) + 2 * (h + w) + 4 + 4 * 64 * 64)
+    for n in (264, 268, 516, 520):
+        assert every(8, n, n) == (plane(8, n, n) + 255) // 256 * 256 + pair(8, n, n)
+        assert [lib.cvb_takes_pairs(B, n, n, 1) for B in (1, 2, 3, 4, 5, 7)] == [0, 2, 0, 2, 2, 2]
+        assert lib.cvb_takes_pairs(8, n, n, 2) == 0
+    for n in (68, 132, 136):
+        assert every(8, n, n) == pair(8, n, n) > plane(8, n, n) > 0
+        assert [lib.cvb_takes_pairs(B, n, n, 2) for B in (1, 2, 3, 4, 5, 7)] == [0, 1, 0, 1, 1, 1]
+    assert plane(4, 2048, 64) == 0 and every(4, 2048, 64) == pair(4, 2048, 64) > 0
+    one = ctypes.c_void_p(16)
+    assert lib.cvb_build_plane_transfer(one, one, 4, 3, 1, 2048, 64, 1e-5, one, None) == -3
+
+
 def test_module_mirror_cpu_behaviour():
     import torch
     from conversenet_b200 import Converse2D, ConverseBlock, ConverseBlockAlphaVariant

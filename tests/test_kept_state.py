@@ -256,3 +256,35 @@ def test_backend_variable_is_read_at_every_call(monkeypatch):
             else:
                 with pytest.raises(error):
                     m._check_backend()
+
+
+@pytest.mark.gpu
+def test_a_layer_holds_only_the_tables_its_calls_read():
+    from conversenet_b200 import Converse2D, _cabi
+    from conversenet_b200 import functional as CF
+    lib = _cabi.load()
+    torch.manual_seed(14)
+    C, k = 16, 5
+    for n, scale in ((264, 1), (268, 1), (68, 2), (132, 1)):
+        m = Converse2D(C, C, k, scale=scale, padding=2).cuda().eval()
+        H = n - 4
+        x = torch.randn(4, C, H, H, device="cuda")
+        held = lambda: sum(e.value[0].numel() for e in m._tables.entries.values())
+        with torch.no_grad():
+            four = m(x)
+            assert held() == lib.cvb_pair_transfer_bytes(C, n, n)
+            one = m(x[1:2])
+            assert held() == lib.cvb_pair_transfer_bytes(C, n, n) + lib.cvb_plane_transfer_bytes(C, n, n)
+            m(x[:2])
+            assert held() == lib.cvb_pair_transfer_bytes(C, n, n) + lib.cvb_plane_transfer_bytes(C, n, n)
+            # a table for every batch gives the same results
+            table, wf = CF.build_transfer(m.weight, m.bias, scale, m.eps, n, n)
+            every = CF.converse2d_forward(x, table, wf, k, scale, 2, "circular")
+        assert _rel(every, four) <= 2e-6 and _rel(one, four[1:2]) <= 6e-6      # (268: split TF32 products)
+        # a table that a call would read past is refused
+        table, wf = CF.build_transfer(m.weight, m.bias, scale, m.eps, n, n, batch=1)
+        with pytest.raises(RuntimeError):
+            CF.converse2d_forward(x, table, wf, k, scale, 2, "circular", pairs=True)
+        if CF.takes_pairs(4, n, n, scale) and n > 136:
+            with pytest.raises(RuntimeError):
+                CF.converse2d_forward(x, table, wf, k, scale, 2, "circular")
