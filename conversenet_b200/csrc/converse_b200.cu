@@ -142,14 +142,29 @@ static bool needs_strip(int h, int w, int k, bool big) {
 // chunk workspace of the multi-launch real-plane kernels
 constexpr size_t kRpWorkspace = (size_t)64 << 20;
 
-// Planes whose two lengths have a compile-time multi-pass plan that beats the run-time ones on FULL pairs of planes (two
-// images of a batch share their taps and travel as one complex plane) keep the tables of both kernel families:
+// Planes whose two lengths have a multi-pass pair plan that beats the real-plane kernels on FULL pairs of planes (two
+// images of a batch share their taps and travel as one complex plane) have the tables of both kernel families:
 //   tensor-core plans   268 x 268, 8 x 128 planes: 1.01 ms against 1.26;  1 x 128 planes: 0.25 against 0.16
 //   264 and 520         4 x 128 planes of 264 x 264: 280 us against 309, of 520 x 520: 1256 against 1463
-// At scale >= 2 the run-time kernels' epilogue wins (260 x 260 by 2, 4 x 64 planes: 270 us against 596).
+//   dense stages that cost more than the two cheap butterflies of a three-stage plan (16 planes of n x n, one pair per
+//   channel, real-plane kernels / pair kernels): 918 = 102 x 9 1.58, 1071 = 119 x 9 1.66, 1000 = 100 x 10 1.25,
+//   1300 = 100 x 13 1.30, 891 = 81 x 11 1.14; but 1024 = 64 x 16 0.73, 1280 = 80 x 16 0.76, 900 = 60 x 15 0.88,
+//   847 = 77 x 11 0.98.  Only on both axes (1000 x 1024: 1.01, 1000 x 720: 0.82), not with a large prime in the length
+//   (776 = 97 x 8: 0.62), not for single planes (1000 x 1000, batch 1: 0.65)
+// At scale >= 2 the run-time kernels' epilogue wins (260 x 260 by 2, 4 x 64 planes: 270 us against 596; 1071 x 1071 by 2,
+// 2 x 8 planes: 1482 us against 1716).
 static bool strip_axis(int n) { return n == 264 || n == 520; }
+static bool three_stage_axis(int n) {
+  int r0, r1;
+  Plan1D pl;
+  bool big = false;
+  if (n <= 800 || !rp::axis_plan(n, r0, r1)) return false;
+  const int width = rp::matrix_width(r0);
+  return (width >= 56 || (width > 0 && r1 <= 11 && n > 860)) && make_plan(n, pl, &big) && !big;
+}
 static bool dual_tables(int h, int w) {
-  return ((gemm_axis(h) && gemm_axis(w) && !gemm_disabled()) || (strip_axis(h) && strip_axis(w))) && rp::supported(h, w);
+  return ((gemm_axis(h) && gemm_axis(w) && !gemm_disabled()) || (strip_axis(h) && strip_axis(w)) ||
+          (three_stage_axis(h) && three_stage_axis(w))) && rp::supported(h, w);
 }
 static size_t dual_offset(int C, int h, int w) { return (rp::table_bytes(C, h, w) + 255) / 256 * 256; }
 // Compile-time-plan kernels on pairs of planes that share their taps (k_static.cu), for the sizes that have one: with
@@ -164,7 +179,10 @@ static bool full_pairs(int B) { return B >= 2 && (B % 2 == 0 || B >= 5); }
 static bool takes_static_pairs(int B, int h, int w) {
   return full_pairs(B) && !option(CVB_OPT_RUNTIME_PLAN) && !option(CVB_OPT_MULTIPASS) && static_plan(h, w) && rp::supported(h, w);
 }
-static bool takes_multipass_pairs(int B, int h, int w, int s) { return s == 1 && full_pairs(B) && dual_tables(h, w); }
+// (from seven images on where a full pair gains least: 1000 x 1000, 5 x 8 planes: 1755 us against 1661)
+static bool takes_multipass_pairs(int B, int h, int w, int s) {
+  return s == 1 && full_pairs(B) && dual_tables(h, w) && !(B == 5 && three_stage_axis(h));
+}
 
 static int check_padding(int H, int W, int p, int pad_mode) {
   if (p < 0) return CVB_ERR_BAD_ARGUMENT;

@@ -90,6 +90,13 @@ def test_table_sizes(lib):
     for n in (68, 132, 136):
         assert every(8, n, n) == pair(8, n, n) > plane(8, n, n) > 0
         assert [lib.cvb_takes_pairs(B, n, n, 2) for B in (1, 2, 3, 4, 5, 7)] == [0, 1, 0, 1, 1, 1]
+    # lengths whose dense stage costs more than a three-stage plan, on both axes, at scale 1
+    for h, w in ((918, 1071), (1000, 1300), (805, 891), (875, 1254)):
+        assert every(2, h, w) == (plane(2, h, w) + 255) // 256 * 256 + pair(2, h, w)
+        assert [lib.cvb_takes_pairs(B, h, w, 1) for B in (1, 2, 3, 4, 5, 6, 7)] == [0, 2, 0, 2, 0, 2, 2]
+        assert lib.cvb_takes_pairs(2, h, w, 2) == 0
+    for h, w in ((1024, 1024), (1280, 720), (1000, 1024), (960, 1080), (665, 665), (847, 847), (776, 970), (832, 832)):
+        assert lib.cvb_takes_pairs(2, h, w, 1) == 0 and every(2, h, w) == plane(2, h, w)
     assert plane(4, 2048, 64) == 0 and every(4, 2048, 64) == pair(4, 2048, 64) > 0
     one = ctypes.c_void_p(16)
     assert lib.cvb_build_plane_transfer(one, one, 4, 3, 1, 2048, 64, 1e-5, one, None) == -3

@@ -59,6 +59,45 @@ def test_forward_matches_oracle(case):
     assert orc.rel_l2(y, ref) <= (2e-6 if dt == "fp32" else 3e-3)
 
 
+@pytest.mark.parametrize("case", [
+    # lengths above 680: dense stages of 64, 80, 60 and 95 points (real planes), two register radices (832 = 32 * 26)
+    (2, 1, 1022, 130, 3, 1, 1, "circular", "fp32"),
+    (1, 2, 60, 1278, 5, 1, 1, "replicate", "bf16"),
+    (2, 1, 896, 77, 3, 2, 2, "reflect", "fp32"),
+    (1, 1, 1043, 828, 3, 1, 2, "constant", "fp32"),       # 1047 = 3 * 349 is refused
+    (1, 1, 1040, 828, 3, 1, 2, "constant", "fp32"),       # 1044 = 87 * 12
+    (1, 1, 1300, 805, 3, 1, 0, "circular", "fp32"),       # the longest dense axis; alone in its batch
+    # both lengths with a costly dense stage: full pairs take the three-stage plans of the pair kernels
+    (2, 1, 803, 889, 3, 1, 1, "circular", "fp32"),
+    (7, 1, 914, 914, 7, 1, 2, "reflect", "bf16"),         # an odd batch: the last pair holds one plane
+    (2, 1, 874, 1249, 3, 1, 0, "replicate", "fp32"),      # 874 has the prime 23, 1249 is prime: refused
+    (2, 1, 873, 1248, 3, 1, 1, "constant", "fp32"),       # 875 = 7 * 5 * 5 * 5, 1250: four stages
+    (4, 1, 803, 889, 3, 2, 1, "circular", "fp32"),        # scale 2: real planes
+])
+def test_long_axes_match_the_oracle(case):
+    from conversenet_b200 import Converse2D
+    B, C, H, W, k, s, p, mode, dt = case
+    rng = np.random.default_rng(H + W)
+    w, b = orc.init_weight(C, k, rng)
+    dtype = torch.float32 if dt == "fp32" else torch.bfloat16
+    x = torch.from_numpy(rng.standard_normal((B, C, H, W)).astype(np.float32)).to(dtype)
+    m = Converse2D(C, C, k, scale=s, padding=p, padding_mode=mode).cuda().eval()
+    with torch.no_grad():
+        m.weight.copy_(torch.from_numpy(w))
+        m.bias.copy_(torch.from_numpy(b))
+        if H + 2 * p == 1047 or W + 2 * p == 1249:
+            with pytest.raises(RuntimeError):
+                m(x.cuda())
+            return
+        y = m(x.cuda()).float().cpu().numpy()
+        m.fuse_gelu = True
+        gelu = m(x.cuda()).float().cpu()
+    ref = orc.converse2d_forward(x.float().numpy(), w, b, s, p, mode, 1e-5, dtype=np.float64)
+    assert orc.rel_l2(y, ref) <= (2e-6 if dt == "fp32" else 3e-3)
+    want = torch.nn.functional.gelu(torch.from_numpy(ref)).numpy()
+    assert orc.rel_l2(gelu.numpy(), want) <= (4e-6 if dt == "fp32" else 3e-3)
+
+
 def test_chunks_of_the_workspace_agree_with_single_planes():
     # 320 planes of 300 x 260 need several chunks; one plane alone needs one
     from conversenet_b200 import Converse2D
