@@ -105,7 +105,16 @@ inline size_t ws_plane_bytes(int h, int w, int s) {
   return s > 1 ? spec + ((size_t)h * wp * sizeof(float) + 15) / 16 * 16 : spec;
 }
 
-constexpr size_t kPlaneWide = 24 * 1024;   // (132 x 132, 64 planes: 41 us against 21 in three launches)
+// One block per plane (plane_body) or three launches, by the shared memory a plane takes:
+//   more planes than SMs: while three planes share an SM's memory
+//   no more planes than SMs, a block of up to 512 threads each: up to 96 KB; up to 148 KB when the planes occupy two
+//   thirds of the SMs, because the time of the launches grows with the planes and that of the block does not
+// (one block / three launches, us at scale 1, planes per call: 28 x 24, 16 6.4 / 8.8; 76 x 76, 47 KB, 64 13.3 / 18.1,
+// 148 13.5 / 21.6; 108 x 108, 94 KB, 16 13.7 / 14.7, 148 14.1 / 23.9; 132 x 132, 139 KB, 64 20.5 / 17.9, 128 20.6 / 26.9)
+constexpr size_t kPlaneThree = 75 * 1024, kPlaneWide = 96 * 1024, kPlaneMost = 148 * 1024;
+inline size_t one_block_limit(int planes, int sms) {
+  return planes > sms ? kPlaneThree : 3 * planes >= 2 * sms ? kPlaneMost : kPlaneWide;
+}
 
 struct Route {
   bool one_block;       // plane_body, no workspace
@@ -113,8 +122,7 @@ struct Route {
   int chunk;            // multi-launch form: planes per chunk
   size_t ws_bytes;
 };
-// One block per plane while three of them share an SM's memory, or while there are no more planes than SMs and one
-// fits (blocks of up to 512 threads then); else the multi-launch form over chunks of at most ws_cap bytes of workspace.
+// One block per plane up to one_block_limit, else the multi-launch form over chunks of at most ws_cap bytes of workspace.
 inline Route route(int B, int C, int H, int W, int s, int p, int sms, bool force_multi, size_t ws_cap) {
   const int h = H + 2 * p, w = W + 2 * p, planes = B * C;
   Route r;
@@ -122,7 +130,7 @@ inline Route route(int B, int C, int H, int W, int s, int p, int sms, bool force
   int a, b, c, d;
   axis_plan(h, a, b);
   axis_plan(w, c, d);
-  r.one_block = !force_multi && register_radix(a) && register_radix(c) && (planes <= sms ? sm <= kPlaneWide : sm <= 75 * 1024);
+  r.one_block = !force_multi && register_radix(a) && register_radix(c) && sm <= one_block_limit(planes, sms);
   r.threads = 256;
   const size_t per = ws_plane_bytes(h, w, s);
   size_t n = ws_cap / per;

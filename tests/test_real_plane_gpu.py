@@ -98,6 +98,29 @@ def test_long_axes_match_the_oracle(case):
     assert orc.rel_l2(gelu.numpy(), want) <= (4e-6 if dt == "fp32" else 3e-3)
 
 
+@pytest.mark.parametrize("n,planes,s", [
+    (76, 2, 2), (108, 98, 1), (108, 99, 2),          # below 96 KB of shared memory: one block at any count
+    (110, 98, 1), (110, 99, 1), (132, 99, 2),        # above: from two thirds of the SMs on
+    (96, 148, 1), (96, 149, 1), (110, 149, 2),       # one plane more than SMs
+    (136, 148, 1),                                   # the largest that one block takes
+])
+def test_one_block_per_plane_and_three_launches_agree(n, planes, s):
+    """Both sides of the lines between the two forms (148 SMs), and the same call forced through the launches."""
+    from conversenet_b200 import Converse2D, _cabi
+    torch.manual_seed(n + planes)
+    m = Converse2D(planes, planes, 5, scale=s, padding=2).cuda().eval()
+    x = torch.randn(1, planes, n - 4, n - 4, device="cuda")
+    with torch.no_grad():
+        y = m(x)
+        with _cabi.option(_cabi.OPT_MULTIPASS, 1):
+            z = m(x)
+    assert _rel(y, z) <= 1e-6
+    c = planes // 2
+    ref = orc.converse2d_forward(x[:, c:c + 1].cpu().numpy(), m.weight[:, c:c + 1].detach().cpu().numpy(),
+                                 m.bias[:, c:c + 1].detach().cpu().numpy(), s, 2, "circular", 1e-5, dtype=np.float64)
+    assert orc.rel_l2(y[:, c:c + 1].cpu().numpy(), ref) <= 2e-6
+
+
 def test_chunks_of_the_workspace_agree_with_single_planes():
     # 320 planes of 300 x 260 need several chunks; one plane alone needs one
     from conversenet_b200 import Converse2D
