@@ -173,6 +173,16 @@ def grad_params(x, g, weight, bias, scale, padding, padding_mode, eps, table=Non
     return None if out is None else out[1:]
 
 
+def _once_differentiable(backward):
+    """torch's once_differentiable, which a backward without create_graph need not enter (3 us a call)."""
+    guarded = once_differentiable(backward)
+    return lambda ctx, g: guarded(ctx, g) if torch.is_grad_enabled() else backward(ctx, g)
+
+
+def _as(t, like):
+    return t if t is None or t.dtype == like.dtype else t.to(like.dtype)
+
+
 class Converse2DFunction(torch.autograd.Function):
     """Native forward and gradients; `grad_input_composed` and `spectral_forward` for planes the gradient kernels do
     not take.  Everything the backward reads is a saved tensor: released by it, and seen by saved-tensor hooks and
@@ -192,22 +202,20 @@ class Converse2DFunction(torch.autograd.Function):
         return out
 
     @staticmethod
-    @once_differentiable
+    @_once_differentiable
     def backward(ctx, g):
         x, weight, bias, table, r = ctx.saved_tensors
         k, s, p, mode, eps = ctx.cfg
-        want_x = ctx.needs_input_grad[0]
-        want_p = ctx.needs_input_grad[1] or ctx.needs_input_grad[2]
-        gx = gw = gb = None
+        want_x, want_w, want_b = ctx.needs_input_grad[:3]
+        want_p = want_w or want_b
+        gx = gw = gb = out = None
         native_p = want_p and NATIVE_PARAM_GRADS and (s == 1 or r is not None)
-        out = None
         if want_x or native_p:
-            out = _cabi.host().backward(x, g, r, table, weight, bias, tuple(x.shape), s, p, mode, eps, want_x,
-                                        native_p)
+            native = _cabi.host().backward
+            out = native(x, g, r, table, weight, bias, x.shape, s, p, mode, eps, want_x, native_p)
             if out is None and native_p and want_x:      # perhaps dL/dx alone
                 native_p = False
-                out = _cabi.host().backward(None, g, None, table, weight, bias, tuple(x.shape), s, p, mode, eps, True,
-                                            False)
+                out = native(None, g, None, table, weight, bias, x.shape, s, p, mode, eps, True, False)
         if out is not None:
             gx, gw, gb = out
         elif want_x:
@@ -218,11 +226,8 @@ class Converse2DFunction(torch.autograd.Function):
                 b_ = bias.detach().float().requires_grad_(True)
                 y = spectral_forward(x.detach().float(), w_, b_, s, p, mode, eps)
                 gw, gb = torch.autograd.grad(y, (w_, b_), g.float())
-        if gx is not None:
-            gx = gx.to(x.dtype)
-        gw = gw.to(weight.dtype) if gw is not None and ctx.needs_input_grad[1] else None
-        gb = gb.to(bias.dtype) if gb is not None and ctx.needs_input_grad[2] else None
-        return gx, gw, gb, None, None, None, None, None, None, None
+        return (_as(gx, x), _as(gw, weight) if want_w else None, _as(gb, bias) if want_b else None, None, None, None, None,
+                None, None, None)
 
 
 class ConverseBlockFunction(torch.autograd.Function):
@@ -238,7 +243,7 @@ class ConverseBlockFunction(torch.autograd.Function):
         return out
 
     @staticmethod
-    @once_differentiable
+    @_once_differentiable
     def backward(ctx, g):
         x, t1, z1, u, x1, z3, table, conv_w, conv_b, *params = ctx.saved_tensors
         eps1, eps2, conv_eps, p, mode = ctx.cfg

@@ -266,12 +266,31 @@ bool capturing(cudaStream_t st) {
   return s != cudaStreamCaptureStatusNone;
 }
 
+// Events that no Ready holds any more, at most kSpareEvents a device; the interpreter's lock guards them.  (Training lays its
+// tables out at every step: making and destroying an event each time takes 1 us.)
+constexpr size_t kSpareEvents = 32;
+std::vector<cudaEvent_t>& spare_events(int device) {
+  static std::vector<cudaEvent_t> spare[64];
+  return spare[device & 63];
+}
 // What a kept value needs beside itself: an event behind the work that makes it, and the storages whose addresses name it
 struct Ready {
+  int device;
   cudaEvent_t event = nullptr;
   std::vector<c10::Storage> pins;
+  explicit Ready(int d) : device(d) {
+    auto& spare = spare_events(device);
+    if (spare.empty()) {
+      cuda(cudaEventCreateWithFlags(&event, cudaEventDisableTiming), "cudaEventCreate");
+    } else {
+      event = spare.back();
+      spare.pop_back();
+    }
+  }
   ~Ready() {
-    if (event) cudaEventDestroy(event);
+    auto& spare = spare_events(device);
+    if (spare.size() < kSpareEvents) spare.push_back(event);
+    else cudaEventDestroy(event);
   }
 };
 
@@ -284,10 +303,9 @@ PyObject* py_ready(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const c10::cuda::CUDAGuard dev(t.device());
     const cudaStream_t st = (cudaStream_t)stream(t);
     if (capturing(st)) Py_RETURN_NONE;
-    auto r = std::make_unique<Ready>();
+    auto r = std::make_unique<Ready>((int)t.device().index());
     for (Py_ssize_t i = 1; i < n; ++i)
       if (a[i] != Py_None) r->pins.push_back(tensor(a[i], "parameter").storage());
-    cuda(cudaEventCreateWithFlags(&r->event, cudaEventDisableTiming), "cudaEventCreate");
     cuda(cudaEventRecord(r->event, st), "cudaEventRecord");
     PyObject* o = PyCapsule_New(r.get(), "cvb.ready", [](PyObject* c) { delete (Ready*)PyCapsule_GetPointer(c, "cvb.ready"); });
     if (o) r.release();

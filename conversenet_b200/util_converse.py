@@ -10,6 +10,7 @@ import torch.nn.functional as F
 
 from . import _cabi, functional as CF
 from ._kept import Kept
+from .autograd import Converse2DFunction, ConverseBlockFunction
 
 
 # False: ConverseBlock runs its layers one by one (PyTorch LayerNorm / 1x1 / GELU around the native
@@ -159,7 +160,6 @@ class Converse2D(nn.Module):
         if torch.is_grad_enabled() and (x.requires_grad or self.weight.requires_grad or self.bias.requires_grad):
             # differentiable route (the reference is differentiable through torch.fft, converse2d.cpp:223)
             # its gradients read the real-plane table; so does the forward, but for the multi-pass pair kernels
-            from .autograd import Converse2DFunction
             table, wf = self._table_for(h, w, x.device, 0 if pairs == 2 else 2)
             out = Converse2DFunction.apply(x, self.weight, self.bias, table, wf, self.kernel_size, self.scale,
                                            self.padding, self.padding_mode, self.eps)
@@ -251,7 +251,6 @@ class ConverseBlock(nn.Module):
         kept = host.block_train(x, table, wf, pack, conv.kernel_size, p, conv.padding_mode, eps1, eps2)
         if kept is None:
             return None
-        from .autograd import ConverseBlockFunction
         return ConverseBlockFunction.apply(kept, x, conv.weight, conv.bias, table,
                                            (eps1, eps2, conv.eps, p, conv.padding_mode), *params)
 
