@@ -20,7 +20,6 @@ __device__ __forceinline__ void pdl_start() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
@@ -64,7 +63,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 }
 #else
 inline void pdl_start() {}
-inline void pdl_wait() {}
 inline uint32_t smem_u32(const void*) { return 0; }
 inline void mbar_init(uint64_t*, int) {}
 inline void mbar_fence_init() {}

@@ -137,7 +137,7 @@ int cvb_converse2d_fwd(const void* x, void* out, const void* table, const float*
  * The same operator on the kernels that carry two planes with the same taps (two images of a batch) as one complex plane,
  * whatever the size and batch, with a table of their own.  cvb_converse2d_fwd takes them where they are the faster ones;
  * called directly they keep their order of sums, on which the outputs of a deep network with bf16 activations depend
- * (its rounding amplifies the last bit of any value).
+ * (its rounding amplifies the last bit of any value; neither order is the more accurate one by design).
  *
  * cvb_takes_pairs: whether cvb_converse2d_fwd takes them for a batch of B on padded planes h x w at scale s: 0 no; 1 yes,
  * reading the real-plane table of cvb_build_transfer (cvb_pair_fwd with the pair table is 1.5 to 2 us faster: the table is
