@@ -57,7 +57,7 @@ CONFIGS = {
 
 
 LARGE = {
-    # planes that take the multi-pass path (workspace): layers of the three benchmark networks, batch reduced
+    # planes that take several launches (workspace): layers of the three benchmark networks, batch reduced
     "dncnn_body_268": dict(B=2, C=8, H=256, W=256, k=7, s=1, p=6, mode="circular", eps=1e-5),
     "srres_264": dict(B=2, C=6, H=256, W=256, k=5, s=1, p=4, mode="replicate", eps=1e-5),
     "srres_up2_260": dict(B=2, C=4, H=256, W=256, k=2, s=2, p=2, mode="replicate", eps=1e-3),
@@ -65,8 +65,8 @@ LARGE = {
     "usrnet_block_516": dict(B=1, C=4, H=512, W=512, k=3, s=1, p=2, mode="circular", eps=1e-5),
     "usrnet_data_512": dict(B=2, C=2, H=512, W=512, k=7, s=1, p=0, mode="circular", eps=1e-3),
     "odd_rect_prime": dict(B=3, C=3, H=83, W=55, k=3, s=3, p=2, mode="reflect", eps=1e-5),  # 87 x 59
-    # 268 = 67 * 4: the 67-point stage on the tensor cores; with the upsampling epilogue (halo columns in
-    # the 16-line tiles, odd plane count), and mixed with a register-radix axis both ways round
+    # 268 = 67 * 4, on the pair kernels the 67-point stage on the tensor cores: with the upsampling epilogue (halo columns
+    # in the 16-line tiles, odd plane count), and mixed with a register-radix axis both ways round
     "tc_268_up2": dict(B=3, C=3, H=264, W=264, k=3, s=2, p=2, mode="replicate", eps=1e-5),
     "tc_268x264": dict(B=2, C=5, H=256, W=252, k=7, s=1, p=6, mode="circular", eps=1e-5),
     "tc_264x268": dict(B=1, C=6, H=252, W=256, k=5, s=1, p=6, mode="reflect", eps=1e-5),
@@ -80,6 +80,19 @@ def test_large_planes_multi_pass(name):
     out = _run(x, w, b, cfg["s"], cfg["p"], cfg["mode"], cfg["eps"])
     ref64 = orc.converse2d_forward(x, w, b, cfg["s"], cfg["p"], cfg["mode"], cfg["eps"], dtype=np.float64)
     assert orc.rel_l2(out, ref64) <= TOL_FP32
+
+
+@pytest.mark.parametrize("name", list(LARGE))
+def test_large_planes_pair_kernels(name):
+    """The same planes on the pair kernels, which the call above takes for few of them."""
+    from conversenet_b200 import _cabi
+    from tests.test_gemmdft_gpu import run_pair_kernels
+    cfg = LARGE[name]
+    x, w, b = _seeded(cfg, 4)
+    out = run_pair_kernels(cfg, x, w, b)
+    ref64 = orc.converse2d_forward(x, w, b, cfg["s"], cfg["p"], cfg["mode"], cfg["eps"], dtype=np.float64)
+    assert orc.rel_l2(out, ref64) <= TOL_FP32
+    assert _cabi.load().cvb_last_device_status(1) == 0
 
 
 def test_tensor_core_stage_bf16_io_and_status_word():
