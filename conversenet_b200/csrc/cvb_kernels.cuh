@@ -248,11 +248,12 @@ enum {
   PASS_MID = 8,         // last row stage: butterfly, transfer multiply, conjugate, butterfly
   PASS_CONJ_OUT = 16,   // negate the imaginary part on the way out
   PASS_SRC_WS = 32,     // read the complex elements from a global workspace (io.ws, strides wes / wls)
-  PASS_DST_WS = 64      // write them to the workspace instead of shared memory
+  PASS_DST_WS = 64,     // write them to the workspace instead of shared memory
+  PASS_HALF = 128       // PASS_MID on the real-plane table (FwdParams::hh); compile-time flag
 };
 
 // Transfer-table values of work item wi of a PASS_MID stage (same index arithmetic as fft_pass).
-template <int R, int CN, int CL, int CM, int CNL>
+template <int R, int CN, int CL, int CM, int CNL, bool HALF>
 CVB_HD void mid_table_load(const PassArgs& a, const IoArgs& io, int wi, float2 (&g)[R]) {
   int t, line;
   if constexpr (CNL != 0) {
@@ -261,27 +262,25 @@ CVB_HD void mid_table_load(const PassArgs& a, const IoArgs& io, int wi, float2 (
   } else {
     divmod_small(wi, a.nlines, a.inv_nlines, t, line);
   }
-  if constexpr (CN != 0) {
-    if (io.hh) {
-      // The real-plane table (any-batch blobs, training): half as large, but the index of a mirrored row costs the stage
-      // 1.3 us of 37.6 (16 x 64 planes of 68 x 68 upsampled by 2), so calls that know their batch bring the pair table.
-      // lanes are consecutive positions: RY1 runs of consecutive frequencies, so natural order stays coalesced
-      int k0, j;
-      divmod_small(line, io.ry1, io.inv_ry1, k0, j);
-      const int u = k0 + io.ry0 * j;
-      const bool mir = 2 * u > io.h;
-      const int step = (CN / R) * io.hh;
-      const float2* tp = io.tab + (mir ? (CN - t) * io.hh + (io.h - u) : t * io.hh + u);
-      const float sy = mir ? -2.f : 2.f;       // the stored multiplier carries a factor 1 / 2
+  if constexpr (HALF) {
+    // lanes are consecutive positions: RY1 runs of consecutive frequencies, so natural order stays coalesced.
+    // The real-plane table (any-batch blobs, training): half as large, but the index of a mirrored row costs the stage
+    // 1.3 us of 37.6 (16 x 64 planes of 68 x 68 upsampled by 2), so calls that know their batch bring the pair table.
+    int k0, j;
+    divmod_small(line, io.ry1, io.inv_ry1, k0, j);
+    const int u = k0 + io.ry0 * j;
+    const bool mir = 2 * u > io.h;
+    const int step = (CN / R) * io.hh;
+    const float2* tp = io.tab + (mir ? (CN - t) * io.hh + (io.h - u) : t * io.hh + u);
+    const float sy = mir ? -2.f : 2.f;       // the stored multiplier carries a factor 1 / 2
 #pragma unroll
-      for (int p = 0; p < R; ++p) {
-        // frequency t + (CN / R) p, mirrored CN - that; frequency 0 is its own mirror
-        const float2* q = mir ? tp - p * step : tp + p * step;
-        const float2 z = *(p == 0 && mir && t == 0 ? q - CN * io.hh : q);
-        g[p] = make_float2(2.f * z.x, sy * z.y);
-      }
-      return;
+    for (int p = 0; p < R; ++p) {
+      // frequency t + (CN / R) p, mirrored CN - that; frequency 0 is its own mirror
+      const float2* q = mir ? tp - p * step : tp + p * step;
+      const float2 z = *(p == 0 && mir && t == 0 ? q - CN * io.hh : q);
+      g[p] = make_float2(2.f * z.x, sy * z.y);
     }
+    return;
   }
   const int tes = a.tab ? a.tab_es : io.h;
   const float2* tp = a.tab ? a.tab + (t * R) * a.tab_es + line * a.tab_ls
@@ -304,9 +303,10 @@ CVB_HD void fft_pass(int tid, int nthr, const PassArgs& a, const IoArgs& io, int
   const float osign = (flags & PASS_CONJ_OUT) ? -1.0f : 1.0f;
   const bool twiddle = aM > 1;
   constexpr bool kMidStatic = CFLAGS >= 0 && (CFLAGS & PASS_MID) != 0;
+  constexpr bool kHalf = kMidStatic && (CFLAGS & PASS_HALF) != 0;
   float2 gtab[kMidStatic ? R : 1], gnext[kMidStatic ? R : 1];
   if constexpr (kMidStatic) {
-    if (tid < total) mid_table_load<R, CN, CL, CM, CNL>(a, io, tid, gnext);
+    if (tid < total) mid_table_load<R, CN, CL, CM, CNL, kHalf>(a, io, tid, gnext);
   }
   for (int wi = tid; wi < total; wi += nthr) {
     int t, line, blk, j;
@@ -336,7 +336,7 @@ CVB_HD void fft_pass(int tid, int nthr, const PassArgs& a, const IoArgs& io, int
 #pragma unroll
       for (int p = 0; p < R; ++p) gtab[p] = gnext[p];
       const int wn = wi + nthr;
-      if (wn < total) mid_table_load<R, CN, CL, CM, CNL>(a, io, wn, gnext);
+      if (wn < total) mid_table_load<R, CN, CL, CM, CNL, kHalf>(a, io, wn, gnext);
     }
 
     if (flags & PASS_SRC_GLOBAL) {
@@ -1097,7 +1097,8 @@ __host__ __device__ inline void smem_block_xspec(const XspecParams& Q, int c, in
 // The seven FFT stages and the epilogue of one plane pair, every stage compiled with
 // its own flags.  `io.xa/xb` may point to global memory or to a staged copy in shared
 // memory; the stage code is the same.
-template <typename IO, int RY0, int RY1, int RX0, int RX1, int NT>
+// HALF: `table` is the real-plane table (P.hh set), and r may be kept (training).
+template <typename IO, int RY0, int RY1, int RX0, int RX1, int NT, bool HALF>
 CVB_HD void static_stages(const FwdParams& P, const IoArgs& io, float2* plane, const float2* twy,
                           const float2* twx, const float* wk) {
   constexpr int h = RY0 * RY1, w = RX0 * RX1;
@@ -1110,7 +1111,7 @@ CVB_HD void static_stages(const FwdParams& P, const IoArgs& io, float2* plane, c
   if (!(sk & 2)) CVB_PHASE_CT((fft_pass<RY0, IO, h, h, RY1, w, PASS_SRC_GLOBAL>(tid, nthr, ay0, io, 0)));
   if (!(sk & 4)) CVB_PHASE_CT((fft_pass<RY1, IO, h, RY1, 1, w, 0>(tid, nthr, ay1, io, 0)));
   if (!(sk & 8)) CVB_PHASE_CT((fft_pass<RX0, IO, w, w, RX1, h, 0>(tid, nthr, ax0, io, 0)));
-  if (!(sk & 16)) CVB_PHASE_CT((fft_pass<RX1, IO, w, RX1, 1, h, PASS_MID>(tid, nthr, ax1, io, 0)));
+  if (!(sk & 16)) CVB_PHASE_CT((fft_pass<RX1, IO, w, RX1, 1, h, PASS_MID | (HALF ? PASS_HALF : 0)>(tid, nthr, ax1, io, 0)));
   if (!(sk & 32)) CVB_PHASE_CT((fft_pass<RX0, IO, w, w, RX1, h, PASS_PRE>(tid, nthr, ax0, io, 0)));
   if (!(sk & 64)) CVB_PHASE_CT((fft_pass<RY1, IO, h, RY1, 1, w, PASS_PRE>(tid, nthr, ay1, io, 0)));
   if (!(sk & 128)) {
@@ -1120,7 +1121,7 @@ CVB_HD void static_stages(const FwdParams& P, const IoArgs& io, float2* plane, c
       CVB_PHASE_CT((fft_pass<RY0, IO, h, h, RY1, w, PASS_PRE | PASS_CONJ_OUT>(tid, nthr, ay0, io, 0)));
     }
   }
-  if (P.s != 1 && P.rsave) {
+  if (HALF && P.s != 1 && P.rsave) {
     // io.oa / ob are the planes' outputs: their numbers place the copies of r
     constexpr int wp = (w + 1) / 2 * 2;
     const size_t out_plane = (size_t)P.H * P.W * P.s * P.s;
@@ -1139,7 +1140,7 @@ CVB_HD void static_stages(const FwdParams& P, const IoArgs& io, float2* plane, c
 }
 
 // One block = one plane pair.
-template <typename IO, int RY0, int RY1, int RX0, int RX1, int NT>
+template <typename IO, int RY0, int RY1, int RX0, int RX1, int NT, bool HALF = false>
 __host__ __device__ void smem_block_static(const FwdParams& P, int pair, float2* smem) {
   constexpr int h = RY0 * RY1, w = RX0 * RX1;
   constexpr int pitch = w | 1;
@@ -1157,7 +1158,7 @@ __host__ __device__ void smem_block_static(const FwdParams& P, int pair, float2*
   io.cmap = maps + h;
   if (P.ystash) { io.ycopy = (float2*)maps + lay.maps; io.yoff = (int)(io.ycopy - plane); }
   CVB_PHASE_CT(load_tables(tid, nthr, P, c, twy, twx, wk, maps));
-  static_stages<IO, RY0, RY1, RX0, RX1, NT>(P, io, plane, twy, twx, wk);
+  static_stages<IO, RY0, RY1, RX0, RX1, NT, HALF>(P, io, plane, twy, twx, wk);
 }
 
 // Persistent variant: a block loops over plane pairs (pair = block, block + nblocks, ...).
@@ -1185,7 +1186,7 @@ CVB_HD void persistent_issue(const FwdParams& P, int pair, IO* dst, uint64_t* ba
   if (pb >= 0) bulk_g2s(dst + HW, (const IO*)P.x + (size_t)pb * HW, bytes, bar);
 }
 
-template <typename IO, int RY0, int RY1, int RX0, int RX1, int NT>
+template <typename IO, int RY0, int RY1, int RX0, int RX1, int NT, bool HALF = false>
 __host__ __device__ void smem_persistent_static(const FwdParams& P, unsigned char* smem, int block, int nblocks) {
   constexpr int h = RY0 * RY1, w = RX0 * RX1;
   constexpr int pitch = w | 1;
@@ -1250,7 +1251,7 @@ __host__ __device__ void smem_persistent_static(const FwdParams& P, unsigned cha
     if (P.s > 1)
       for (int i = 0; i < P.k * P.k; ++i) wk[i] = P.weight[(size_t)c * P.k * P.k + i];
 #endif
-    static_stages<IO, RY0, RY1, RX0, RX1, NT>(P, io, plane, twy, twx, wk);
+    static_stages<IO, RY0, RY1, RX0, RX1, NT, HALF>(P, io, plane, twy, twx, wk);
   }
 }
 

@@ -14,23 +14,24 @@ namespace cvb {
 
 // The radices are template parameters so that every registry line gets its own
 // kernel symbol: this file is compiled several times into one library.
-template <typename IO, int RY0, int RY1, int RX0, int RX1, int NT, int MB>
+template <typename IO, int RY0, int RY1, int RX0, int RX1, int NT, int MB, bool HALF>
 __global__ void __launch_bounds__(NT, MB) smem_static_kernel(const FwdParams P) {
   extern __shared__ float2 smem[];
   pdl_start();
-  smem_block_static<IO, RY0, RY1, RX0, RX1, NT>(P, blockIdx.x, smem);
+  smem_block_static<IO, RY0, RY1, RX0, RX1, NT, HALF>(P, blockIdx.x, smem);
 }
 
-template <typename IO, int RY0, int RY1, int RX0, int RX1, int NT, int MB>
+template <typename IO, int RY0, int RY1, int RX0, int RX1, int NT, int MB, bool HALF>
 __global__ void __launch_bounds__(NT, MB) smem_persistent_kernel(const FwdParams P) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  smem_persistent_static<IO, RY0, RY1, RX0, RX1, NT>(P, smem_raw, blockIdx.x, gridDim.x);
+  smem_persistent_static<IO, RY0, RY1, RX0, RX1, NT, HALF>(P, smem_raw, blockIdx.x, gridDim.x);
 }
 
 namespace {
 template <typename IO>
 int launch_t(const FwdParams& P, size_t smem, cudaStream_t st) {
-  auto kernel = smem_static_kernel<IO, CVB_RY0, CVB_RY1, CVB_RX0, CVB_RX1, CVB_NT, CVB_MB>;
+  auto kernel = P.hh ? smem_static_kernel<IO, CVB_RY0, CVB_RY1, CVB_RX0, CVB_RX1, CVB_NT, CVB_MB, true>
+                     : smem_static_kernel<IO, CVB_RY0, CVB_RY1, CVB_RX0, CVB_RX1, CVB_NT, CVB_MB, false>;
   const int rc = allow_smem(kernel, smem);
   // (the block size is baked into the index arithmetic)
   return rc != CVB_OK ? rc : launch_chained(kernel, dim3(num_pairs(P)), CVB_NT, smem, st, P);
@@ -38,7 +39,8 @@ int launch_t(const FwdParams& P, size_t smem, cudaStream_t st) {
 
 template <typename IO>
 int launch_p(const FwdParams& P, size_t smem, int blocks, cudaStream_t st) {
-  auto kernel = smem_persistent_kernel<IO, CVB_RY0, CVB_RY1, CVB_RX0, CVB_RX1, CVB_NT, CVB_MB>;
+  auto kernel = P.hh ? smem_persistent_kernel<IO, CVB_RY0, CVB_RY1, CVB_RX0, CVB_RX1, CVB_NT, CVB_MB, true>
+                     : smem_persistent_kernel<IO, CVB_RY0, CVB_RY1, CVB_RX0, CVB_RX1, CVB_NT, CVB_MB, false>;
   CVB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kernel<<<blocks, CVB_NT, smem, st>>>(P);
   CVB_CUDA(cudaGetLastError());
