@@ -29,14 +29,15 @@ STATIC_PLANS = [
 
 # Compile-time axis plans of the register-FFT multi-pass path: (R0, R1, S0, S1); axis length R0*R1, and
 # for a large prime R0 the Rader sub-plan R0-1 = S0*S1 (else 0, 0).  268 = 67 * 4 (ConverseDnCNN) is
-# served by the tensor-core multi-pass kernels (GEMM_PLANS) instead.
+# served by the tensor-core multi-pass kernels (GEMM_PLANS) instead.  Reached by full pairs of 264 and 520 planes, and by
+# every size through cvb_pair_fwd (bf16 networks: 260 is ConverseDnCNN at 248 x 248).
 STRIP2_PLANS = [
     (22, 12, 0, 0),   # 264  SRResNet 256+8
     (20, 13, 0, 0),   # 260  SRResNet up2 256+4
     (26, 20, 0, 0),   # 520  SRResNet 512+8
     (43, 12, 7, 6),   # 516  USRNet blocks 512+4
-    (17, 8, 0, 0),    # 136  (also reachable with CVB_FORCE_STRIP)
-    (17, 4, 0, 0),    # 68
+    (17, 8, 0, 0),    # 136  (cvb_pair_fwd with CVB_OPT_MULTIPASS)
+    (17, 4, 0, 0),    # 68   (likewise)
 ]
 
 # First factor R0 of the tensor-core multi-pass plans (padded length 4 * R0, both axes of a plane):

@@ -131,7 +131,10 @@ __device__ __forceinline__ void twiddle(float (&re)[R], float (&im)[R], const fl
 // a_k = x_0 + sum_q cos(2 pi q k / R) p_q,  b_k = sum_q sin(2 pi q k / R) m_q.  One thread keeps the p (or the m) of a
 // vector in registers and runs over the k: two FMAs per (k, q), the cosines four at a time from shared memory.  Element
 // k then holds a_k and element R - k holds b_k (matrix_value puts them together), so that the two threads of a vector
-// never have to meet.  FMA-bound by construction: about R FMAs per point.
+// never have to meet.  About R FMAs per point; a 16-byte read of cosines (four cycles of the shared-memory port a warp)
+// feeds eight of them a thread (two cycles of the FMA pipes), so the port is the nearer limit of the two.  Neither is
+// reached: 1 x 128 planes of 268 x 268 keep the port below half busy, the FMA pipes a third and the issue slots a half, at
+// 15 warps an SM (128 registers), waiting for memory.
 template <int MP, class Base>
 __device__ __forceinline__ void matrix_stage(int R, int nvec, int stride, const float* mats, Base base) {
   const int tid = threadIdx.x, half = blockDim.x >> 1;

@@ -244,7 +244,7 @@ int cvb_block_bwd(const cvb_block_bwd_args* args);
  * Converse2D forward for callers that cannot allocate device memory.
  *
  * Same arguments, result and error codes as cvb_converse2d_fwd, minus the workspace:
- * the multi-pass kernels run with their scratch in a fixed array inside the library
+ * the kernels of several launches run with their scratch in a fixed array inside the library
  * (CVB_STATIC_SCRATCH_BYTES, held by every GPU that loads the library until the process
  * ends).  Meant for code that runs where an allocator call is impossible or unwelcome:
  * a plug-in that owns nothing but its input and output buffers, a region whose memory
@@ -254,11 +254,8 @@ int cvb_block_bwd(const cvb_block_bwd_args* args);
  *   - Limit: one padded plane pair, 8*(H+2p)*(W+2p) bytes, must fit the array
  *     (about 1440 x 1440); larger planes return CVB_ERR_TOO_LARGE.
  *   - Set-up on first use: the first call on each device looks up the device addresses
- *     of the array and of the status word (runtime queries, no allocation), and the
- *     first call per device that meets a padded length with a large prime factor (268,
- *     for instance) also runs one small kernel that fills a constant table inside the
- *     library and waits for it on `stream` (cudaStreamSynchronize).  Make those first
- *     calls outside any stream capture.
+ *     of the array and of the status word (runtime queries, no allocation).  Make it
+ *     outside any stream capture.
  *   - A bounded wait that gives up inside a kernel is reported through
  *     cvb_last_device_status, as for cvb_converse2d_fwd.
  *   - All calls share the one array and it keeps the previous call's contents.  Nothing
