@@ -1,0 +1,152 @@
+"""Host emulation of the real-plane kernels (tests/emu/emu_rp.cpp) against the oracle: their index arithmetic, barriers,
+shuffles, alignment and buffer bounds, without a GPU, at sizes where they can go wrong."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import converse2d_oracle as orc
+from tests.emu.build_emu import build_emu_rp
+
+PAD = {"circular": 0, "replicate": 1, "reflect": 2, "constant": 3}
+SMS = 148
+
+
+@pytest.fixture(scope="module")
+def emu():
+    lib = ctypes.CDLL(build_emu_rp())
+    lib.emu_rp_message.restype = ctypes.c_char_p
+    return lib
+
+
+def _ptr(a):
+    return None if a is None else a.ctypes.data_as(ctypes.c_void_p)
+
+
+def _check(lib, rc):
+    assert rc == 0, (rc, lib.emu_rp_message())
+
+
+def _weights(C, k, seed):
+    rng = np.random.default_rng(seed)
+    w, b = orc.init_weight(C, k, rng)
+    return w, (b + rng.standard_normal(b.shape)).astype(np.float32), rng
+
+
+def _forward(lib, x, w, b, s, p, mode, gelu=0, multi=0, ws_planes=0, keep=False):
+    """x: float32, or uint16 holding bf16"""
+    B, C, H, W = x.shape
+    k, bf16 = w.shape[-1], x.dtype == np.uint16
+    out = np.zeros((B, C, H * s, W * s), x.dtype)
+    h, wp = H + 2 * p, (W + 2 * p + 1) // 2 * 2
+    r = np.zeros((B, C, h, wp), np.float32) if keep else None
+    wf = np.ascontiguousarray(w.reshape(C, k, k), np.float32)
+    _check(lib, lib.emu_rp_forward(_ptr(x), _ptr(out), _ptr(r), _ptr(wf), _ptr(np.ascontiguousarray(b.reshape(C))), B, C, H, W, k,
+                                   s, p, PAD[mode], ctypes.c_float(1e-5), gelu, int(bf16), multi, ws_planes, SMS))
+    return (out, r) if keep else out
+
+
+CASES = [
+    # B, C, H, W, k, s, p, mode
+    (1, 1, 2, 3, 1, 1, 0, "circular"),            # the smallest axes
+    (1, 3, 29, 32, 3, 1, 0, "circular"),          # the largest register radices, one stage
+    (2, 2, 20, 17, 5, 1, 2, "replicate"),         # 24 x 21: odd width, an unpaired column
+    (1, 2, 30, 26, 3, 1, 3, "reflect"),
+    (1, 1, 22, 23, 3, 1, 2, "constant"),          # 26 x 27: zero margins
+    (1, 2, 33, 37, 3, 1, 0, "circular"),          # dense stages of both parities
+    (1, 1, 43, 47, 3, 1, 0, "replicate"),
+    (1, 1, 51, 61, 3, 1, 0, "circular"),
+    (1, 1, 67, 74, 3, 1, 0, "circular"),          # 74 = 37 x 2
+    (1, 1, 79, 86, 3, 1, 0, "reflect"),
+    (1, 1, 111, 53, 3, 1, 1, "circular"),         # 113
+    (1, 1, 53, 125, 3, 1, 1, "constant"),         # 127
+    (2, 2, 16, 14, 5, 2, 2, "circular"),          # upsampling: every window, runs and bands
+    (1, 2, 13, 15, 3, 3, 1, "reflect"),
+    (1, 1, 10, 12, 7, 4, 3, "replicate"),
+    (1, 1, 9, 11, 4, 2, 2, "constant"),           # a tap count without a compile-time epilogue
+    (1, 1, 33, 35, 3, 2, 1, "circular"),          # dense stages with the epilogue
+]
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_forward_matches_the_oracle(emu, case):
+    B, C, H, W, k, s, p, mode = case
+    w, b, rng = _weights(C, k, H * 100 + W)
+    x = rng.standard_normal((B, C, H, W)).astype(np.float32)
+    ref = orc.converse2d_forward(x, w, b, s, p, mode, 1e-5, dtype=np.float64)
+    outs = [_forward(emu, x, w, b, s, p, mode), _forward(emu, x, w, b, s, p, mode, multi=1, ws_planes=1 if B * C > 1 else 0)]
+    for out in outs:
+        assert orc.rel_l2(out, ref) <= 2e-6
+    gelu = _forward(emu, x, w, b, s, p, mode, gelu=1)
+    assert orc.rel_l2(gelu, torch.nn.functional.gelu(torch.from_numpy(ref)).numpy()) <= 4e-6
+
+
+@pytest.mark.parametrize("case", [(1, 2, 20, 18, 3, 1, 2, "circular"), (1, 1, 21, 15, 5, 1, 2, "constant"),
+                                  (1, 1, 49, 28, 3, 1, 0, "circular"), (1, 2, 11, 14, 3, 3, 1, "reflect"),
+                                  (1, 2, 12, 10, 5, 2, 2, "replicate")])
+def test_bf16_tensors(emu, case):
+    B, C, H, W, k, s, p, mode = case
+    w, b, rng = _weights(C, k, H + W)
+    x = torch.from_numpy(rng.standard_normal((B, C, H, W)).astype(np.float32)).bfloat16()
+    ref = orc.converse2d_forward(x.float().numpy(), w, b, s, p, mode, 1e-5, dtype=np.float64)
+    bits = x.view(torch.int16).numpy().view(np.uint16)
+    for multi in (0, 1):
+        out = _forward(emu, bits, w, b, s, p, mode, multi=multi)
+        got = torch.from_numpy(out.view(np.int16)).view(torch.bfloat16).float().numpy()
+        assert orc.rel_l2(got, ref) <= 3e-3
+
+
+@pytest.mark.parametrize("case", [
+    (2, 2, 14, 17, 3, 1, 3, "replicate"),
+    (3, 1, 20, 15, 5, 1, 2, "reflect"),
+    (2, 1, 12, 12, 3, 1, 8, "circular"),        # margins almost as wide as the plane
+    (2, 2, 10, 14, 5, 2, 2, "circular"),
+    (2, 1, 9, 12, 7, 3, 3, "reflect"),
+    (1, 2, 8, 7, 3, 4, 1, "constant"),
+    (2, 1, 8, 9, 4, 3, 2, "replicate"),         # run-time taps and scale
+    (2, 1, 14, 39, 3, 1, 1, "circular"),        # 41: dense stage along x
+])
+def test_gradient_kernels_match_fp64_autograd(emu, case):
+    from conversenet_b200.autograd import spectral_forward
+    B, C, H, W, k, s, p, mode = case
+    w, b, rng = _weights(C, k, H * W)
+    x = rng.standard_normal((B, C, H, W)).astype(np.float32)
+    g = rng.standard_normal((B, C, H * s, W * s)).astype(np.float32)
+    out, r = _forward(emu, x, w, b, s, p, mode, keep=True)
+    h, wd = H + 2 * p, W + 2 * p
+    nseg, hh = (2 if B > 1 else 1), h // 2 + 1
+    gx, D, taps = np.zeros_like(x), np.zeros((C, wd, hh, 2), np.float32), np.zeros((B, C, k, k), np.float32)
+    wf, bf = np.ascontiguousarray(w.reshape(C, k, k)), np.ascontiguousarray(b.reshape(C))
+    _check(emu, emu.emu_rp_backward(_ptr(x), _ptr(g), _ptr(r), _ptr(gx), _ptr(D), _ptr(taps), _ptr(wf), _ptr(bf), B, C, H, W, k, s,
+                                    p, PAD[mode], ctypes.c_float(1e-5), nseg, SMS))
+    X, Wt, Bt = (torch.from_numpy(a).double().requires_grad_(True) for a in (x, w, b))
+    y = spectral_forward(X, Wt, Bt, s, p, mode, 1e-5)
+    ref, = torch.autograd.grad(y, X, torch.from_numpy(g).double())
+    assert orc.rel_l2(gx, ref.numpy()) <= 2e-6
+    # D = 4 sum_b FFT2(pad(x_b)) conj(FFT2(q_b)): q is the extended cotangent, at scale >= 2 its strided correlation
+    from conversenet_b200.autograd import _Cotangent, _pad
+    cot = _Cotangent(torch.from_numpy(g), torch.from_numpy(wf), k, s, p)
+    q = (cot.g_full if s == 1 else cot.v).double()
+    d = (torch.fft.fft2(_pad(torch.from_numpy(x).double(), p, mode)) * torch.fft.fft2(q).conj()).sum(0)[:, :hh]
+    got = torch.view_as_complex(torch.from_numpy(D).double()).transpose(1, 2) / 4
+    assert float((got - d).abs().pow(2).sum().sqrt() / d.abs().pow(2).sum().sqrt()) <= 2e-6
+    if s > 1:
+        full, rr = cot.g_full.double(), torch.from_numpy(r[..., :wd]).double()
+        for a in range(k):
+            for c in range(k):
+                moved = torch.roll(full, (a - k // 2, c - k // 2), (-2, -1))[..., ::s, ::s]
+                assert orc.rel_l2(taps[:, :, a, c], (moved * rr).sum((-2, -1)).numpy()) <= 2e-5
+
+
+def test_routes_and_shared_memory(emu):
+    one = lambda n, planes: emu.emu_rp_one_block(1, planes, n, n, 1, 0, SMS)
+    assert [one(76, 64), one(108, 1), one(110, 98), one(110, 99), one(132, 99), one(132, 64)] == [1, 1, 0, 1, 1, 0]
+    assert [one(96, 149), one(98, 149), one(136, 148), one(140, 148), one(74, 10)] == [1, 0, 1, 0, 0]     # 74: dense stage
+    r0, r1 = ctypes.c_int(), ctypes.c_int()
+    for n in range(2, 1400):
+        width = emu.emu_rp_plan(n, ctypes.byref(r0), ctypes.byref(r1))
+        if width < 0:
+            continue
+        assert r0.value * r1.value == n and r0.value <= 127 and r1.value <= 26 and (width == 0 or r1.value <= 16)
+        assert emu.emu_rp_fits(n, n, 1, SMS) == 1 and emu.emu_rp_fits(n, n, 1000, SMS) == 1
