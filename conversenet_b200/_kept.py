@@ -36,6 +36,11 @@ class Kept:
     def __deepcopy__(self, memo):
         return Kept(self.slots)
 
+    def values(self):
+        """Every value kept now (a captured graph holds on to those that its kernels read)."""
+        with _LOCK:
+            return [e.value for e in self.entries.values()] + ([] if self.last is None else [self.last[1]])
+
     def clear(self):
         with _LOCK:
             self.entries.clear()

@@ -85,7 +85,7 @@ def cross_spectrum(x, q, table, padding, padding_mode):
 
     x (B,C,H,W), q (B,C,h,w) with h = H + 2*padding: the batch reduction behind dL/dweight and
     dL/dbias (the reference leaves it to autograd through `torch.fft`, `converse2d.cpp:223`).
-    `table`: a transfer table of the same (C,h,w) (its twiddle tables are used)."""
+    `table`: a transfer table of the same (C,h,w) (its twiddle tables are used); not the pair table alone."""
     lib = _cabi.load()
     if not (x.is_cuda and q.is_cuda):
         raise RuntimeError("cross_spectrum needs CUDA tensors; this build has no CPU path")

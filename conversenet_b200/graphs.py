@@ -5,10 +5,12 @@ and at one image the host needs longer to enqueue them than the GPU needs to run
 captures one forward (this package's kernels, PyTorch's few 1x1 convolutions and copies, and the
 allocations between them) in a CUDA graph with static input and output buffers and replays it: one
 launch per forward.  Inference only (no autograd); tensor shapes, dtypes and the non-tensor arguments
-are fixed at capture time; the parameters are read at replay time, but a transfer table is rebuilt only
-on a new capture, so re-capture after changing a Converse2D weight.  The reference has no counterpart
+are fixed at capture time; transfer tables and packed block weights are those of the capture (the graph holds
+them), so re-capture after changing a parameter.  The reference has no counterpart
 (its scripts run eager PyTorch, `main_test_converse_dncnn.py:133-136`)."""
 import torch
+
+from ._kept import Kept
 
 
 class GraphedForward:
@@ -29,6 +31,9 @@ class GraphedForward:
         self.graph = torch.cuda.CUDAGraph()
         with torch.no_grad(), torch.cuda.graph(self.graph):
             self.static_out = net(*self.static_args)
+        # The captured kernels read the tables and packed weights that the modules keep now; the modules drop them when
+        # other sizes or parameters come, the graph must not.
+        self._held = [k.values() for m in net.modules() for k in vars(m).values() if isinstance(k, Kept)]
 
     def __call__(self, *args):
         """Copy the tensor arguments into the static buffers, replay, return the static output

@@ -257,7 +257,9 @@ def test_registered_torch_op_matches_reference_contract(golden):
 
 
 @pytest.mark.parametrize("shape,k,s", [((2, 3, 20, 26), 5, 2), ((1, 4, 32, 32), 3, 1), ((2, 2, 18, 24), 2, 2),
-                                       ((1, 2, 24, 15), 5, 3)])
+                                       ((1, 2, 24, 15), 5, 3),
+                                       # pairs of planes: compile-time and multi-pass kernels, with tables of their own
+                                       ((2, 1, 68, 68), 5, 2), ((2, 1, 264, 264), 3, 1), ((2, 1, 268, 268), 3, 1)])
 def test_registered_torch_op_with_an_arbitrary_x0(shape, k, s):
     """The raw operator with an x0 that is NOT the upsampled input (`converse2d.cpp:165,193`; this is what
     `test/test_error.py:30` builds): checked against the oracle's closed-form solve."""

@@ -136,7 +136,9 @@ def test_gradient_kernels_match_fp64_autograd(emu, case):
         for a in range(k):
             for c in range(k):
                 moved = torch.roll(full, (a - k // 2, c - k // 2), (-2, -1))[..., ::s, ::s]
-                assert orc.rel_l2(taps[:, :, a, c], (moved * rr).sum((-2, -1)).numpy()) <= 2e-5
+                want, most = (moved * rr).sum((-2, -1)), moved.norm(dim=(-2, -1)) * rr.norm(dim=(-2, -1))
+                # r itself is within 1e-6 of its norm; a sum that cancels has no relative error to speak of
+                assert bool((torch.from_numpy(taps[:, :, a, c]).double() - want).abs().le(2e-6 * most).all())
 
 
 def test_routes_and_shared_memory(emu):

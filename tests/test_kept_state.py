@@ -288,3 +288,24 @@ def test_a_layer_holds_only_the_tables_its_calls_read():
         if CF.takes_pairs(4, n, n, scale) and n > 136:
             with pytest.raises(RuntimeError):
                 CF.converse2d_forward(x, table, wf, k, scale, 2, "circular")
+
+
+@pytest.mark.gpu
+def test_a_captured_graph_holds_the_tables_it_reads():
+    from conversenet_b200 import ConverseBlock
+    from conversenet_b200.graphs import GraphedForward
+    torch.manual_seed(15)
+    blk = ConverseBlock(64, 64, 3, 1, 1).cuda().eval()
+    x = torch.randn(1, 64, 30, 22, device="cuda")
+    ref = _block_step(blk, x)
+    g = GraphedForward(blk, x)
+    for n in range(12):                  # more sizes than a layer keeps tables for, then new versions of all weights
+        _block_step(blk, torch.randn(1, 64, 12 + n, 16, device="cuda"))
+    with torch.no_grad():
+        for q in blk.parameters():
+            q.add_(1.0)
+    _block_step(blk, x)
+    filler = [torch.full((1 << 20,), float("nan"), device="cuda") for _ in range(16)]
+    filler += [torch.full((n,), float("nan"), device="cuda") for n in (1 << 10, 1 << 14, 50000, 1 << 17) for _ in range(32)]
+    assert torch.equal(g(x), ref)
+    del filler
