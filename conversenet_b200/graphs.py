@@ -1,8 +1,8 @@
 """CUDA-graph replay of a network's forward.
 
-A Converse network at a small batch is launch-bound: ConverseDnCNN issues about 520 kernels per forward,
-and at one image the host needs longer to enqueue them than the GPU needs to run them.  `GraphedForward`
-captures one forward (this package's kernels, PyTorch's few 1x1 convolutions and copies, and the
+A forward is many launches: ConverseDnCNN issues about 100 kernels on one 256 x 256 image and 700 on eight
+(chunks of the multi-pass kernels), and on small images the host needs longer to enqueue them than the GPU
+needs to run them.  `GraphedForward` captures one forward (this package's kernels, PyTorch's few 1x1 convolutions and copies, and the
 allocations between them) in a CUDA graph with static input and output buffers and replays it: one
 launch per forward.  Inference only (no autograd); tensor shapes, dtypes and the non-tensor arguments
 are fixed at capture time; transfer tables and packed block weights are those of the capture (the graph holds

@@ -238,7 +238,7 @@ def test_a_call_that_waits_for_the_launch_queue_lets_other_threads_run():
         t.join()
         torch.cuda.synchronize()
     assert waited > 0.4                       # the queue did fill
-    assert max(gaps) < 0.3 * waited
+    assert sum(g for g in gaps if g > 0.05) < 0.5 * waited
 
 
 def test_backend_variable_is_read_at_every_call(monkeypatch):
