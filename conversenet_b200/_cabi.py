@@ -58,6 +58,9 @@ SIGNATURES = {
                                             _c.c_int, _c.c_float, _c.c_void_p, _c.c_void_p]),
     "cvb_pair_workspace_bytes": (_c.c_size_t, [_c.c_int] * 6),
     "cvb_pair_fwd": (_c.c_int, [_c.c_void_p] * 4 + [_c.c_int] * 10 + [_c.c_void_p, _c.c_size_t, _c.c_void_p]),
+    "cvb_takes_planes": (_c.c_int, [_c.c_int] * 5),
+    "cvb_plane_workspace_bytes": (_c.c_size_t, [_c.c_int] * 6),
+    "cvb_plane_fwd": (_c.c_int, [_c.c_void_p] * 4 + [_c.c_int] * 10 + [_c.c_void_p, _c.c_size_t, _c.c_void_p]),
     "cvb_plan_radices": (_c.c_int, [_c.c_int, _c.POINTER(_c.c_int), _c.c_int]),
     "cvb_fits_shared": (_c.c_int, [_c.c_int, _c.c_int]),
     "cvb_cross_spectrum": (_c.c_int, [_c.c_void_p] * 4 + [_c.c_int] * 7 + [_c.c_void_p]),

@@ -89,7 +89,7 @@ def _units():
     units = [("converse_b200", "converse_b200.cu", []), ("k_dynamic", "k_dynamic.cu", []),
              ("k_strip", "k_strip.cu", []), ("k_block", "k_block.cu", []), ("k_block_tc", "k_block_tc.cu", []), ("k_block_tc2", "k_block_tc2.cu", []),
              ("k_block_tc3", "k_block_tc3.cu", []), ("k_block_mlp", "k_block_mlp.cu", []), ("k_block_train", "k_block_train.cu", [])]
-    units += [("k_rp", "k_rp.cu", []), ("k_rp_rows", "k_rp_rows.cu", []), ("k_rp_bwd", "k_rp_bwd.cu", [])]
+    units += [("k_rp", "k_rp.cu", []), ("k_rp_rows", "k_rp_rows.cu", []), ("k_rp_bwd", "k_rp_bwd.cu", []), ("k_fix", "k_fix.cu", [])]
     for name, io in (("f32", "float"), ("bf16", "__nv_bfloat16")):
         for unit in ("k_rp_cols", "k_rp_plane"):
             units.append(("%s_%s" % (unit, name), unit + ".cu", ["-DCVB_IO=" + io, "-DCVB_IO_NAME=" + name]))

@@ -44,7 +44,7 @@ static const StaticEntry kStatic[] = {
 
 // Device word set by a kernel whose bounded wait gave up (one per device).
 __device__ int g_device_status;
-static int* status_ptr() {
+int* status_ptr() {
   static int* ptrs[64] = {nullptr};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
@@ -144,7 +144,7 @@ constexpr size_t kRpWorkspace = (size_t)64 << 20;
 
 // Planes whose two lengths have a multi-pass pair plan that beats the real-plane kernels on FULL pairs of planes (two
 // images of a batch share their taps and travel as one complex plane) have the tables of both kernel families:
-//   tensor-core plans   268 x 268, 8 x 128 planes: 1.01 ms against 1.26;  1 x 128 planes: 0.25 against 0.16
+//   tensor-core plans   268 and 516 (but see takes_contractions)
 //   264 and 520         4 x 128 planes of 264 x 264: 280 us against 309, of 520 x 520: 1256 against 1463
 //   dense stages that cost more than the two cheap butterflies of a three-stage plan (16 planes of n x n, one pair per
 //   channel, real-plane kernels / pair kernels): 918 = 102 x 9 1.58, 1071 = 119 x 9 1.66, 1000 = 100 x 10 1.25,
@@ -182,6 +182,13 @@ static bool takes_static_pairs(int B, int h, int w) {
 // (from seven images on where a full pair gains least: 1000 x 1000, 5 x 8 planes: 1755 us against 1661)
 static bool takes_multipass_pairs(int B, int h, int w, int s) {
   return s == 1 && full_pairs(B) && dual_tables(h, w) && !(B == 5 && three_stage_axis(h));
+}
+// Of those, the ones whose real planes are faster all the same when the caller has the table for them: 268 x 268, whose
+// 67-point stages run as integer contractions (cvb_fix.cuh): 8 x 128 planes 956 us against 1063, 2 x 128 255 against 276,
+// with a tenth of the rounding error.  From 128 planes on: smaller batches keep the one table that they always had.
+static bool takes_contractions(int B, int C, int h, int w, int s) {
+  return takes_multipass_pairs(B, h, w, s) && gemm_axis(h) && gemm_axis(w) && rp::fix_length(h) && rp::fix_length(w) &&
+         (long long)B * C >= 128;
 }
 
 static int check_padding(int H, int W, int p, int pad_mode) {
@@ -395,18 +402,40 @@ int cvb_pair_fwd(const void* x, void* out, const void* table, const float* weigh
                       workspace_bytes, (cudaStream_t)stream);
 }
 
+static rp::Route plane_route(int B, int C, int H, int W, int s, int p) {
+  return rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0,
+                   std::max(kRpWorkspace, rp::ws_plane_bytes(H + 2 * p, W + 2 * p, s)));
+}
+
 size_t cvb_converse2d_workspace_bytes(int B, int C, int H, int W, int s, int p, int io_dtype) {
   (void)io_dtype;
   if (B < 1 || C < 1 || H < 1 || W < 1 || p < 0 || s < 1) return 0;
   const int h = H + 2 * p, w = W + 2 * p;
   if (takes_static_pairs(B, h, w)) return 0;
   if (rp::supported(h, w) && !takes_multipass_pairs(B, h, w, s))
-    return rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0, std::max(kRpWorkspace, rp::ws_plane_bytes(h, w, s))).ws_bytes;
+    return plane_route(B, C, H, W, s, p).ws_bytes;
   return pair_workspace(B, C, h, w, s);
 }
 size_t cvb_pair_workspace_bytes(int B, int C, int H, int W, int s, int p) {
   if (B < 1 || C < 1 || H < 1 || W < 1 || p < 0 || s < 1) return 0;
   return pair_workspace(B, C, H + 2 * p, W + 2 * p, s);
+}
+
+int cvb_takes_planes(int B, int C, int h, int w, int s) {
+  return B > 0 && C > 0 && h > 1 && w > 1 && s > 0 && takes_contractions(B, C, h, w, s) ? 1 : 0;
+}
+size_t cvb_plane_workspace_bytes(int B, int C, int H, int W, int s, int p) {
+  if (B < 1 || C < 1 || H < 1 || W < 1 || p < 0 || s < 1 || !rp::supported(H + 2 * p, W + 2 * p)) return 0;
+  return plane_route(B, C, H, W, s, p).ws_bytes;
+}
+int cvb_plane_fwd(const void* x, void* out, const void* table, const float* weight, int B, int C, int H, int W, int k, int s,
+                  int p, int pad_mode, int io_dtype, int fuse_gelu, void* workspace, size_t workspace_bytes, void* stream) {
+  const int rc = check_forward(x, out, table, weight, B, C, H, W, k, s, p, pad_mode, io_dtype);
+  if (rc != CVB_OK) return rc;
+  rp::Params Q;
+  if (!rp::fill_params(Q, table, B, C, H, W, k, s, p, pad_mode)) return CVB_ERR_UNSUPPORTED_SIZE;
+  Q.x = x; Q.out = out; Q.weight = weight; Q.gelu = fuse_gelu ? 1 : 0;
+  return rp::run(Q, plane_route(B, C, H, W, s, p), io_dtype, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 int cvb_converse2d_fwd(const void* x, void* out, const void* table, const float* weight, int B,
@@ -423,9 +452,7 @@ int cvb_converse2d_fwd(const void* x, void* out, const void* table, const float*
     hh = h / 2 + 1;
   } else if (rp::fill_params(Q, table, B, C, H, W, k, s, p, pad_mode)) {
     Q.x = x; Q.out = out; Q.weight = weight; Q.gelu = fuse_gelu ? 1 : 0;
-    const rp::Route r = rp::route(B, C, H, W, s, p, sm_count(), option(CVB_OPT_MULTIPASS) != 0,
-                                  std::max(kRpWorkspace, rp::ws_plane_bytes(h, w, s)));
-    return rp::run(Q, r, io_dtype, workspace, workspace_bytes, (cudaStream_t)stream);
+    return rp::run(Q, plane_route(B, C, H, W, s, p), io_dtype, workspace, workspace_bytes, (cudaStream_t)stream);
   }
   return pair_forward(x, out, table, weight, B, C, H, W, k, s, p, pad_mode, io_dtype, fuse_gelu, hh, workspace,
                       workspace_bytes, (cudaStream_t)stream);

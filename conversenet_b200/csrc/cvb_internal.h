@@ -49,6 +49,7 @@ int env_int(const char* name, int dflt);
 // Process-wide routing options (cvb_set_option / cvb_get_option in the C ABI).
 int option(int which);
 int sm_count();  // multiprocessors of the current device
+int* status_ptr();  // the current device's status word (null: cannot be had)
 
 // Number of (channel, batch-pair) work items = blocks of the shared-memory kernels.
 inline int num_pairs(const FwdParams& P) { return P.C * ((P.B + 1) / 2); }

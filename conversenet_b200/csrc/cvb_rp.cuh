@@ -35,6 +35,7 @@ struct Axis {
   float inv_r1;
   const float2* tw;     // twiddles in position order: [k0 r1 + j] = (cos, sin)(2 pi k0 j / n)
   const float* dm;      // matrix stage: cos(2 pi q k / R0) as [k = 0 .. R0/2][q = 1 .. mp], then sin likewise
+  const unsigned char* fix;   // operand of the integer contractions (cvb_fix.cuh), or null
 };
 
 struct Params {
@@ -53,6 +54,7 @@ struct Params {
   float* rsave;         // scale >= 2: all planes' r kept for the backward ([B C][h][wp]), or null
   int pitch;            // rows kernel / plane kernel: odd row pitch (complex) of the shared-memory rows
   float inv_wc, inv_hh;
+  int* status;          // device word set non-zero when a bounded wait gives up; may be null
   Axis ay, ax;
 };
 

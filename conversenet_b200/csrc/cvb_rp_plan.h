@@ -1,7 +1,7 @@
 // Host side of the real-plane kernels (cvb_rp.cuh): axis plans, table layout, launch geometry.  Allocates nothing.
 #pragma once
 #include "cvb_plan.h"
-#include "cvb_rp.cuh"
+#include "cvb_fix.cuh"
 
 namespace cvb {
 namespace rp {
@@ -34,11 +34,14 @@ inline bool supported(int h, int w) {
   return h >= 2 && w >= 2 && axis_plan(h, a, b) && axis_plan(w, a, b);
 }
 
+// Axes that carry an operand for the integer contractions
+inline bool fix_axis(int n, int r0) { return fix_length(n) && matrix_width(r0) > 0; }
+
 inline int matrix_entries(int r0) { return 2 * (r0 / 2 + 1) * matrix_width(r0); }   // floats, a multiple of 8
 
 // Blob in float2 units: multiplier [C][w][hh]; twiddles of h and of w in natural order (tw), then in position order
-// (twy, twx); matrix rows of R0(h) and of R0(w)
-struct Blob { size_t tw, twy, twx, dmy, dmx, total; };
+// (twy, twx); matrix rows of R0(h) and of R0(w); operands of the integer contractions along h and w
+struct Blob { size_t tw, twy, twx, dmy, dmx, fixy, fixx, total; };
 inline Blob blob_layout(int C, int h, int w, int r0y, int r0x) {
   Blob b;
   b.tw = (size_t)C * w * (h / 2 + 1);
@@ -46,7 +49,9 @@ inline Blob blob_layout(int C, int h, int w, int r0y, int r0x) {
   b.twx = (b.twy + h + 1) & ~(size_t)1;
   b.dmy = (b.twx + w + 1) & ~(size_t)1;
   b.dmx = b.dmy + matrix_entries(r0y) / 2;
-  b.total = b.dmx + matrix_entries(r0x) / 2;
+  b.fixy = (b.dmx + matrix_entries(r0x) / 2 + 1) & ~(size_t)1;
+  b.fixx = b.fixy + (fix_axis(h, r0y) ? fix_bytes(h) / 8 : 0);
+  b.total = b.fixx + (fix_axis(w, r0x) ? fix_bytes(w) / 8 : 0);
   return b;
 }
 
@@ -54,7 +59,7 @@ inline void fill_axis(Axis& a, int n, int r0, int r1, const float2* tw, const fl
   a.n = n; a.r0 = r0; a.r1 = r1;
   a.mp = matrix_width(r0);
   a.inv_r1 = 1.0f / (float)r1;
-  a.tw = tw; a.dm = (const float*)dm;
+  a.tw = tw; a.dm = (const float*)dm; a.fix = nullptr;
 }
 
 inline size_t cols_smem(const Params& P) {
@@ -93,9 +98,26 @@ inline bool fill_params(Params& P, const void* table, int B, int C, int H, int W
   P.inv_wc = 1.0f / (float)P.wc; P.inv_hh = 1.0f / (float)P.hh;
   fill_axis(P.ay, h, r0y, r1y, t + bl.twy, t + bl.dmy);
   fill_axis(P.ax, w, r0x, r1x, t + bl.twx, t + bl.dmx);
+  if (fix_axis(h, r0y)) P.ay.fix = (const unsigned char*)(t + bl.fixy);
+  if (fix_axis(w, r0x)) P.ax.fix = (const unsigned char*)(t + bl.fixx);
+  P.status = nullptr;
   P.gelu = 0; P.conj = 0; P.plane0 = 0; P.nplane = 0; P.vec = 0; P.vec_out = 0; P.po = p; P.OH = H; P.OW = W; P.rsave = nullptr;
   P.ws = nullptr; P.r = nullptr; P.x = nullptr; P.out = nullptr; P.weight = nullptr;
   return true;
+}
+
+// Strip kernels (kFixFwd, kFixRows, kFixInv) that run as integer contractions (cvb_fix.cuh): along axes that would need a
+// matrix stage, from the number of lines on that gives 55 of 100 SMs a tile (a launch takes as long with fewer).  Matrix
+// stage / contractions on all three kernels, us, planes of N x N: 244 48 planes (91 tiles) 70.7 / 51.9, 32 planes 43.6 / 50.6;
+// 80 planes (153 tiles, two rounds) 112 / 93; 128 planes of 268 155 / 125, 218 157 / 94, 178 122 / 74, 134 49.4 / 38.5; 64
+// planes of 134 (67 tiles) 34.9 / 38.4.  Wide matrix stages (R0 > 88) lose to any number of lines: 8 planes of 202 54.8 / 47.
+// The narrowest (R0 = 37, 41) keep the rows below 240: 128 planes of 164 64.4 with the columns alone, 71.7 with all three;
+// 246 105 / 101.  Register radices stay: 128 planes of 264 79 / 124.
+inline bool takes_fix(const Params& P, int kind, int sms) {
+  const Axis& a = kind == kFixRows ? P.ax : P.ay;
+  if (!a.fix || (kind == kFixRows && a.mp <= 20 && a.n < 240)) return false;
+  const long long tiles = (fix_lines(kind, P) + kFixLines - 1) / kFixLines;
+  return a.mp >= 56 || 100 * tiles >= 55 * (long long)sms;
 }
 
 // Bytes of workspace one plane takes in the multi-launch form
@@ -135,7 +157,22 @@ inline Route route(int B, int C, int H, int W, int s, int p, int sms, bool force
   const size_t per = ws_plane_bytes(h, w, s);
   size_t n = ws_cap / per;
   if (n > (size_t)planes) n = planes;
-  if (n > 0) n = (planes + (planes + n - 1) / n - 1) / ((planes + n - 1) / n);   // chunks of equal size
+  if (n > 0) {                            // chunks of equal size, as many as
+    const int least = (planes + (int)n - 1) / (int)n;
+    const bool fy = fix_axis(h, a), fx = fix_axis(w, c);
+    // rounds of tiles that the integer contractions take for m planes: 4 x 128 planes of 268 x 268, 512 us in four chunks
+    // (two rounds a kernel each), 561 in three (2.4, that is three)
+    auto rounds = [&](int m) {
+      auto of = [&](long long lines) { return (int)((lines + (long long)kFixLines * sms - 1) / ((long long)kFixLines * sms)); };
+      return (fy ? 2 * of((long long)m * (w + 1)) : 0) + (fx ? 2 * of(2LL * m * (h / 2 + 1)) : 0);
+    };
+    int best = least, most = 0x7fffffff;
+    for (int q = least; q < least + 4 && (q == least || ((fy || fx) && q <= planes)); ++q) {
+      const int m = (planes + q - 1) / q, whole = planes / m, total = whole * rounds(m) + (planes % m ? rounds(planes % m) : 0);
+      if (total < most) { most = total; best = q; }
+    }
+    n = (planes + best - 1) / best;
+  }
   r.chunk = (int)n;
   r.ws_bytes = r.one_block ? 0 : n * per;
   return r;

@@ -51,6 +51,9 @@ struct Api {
   decltype(&cvb_build_pair_transfer) build_pair = nullptr;
   decltype(&cvb_pair_workspace_bytes) pair_workspace_bytes = nullptr;
   decltype(&cvb_pair_fwd) pair_fwd = nullptr;
+  decltype(&cvb_takes_planes) takes_planes = nullptr;
+  decltype(&cvb_plane_workspace_bytes) plane_workspace_bytes = nullptr;
+  decltype(&cvb_plane_fwd) plane_fwd = nullptr;
 } api;
 
 struct Failed : std::runtime_error { using std::runtime_error::runtime_error; };
@@ -108,18 +111,21 @@ at::Tensor f32(const at::Tensor& t) {
 }
 
 // `pairs`: `table` is the pair table and the pair kernels run; else the table of build_transfer for any batch, or the
-// real-plane one
+// real-plane one (both begin with what cvb_plane_fwd reads)
 at::Tensor forward(const at::Tensor& x, const at::Tensor& table, const at::Tensor& wf, int k, int s, int p, int mode,
                    int gelu, at::Tensor out, bool pairs) {
   const int B = (int)x.size(0), C = (int)x.size(1), H = (int)x.size(2), W = (int)x.size(3), io = io_type(x);
   if (!out.defined()) out = at::empty({B, C, (int64_t)H * s, (int64_t)W * s}, x.options().requires_grad(false));
   const size_t full = sizeof(float) * 2 * (size_t)C * (H + 2 * p) * (W + 2 * p);   // below that: no pair table in it
-  if ((size_t)table.numel() < full && (pairs || api.takes_pairs(B, H + 2 * p, W + 2 * p, s) == 2))
+  const bool planes = !pairs && api.takes_planes(B, C, H + 2 * p, W + 2 * p, s);
+  if ((size_t)table.numel() < full && !planes && (pairs || api.takes_pairs(B, H + 2 * p, W + 2 * p, s) == 2))
     throw Failed("the transfer table was built for another batch size");
-  const size_t ws = pairs ? api.pair_workspace_bytes(B, C, H, W, s, p) : api.workspace_bytes(B, C, H, W, s, p, io);
+  const size_t ws = pairs    ? api.pair_workspace_bytes(B, C, H, W, s, p)
+                    : planes ? api.plane_workspace_bytes(B, C, H, W, s, p)
+                             : api.workspace_bytes(B, C, H, W, s, p, io);
   at::Tensor w;
   if (ws) w = bytes_like(x, ws);
-  check((pairs ? api.pair_fwd : api.converse2d_fwd)(x.data_ptr(), out.data_ptr(), table.data_ptr(), (const float*)wf.data_ptr(), B, C,
+  check((pairs ? api.pair_fwd : planes ? api.plane_fwd : api.converse2d_fwd)(x.data_ptr(), out.data_ptr(), table.data_ptr(), (const float*)wf.data_ptr(), B, C,
                                                     H, W, k, s, p, mode, io, gelu, ws ? w.data_ptr() : nullptr, ws, stream(x)),
         "cvb_converse2d_fwd");
   return out;
@@ -170,11 +176,13 @@ PyObject* py_converse2d(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
-// takes_pairs(B, h, w, scale) -> cvb_takes_pairs
+// takes_pairs(B, h, w, scale) -> cvb_takes_pairs; with the channels behind them, 0 where cvb_takes_planes answers 1
 PyObject* py_takes_pairs(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    want(n, 4);
-    return PyLong_FromLong(api.takes_pairs((int)integer(a[0]), (int)integer(a[1]), (int)integer(a[2]), (int)integer(a[3])));
+    if (n != 5) want(n, 4);
+    const int B = (int)integer(a[0]), h = (int)integer(a[1]), w = (int)integer(a[2]), s = (int)integer(a[3]);
+    const int pairs = api.takes_pairs(B, h, w, s);
+    return PyLong_FromLong(pairs == 2 && n == 5 && api.takes_planes(B, (int)integer(a[4]), h, w, s) ? 0 : pairs);
   });
 }
 
@@ -562,9 +570,9 @@ PyObject* py_block_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // init(address of each C ABI function in the order of `names`)
 PyObject* py_init(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    want(n, 27);
-    void* p[27];
-    for (int i = 0; i < 27; ++i) p[i] = PyLong_AsVoidPtr(a[i]);
+    want(n, 30);
+    void* p[30];
+    for (int i = 0; i < 30; ++i) p[i] = PyLong_AsVoidPtr(a[i]);
     int i = 0;
     auto set = [&](auto& f) { f = (std::decay_t<decltype(f)>)p[i++]; };
     set(api.strerror_); set(api.last_cuda_error); set(api.transfer_bytes); set(api.build_transfer); set(api.build_x0_table);
@@ -573,6 +581,7 @@ PyObject* py_init(PyObject*, PyObject* const* a, Py_ssize_t n) {
     set(api.block_pre_train); set(api.block_post_train); set(api.block_grad_floats); set(api.block_bwd_workspace);
     set(api.block_bwd); set(api.takes_pairs); set(api.plane_bytes); set(api.build_plane); set(api.pair_bytes);
     set(api.build_pair); set(api.pair_workspace_bytes); set(api.pair_fwd);
+    set(api.takes_planes); set(api.plane_workspace_bytes); set(api.plane_fwd);
     Py_RETURN_NONE;
   });
 }
@@ -600,7 +609,7 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, null
 PyMODINIT_FUNC PyInit__host(void) {
   PyObject* m = PyModule_Create(&module);
   if (!m) return nullptr;
-  PyObject* names = Py_BuildValue("(sssssssssssssssssssssssssss)", "cvb_strerror", "cvb_last_cuda_error", "cvb_transfer_bytes",
+  PyObject* names = Py_BuildValue("(ssssssssssssssssssssssssssssss)", "cvb_strerror", "cvb_last_cuda_error", "cvb_transfer_bytes",
                                   "cvb_build_transfer", "cvb_build_x0_table", "cvb_converse2d_workspace_bytes",
                                   "cvb_converse2d_fwd", "cvb_block_pack_bytes", "cvb_block_pack", "cvb_block_pre_fwd",
                                   "cvb_block_post_fwd", "cvb_converse2d_train_workspace_bytes",
@@ -608,7 +617,8 @@ PyMODINIT_FUNC PyInit__host(void) {
                                   "cvb_block_pre_train", "cvb_block_post_train", "cvb_block_grad_floats",
                                   "cvb_block_bwd_workspace_bytes", "cvb_block_bwd", "cvb_takes_pairs",
                                   "cvb_plane_transfer_bytes", "cvb_build_plane_transfer", "cvb_pair_transfer_bytes",
-                                  "cvb_build_pair_transfer", "cvb_pair_workspace_bytes", "cvb_pair_fwd");
+                                  "cvb_build_pair_transfer", "cvb_pair_workspace_bytes", "cvb_pair_fwd",
+                                  "cvb_takes_planes", "cvb_plane_workspace_bytes", "cvb_plane_fwd");
   if (!names || PyModule_AddObject(m, "names", names) < 0) return nullptr;
   return m;
 }

@@ -16,6 +16,7 @@ int launch_epilogue_bf16(const Params&, cudaStream_t);
 int launch_rows(const Params&, bool, int, int, size_t, cudaStream_t);
 int launch_plane_f32(const Params&, bool, int, size_t, cudaStream_t);
 int launch_plane_bf16(const Params&, bool, int, size_t, cudaStream_t);
+int launch_fix(int kind, const Params&, int io_dtype, int sms, cudaStream_t);   // integer contractions (k_fix.cu)
 typedef int (*MatrixLauncher)(const Params&, int, int, int, size_t, cudaStream_t);   // (.., tensor type, threads, grid, ..)
 struct MatrixEntry { int width; MatrixLauncher cols_fwd, rows, cols_inv; };
 #define CVB_RP_X(M)                                                            \
@@ -44,7 +45,8 @@ struct TableParams {
   float eps;
   int tk, tf;            // tiles of 32 rows, of 16 frequencies along x
   int r0y, r1y, r0x, r1x, ey, ex;  // plans; entries of the matrix stages (0 = none)
-  size_t tw, twy, twx, dmy, dmx;
+  size_t tw, twy, twx, dmy, dmx, fixy, fixx;
+  int fy, fx;                      // values of the operands of the integer contractions (0 = none)
 };
 constexpr int kTK = 32, kTF = 16;
 
@@ -58,9 +60,35 @@ __device__ __forceinline__ double2 cis(long long m, int N) {
   return r;
 }
 
-// twiddles and matrix rows behind the multiplier
+// Operand of the integer contractions along an axis of length N: value i = (parity, cosine / sine, row, q < 64), three
+// digits; then the fp32 values q = 64 .. 67 of every row.
+__device__ void fix_value_out(unsigned char* out, int N, int i) {
+  const int nr = fix_rows(N), M = N / 2, QH = M / 2;
+  const bool whole = i >= 256 * nr;
+  const int e = whole ? i - 256 * nr : i, per = whole ? 4 : 64;
+  const int q = e % per + (whole ? 64 : 0), j = (e / per) % nr, cs = (e / (per * nr)) & 1, par = e / (2 * per * nr), k = 2 * j + par;
+  double sn, cn;
+  sincospi(2.0 * (double)((q * k) % N) / (double)N, &sn, &cn);
+  double v = k <= M && q <= QH ? (cs ? sn : cn) : 0.0;
+  if (q == 0 || 2 * q == M) v *= 0.5;
+  if (whole) {
+    ((float*)(out + fix_operand(N)))[((par * 2 + cs) * 4 + q - 64) * nr + j] = (float)v;
+    return;
+  }
+  const int n = __double2int_rn(v / (double)kFixUnit);
+  const uint32_t t = ((uint32_t)n + 0x808080u) ^ 0x808080u;
+  int step;
+  const int o = fix_row_offset(nr, par, cs, j, q, step);
+  out[o] = (unsigned char)(t >> 16); out[o + step] = (unsigned char)(t >> 8); out[o + 2 * step] = (unsigned char)t;
+}
+
+// twiddles, matrix rows and contraction operands behind the multiplier
 __device__ void table_tail(const TableParams& T, int i0, int step) {
   const int nt = T.h + T.w;
+  for (int i = i0; i < T.fy + T.fx; i += step) {
+    if (i < T.fy) fix_value_out((unsigned char*)(T.out + T.fixy), T.h, i);
+    else fix_value_out((unsigned char*)(T.out + T.fixx), T.w, i - T.fy);
+  }
   for (int i = i0; i < 2 * nt + T.ey + T.ex; i += step) {
     double sn, cs;
     if (i < 2 * nt) {
@@ -188,8 +216,9 @@ int build_table(const float* weight, const float* bias, int C, int k, int s, int
   T.C = C; T.k = k; T.s = s; T.h = h; T.w = w; T.hh = h / 2 + 1; T.kind = kind; T.eps = eps;
   T.tk = (T.hh + kTK - 1) / kTK; T.tf = (w + kTF - 1) / kTF;
   T.r0y = r0y; T.r1y = r1y; T.r0x = r0x; T.r1x = r1x; T.ey = matrix_entries(r0y); T.ex = matrix_entries(r0x);
-  T.tw = bl.tw; T.twy = bl.twy; T.twx = bl.twx; T.dmy = bl.dmy; T.dmx = bl.dmx;
-  const int tail = (2 * (h + w) + T.ey + T.ex + 255) / 256;
+  T.tw = bl.tw; T.twy = bl.twy; T.twx = bl.twx; T.dmy = bl.dmy; T.dmx = bl.dmx; T.fixy = bl.fixy; T.fixx = bl.fixx;
+  T.fy = fix_axis(h, r0y) ? 272 * fix_rows(h) : 0; T.fx = fix_axis(w, r0x) ? 272 * fix_rows(w) : 0;
+  const int tail = (std::max(2 * (h + w) + T.ey + T.ex, T.fy + T.fx) + 255) / 256;
   const size_t smem = (size_t)(s * (kTF + kTK) * (k + 1) + 1) * sizeof(double2);
   const long long nblk = (long long)C * T.tk * T.tf;
   if (nblk + tail > 0x7fffffffLL) return CVB_ERR_TOO_LARGE;
@@ -214,7 +243,8 @@ static void set_vec(Params& P, bool f32) {
 // one launch of each strip kernel over planes 0 .. planes - 1 (fp32 tensors)
 static int strip(Params& P, int planes, int which, cudaStream_t st) {
   set_vec(P, true);
-  P.plane0 = 0; P.nplane = planes;
+  P.plane0 = 0; P.nplane = planes; P.status = status_ptr();
+  if (takes_fix(P, which, sm_count())) return launch_fix(which, P, CVB_F32, sm_count(), st);
   const int gc = (planes * P.wc + kLines - 1) / kLines, gr = (planes * P.hh + kLines - 1) / kLines;
   const int tc = strip_threads(cols_smem(P), gc, sm_count()), tr = strip_threads(rows_smem(P), gr, sm_count());
   if (which == 1)
@@ -247,6 +277,7 @@ int run(Params& P, const Route& r, int io_dtype, void* workspace, size_t ws_byte
   if (smem_c > kSmemLimit || smem_r > kSmemLimit) return CVB_ERR_UNSUPPORTED_SIZE;
   const bool sy = small_axis(P.ay), sx = small_axis(P.ax);
   P.ws = (float2*)workspace;
+  P.status = status_ptr();
   for (int p0 = 0; p0 < planes; p0 += r.chunk) {
     P.plane0 = p0;
     P.nplane = planes - p0 < r.chunk ? planes - p0 : r.chunk;
@@ -255,13 +286,16 @@ int run(Params& P, const Route& r, int io_dtype, void* workspace, size_t ws_byte
                     : (float*)((char*)workspace + (size_t)P.nplane * P.hh * P.wp * sizeof(float2));
     const int gc = (P.nplane * P.wc + kLines - 1) / kLines, gr = (P.nplane * P.hh + kLines - 1) / kLines;
     const int tc = strip_threads(smem_c, gc, sm_count()), tr = strip_threads(smem_r, gr, sm_count());
-    int rc = P.ay.mp ? matrix_entry(P.ay.mp).cols_fwd(P, io_dtype, tc, gc, smem_c, st)
+    int rc = takes_fix(P, 0, sm_count()) ? launch_fix(0, P, io_dtype, sm_count(), st)
+             : P.ay.mp ? matrix_entry(P.ay.mp).cols_fwd(P, io_dtype, tc, gc, smem_c, st)
              : f32   ? launch_cols_fwd_f32(P, sy, tc, gc, smem_c, st)
                      : launch_cols_fwd_bf16(P, sy, tc, gc, smem_c, st);
     if (rc == CVB_OK)
-      rc = P.ax.mp ? matrix_entry(P.ax.mp).rows(P, io_dtype, tr, gr, smem_r, st) : launch_rows(P, sx, tr, gr, smem_r, st);
+      rc = takes_fix(P, 1, sm_count()) ? launch_fix(1, P, io_dtype, sm_count(), st)
+           : P.ax.mp ? matrix_entry(P.ax.mp).rows(P, io_dtype, tr, gr, smem_r, st) : launch_rows(P, sx, tr, gr, smem_r, st);
     if (rc == CVB_OK)
-      rc = P.ay.mp ? matrix_entry(P.ay.mp).cols_inv(P, io_dtype, tc, gc, smem_c, st)
+      rc = takes_fix(P, 2, sm_count()) ? launch_fix(2, P, io_dtype, sm_count(), st)
+           : P.ay.mp ? matrix_entry(P.ay.mp).cols_inv(P, io_dtype, tc, gc, smem_c, st)
            : f32   ? launch_cols_inv_f32(P, sy, tc, gc, smem_c, st)
                    : launch_cols_inv_bf16(P, sy, tc, gc, smem_c, st);
     if (rc == CVB_OK && P.s > 1) rc = f32 ? launch_epilogue_f32(P, st) : launch_epilogue_bf16(P, st);

@@ -164,6 +164,16 @@ int cvb_build_plane_transfer(const float* weight, const float* bias, int C, int 
                              void* table, void* stream);
 
 /*
+ * The same operator on one real plane after the other with that table, whatever the batch.  cvb_takes_planes: 1 for batches
+ * that cvb_takes_pairs answers 2 for although the real planes are the faster ones, so that a caller that knows its batch
+ * keeps the real-plane table and calls cvb_plane_fwd; else 0.
+ */
+int cvb_takes_planes(int B, int C, int h, int w, int s);
+size_t cvb_plane_workspace_bytes(int B, int C, int H, int W, int s, int p);
+int cvb_plane_fwd(const void* x, void* out, const void* table, const float* weight, int B, int C, int H, int W, int k, int s,
+                  int p, int pad_mode, int io_dtype, int fuse_gelu, void* workspace, size_t workspace_bytes, void* stream);
+
+/*
  * ConverseBlock, first fused kernel: out = GELU( W . LayerNorm(x) + b ), C -> 2C channels,
  * i.e. conv1[0..2] of the block: channels_first LayerNorm (models/util_converse.py:60-68),
  * 1x1 Conv2d (:279), GELU (:280).  x (B,C,HW), out (B,2C,HW) contiguous, io_dtype;

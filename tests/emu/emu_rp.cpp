@@ -6,6 +6,7 @@
 #include <cuda_bf16.h>
 #include <ucontext.h>
 
+#include <cmath>
 #include <csetjmp>
 #include <csignal>
 #include <functional>
@@ -95,7 +96,7 @@ void run_block(int nthr) {
     }
     for (int t = 0; t < nthr; ++t) ++count[fibers[t].state];
     if (count[Fiber::kDone] == nthr) return;
-    bool moved = false;
+    bool moved = count[Fiber::kReady] > 0;      // (polling a barrier in shared memory)
     for (int w = 0; w < nthr / 32; ++w) {
       int waiting = 0;
       for (int l = 0; l < 32; ++l) waiting += fibers[32 * w + l].state == Fiber::kWarp;
@@ -162,6 +163,125 @@ static inline void __stcs(T* p, T v) { *p = v; }
 template <class T>
 static inline T __ldg(const T* p) { return *p; }
 
+static inline unsigned __float_as_uint(float f) {
+  unsigned v;
+  __builtin_memcpy(&v, &f, 4);
+  return v;
+}
+static inline int __float2int_rn(float f) { return f != f ? 0 : (int)nearbyintf(f); }
+static inline unsigned __byte_perm(unsigned a, unsigned b, unsigned s) {
+  const unsigned long long v = ((unsigned long long)b << 32) | a;
+  unsigned r = 0;
+  for (int i = 0; i < 4; ++i) r |= (unsigned)((v >> (8 * ((s >> (4 * i)) & 7))) & 0xff) << (8 * i);
+  return r;
+}
+static inline unsigned atomicMax(unsigned* p, unsigned v) {
+  const unsigned o = *p;
+  if (v > o) *p = v;
+  return o;
+}
+static inline int atomicExch(int* p, int v) {
+  const int o = *p;
+  *p = v;
+  return o;
+}
+static inline unsigned max(unsigned a, unsigned b) { return a > b ? a : b; }
+#define __noinline__
+#define __syncwarp() emu::wait(emu::Fiber::kWarp)
+
+// Tensor memory, the integer MMA (the second operand in rows of 16 bytes, eight rows a core matrix, K = 32), barriers in
+// shared memory and asynchronous copies of cvb_fix.cuh.  MMAs and copies happen at once.
+#include <cstdint>
+#include <map>
+namespace cvb {
+namespace rp {
+static int tensor_memory[128][512];
+struct Barrier { int pending; long long bytes; uint32_t phase; };
+static std::map<uint64_t*, Barrier> barriers;
+inline Barrier& barrier(uint64_t* b) {
+  auto it = barriers.find(b);
+  if (it == barriers.end()) throw std::runtime_error("barrier not initialised");
+  return it->second;
+}
+inline void settle(Barrier& b) {
+  if (b.pending < 0) throw std::runtime_error("too many arrivals");
+  if (b.pending == 0 && b.bytes == 0) { b.phase ^= 1; b.pending = 1; }
+}
+inline void fx_init(uint64_t* b) { barriers[b] = {1, 0, 0}; }
+inline void fx_init_done() {}
+inline void fx_expect(uint64_t* p, uint32_t bytes) { Barrier& b = barrier(p); b.bytes += bytes; --b.pending; settle(b); }
+inline void fx_bulk(void* dst, const void* src, uint32_t bytes, uint64_t* p) {
+  if (((size_t)dst | (size_t)src | bytes) % 16) throw std::runtime_error("bulk copy alignment");
+  memcpy(dst, src, bytes);
+  Barrier& b = barrier(p);
+  b.bytes -= bytes;
+  settle(b);
+}
+inline bool fx_wait(uint64_t* p, uint32_t parity) {
+  for (int i = 0; barrier(p).phase == parity; ++i) {
+    if (i > 100000) throw std::runtime_error("a wait that does not end");
+    swapcontext(&emu::fiber->context, &emu::scheduler);
+  }
+  return true;
+}
+inline void fx_commit(uint64_t* p) { Barrier& b = barrier(p); --b.pending; settle(b); }
+inline unsigned fx_count(unsigned* c) { return (*c)++; }
+inline uint32_t fx_elect() { return emu::fiber->lane == 0; }
+inline unsigned fx_from_first(unsigned v) { return (unsigned)emu::exchange(&emu::WarpSlots::i, (int)v, 0); }
+inline void fx_alloc(uint32_t* holder) {
+  if (emu::fiber->lane) return;
+  *holder = 0;
+  for (auto& l : tensor_memory)
+    for (int& v : l) v = 0x5a5a5a5a;
+}
+inline void fx_free(uint32_t) {}
+inline void fx_before_sync() {}
+inline void fx_after_sync() {}
+struct Operand { const unsigned char* at; int rows; };
+inline Operand fx_operand(const unsigned char* b, int brows) { return {b, brows}; }
+inline Operand fx_further(Operand b, int bytes) { return {b.at + bytes, b.rows}; }
+inline void fx_mma(uint32_t d, uint32_t a, Operand o, int n, bool add, uint32_t elected) {
+  if (!elected) return;
+  const unsigned char* b = o.at;
+  const int brows = o.rows;
+  if (n % 16 || n < 16 || n > 256 || d < 256 || d + n > 512 || a + 8 > 256 || (size_t)b % 16) throw std::runtime_error("MMA form");
+  for (int m = 0; m < 128; ++m) {
+    const signed char* l = (const signed char*)&tensor_memory[m][a];
+    for (int j = 0; j < n; ++j) {
+      int sum = add ? tensor_memory[m][d + j] : 0;
+      for (int k = 0; k < 32; ++k) sum += (int)l[k] * (int)(signed char)b[(k >> 4) * 16 * brows + j * 16 + (k & 15)];
+      tensor_memory[m][d + j] = sum;
+    }
+  }
+}
+inline int* tensor_lane(uint32_t t, uint32_t n) {
+  if (t >> 16 != (unsigned)(32 * (emu::fiber->warp & 3)) || (t & 0xffff) + n > 512) throw std::runtime_error("tensor-memory access");
+  return &tensor_memory[(t >> 16) + emu::fiber->lane][t & 0xffff];
+}
+template <int N>
+inline void fx_ld(uint32_t t, int (&v)[N]) { memcpy(v, tensor_lane(t, N), sizeof(v)); }
+inline void fx_ld_wait() {}
+template <int N>
+inline void fx_st(uint32_t t, const uint32_t (&v)[N]) { memcpy(tensor_lane(t, N), v, sizeof(v)); }
+inline void fx_st_wait() {}
+template <int BYTES>
+inline void fx_copy(void* dst, const void* src, bool ok) {
+  if (((size_t)dst | (size_t)src) % BYTES) throw std::runtime_error("asynchronous copy alignment");
+  if (ok) memcpy(dst, src, BYTES);
+  else memset(dst, 0, BYTES);
+}
+inline void fx_copies_done() {}
+inline float fx_largest(float m, float a, float b) {
+  const float v[3] = {m, fabsf(a), fabsf(b)};
+  float r = 0.f;
+  for (float x : v) r = r != r || x != x ? NAN : x > r ? x : r;
+  return r;
+}
+inline float2 fx_fma2(float2 a, float2 b, float2 c) { return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)); }
+inline float2 fx_mul2(float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); }
+}  // namespace rp
+}  // namespace cvb
+
 #include "../../conversenet_b200/csrc/cvb_rp_plan.h"
 #include "../../conversenet_b200/csrc/cvb_rp_bwd.cuh"
 
@@ -189,6 +309,31 @@ void fill_tail(float2* t, const Blob& bl, int h, int w, int r0y, int r1y, int r0
           const float2 u = unit((q * k) % r0, r0);
           dm[(half * (r0 / 2 + 1) + k) * mp + q - 1] = q > r0 / 2 ? 0.f : half ? u.y : u.x;
         }
+  }
+  for (int a = 0; a < 2; ++a) {
+    const int n = a ? w : h, nr = fix_rows(n), M = n / 2;
+    if (!fix_axis(n, a ? r0x : r0y)) continue;
+    unsigned char* out = (unsigned char*)(t + (a ? bl.fixx : bl.fixy));
+    for (int par = 0; par < 2; ++par)
+      for (int cs = 0; cs < 2; ++cs)
+        for (int j = 0; j < nr; ++j)
+          for (int q = 0; q < 68; ++q) {
+            const int k = 2 * j + par;
+            const double u = 2.0 * M_PI * ((q * k) % n) / n;
+            double v = k <= M && q <= M / 2 ? (cs ? sin(u) : cos(u)) : 0.0;
+            if (q == 0 || 2 * q == M) v *= 0.5;
+            if (q >= 64) {
+              ((float*)(out + fix_operand(n)))[((par * 2 + cs) * 4 + q - 64) * nr + j] = (float)v;
+              continue;
+            }
+            int m = (int)nearbyint(v / (double)kFixUnit), step;
+            const int o = fix_row_offset(nr, par, cs, j, q, step);
+            for (int d = 2; d >= 0; --d) {
+              const int digit = (signed char)(m & 0xff);
+              out[o + d * step] = (unsigned char)digit;
+              m = (m - digit) / 256;
+            }
+          }
   }
 }
 
@@ -229,6 +374,24 @@ void strip_body(const Params& P, Kernel which, float2* sm, int nthr, int grid) {
 template <typename IO>
 void strip(const Params& P, Kernel which, int sms) {
   const Axis& a = which == kRows ? P.ax : P.ay;
+  if (takes_fix(P, which, sms)) {
+    const size_t bytes = fix_smem(which, a.n);
+    emu::Guarded sm(bytes);
+    if (bytes > kSmemLimit) throw std::runtime_error("shared memory");
+    const int tiles = (fix_lines(which, P) + kFixLines - 1) / kFixLines;
+    const int grid = tiles > 2 ? tiles / 2 : tiles;     // blocks walk over several tiles
+    auto run = [&](auto extra) {
+      constexpr bool E = decltype(extra)::value;
+      unsigned char* m = (unsigned char*)sm.get();
+      if (which == kColsFwd) emu::launch(grid, 1, 1, kFixThreads, [&] { fix_body<kFixFwd, IO, E>(P, m); });
+      if (which == kRows) emu::launch(grid, 1, 1, kFixThreads, [&] { fix_body<kFixRows, IO, E>(P, m); });
+      if (which == kColsInv) emu::launch(grid, 1, 1, kFixThreads, [&] { fix_body<kFixInv, IO, E>(P, m); });
+    };
+    if (a.n >= 256) run(std::true_type());
+    else run(std::false_type());
+    sm.check("shared memory");
+    return;
+  }
   const int lines = which == kRows ? P.hh : P.wc, grid = (P.nplane * lines + kLines - 1) / kLines;
   const size_t bytes = which == kRows ? rows_smem(P) : cols_smem(P);
   if (bytes > kSmemLimit) throw std::runtime_error("shared memory");

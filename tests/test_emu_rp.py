@@ -34,7 +34,7 @@ def _weights(C, k, seed):
     return w, (b + rng.standard_normal(b.shape)).astype(np.float32), rng
 
 
-def _forward(lib, x, w, b, s, p, mode, gelu=0, multi=0, ws_planes=0, keep=False):
+def _forward(lib, x, w, b, s, p, mode, gelu=0, multi=0, ws_planes=0, keep=False, sms=SMS):
     """x: float32, or uint16 holding bf16"""
     B, C, H, W = x.shape
     k, bf16 = w.shape[-1], x.dtype == np.uint16
@@ -43,7 +43,7 @@ def _forward(lib, x, w, b, s, p, mode, gelu=0, multi=0, ws_planes=0, keep=False)
     r = np.zeros((B, C, h, wp), np.float32) if keep else None
     wf = np.ascontiguousarray(w.reshape(C, k, k), np.float32)
     _check(lib, lib.emu_rp_forward(_ptr(x), _ptr(out), _ptr(r), _ptr(wf), _ptr(np.ascontiguousarray(b.reshape(C))), B, C, H, W, k,
-                                   s, p, PAD[mode], ctypes.c_float(1e-5), gelu, int(bf16), multi, ws_planes, SMS))
+                                   s, p, PAD[mode], ctypes.c_float(1e-5), gelu, int(bf16), multi, ws_planes, sms))
     return (out, r) if keep else out
 
 
@@ -80,6 +80,50 @@ def test_forward_matches_the_oracle(emu, case):
         assert orc.rel_l2(out, ref) <= 2e-6
     gelu = _forward(emu, x, w, b, s, p, mode, gelu=1)
     assert orc.rel_l2(gelu, torch.nn.functional.gelu(torch.from_numpy(ref)).numpy()) <= 4e-6
+
+
+FIXED = [
+    # integer contractions (one SM: every tile count takes them): B, C, H, W, k, s, p, mode
+    (1, 1, 132, 140, 3, 1, 1, "circular"),        # 134 x 142: the shortest axes, odd halves
+    (3, 1, 130, 131, 5, 1, 2, "replicate"),       # 134 x 135: an odd width, columns alone; tiles across planes
+    (1, 2, 20, 140, 3, 1, 3, "constant"),         # 26 x 146: rows alone
+    (1, 1, 250, 146, 5, 1, 4, "reflect"),         # 258 x 154: one frequency and one q above 64
+    (1, 1, 252, 130, 3, 1, 1, "constant"),        # 254: the longest without
+    (1, 1, 32, 256, 5, 1, 6, "circular"),         # 44 x 268: four q above 64
+    (1, 1, 256, 234, 7, 1, 6, "replicate"),       # 268 x 246
+    (1, 2, 64, 132, 3, 2, 1, "circular"),         # 66 x 134 by 2: rows; the plane r
+    (1, 1, 132, 20, 3, 3, 1, "reflect"),          # 134 x 22 by 3: columns and r
+]
+
+
+@pytest.mark.parametrize("case", FIXED)
+def test_integer_contractions(emu, case):
+    B, C, H, W, k, s, p, mode = case
+    w, b, rng = _weights(C, k, H * 100 + W)
+    x = rng.standard_normal((B, C, H, W)).astype(np.float32)
+    ref = orc.converse2d_forward(x, w, b, s, p, mode, 1e-5, dtype=np.float64)
+    out, r = _forward(emu, x, w, b, s, p, mode, multi=1, keep=True, sms=1)
+    # the constants' 24 bits, two roundings of the folds and one of the result on each of four passes: 2e-7
+    assert orc.rel_l2(out, ref) <= 4e-7
+    gelu = _forward(emu, x, w, b, s, p, mode, gelu=1, multi=1, ws_planes=1 if B * C > 1 else 0, sms=1)
+    assert orc.rel_l2(gelu, torch.nn.functional.gelu(torch.from_numpy(ref)).numpy()) <= 2e-6
+    if s > 1:
+        other = _forward(emu, x, w, b, s, p, mode, multi=1, keep=True)[1]
+        assert orc.rel_l2(r, other) <= 2e-6
+
+
+def test_integer_contractions_on_values_of_any_size(emu):
+    """Lines are scaled one by one: planes of very different magnitudes, zeros, an infinity and a NaN do not meet."""
+    w, b, rng = _weights(6, 3, 7)
+    w[:], b[:] = w[:, :1], b[:, :1]
+    x = np.repeat(rng.standard_normal((1, 1, 132, 140)).astype(np.float32), 6, axis=1)
+    for c, f in enumerate((1.0, 2.0 ** -80, 2.0 ** 90, 0.0)):
+        x[:, c] *= np.float32(f)
+    x[0, 4, 60, 70], x[0, 5, 5, 9] = np.inf, np.nan
+    out = _forward(emu, x, w, b, 1, 1, "circular", multi=1, sms=1)[0]
+    for c, f in ((1, 2.0 ** -80), (2, 2.0 ** 90)):
+        assert np.array_equal(out[c] / np.float32(f), out[0])      # powers of two: not one bit differs
+    assert not out[3].any() and not np.isfinite(out[4]).any() and np.isnan(out[5]).all()
 
 
 @pytest.mark.parametrize("case", [(1, 2, 20, 18, 3, 1, 2, "circular"), (1, 1, 21, 15, 5, 1, 2, "constant"),

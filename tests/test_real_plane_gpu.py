@@ -60,6 +60,53 @@ def test_forward_matches_oracle(case):
 
 
 @pytest.mark.parametrize("case", [
+    # integer contractions: enough planes that they are taken on the largest chips; a few planes are compared
+    (1, 176, 132, 140, 3, 1, 1, "circular", "fp32"),      # 134 x 142: the shortest
+    (2, 64, 252, 156, 5, 1, 1, "constant", "fp32"),       # 254 x 158: columns too long for one more q
+    (1, 96, 256, 240, 7, 1, 6, "replicate", "bf16"),      # 268 x 252: four q above 64; bf16 columns
+    (3, 40, 250, 232, 3, 1, 4, "reflect", "fp32"),        # 258 x 240
+    (1, 80, 40, 256, 3, 1, 6, "circular", "fp32"),        # 52 x 268: rows alone
+    (1, 70, 242, 243, 3, 2, 1, "circular", "fp32"),       # 244 x 245 by 2: an odd width
+    (1, 3, 200, 192, 3, 1, 1, "circular", "fp32"),        # 202 x 194: wide dense stages, any number of planes
+])
+def test_integer_contractions(case):
+    from conversenet_b200 import Converse2D, _cabi
+    B, C, H, W, k, s, p, mode, dt = case
+    rng = np.random.default_rng(H * 1000 + W)
+    w, b = orc.init_weight(C, k, rng)
+    b = b + rng.standard_normal(b.shape).astype(np.float32)
+    dtype = torch.float32 if dt == "fp32" else torch.bfloat16
+    x = torch.from_numpy(rng.standard_normal((B, C, H, W)).astype(np.float32)).to(dtype)
+    m = Converse2D(C, C, k, scale=s, padding=p, padding_mode=mode).cuda().eval()
+    with torch.no_grad():
+        m.weight.copy_(torch.from_numpy(w))
+        m.bias.copy_(torch.from_numpy(b))
+        y = m(x.cuda()).float().cpu().numpy()
+    some = sorted({0, C // 2, C - 1})
+    ref = orc.converse2d_forward(x.float().numpy()[-1:, some], np.ascontiguousarray(w[:, some]), np.ascontiguousarray(b[:, some]),
+                                 s, p, mode, 1e-5, dtype=np.float64)
+    # fp32: see tests/test_emu_rp.py; at scale 2 the epilogue's sums of nine come on top
+    assert orc.rel_l2(y[-1:, some], ref) <= (4e-7 if dt == "fp32" else 3e-3)
+    assert _cabi.load().cvb_last_device_status(1) == 0      # no bounded wait has run out
+
+
+def test_integer_contractions_keep_planes_apart():
+    from conversenet_b200 import Converse2D
+    g = torch.Generator(device="cuda").manual_seed(3)
+    m = Converse2D(96, 96, 3, padding=1, padding_mode="circular").cuda().eval()
+    x = torch.randn(1, 96, 242, 266, device="cuda", generator=g)
+    with torch.no_grad():
+        y = m(x)
+        z = x.clone()
+        z[0, 7, 100, 3], z[0, 50, 0, 0] = float("nan"), float("inf")
+        z[0, 20] *= 2.0 ** 60
+        t = m(z)
+    same = [c for c in range(96) if c not in (7, 20, 50)]
+    assert torch.equal(t[:, same], y[:, same]) and torch.equal(t[:, 20], y[:, 20] * 2.0 ** 60)
+    assert bool(t[0, 7].isnan().all()) and not bool(t[0, 50].isfinite().any())
+
+
+@pytest.mark.parametrize("case", [
     # lengths above 680: dense stages of 64, 80, 60 and 95 points (real planes), two register radices (832 = 32 * 26)
     (2, 1, 1022, 130, 3, 1, 1, "circular", "fp32"),
     (1, 2, 60, 1278, 5, 1, 1, "replicate", "bf16"),
