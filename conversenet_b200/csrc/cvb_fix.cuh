@@ -57,12 +57,7 @@ __device__ __forceinline__ void fx_alloc(uint32_t* holder) { tc::tmem_alloc(hold
 __device__ __forceinline__ void fx_free(uint32_t t) { tc::tmem_dealloc(t, 512); }
 __device__ __forceinline__ void fx_before_sync() { tc::fence_before_sync(); }
 __device__ __forceinline__ void fx_after_sync() { tc::fence_after_sync(); }
-// one lane of a converged warp
-__device__ __forceinline__ uint32_t fx_elect() {
-  uint32_t e;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
-  return e;
-}
+__device__ __forceinline__ uint32_t fx_elect() { return tc::elect_one(); }
 __device__ __forceinline__ void fx_commit(uint64_t* bar) { tc::mma_commit(bar); }
 __device__ __forceinline__ void fx_init(uint64_t* bar) { mbar_init(bar, 1); }
 __device__ __forceinline__ void fx_init_done() { mbar_fence_init(); }
@@ -75,7 +70,7 @@ __device__ __forceinline__ unsigned fx_count(unsigned* counter) {
   asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(old) : "r"(smem_u32(counter)) : "memory");
   return old;
 }
-__device__ __forceinline__ unsigned fx_from_first(unsigned v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ unsigned fx_from_first(unsigned v) { return tc::from_first(v); }
 // the second operand of fx_mma: rows of 16 bytes, eight of them a core matrix, the second half of K `brows` rows further on
 __device__ __forceinline__ uint64_t fx_operand(const unsigned char* b, int brows) { return tc::smem_desc(b, 16 * brows, 128); }
 __device__ __forceinline__ uint64_t fx_further(uint64_t b, int bytes) { return b + (uint32_t)(bytes >> 4); }

@@ -215,10 +215,10 @@ __device__ __forceinline__ void stage_quad_ta(uint32_t taddr, const float (&re)[
 }
 
 // the six MMAs of K-chunk `ch`, accumulating unless ch == 0; operand A in tensor memory (slot = 32 columns at
-// `a_tmem`), the constant operand in shared memory
+// `a_tmem`), the constant operand in shared memory; a whole warp
 template <int R0>
 __device__ __forceinline__ void issue_chunk_ta(uint32_t tmem, uint32_t a_tmem, const float* b_hi, const float* b_lo,
-                                               int ch) {
+                                               int ch, uint32_t elected) {
   typedef Geo<R0> G;
   constexpr uint32_t idesc = tc::idesc_tf32(kVec, G::NB, false, false);
   const uint64_t bh = tc::smem_desc((const char*)b_hi + ch * G::B_KSTEP, G::B_LBO, 128);
@@ -227,9 +227,9 @@ __device__ __forceinline__ void issue_chunk_ta(uint32_t tmem, uint32_t a_tmem, c
   for (int part = 0; part < 2; ++part) {
     const uint32_t ah = a_tmem + (uint32_t)(16 * part), al = ah + 8u;
     const uint32_t d = tmem + (uint32_t)(part * G::NB);
-    tc::mma_tf32_ta(d, ah, bh, idesc, ch > 0 ? 1u : 0u);
-    tc::mma_tf32_ta(d, ah, bl, idesc, 1u);
-    tc::mma_tf32_ta(d, al, bh, idesc, 1u);
+    tc::mma_tf32_ta(d, ah, bh, idesc, ch > 0 ? 1u : 0u, elected);
+    tc::mma_tf32_ta(d, ah, bl, idesc, 1u, elected);
+    tc::mma_tf32_ta(d, al, bh, idesc, 1u, elected);
   }
 }
 
@@ -360,7 +360,7 @@ __device__ void body(const Params& P, unsigned char* smem_raw) {
   constexpr int N = G::N;
   constexpr int BAR_FREE = NS + 1;           // named barrier "accumulators read"; slots use 1 .. NS
   const FwdParams& F = P.f;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = (int)tc::from_first(tid >> 5), lane = tid & 31;
   const bool issuer = warp == kStageThreads / 32;
   const int m = tid & (kVec - 1), hf = (tid >> 7) & 1;
   const int h = F.h, w = F.w;
@@ -396,7 +396,7 @@ __device__ void body(const Params& P, unsigned char* smem_raw) {
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  const uint32_t tmem = *holder;
+  const uint32_t tmem = tc::from_first(*holder);
   bool ok = true;
   // Ring bookkeeping: chunk number g (counted over the block's life) uses slot g % NS for the
   // (g / NS)-th time; that use may start once the commit of the use before it has arrived.
@@ -404,6 +404,7 @@ __device__ void body(const Params& P, unsigned char* smem_raw) {
 
   if (issuer) {
     // ---------------- the issuing warp ----------------
+    const uint32_t elected = tc::elect_one();
     bool first = true;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
       if (!first) bar_sync(BAR_FREE);   // the previous tile's accumulators have been read
@@ -411,11 +412,9 @@ __device__ void body(const Params& P, unsigned char* smem_raw) {
         const uint32_t slot = seq % NS;
         bar_sync(1 + (int)slot);        // chunk staged
         tc::fence_after_sync();
-        if (lane == 0) {
-          if (first && ch == 0) ok = mbar_wait_bounded(&mbar[NS], 0, kWait);   // the constant operand has landed
-          if (ok) issue_chunk_ta<R0>(tmem, tmem + A_BASE + slot * 32u, b_hi, b_lo, ch);
-          tc::mma_commit(&mbar[slot]);
-        }
+        if (first && ch == 0) ok = mbar_wait_bounded(&mbar[NS], 0, kWait);   // the constant operand has landed
+        issue_chunk_ta<R0>(tmem, tmem + A_BASE + slot * 32u, b_hi, b_lo, ch, ok ? elected : 0u);
+        if (elected) tc::mma_commit(&mbar[slot]);
         __syncwarp();
         seq += 1;
       }

@@ -48,9 +48,9 @@ __device__ __forceinline__ void mix_mma(uint32_t tmem, const float* b_hi, int k0
   for (int ks = 0; ks < 8; ++ks) {
     const uint64_t bh = tc::smem_desc((const char*)b_hi + (k0 / 8 + ks) * KSTEP, LBO, 128);
     const uint64_t bl = tc::smem_desc((const char*)(b_hi + kW) + (k0 / 8 + ks) * KSTEP, LBO, 128);
-    tc::mma_tf32_ta(tmem, tmem + kOpHi + ks * 8, bh, idesc, (accumulate || ks > 0) ? 1u : 0u);
-    tc::mma_tf32_ta(tmem, tmem + kOpHi + ks * 8, bl, idesc, 1u);
-    tc::mma_tf32_ta(tmem, tmem + kOpLo + ks * 8, bh, idesc, 1u);
+    tc::mma_tf32_ta(tmem, tmem + kOpHi + ks * 8, bh, idesc, (accumulate || ks > 0) ? 1u : 0u, 1u);
+    tc::mma_tf32_ta(tmem, tmem + kOpHi + ks * 8, bl, idesc, 1u, 1u);
+    tc::mma_tf32_ta(tmem, tmem + kOpLo + ks * 8, bh, idesc, 1u, 1u);
   }
 }
 template <typename IO>

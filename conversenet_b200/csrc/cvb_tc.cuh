@@ -65,17 +65,28 @@ __device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t adesc, uint64
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// One lane of a converged warp.  A whole warp goes through the code that issues MMAs and one lane issues: the operands then
+// stay in uniform registers.  With a branch around it that a single lane takes, each MMA waits about 80 cycles for its
+// operands to be moved there (1 x 128 planes of 268 x 268 in cvb_fix.cuh: 152 us against 129).
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e;
+}
+// the first lane's value, which the compiler then knows to be the warp's
+__device__ __forceinline__ uint32_t from_first(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
 // D[tmem] (+)= A[tmem] * B[smem]: the A operand read from tensor memory (lane = row, one 32-bit column
-// per K element); one thread issues
+// per K element); the lane whose `elected` is not 0 issues
 __device__ __forceinline__ void mma_tf32_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate) {
+                                            uint32_t accumulate, uint32_t elected) {
   asm volatile(
       "{\n\t"
-      ".reg .pred p;\n\t"
+      ".reg .pred p, e;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t"
+      "setp.ne.b32 e, %5, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t"
       "}\n" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(elected)
       : "memory");
 }
 // four consecutive 32-bit columns of this thread's TMEM lane (the warp writes its 32-lane quadrant)

@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(T3Threads<MODE>::value, 1) tc3_pw_kernel(const
   volatile int* abort_flag = (volatile int*)(tmem_holder + 1);
   uint64_t* full = bars; uint64_t* empty = bars + 2; uint64_t* tfull = bars + 4; uint64_t* tempty = bars + 6;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = (int)tc::from_first(tid >> 5), lane = tid & 31;
   const long long ntiles = ((long long)P.B * P.HW) / kT3Tile;
   const long long my_tiles = ((long long)blockIdx.x < ntiles) ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
 
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(T3Threads<MODE>::value, 1) tc3_pw_kernel(const
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  const uint32_t tmem = *tmem_holder;
+  const uint32_t tmem = tc::from_first(*tmem_holder);
   constexpr uint32_t idesc = tc::idesc_tf32(kT3Tile, N, false, false);
 
   if (warp < 4) {
@@ -194,36 +194,38 @@ __global__ void __launch_bounds__(T3Threads<MODE>::value, 1) tc3_pw_kernel(const
     }
     t3_wait_group<0>();
   } else if (warp == 8) {
-    // ================= MMA issuer (one lane) =================
-    if (lane == 0) {
-      long long chunk = 0, it = 0;
-      for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
-        const int acc = (int)(it & 1);
-        // accumulator free again?  (first use of each passes at once)
-        if (!t3_wait(&tempty[acc], (uint32_t)(((it >> 1) & 1) ^ 1), abort_flag)) break;
-        tc::fence_after_sync();
-        const uint32_t d = tmem + (uint32_t)(acc * N);
-        bool ok = true;
+    // ================= MMA issuer =================
+    const uint32_t e = tc::elect_one();
+    long long chunk = 0, it = 0;
+    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
+      const int acc = (int)(it & 1);
+      // accumulator free again?  (first use of each passes at once)
+      if (!__all_sync(0xffffffffu, t3_wait(&tempty[acc], (uint32_t)(((it >> 1) & 1) ^ 1), abort_flag))) break;
+      tc::fence_after_sync();
+      const uint32_t d = tmem + (uint32_t)(acc * N);
+      bool ok = true;
 #pragma unroll 1
-        for (int kc = 0; kc < CPT; ++kc, ++chunk) {
-          const int st = (int)(chunk & 1);
-          if (!t3_wait(&full[st], (uint32_t)((chunk >> 1) & 1), abort_flag)) { ok = false; break; }
-          tc::fence_after_sync();
-          const uint32_t a_hi = tmem + A_BASE + (uint32_t)st * 128u, a_lo = a_hi + 64u;
+      for (int kc = 0; kc < CPT; ++kc, ++chunk) {
+        const int st = (int)(chunk & 1);
+        if (!__all_sync(0xffffffffu, t3_wait(&full[st], (uint32_t)((chunk >> 1) & 1), abort_flag))) { ok = false; break; }
+        tc::fence_after_sync();
+        const uint32_t a_hi = tmem + A_BASE + (uint32_t)st * 128u, a_lo = a_hi + 64u;
 #pragma unroll
-          for (int ks = 0; ks < kT3Chunk / 8; ++ks) {
-            const int kb = kc * (kT3Chunk / 8) + ks;
-            const uint64_t bh = tc::smem_desc((const char*)b_hi + kb * B_KSTEP, B_LBO, B_SBO);
-            const uint64_t bl = tc::smem_desc((const char*)b_lo + kb * B_KSTEP, B_LBO, B_SBO);
-            tc::mma_tf32_ta(d, a_hi + (uint32_t)(ks * 8), bh, idesc, (kc > 0 || ks > 0) ? 1u : 0u);
-            tc::mma_tf32_ta(d, a_hi + (uint32_t)(ks * 8), bl, idesc, 1u);
-            tc::mma_tf32_ta(d, a_lo + (uint32_t)(ks * 8), bh, idesc, 1u);
-          }
-          tc::mma_commit(&empty[st]);     // the stage may be refilled once these MMAs are done
+        for (int ks = 0; ks < kT3Chunk / 8; ++ks) {
+          const int kb = kc * (kT3Chunk / 8) + ks;
+          const uint64_t bh = tc::smem_desc((const char*)b_hi + kb * B_KSTEP, B_LBO, B_SBO);
+          const uint64_t bl = tc::smem_desc((const char*)b_lo + kb * B_KSTEP, B_LBO, B_SBO);
+          tc::mma_tf32_ta(d, a_hi + (uint32_t)(ks * 8), bh, idesc, (kc > 0 || ks > 0) ? 1u : 0u, e);
+          tc::mma_tf32_ta(d, a_hi + (uint32_t)(ks * 8), bl, idesc, 1u, e);
+          tc::mma_tf32_ta(d, a_lo + (uint32_t)(ks * 8), bh, idesc, 1u, e);
         }
-        if (!ok) break;
-        tc::mma_commit(&tfull[acc]);      // accumulator complete
+        if (e) {
+          tc::mma_commit(&empty[st]);     // the stage may be refilled once these MMAs are done
+          if (kc == CPT - 1) tc::mma_commit(&tfull[acc]);      // accumulator complete
+        }
+        __syncwarp();
       }
+      if (!ok) break;
     }
   } else {
     // ================= consumers: warp w reads TMEM lanes 32 (w % 4) .., warps 4-7 the first half of the
