@@ -3,10 +3,11 @@
 #pragma once
 #include "cvb_block.cuh"
 #include "cvb_tc.cuh"
+#include <cuda_fp16.h>
 
 namespace cvb {
 
-constexpr int kW = kBlkC * kBlkM;                               // floats of one weight matrix
+constexpr int kW = kBlkC * kBlkM;                               // values of one weight matrix
 
 // float index of element (n, k) of an operand with N rows (K-major core matrices, no swizzle)
 __host__ __device__ constexpr int pack_index(int N, int n, int k) {
@@ -41,16 +42,54 @@ __device__ __forceinline__ void mix_stage(uint32_t lane, const float (&v)[32]) {
 }
 // D (+)= A[64 channels in the operand columns] . B, B = N rows, K columns k0 .. k0 + 63 of a packed matrix
 template <int N>
-__device__ __forceinline__ void mix_mma(uint32_t tmem, const float* b_hi, int k0, bool accumulate) {
+__device__ __forceinline__ void mix_mma(uint32_t tmem, const float* b_hi, int k0, bool accumulate, uint32_t elected) {
   constexpr uint32_t idesc = tc::idesc_tf32(128, N, false, false);
   constexpr int LBO = (N / 8) * 128, KSTEP = 2 * LBO;
 #pragma unroll
   for (int ks = 0; ks < 8; ++ks) {
     const uint64_t bh = tc::smem_desc((const char*)b_hi + (k0 / 8 + ks) * KSTEP, LBO, 128);
     const uint64_t bl = tc::smem_desc((const char*)(b_hi + kW) + (k0 / 8 + ks) * KSTEP, LBO, 128);
-    tc::mma_tf32_ta(tmem, tmem + kOpHi + ks * 8, bh, idesc, (accumulate || ks > 0) ? 1u : 0u, 1u);
-    tc::mma_tf32_ta(tmem, tmem + kOpHi + ks * 8, bl, idesc, 1u, 1u);
-    tc::mma_tf32_ta(tmem, tmem + kOpLo + ks * 8, bh, idesc, 1u, 1u);
+    tc::mma_tf32_ta(tmem, tmem + kOpHi + ks * 8, bh, idesc, (accumulate || ks > 0) ? 1u : 0u, elected);
+    tc::mma_tf32_ta(tmem, tmem + kOpHi + ks * 8, bl, idesc, 1u, elected);
+    tc::mma_tf32_ta(tmem, tmem + kOpLo + ks * 8, bh, idesc, 1u, elected);
+  }
+}
+
+// ---- the forward's operands: fp16 hi + lo (22 bits, as TF32 hi + lo, at twice the rate and half the space), which need the
+// values of a row scaled by a power of two to below 2^14: both halves are normal numbers then, whatever the row's size.
+// half index of element (n, k) of an operand with N rows (K-major core matrices of 8 x 8, no swizzle)
+__host__ __device__ constexpr int pack_index16(int N, int n, int k) {
+  return (n >> 3) * 64 + (n & 7) * 8 + (k & 7) + ((k >> 3) & 1) * (N / 8) * 64 + (k >> 4) * (N / 8) * 128;
+}
+// this thread's 32 of 64 channel values -> operand columns (two channels a column: hi 32 columns, lo 32); `op`: this
+// thread's lane, its half's first column
+__device__ __forceinline__ void mix_stage16(uint32_t op, const float (&v)[32]) {
+  float hi[16], lo[16];
+#pragma unroll
+  for (int e = 0; e < 16; ++e) {
+    const __half2 h = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(v[2 * e] - f.x, v[2 * e + 1] - f.y);
+    hi[e] = __uint_as_float(*(const uint32_t*)&h);
+    lo[e] = __uint_as_float(*(const uint32_t*)&l);
+  }
+  mix_st16(op, hi);
+  mix_st16(op + 32u, lo);
+  tc::tmem_wait_st();
+}
+// D (+)= A[64 channels in the operand columns from `op` on] . B, B = N rows, K columns k0 .. k0 + 63 of a matrix packed with
+// pack_index16, lo behind hi; a whole warp
+template <int N>
+__device__ __forceinline__ void mix_mma16(uint32_t tmem, uint32_t op, const __half* b, int k0, bool accumulate, uint32_t elected) {
+  constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(N >> 3) << 17) | (8u << 24);     // fp16 operands, fp32 sums, M = 128
+  constexpr int LBO = (N / 8) * 128, KSTEP = 2 * LBO;
+#pragma unroll
+  for (int ks = 0; ks < 4; ++ks) {
+    const uint64_t bh = tc::smem_desc((const char*)b + (k0 / 16 + ks) * KSTEP, LBO, 128);
+    const uint64_t bl = tc::smem_desc((const char*)(b + kW) + (k0 / 16 + ks) * KSTEP, LBO, 128);
+    tc::mma_f16_ta(tmem, op + ks * 8, bh, idesc, (accumulate || ks > 0) ? 1u : 0u, elected);
+    tc::mma_f16_ta(tmem, op + ks * 8, bl, idesc, 1u, elected);
+    tc::mma_f16_ta(tmem, op + 32 + ks * 8, bh, idesc, 1u, elected);
   }
 }
 template <typename IO>
@@ -69,9 +108,9 @@ __device__ __forceinline__ void mix_bar(int g) {
   if (g == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
   else asm volatile("bar.sync 2, 256;" ::: "memory");
 }
-// centre and scale a pixel's 64 values, 32 of them here (the affine part is in the weights).  `mine`, `other`: this and
+// centre and scale a pixel's 64 values (and times `scale`), 32 of them here (the affine part is in the weights).  `mine`, `other`: this and
 // the partner thread's cell for (mean, sum of squared deviations) of a half; the two combine to the whole's.
-__device__ __forceinline__ float mix_norm(float (&v)[32], float eps, float2* mine, const float2* other, int g) {
+__device__ __forceinline__ float mix_norm(float (&v)[32], float eps, float2* mine, const float2* other, int g, float scale = 1.f) {
   float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll
   for (int c = 0; c < 32; c += 4) { s0 += v[c]; s1 += v[c + 1]; s2 += v[c + 2]; s3 += v[c + 3]; }
@@ -89,7 +128,7 @@ __device__ __forceinline__ float mix_norm(float (&v)[32], float eps, float2* min
   const float d = m0 - o.x, mean = 0.5f * (m0 + o.x);
   const float rstd = 1.0f / sqrtf(fmaf(16.f * d, d, q0 + o.y) * (1.0f / 64) + eps);
 #pragma unroll
-  for (int c = 0; c < 32; ++c) v[c] = (v[c] - mean) * rstd;
+  for (int c = 0; c < 32; ++c) v[c] = (v[c] - mean) * (rstd * scale);
   return rstd;
 }
 

@@ -7,19 +7,25 @@
 //
 // A block is two groups of 256 threads; each works on a 128-pixel tile of its own, so that one group's arithmetic
 // covers the other's MMAs.  Two threads share a pixel, 32 channels each (sixteen warps on an SM: with one thread per
-// pixel and eight warps 8 x 256 x 256 pixels of POST took 239 us); they meet only in LayerNorm, whose halves' means and
-// squared deviations go through shared memory.  Per contraction: the thread splits its values into TF32 hi + lo and
-// writes them to its lane of the group's operand columns (tcgen05.st, 64 channels at a time); after a barrier of the
-// group one thread issues hi hi + hi lo + lo hi with the weights from shared memory and commits to the group's mbarrier;
-// every thread then reads its half of its lane of the accumulator.  TMEM columns of group g at 256 g: accumulator
-// [0,128), operand hi [128,192), lo [192,256).  The weights, split and in operand layout, were packed once
-// (block_pack_kernel) and arrive by one bulk copy.  Pixels are addressed one by one (channel rows of any alignment, any
-// image size, fp32 or bf16); the values of the next tile are requested while the current one computes.
+// pixel and eight warps 8 x 256 x 256 pixels of POST took 239 us); they meet only in LayerNorm and in the scale of t, through
+// shared memory.  Per contraction: the thread splits its values into fp16 hi + lo and writes them to its lane of one of the
+// group's two operand buffers (tcgen05.st, 64 channels at a time); after a barrier of the group one warp issues
+// hi hi + hi lo + lo hi with the weights from shared memory and commits to the group's mbarrier; every thread then reads its
+// half of its lane of the accumulator.  TMEM columns of group g at 256 g: accumulator [0,128), operands [128,192) and
+// [192,256).  The weights, scaled, split and in operand layout, were packed once (block_pack_kernel) and arrive by one bulk
+// copy.  Pixels are addressed one by one (channel rows of any alignment, any image size, fp32 or bf16); the values of the
+// next tile are requested while the current one computes.
 //
-// What bounds it: bytes (PRE 3 C, POST 4 C channel planes), the MMAs (24 of 128x128x8 a tile for PRE, 72 of which 48 of
-// 128x64x8 for POST) and instruction issue (about 2400 and 4000 a warp and tile).  8 x 256 x 256 pixels, fp32: PRE and POST
-// take 337 us, their 940 MB would take 144.  PRE has 62 % of its issue slots busy and DRAM at 38 %; POST 43 % and 26 %, the
-// tensor pipe at 39 %, and waits for its 192 channel rows a tile: 202 KB of weights leave one block an SM and no ring.
+// fp16 hi + lo keeps 22 bits of a value like TF32 hi + lo, with K = 16 an MMA instead of 8 and half the space, as long as the
+// values lie high enough in fp16's range: rows of weights and pixels are scaled by powers of two.  A LayerNorm's values stay
+// below 8, the hidden ones below a bound that follows from the weights; t has any size, so a pixel takes its scale from its
+// first 64 channels, and if the others are more than 32 times as large its sums so far are scaled down in tensor memory.
+// With TF32 (twice as many MMAs, whose 46 cycles at least the two groups wait for together, and waits for one operand buffer)
+// 8 x 256 x 256 pixels took 103 us PRE and 232 POST, now 93 and 199; against fp64 PRE's error went from 5.9e-7 to 3.6e-7,
+// POST's from 1.0e-6 to 5.8e-7.
+//
+// What bounds it: bytes (PRE 3 C, POST 4 C channel planes: 61 and 82 us), loads of single 4-byte values, which fill the
+// load queue while a group waits, and instruction issue (about 2400 and 4000 a warp and tile).
 // Every wait is bounded; after a time-out a thread stops working but keeps meeting the group's barriers.
 #include "../../include/converse_b200.h"
 #include "cvb_internal.h"
@@ -27,9 +33,15 @@
 
 namespace cvb {
 
-// ---- packed weights: PRE | POST, each a multiple of 16 bytes
-constexpr int kPreFloats = 2 * kW + kBlkM;                      // W1 hi, lo; b1
-constexpr int kPostFloats = 6 * kW + 4 * kBlkC + kBlkM;         // W2, W3, W4 hi, lo; b2, a1, b4, a2; b3
+// ---- packed weights: PRE | POST, each a multiple of 16 bytes: matrices as fp16 hi and lo (16 KB each), every row scaled by a
+// power of two to below 2^14, then fp32 vectors.  The factors that undo the scales of a row and of its operand are in the
+// vectors: 1 / (row scale x kNormScale) for what follows a LayerNorm (its values stay below 8), for W4 with the scale of the
+// hidden values, of which a bound follows from W3 and b3; t is scaled pixel by pixel.
+constexpr float kNormScale = 1024.f;
+constexpr int kPreFloats = kW + 2 * kBlkM;                      // W1; b1, undo1
+constexpr int kPostFloats = 3 * kW + 6 * kBlkC + 2 * kBlkM + 4; // W2, W3, W4; b2, a1, b4, a2, undo2, undo4; b3, undo3; hidden scale
+enum { kB2 = 0, kA1 = kBlkC, kB4 = 2 * kBlkC, kA2 = 3 * kBlkC, kUndo2 = 4 * kBlkC, kUndo4 = 5 * kBlkC, kB3 = 6 * kBlkC,
+       kUndo3 = 6 * kBlkC + kBlkM, kHidden = 6 * kBlkC + 2 * kBlkM };
 size_t block_pack_bytes() { return (size_t)(kPreFloats + kPostFloats) * sizeof(float); }
 
 struct PackParams {
@@ -37,33 +49,69 @@ struct PackParams {
   float* out;
 };
 
+// the power of two that takes m to [2^13, 2^14) (1 for zero, infinities and NaN)
+__device__ __forceinline__ float to_2_14(float m) {
+  const int e = (int)(__float_as_uint(m) >> 23);
+  if (e == 0 || e >= 255) return 1.f;
+  const int f = 127 + 13 + 127 - e;      // (at most 2^100: its product with other scales stays finite)
+  return __uint_as_float((uint32_t)(f < 1 ? 1 : f > 227 ? 227 : f) << 23);
+}
+
 // grid: 4 matrices x 16 slices.  The LayerNorm affine is folded into the weights that follow it.
 __global__ void __launch_bounds__(256) block_pack_kernel(const PackParams P) {
-  const int which = blockIdx.x >> 4, slice = blockIdx.x & 15;
+  __shared__ float part[8];
+  const int which = blockIdx.x >> 4, slice = blockIdx.x & 15, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* post = P.out + kPreFloats;
   const float* w = which == 0 ? P.w1 : which == 1 ? P.w2 : which == 2 ? P.w3 : P.w4;
   const float* g = which == 0 ? P.ln1_w : which == 2 ? P.ln2_w : nullptr;
   const int N = which == 0 || which == 2 ? kBlkM : kBlkC, K = kW / N;
-  float* hi = which == 0 ? P.out : post + (which - 1) * 2 * kW;
-  for (int i = slice * (kW / 16) + threadIdx.x; i < (slice + 1) * (kW / 16); i += 256) {
-    const int n = i / K, k = i - n * K;
-    float a, b;
-    tc::split_tf32(g ? w[i] * g[k] : w[i], a, b);
-    hi[pack_index(N, n, k)] = a;
-    hi[kW + pack_index(N, n, k)] = b;
-  }
-  if (slice != 0) return;
-  float* vec = post + 6 * kW;
+  __half* hi = (__half*)(which == 0 ? P.out : post + (which - 1) * kW);
+  float* vec = which == 0 ? P.out + kW : post + 3 * kW;
   const float* bias = which == 0 ? P.b1 : which == 1 ? P.b2 : which == 2 ? P.b3 : P.b4;
   const float* beta = which == 0 ? P.ln1_b : which == 2 ? P.ln2_b : nullptr;
-  float* dst = which == 0 ? P.out + 2 * kW : which == 1 ? vec : which == 2 ? vec + 4 * kBlkC : vec + 2 * kBlkC;
-  for (int n = threadIdx.x; n < N; n += 256) {
-    float s = bias[n];
-    if (beta)
-      for (int k = 0; k < K; ++k) s = fmaf(w[n * K + k], beta[k], s);
-    dst[n] = s;
-    if (which == 1) vec[kBlkC + n] = P.a1 ? P.a1[n] : 1.0f;
-    if (which == 3) vec[3 * kBlkC + n] = P.a2 ? P.a2[n] : 1.0f;
+  // the hidden values' bound: |W3 . v + b3'| <= 8 |W3 row| + |b3'| for a normalised v of 64 values
+  float hidden = 1.f;
+  if (which == 3 || (which == 2 && slice == 0)) {
+    float most = 0.f;
+    for (int n = warp; n < kBlkM; n += 8) {
+      float q = 0.f, d = 0.f;
+      for (int k = lane; k < kBlkC; k += 32) {
+        const float a = P.w3[n * kBlkC + k];
+        q = fmaf(a * P.ln2_w[k], a * P.ln2_w[k], q);
+        d = fmaf(a, P.ln2_b[k], d);
+      }
+      for (int o = 16; o; o >>= 1) { q += __shfl_xor_sync(0xffffffffu, q, o); d += __shfl_xor_sync(0xffffffffu, d, o); }
+      most = fmaxf(most, 8.f * sqrtf(q) + fabsf(d + P.b3[n]));
+    }
+    if (lane == 0) part[warp] = most;
+    __syncthreads();
+    for (int i = 0; i < 8; ++i) most = fmaxf(most, part[i]);
+    hidden = to_2_14(1.001f * most);        // (of the rounding of the sums)
+    if (which == 2 && threadIdx.x == 0) vec[kHidden] = hidden;
+  }
+  const int rows = N / 16;
+  for (int r = warp; r < rows; r += 8) {
+    const int n = slice * rows + r;
+    float m = 0.f, d = 0.f;
+    for (int k = lane; k < K; k += 32) {
+      const float a = w[n * K + k];
+      m = fmaxf(m, fabsf(g ? a * g[k] : a));
+      if (beta) d = fmaf(a, beta[k], d);
+    }
+    for (int o = 16; o; o >>= 1) { m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o)); d += __shfl_xor_sync(0xffffffffu, d, o); }
+    const float f = to_2_14(m);
+    for (int k = lane; k < K; k += 32) {
+      const float a = (g ? w[n * K + k] * g[k] : w[n * K + k]) * f;
+      const __half h = __float2half_rn(a);
+      hi[pack_index16(N, n, k)] = h;
+      hi[kW + pack_index16(N, n, k)] = __float2half_rn(a - __half2float(h));
+    }
+    if (lane) continue;
+    const float b = bias[n] + d;
+    if (which == 0) { vec[n] = b; vec[kBlkM + n] = 1.f / (f * kNormScale); }
+    if (which == 1) { vec[kB2 + n] = b; vec[kUndo2 + n] = 1.f / f; vec[kA1 + n] = P.a1 ? P.a1[n] : 1.f; }
+    if (which == 2) { vec[kB3 + n] = b; vec[kUndo3 + n] = 1.f / (f * kNormScale); }
+    if (which == 3) { vec[kB4 + n] = b; vec[kUndo4 + n] = 1.f / f / hidden; vec[kA2 + n] = P.a2 ? P.a2[n] : 1.f; }
   }
 }
 
@@ -96,16 +144,16 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
   pdl_start();
   constexpr int kFloats = POST ? kPostFloats : kPreFloats;
   float* wts = msm;
-  const float* vec = wts + (POST ? 6 : 2) * kW;    // PRE: b1.  POST: b2, a1, b4, a2, b3
-  uint64_t* bars = (uint64_t*)(msm + kFloats);      // MMA of group 0, 1; weights
-  uint32_t* holder = (uint32_t*)(bars + 3);
+  const float* vec = wts + (POST ? 3 : 1) * kW;     // (see block_pack_kernel)
+  uint64_t* bars = (uint64_t*)(msm + kFloats);      // MMA of group 0, 1; weights; first half of t of group 0, 1
+  uint32_t* holder = (uint32_t*)(bars + 5);
   float2* halves = (float2*)(holder + 2);           // [group][half][pixel]
-  const int tid = threadIdx.x, warp = tid >> 5, g = tid >> 8, m = tid & 127, hf = (tid >> 7) & 1;
-  const bool lead = (tid & 255) == 0;
+  const int tid = threadIdx.x, warp = (int)tc::from_first(tid >> 5), g = warp >> 3, m = tid & 127, hf = (tid >> 7) & 1;
+  const bool lead = (warp & 7) == 0;               // the warp that issues the group's MMAs
   float2* mine = halves + (g * 2 + hf) * 128 + m;
   const float2* other = halves + (g * 2 + (hf ^ 1)) * 128 + m;
   if (tid == 0) {
-    for (int i = 0; i < 3; ++i) mbar_init(&bars[i], 1);
+    for (int i = 0; i < 5; ++i) mbar_init(&bars[i], 1);
     mbar_fence_init();
     mbar_expect_tx(&bars[2], kFloats * 4);
     bulk_g2s(wts, P.pack + (POST ? kPreFloats : 0), kFloats * 4, &bars[2]);
@@ -114,10 +162,11 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  const uint32_t tmem = *holder + 256u * (uint32_t)g;
+  const uint32_t tmem = tc::from_first(*holder) + 256u * (uint32_t)g;
   const uint32_t lane = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 32u * (uint32_t)hf;   // 32 columns a thread
+  const uint32_t op = lane + 128u - 16u * (uint32_t)hf;        // its 16 columns of the first operand buffer, the second 64 on
   uint64_t* done = &bars[g];
-  uint32_t uses = 0;                                // commits of this group so far
+  uint32_t uses = 0, tiles = 0;                     // commits of this group so far, tiles
   bool ok = true;
 
   const long long ntiles = (P.npix + 127) / 128, step = 2ll * gridDim.x;
@@ -159,7 +208,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
     int npos = 0;
     if (ntile < ntiles) place(ntile, nvalid, nimg, npos);
     const IO* next = (const IO*)(POST ? P.t : P.x) + (size_t)nimg * Cin * HW + npos + half_off;
-    IO* op = (IO*)P.out + (size_t)img * Cout * HW + pos + (POST ? half_off : 2 * half_off);
+    IO* op_out = (IO*)P.out + (size_t)img * Cout * HW + pos + (POST ? half_off : 2 * half_off);
     {
       // the tile after: rows of its first pixel in this warp
       const long long npix0 = ntile * 128 + (m & ~31);
@@ -175,10 +224,14 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
       }
     }
     if constexpr (!POST) {
-      mix_norm(v, P.eps, mine, other, g);
-      mix_stage(lane, v);
+      mix_norm(v, P.eps, mine, other, g, kNormScale);
+      mix_stage16(op, v);
       publish();
-      if (lead && ok) { mix_mma<128>(tmem, wts, 0, false); tc::mma_commit(done); }
+      if (lead) {
+        const uint32_t e = tc::elect_one() & (ok ? 1u : 0u);
+        mix_mma16<128>(tmem, tmem + 128u, (const __half*)wts, 0, false, e);
+        if (e) tc::mma_commit(done);
+      }
       mix_load<IO>(v, next, HW, nvalid);
       commit_wait();
 #pragma unroll 1
@@ -189,91 +242,123 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
 #ifdef __CUDA_ARCH__
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
-            const float2 b = *(const float2*)(vec + 64 * hf + c0 + j);
-            const float za = a[j] + b.x, zb = a[j + 1] + b.y;
+            const float2 b = *(const float2*)(vec + 64 * hf + c0 + j), u = *(const float2*)(vec + kBlkM + 64 * hf + c0 + j);
+            const float za = fmaf(a[j], u.x, b.x), zb = fmaf(a[j + 1], u.y, b.y);
             const float2 o = gelu_fast2(za, zb);
             if (TRAIN) {
-              float* zp = P.z + (op - (IO*)P.out);
+              float* zp = P.z + (op_out - (IO*)P.out);
               zp[(size_t)(c0 + j) * HW] = za;
               zp[(size_t)(c0 + j + 1) * HW] = zb;
             }
-            st_io<IO>(op, (size_t)(c0 + j) * HW, o.x);
-            st_io<IO>(op, (size_t)(c0 + j + 1) * HW, o.y);
+            st_io<IO>(op_out, (size_t)(c0 + j) * HW, o.x);
+            st_io<IO>(op_out, (size_t)(c0 + j + 1) * HW, o.y);
           }
 #endif
         }
       }
     } else {
-      const float *w2 = wts, *w3 = wts + 2 * kW, *w4 = wts + 4 * kW;
-      const float* vh = vec + 32 * hf;              // this thread's channels of b2, a1, b4, a2
+      const __half *w2 = (const __half*)wts, *w3 = w2 + 2 * kW, *w4 = w3 + 2 * kW;
+      const float* vh = vec + 32 * hf;              // this thread's channels of the vectors
       float x1[32];
       mix_load<IO>(x1, (const IO*)P.x + (size_t)img * kBlkC * HW + pos + half_off, HW, valid);
-      // five operands of 64 channels: t (two halves), LN(x1), GELU (two halves).  One copy of the staging code: the whole
-      // kernel has to stay in the instruction cache.
+      float undo = 1.f;                             // of the scale of t
+      int top = 0;                                  //   and its exponent
+      // five operands of 64 channels: t (two halves), LN(x1), GELU (two halves), in two buffers by turns.  One copy of the
+      // staging code: the whole kernel has to stay in the instruction cache.
 #pragma unroll 1
       for (int ph = 0; ph < 5; ++ph) {
-        if (ph == 1) {
-          commit_wait();
-        } else if (ph == 2) {                       // x1 = x + a1 (W2 . t + b2)
+        if (ph == 2) {                              // x1 = x + a1 (W2 . t + b2)
           commit_wait();
           float a[32];
           tc::tmem_ld32(lane, a);
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            x1[j] = fmaf(vh[kBlkC + j], a[j] + vh[j], x1[j]);
+            x1[j] = fmaf(vh[kA1 + j], fmaf(a[j] * undo, vh[kUndo2 + j], vh[kB2 + j]), x1[j]);
             v[j] = x1[j];
-            if (TRAIN && valid) P.x1[(op - (IO*)P.out) + (size_t)j * HW] = x1[j];
+            if (TRAIN && valid) P.x1[(op_out - (IO*)P.out) + (size_t)j * HW] = x1[j];
           }
-          mix_norm(v, P.eps, mine, other, g);
+          mix_norm(v, P.eps, mine, other, g, kNormScale);
         } else if (ph >= 3) {                       // GELU of 32 of 64 hidden channels
           const int h0 = 64 * (ph - 3);
           if (ph == 3) commit_wait();
           float a[32];
           tc::tmem_ld32(lane + (uint32_t)h0, a);
 #ifdef __CUDA_ARCH__
+          const float hs = vec[kHidden];
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
-            const float2 b = *(const float2*)(vh + 4 * kBlkC + h0 + j);
-            const float za = a[j] + b.x, zb = a[j + 1] + b.y;
+            const float2 b = *(const float2*)(vh + kB3 + h0 + j), u = *(const float2*)(vh + kUndo3 + h0 + j);
+            const float za = fmaf(a[j], u.x, b.x), zb = fmaf(a[j + 1], u.y, b.y);
             const float2 o = gelu_fast2(za, zb);
             if (TRAIN && valid) {
               float* zp = P.z + ((size_t)img * kBlkM + h0) * HW + pos + half_off;
               zp[(size_t)j * HW] = za;
               zp[(size_t)(j + 1) * HW] = zb;
             }
-            v[j] = o.x; v[j + 1] = o.y;
+            v[j] = o.x * hs; v[j + 1] = o.y * hs;
           }
 #endif
-          if (ph == 4) commit_wait();               // the MMAs of the first half have read the operand columns
-        }
+        } else {                                    // 64 channels of t
 #ifdef __CUDA_ARCH__
-        if (TRAIN && ph < 2) {
+          if (TRAIN) {
 #pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const float2 o = gelu_fast2(v[j], v[j + 1]);
-            v[j] = o.x; v[j + 1] = o.y;
+            for (int j = 0; j < 32; j += 2) {
+              const float2 o = gelu_fast2(v[j], v[j + 1]);
+              v[j] = o.x; v[j + 1] = o.y;
+            }
           }
-        }
 #endif
-        mix_stage(lane, v);
+          // the pixel's largest magnitude goes to [2^10, 2^11): the other half may be 32 times as large
+          float m = 0.f;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) m = fmaxf(m, fabsf(v[j]));
+          mine->x = m;
+          mix_bar(g);
+          const int e = min(max((int)(__float_as_uint(fmaxf(m, other->x)) >> 23), 32), 254);
+          if (ph == 0) {
+            top = e;
+          } else if (__any_sync(0xffffffffu, e > top + 4)) {       // it is larger still: the sums so far are scaled down
+            if (ok) ok = mbar_wait_bounded(&bars[3 + g], tiles & 1u, kWaitLimit);
+            tc::fence_after_sync();
+            const int by = e > top + 4 ? e - top : 0;
+            const float f = by > 126 ? 0.f : __uint_as_float((uint32_t)(127 - by) << 23);
+            top += by;
+            float a[32];
+            tc::tmem_ld32(lane, a);
+            float b0[16], b1[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) { b0[j] = a[j] * f; b1[j] = a[16 + j] * f; }
+            mix_st16(lane, b0);
+            mix_st16(lane + 16u, b1);
+            tc::tmem_wait_st();
+          }
+          const float s = __uint_as_float((uint32_t)min(264 - top, 254) << 23);       // 2^(10 - exponent)
+          undo = 1.f / s;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] *= s;
+        }
+        const uint32_t buf = 64u * (uint32_t)(ph & 1);
+        mix_stage16(op + buf, v);
         publish();                                  // (the accumulator's first 64 columns have been read by ph = 3)
-        if (lead && ok) {
-          if (ph == 2) mix_mma<128>(tmem, w3, 0, false);
-          else mix_mma<64>(tmem, ph < 2 ? w2 : w4, ph == 1 || ph == 4 ? 64 : 0, ph == 1 || ph == 4);
-          tc::mma_commit(done);
+        if (lead) {
+          const uint32_t e = tc::elect_one() & (ok ? 1u : 0u);
+          if (ph == 2) mix_mma16<128>(tmem, tmem + 128u + buf, w3, 0, false, e);
+          else mix_mma16<64>(tmem, tmem + 128u + buf, ph < 2 ? w2 : w4, ph == 1 || ph == 4 ? 64 : 0, ph == 1 || ph == 4, e);
+          if (e && ph != 3) tc::mma_commit(ph == 0 ? &bars[3 + g] : done);
         }
         if (ph == 0 || ph == 4) {                   // the second half of t; the next tile
           const IO* q = ph == 0 ? (const IO*)P.t + ((size_t)img * Cin + 64) * HW + pos + half_off : next;
           mix_load<IO>(v, q, HW, ph == 0 ? valid : nvalid);
         }
       }
+      tiles += 1;
       commit_wait();
       float a[32];
       tc::tmem_ld32(lane, a);
       if (valid && ok) {
 #pragma unroll
         for (int j = 0; j < 32; ++j)
-          st_io<IO>(op, (size_t)j * HW, fmaf(vh[3 * kBlkC + j], a[j] + vh[2 * kBlkC + j], x1[j]));
+          st_io<IO>(op_out, (size_t)j * HW, fmaf(vh[kA2 + j], fmaf(a[j], vh[kUndo4 + j], vh[kB4 + j]), x1[j]));
       }
     }
     valid = nvalid; img = nimg; pos = npos;
@@ -286,7 +371,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
 
 template <bool POST, typename IO, bool TRAIN = false>
 static int launch_mix(const MixParams& P, int sms, cudaStream_t st) {
-  const size_t smem = (size_t)(POST ? kPostFloats : kPreFloats) * sizeof(float) + 3 * sizeof(uint64_t) + 8 + 512 * sizeof(float2) + 16;
+  const size_t smem = (size_t)(POST ? kPostFloats : kPreFloats) * sizeof(float) + 5 * sizeof(uint64_t) + 8 + 512 * sizeof(float2) + 16;
   const int rc = allow_smem(block_mix_kernel<POST, IO, TRAIN>, smem);
   if (rc != CVB_OK) return rc;
   const long long ntiles = (P.npix + 127) / 128;

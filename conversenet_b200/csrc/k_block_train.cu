@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_grad_kernel(const __grid
       mix_load<float>(v, P.in + at64, HW, valid);
       mix_stage(lane, v);
       publish();
-      if (lead && ok) { mix_mma<128>(tmem, wts, 0, false); tc::mma_commit(done); }
+      if (lead && ok) { mix_mma<128>(tmem, wts, 0, false, 1u); tc::mma_commit(done); }
       const size_t at = ((size_t)img * kBlkM + 64 * hf) * HW + pos;
       mix_load<float>(v, P.z + at, HW, valid);
       commit_wait();
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_grad_kernel(const __grid
         if (ph) commit_wait();
         mix_stage(lane, v);
         publish();
-        if (lead && ok) { mix_mma<64>(tmem, wts, 64 * ph, ph != 0); tc::mma_commit(done); }
+        if (lead && ok) { mix_mma<64>(tmem, wts, 64 * ph, ph != 0, 1u); tc::mma_commit(done); }
       }
       mix_load<float>(v, P.x + at64, HW, valid);
       const float rstd = mix_norm(v, P.eps, mine, other, g);
