@@ -97,13 +97,6 @@ __device__ __forceinline__ void mix_load(float (&v)[32], const IO* p, int HW, bo
 #pragma unroll
   for (int c = 0; c < 32; ++c) v[c] = valid ? ld_io<IO>(p, (size_t)c * HW) : 0.f;
 }
-// Ask L2 for a warp's 32 pixels of 32 channel rows, one row a lane: loads issued a phase before their use arrive from DRAM
-// too late, loads of prefetched rows less so (waits for loads are still the largest share of POST's stalls, three of nine
-// warps per issue).  `p`: the first pixel of the thread's first channel.
-template <typename IO>
-__device__ __forceinline__ void mix_prefetch(const IO* p, int HW) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(p + (size_t)(threadIdx.x & 31) * HW));
-}
 __device__ __forceinline__ void mix_bar(int g) {
   if (g == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
   else asm volatile("bar.sync 2, 256;" ::: "memory");

@@ -13,19 +13,20 @@
 // hi hi + hi lo + lo hi with the weights from shared memory and commits to the group's mbarrier; every thread then reads its
 // half of its lane of the accumulator.  TMEM columns of group g at 256 g: accumulator [0,128), operands [128,192) and
 // [192,256).  The weights, scaled, split and in operand layout, were packed once (block_pack_kernel) and arrive by one bulk
-// copy.  Pixels are addressed one by one (channel rows of any alignment, any image size, fp32 or bf16); the values of the
-// next tile are requested while the current one computes.
+// copy.  Rows that are 16-byte aligned are copied to shared memory two phases and more ahead of their use, each warp its own
+// 32 channels x 32 pixels; others are loaded pixel by pixel (any image size and alignment, fp32 or bf16).
 //
 // fp16 hi + lo keeps 22 bits of a value like TF32 hi + lo, with K = 16 an MMA instead of 8 and half the space, as long as the
 // values lie high enough in fp16's range: rows of weights and pixels are scaled by powers of two.  A LayerNorm's values stay
 // below 8, the hidden ones below a bound that follows from the weights; t has any size, so a pixel takes its scale from its
 // first 64 channels, and if the others are more than 32 times as large its sums so far are scaled down in tensor memory.
 // With TF32 (twice as many MMAs, whose 46 cycles at least the two groups wait for together, and waits for one operand buffer)
-// 8 x 256 x 256 pixels took 103 us PRE and 232 POST, now 93 and 199; against fp64 PRE's error went from 5.9e-7 to 3.6e-7,
-// POST's from 1.0e-6 to 5.8e-7.
+// 8 x 256 x 256 pixels took 103 us PRE and 232 POST, with fp16 93 and 199, with the copies ahead 81 and 164; against fp64
+// PRE's error went from 5.9e-7 to 3.6e-7, POST's from 1.0e-6 to 5.8e-7.
 //
-// What bounds it: bytes (PRE 3 C, POST 4 C channel planes: 61 and 82 us), loads of single 4-byte values, which fill the
-// load queue while a group waits, and instruction issue (about 2400 and 4000 a warp and tile).
+// What bounds it: bytes (PRE 3 C, POST 4 C channel planes: 61 and 82 us) and, in POST, a group's chain of five contractions
+// with the arithmetic between them.  Registers spilled to local memory cost far more than their number suggests, because the
+// shared memory leaves the L1 cache next to nothing (POST with 33 words spilled: 192 us).
 // Every wait is bounded; after a time-out a thread stops working but keeps meeting the group's barriers.
 #include "../../include/converse_b200.h"
 #include "cvb_internal.h"
@@ -136,22 +137,28 @@ struct MixParams {
   float *z, *x1;        // TRAIN: (B,128,HW), (B,64,HW)
 };
 
+// Shared memory behind the weights: every warp has two slots for 32 channels of its 32 pixels
+constexpr int kSlot = 32 * 32 * 4, kRing = 16 * 2 * kSlot;
+
+__device__ __forceinline__ void mix_copy(void* dst, const void* src, bool in) {       // zeros where `in` is false
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+
 // TRAIN (fp32): also keeps what the gradients need -- PRE the hidden layer before its GELU (z), POST x1 and the hidden
-// layer before its GELU -- and POST takes t before ITS GELU.
-template <bool POST, typename IO, bool TRAIN>
+// layer before its GELU -- and POST takes t before ITS GELU.  COPIES: rows are 16-byte aligned and reach shared memory by
+// asynchronous copies ahead of their use.
+template <bool POST, typename IO, bool TRAIN, bool COPIES>
 __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_constant__ MixParams P) {
   extern __shared__ __align__(128) float msm[];
   pdl_start();
   constexpr int kFloats = POST ? kPostFloats : kPreFloats;
   float* wts = msm;
   const float* vec = wts + (POST ? 3 : 1) * kW;     // (see block_pack_kernel)
-  uint64_t* bars = (uint64_t*)(msm + kFloats);      // MMA of group 0, 1; weights; first half of t of group 0, 1
+  unsigned char* ring = (unsigned char*)(msm + kFloats);
+  uint64_t* bars = (uint64_t*)(ring + kRing);       // MMA of group 0, 1; weights; first half of t of group 0, 1
   uint32_t* holder = (uint32_t*)(bars + 5);
-  float2* halves = (float2*)(holder + 2);           // [group][half][pixel]
-  const int tid = threadIdx.x, warp = (int)tc::from_first(tid >> 5), g = warp >> 3, m = tid & 127, hf = (tid >> 7) & 1;
+  const int tid = threadIdx.x, warp = (int)tc::from_first(tid >> 5), ln = tid & 31, g = warp >> 3, m = tid & 127, hf = (warp >> 2) & 1;
   const bool lead = (warp & 7) == 0;               // the warp that issues the group's MMAs
-  float2* mine = halves + (g * 2 + hf) * 128 + m;
-  const float2* other = halves + (g * 2 + (hf ^ 1)) * 128 + m;
   if (tid == 0) {
     for (int i = 0; i < 5; ++i) mbar_init(&bars[i], 1);
     mbar_fence_init();
@@ -171,13 +178,17 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
 
   const long long ntiles = (P.npix + 127) / 128, step = 2ll * gridDim.x;
   const int HW = P.HW;
-  const int Cin = POST ? kBlkM : kBlkC, Cout = POST ? kBlkC : kBlkM;
-  // this thread's pixel of a tile: image, position
-  auto place = [&](long long tile, bool& valid, long long& img, int& pos) {
-    const long long pix = tile * 128 + m;
-    valid = pix < P.npix;
-    img = valid ? pix / HW : 0;
-    pos = valid ? (int)(pix - img * HW) : 0;
+  constexpr int Cin = POST ? kBlkM : kBlkC, Cout = POST ? kBlkC : kBlkM;
+  const IO* const in = (const IO*)(POST ? P.t : P.x) + (size_t)(32 * hf) * HW;      // this warp's channels of the first item
+  // a pixel of a tile: image, position in it
+  struct Place { bool valid; int img, pos; };
+  auto place = [&](long long tile, int at) {
+    const long long pix = tile * 128 + at;
+    Place q;
+    q.valid = pix < P.npix;
+    q.img = !q.valid ? 0 : P.npix <= 0xffffffffll ? (int)((uint32_t)pix / (uint32_t)HW) : (int)(pix / HW);
+    q.pos = q.valid ? (int)(pix - (long long)q.img * HW) : 0;
+    return q;
   };
   auto commit_wait = [&]() {                        // the group's last MMAs have finished
     if (ok) ok = mbar_wait_bounded(done, uses & 1u, kWaitLimit);
@@ -189,42 +200,53 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
     mix_bar(g);
     tc::fence_after_sync();
   };
+  // ---- the way of the input: items of 32 channels x 32 pixels, a warp's own, in the order they are needed (POST: t, t, x of
+  // a tile), two slots by turns.  An item is asked for when the one before last has been used up, two phases or more before
+  // its use; single 4-byte loads into registers, a phase ahead, had the warps wait for their load queue two fifths of the
+  // time.  Rows that are not 16-byte aligned keep those: 4-byte copies are slower (2 x 111 x 167 pixels: 23.3 us against 18.5).
+  constexpr int PX = 16 / (int)sizeof(IO), CH = 32 / PX, RS = 32 / CH;      // pixels of a copy, copies of a row, rows a step
+  const int first_px = (m & ~31) + ln % CH * PX;
+  uint32_t item = 0;                                // items used so far
+  auto slot = [&](int w, uint32_t i) { return ring + (w * 2 + (int)(i & 1u)) * kSlot; };
+  auto ask = [&](uint32_t i, const IO* from, int channels, const Place& q) {
+    const int r = ln / CH;
+    unsigned char* dst = slot(warp, i) + r * 32 * (int)sizeof(IO) + ln % CH * 16;
+    const IO* src = q.valid ? from + ((size_t)q.img * channels + r) * HW + q.pos : from;
+    const size_t rows = q.valid ? (size_t)RS * HW : 0;
+#pragma unroll
+    for (int c = 0; c < 32; c += RS, src += rows) mix_copy(dst + c * 32 * (int)sizeof(IO), src, q.valid);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // the next item's values of this thread's pixel (without copies: they are in v already)
+  auto take = [&](float (&v)[32]) {
+    if (!COPIES) return;
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+    const IO* p = (const IO*)slot(warp, item) + ln;
+#pragma unroll
+    for (int c = 0; c < 32; ++c) v[c] = ld_io<IO>(p, (size_t)(c * 32));
+    __syncwarp();
+  };
+  // a cell of the slot just used up, and the one of the other thread of the pixel
+  auto mine = [&]() { return (float2*)slot(warp, item) + ln; };
+  auto other = [&]() { return (const float2*)slot(warp ^ 4, item) + ln; };
 
   long long tile = blockIdx.x + (long long)g * gridDim.x;
-  bool valid = false;
-  long long img = 0;
-  int pos = 0;
-  const size_t half_off = (size_t)(32 * hf) * HW;
+  Place here = place(tile, m);
   float v[32];
-  if (tile < ntiles) {
-    place(tile, valid, img, pos);
-    mix_load<IO>(v, (const IO*)(POST ? P.t : P.x) + (size_t)img * Cin * HW + pos + half_off, HW, valid);
+  if (!COPIES) {
+    mix_load<IO>(v, in + (size_t)here.img * Cin * HW + here.pos, HW, here.valid);
+  } else {
+    ask(0, in, Cin, place(tile, first_px));
+    ask(1, in + (POST ? (size_t)64 * HW : 0), Cin, place(POST ? tile : tile + step, first_px));
   }
   if (ok) ok = mbar_wait_bounded(&bars[2], 0, kWaitLimit);   // weights
   for (; tile < ntiles; tile += step) {
-    const long long ntile = tile + step;
-    bool nvalid = false;
-    long long nimg = 0;
-    int npos = 0;
-    if (ntile < ntiles) place(ntile, nvalid, nimg, npos);
-    const IO* next = (const IO*)(POST ? P.t : P.x) + (size_t)nimg * Cin * HW + npos + half_off;
-    IO* op_out = (IO*)P.out + (size_t)img * Cout * HW + pos + (POST ? half_off : 2 * half_off);
-    {
-      // the tile after: rows of its first pixel in this warp
-      const long long npix0 = ntile * 128 + (m & ~31);
-      if (npix0 < P.npix) {
-        const long long i0 = npix0 / HW;
-        const size_t p0 = (size_t)(npix0 - i0 * HW) + half_off;
-        const IO* q = (const IO*)(POST ? P.t : P.x) + (size_t)i0 * Cin * HW + p0;
-        mix_prefetch<IO>(q, HW);
-        if (POST) {
-          mix_prefetch<IO>(q + (size_t)64 * HW, HW);
-          mix_prefetch<IO>((const IO*)P.x + (size_t)i0 * kBlkC * HW + p0, HW);
-        }
-      }
-    }
+    const bool valid = here.valid;
+    IO* op_out = (IO*)P.out + ((size_t)here.img * Cout + (POST ? 32 : 64) * hf) * HW + here.pos;
     if constexpr (!POST) {
-      mix_norm(v, P.eps, mine, other, g, kNormScale);
+      take(v);
+      mix_norm(v, P.eps, mine(), other(), g, kNormScale);
       mix_stage16(op, v);
       publish();
       if (lead) {
@@ -232,7 +254,13 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
         mix_mma16<128>(tmem, tmem + 128u, (const __half*)wts, 0, false, e);
         if (e) tc::mma_commit(done);
       }
-      mix_load<IO>(v, next, HW, nvalid);
+      if (!COPIES) {
+        const Place q = place(tile + step, m);
+        mix_load<IO>(v, in + (size_t)q.img * Cin * HW + q.pos, HW, q.valid);
+      } else {
+        ask(item + 2, in, Cin, place(tile + 2 * step, first_px));
+      }
+      item += 1;
       commit_wait();
 #pragma unroll 1
       for (int c0 = 0; c0 < 64; c0 += 32) {         // 64 of the 128 output channels
@@ -260,7 +288,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
       const __half *w2 = (const __half*)wts, *w3 = w2 + 2 * kW, *w4 = w3 + 2 * kW;
       const float* vh = vec + 32 * hf;              // this thread's channels of the vectors
       float x1[32];
-      mix_load<IO>(x1, (const IO*)P.x + (size_t)img * kBlkC * HW + pos + half_off, HW, valid);
+      if (!COPIES) mix_load<IO>(x1, (const IO*)P.x + ((size_t)here.img * kBlkC + 32 * hf) * HW + here.pos, HW, valid);
       float undo = 1.f;                             // of the scale of t
       int top = 0;                                  //   and its exponent
       // five operands of 64 channels: t (two halves), LN(x1), GELU (two halves), in two buffers by turns.  One copy of the
@@ -268,16 +296,17 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
 #pragma unroll 1
       for (int ph = 0; ph < 5; ++ph) {
         if (ph == 2) {                              // x1 = x + a1 (W2 . t + b2)
+          if (COPIES) take(v);
           commit_wait();
           float a[32];
           tc::tmem_ld32(lane, a);
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            x1[j] = fmaf(vh[kA1 + j], fmaf(a[j] * undo, vh[kUndo2 + j], vh[kB2 + j]), x1[j]);
+            x1[j] = fmaf(vh[kA1 + j], fmaf(a[j] * undo, vh[kUndo2 + j], vh[kB2 + j]), COPIES ? v[j] : x1[j]);
             v[j] = x1[j];
             if (TRAIN && valid) P.x1[(op_out - (IO*)P.out) + (size_t)j * HW] = x1[j];
           }
-          mix_norm(v, P.eps, mine, other, g, kNormScale);
+          mix_norm(v, P.eps, mine(), other(), g, kNormScale);
         } else if (ph >= 3) {                       // GELU of 32 of 64 hidden channels
           const int h0 = 64 * (ph - 3);
           if (ph == 3) commit_wait();
@@ -291,7 +320,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
             const float za = fmaf(a[j], u.x, b.x), zb = fmaf(a[j + 1], u.y, b.y);
             const float2 o = gelu_fast2(za, zb);
             if (TRAIN && valid) {
-              float* zp = P.z + ((size_t)img * kBlkM + h0) * HW + pos + half_off;
+              float* zp = P.z + ((size_t)here.img * kBlkM + h0 + 32 * hf) * HW + here.pos;
               zp[(size_t)j * HW] = za;
               zp[(size_t)(j + 1) * HW] = zb;
             }
@@ -299,6 +328,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
           }
 #endif
         } else {                                    // 64 channels of t
+          take(v);
 #ifdef __CUDA_ARCH__
           if (TRAIN) {
 #pragma unroll
@@ -309,12 +339,12 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
           }
 #endif
           // the pixel's largest magnitude goes to [2^10, 2^11): the other half may be 32 times as large
-          float m = 0.f;
+          float most = 0.f;
 #pragma unroll
-          for (int j = 0; j < 32; ++j) m = fmaxf(m, fabsf(v[j]));
-          mine->x = m;
+          for (int j = 0; j < 32; ++j) most = fmaxf(most, fabsf(v[j]));
+          mine()->x = most;
           mix_bar(g);
-          const int e = min(max((int)(__float_as_uint(fmaxf(m, other->x)) >> 23), 32), 254);
+          const int e = min(max((int)(__float_as_uint(fmaxf(most, other()->x)) >> 23), 32), 254);
           if (ph == 0) {
             top = e;
           } else if (__any_sync(0xffffffffu, e > top + 4)) {       // it is larger still: the sums so far are scaled down
@@ -346,10 +376,17 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
           else mix_mma16<64>(tmem, tmem + 128u + buf, ph < 2 ? w2 : w4, ph == 1 || ph == 4 ? 64 : 0, ph == 1 || ph == 4, e);
           if (e && ph != 3) tc::mma_commit(ph == 0 ? &bars[3 + g] : done);
         }
-        if (ph == 0 || ph == 4) {                   // the second half of t; the next tile
-          const IO* q = ph == 0 ? (const IO*)P.t + ((size_t)img * Cin + 64) * HW + pos + half_off : next;
-          mix_load<IO>(v, q, HW, ph == 0 ? valid : nvalid);
+        // what comes after next: x after the first half of t, then the next tile's two halves
+        if (!COPIES) {
+          if (ph == 0 || ph == 4) {
+            const Place q = ph == 4 ? place(tile + step, m) : here;
+            mix_load<IO>(v, in + (ph == 0 ? (size_t)64 * HW : 0) + (size_t)q.img * Cin * HW + q.pos, HW, q.valid);
+          }
+        } else if (ph < 3) {
+          ask(item + 2, ph == 0 ? (const IO*)P.x + (size_t)(32 * hf) * HW : in + (ph == 2 ? (size_t)64 * HW : 0),
+              ph == 0 ? kBlkC : kBlkM, place(ph == 0 ? tile : tile + step, first_px));
         }
+        if (ph < 3) item += 1;
       }
       tiles += 1;
       commit_wait();
@@ -361,7 +398,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
           st_io<IO>(op_out, (size_t)j * HW, fmaf(vh[kA2 + j], fmaf(a[j], vh[kUndo4 + j], vh[kB4 + j]), x1[j]));
       }
     }
-    valid = nvalid; img = nimg; pos = npos;
+    here = place(tile + step, m);
   }
   if (!ok && P.status) atomicExch(P.status, 3);
   tc::fence_before_sync();
@@ -369,14 +406,19 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
   if (warp == 0) tc::tmem_dealloc(*holder, 512);
 }
 
-template <bool POST, typename IO, bool TRAIN = false>
-static int launch_mix(const MixParams& P, int sms, cudaStream_t st) {
-  const size_t smem = (size_t)(POST ? kPostFloats : kPreFloats) * sizeof(float) + 5 * sizeof(uint64_t) + 8 + 512 * sizeof(float2) + 16;
-  const int rc = allow_smem(block_mix_kernel<POST, IO, TRAIN>, smem);
+template <bool POST, typename IO, bool TRAIN, bool COPIES>
+static int launch_one(const MixParams& P, int sms, cudaStream_t st) {
+  const size_t smem = (size_t)(POST ? kPostFloats : kPreFloats) * sizeof(float) + kRing + 5 * sizeof(uint64_t) + 8;
+  const int rc = allow_smem(block_mix_kernel<POST, IO, TRAIN, COPIES>, smem);
   if (rc != CVB_OK) return rc;
   const long long ntiles = (P.npix + 127) / 128;
   const int grid = (int)(ntiles < sms ? ntiles : sms);     // one block per SM; tiles go round the blocks first
-  return launch_chained(block_mix_kernel<POST, IO, TRAIN>, dim3(grid), kMixThreads, smem, st, P);
+  return launch_chained(block_mix_kernel<POST, IO, TRAIN, COPIES>, dim3(grid), kMixThreads, smem, st, P);
+}
+template <bool POST, typename IO, bool TRAIN = false>
+static int launch_mix(const MixParams& P, int sms, cudaStream_t st) {
+  const size_t at = (size_t)P.x | (size_t)(POST ? P.t : P.x) | (size_t)P.HW * sizeof(IO);
+  return at % 16 == 0 ? launch_one<POST, IO, TRAIN, true>(P, sms, st) : launch_one<POST, IO, TRAIN, false>(P, sms, st);
 }
 
 int launch_block_mix(bool post, const void* x, const void* t, void* out, const void* pack, float eps, int B, int HW,

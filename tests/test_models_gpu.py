@@ -240,3 +240,61 @@ def test_block_kernels_with_the_operand_in_tensor_memory(dtype):
         assert float((got2.float() - want2).norm() / want2.norm()) <= tol, shape
         assert float((out.float() - ref.float()).norm() / ref.float().norm()) <= tol
         assert float((got2.float() - ref2.float()).norm() / ref2.float().norm()) <= tol
+
+
+@pytest.mark.parametrize("B, H, W, dtype, t_kind", [
+    (1, 8, 16, torch.float32, "plain"),           # one tile
+    (3, 20, 25, torch.float32, "up"),             # 500 pixels: 16-byte rows, tiles across images, the last one short
+    (3, 20, 24, torch.bfloat16, "wild"),
+    (2, 21, 25, torch.float32, "down"),           # odd rows: no copies
+    (1, 3, 3, torch.float32, "wild"),
+    (2, 5, 7, torch.bfloat16, "plain"),
+    (1, 150, 160, torch.float32, "zeros"),        # more tiles than one round of blocks takes
+])
+def test_block_kernels_at_any_magnitude(B, H, W, dtype, t_kind):
+    """Both 1x1 kernels against fp64: a pixel's values and its two halves of t may have any size next to each other."""
+    from conversenet_b200 import ConverseBlock, _cabi
+    from conversenet_b200 import functional as CF
+    g = torch.Generator(device="cuda").manual_seed(B * 100 + H)
+    blk = ConverseBlock(64, 64, 3, 1, 1).cuda().eval()
+    rand = lambda *n: torch.randn(*n, device="cuda", generator=g)
+    with torch.no_grad():
+        for q in blk.parameters():
+            if q.dim() == 1:
+                q.add_(0.1 * rand(*q.shape))
+        x, t = rand(B, 64, H, W), torch.nn.functional.gelu(rand(B, 128, H, W))
+        if t_kind == "up":
+            t[:, 64:] *= 1e6
+        elif t_kind == "down":
+            t[:, 64:] *= 1e-6
+        elif t_kind == "zeros":
+            t[:, :64] = 0
+        elif t_kind == "wild":
+            t *= torch.exp(5 * rand(B, 128, H, W))
+        x, t = x.to(dtype), t.to(dtype)
+        t[0, 5, 0, 0] = float("nan")
+        c1, c2 = blk.conv1._modules, blk.conv2._modules
+        pack = blk._packed(CF.block_parameters(c1["0"], c1["1"], c1["5"], None, c2["0"], c2["1"], c2["3"], None))
+        eps, lib, st, io = c1["0"].eps, _cabi.load(), torch.cuda.current_stream().cuda_stream, int(dtype == torch.bfloat16)
+        pre, post = torch.empty_like(t), torch.empty_like(x)
+        assert lib.cvb_block_pre_fwd(x.data_ptr(), pre.data_ptr(), pack.data_ptr(), eps, B, H * W, io, st) == 0
+        assert lib.cvb_block_post_fwd(t.data_ptr(), x.data_ptr(), post.data_ptr(), pack.data_ptr(), eps, B, H * W, io, st) == 0
+        F = torch.nn.functional
+        conv = lambda v, m: F.conv2d(v, m.weight.double(), m.bias.double())
+
+        def norm(v, m):
+            u = v.mean(1, keepdim=True)
+            s = (v - u).pow(2).mean(1, keepdim=True)
+            return (v - u) / torch.sqrt(s + eps) * m.weight.double()[:, None, None] + m.bias.double()[:, None, None]
+        xd, td = x.double(), t.double()
+        want_pre = F.gelu(conv(norm(xd, c1["0"]), c1["1"]))
+        x1 = xd + conv(td, c1["5"])
+        want = x1 + conv(F.gelu(conv(norm(x1, c2["0"]), c2["1"])), c2["3"])
+    nan = torch.zeros_like(post, dtype=torch.bool)
+    nan[0, :, 0, 0] = True
+    assert torch.equal(post.isnan(), nan)         # the pixel, and no other
+    # 22 bits of each operand and fp32 sums of 64 and 128 products; bf16 results 8 bits
+    bar = 1e-6 if dtype == torch.float32 else 4e-3
+    rel = lambda a, r: float((a.double() - r).norm() / r.norm())
+    assert rel(pre, want_pre) <= bar and rel(post[~nan], want[~nan]) <= bar
+    assert lib.cvb_last_device_status(1) == 0
