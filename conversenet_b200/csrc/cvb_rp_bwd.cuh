@@ -11,6 +11,7 @@
 // and lambda is closed form (chain_body); the taps also enter the epilogue's correlation directly (tap sums of
 // adjoint_epilogue_body).
 #pragma once
+#include "cvb_fix.cuh"
 #include "cvb_rp.cuh"
 
 namespace cvb {
@@ -213,91 +214,204 @@ struct AdjointParams {
   float* v;               // (B,C,h,w)
   float* taps;            // [B C][k k]
   int C, H, W, k, s, p, h, w, wp;
+  int tw, th, nx, ny, pitch;     // plan_adjoint: a tile is th x tw items of 2 x 2 cells
+  float inv_tw;
 };
-// One block per plane.  A thread owns two neighbouring cells at a time; the (k + s) x k window of g that they share is
-// read once, row by row, and serves both the correlation and the tap products.
+// One block per plane walks over tiles of it: the part of g that a tile's cells read, wrapped and extended by zeros, and r are
+// copied to shared memory asynchronously while the previous tile is worked on.  A thread owns 2 x 2 neighbouring cells; the
+// (K + s) x (K + s) window that they share is read row by row, 16 bytes at a time (two cells apart: no bank conflicts at
+// scale 2), and serves both the correlation and the tap products, two columns an instruction.  1024 planes of 68 x 68, scale
+// 2, 5 x 5 taps: 43 us, issue slots 62 % busy, the port to shared memory 56 %, 17 % of the blocks' time the third, short wave;
+// 105 MB take 16 us.  With rows of g loaded by each thread as it needed them, one row's latency after the other: 112 us.
+// Tried: taps in registers and two blocks an SM 59 us; without the packed products 55 (copies indexed chunk by chunk in both).
 template <int K, int S>
-__device__ __forceinline__ void adjoint_epilogue_body(const AdjointParams& A, float* red) {
+struct AdjointTile {
+  static constexpr int c = K / 2, NW = K + S, SHIFT = ((c - K + 1) % 4 + 4) % 4, NV = (SHIFT + NW + 3) / 4;
+  static constexpr int threads = 256, sums = threads + 8, blocks = K < 7 && K * S < 20 ? 3 : 2, area = 216 * 1024 / blocks;    // an SM's blocks; their tiles
+  __host__ __device__ static int rows(int th) { return 2 * S * th + K - S; }
+  __host__ __device__ static int floats(const AdjointParams& A) {
+    const int t = 2 * buffer(A), red = K * K * sums;
+    return taps + (t > red ? t : red);
+  }
+  // Taps in ascending order of the columns that they meet, two at a time where the window has them in one aligned pair:
+  // LEAD alone, NP pairs, TAIL alone; in shared memory rows of KP, the pairs aligned
+  static constexpr int LEAD = SHIFT & 1, NP = (K - LEAD) / 2, TAIL = (K - LEAD) & 1, KP = (K + LEAD + 3) & ~3, taps = K * KP;
+  // g's part of a tile, then r's
+  __host__ __device__ static int buffer(const AdjointParams& A) { return rows(A.th) * A.pitch + 4 * A.th * A.tw; }
+};
+// At most 64 items side by side (524 floats a row at scale 4: two tiles of one item's rows always fit); as many rows of items
+// as make the walk shortest by a rough count of a block's cycles -- 520 for every 256 items, 15 floats copied per cycle, 150
+// a tile -- in at most 56 KB, so that blocks overlap on an SM.
+template <int K, int S>
+inline void plan_adjoint(AdjointParams& A) {
+  using T = AdjointTile<K, S>;
+  const int cols = (A.w + 1) / 2, lines = (A.h + 1) / 2;
+  A.nx = (cols + 63) / 64;
+  A.tw = ((cols + A.nx - 1) / A.nx + 1) & ~1;          // even: tiles start at a multiple of four columns at every scale
+  A.pitch = (2 * S * A.tw - S + K + T::SHIFT + S + 3) & ~3;
+  if (A.pitch < 2 * S * (A.tw - 1) + 4 * T::NV) A.pitch = (2 * S * (A.tw - 1) + 4 * T::NV + 3) & ~3;
+  A.inv_tw = 1.0f / (float)A.tw;
+  long long best = -1;
+  for (int th = 1; th <= lines; ++th) {
+    const int area = T::rows(th) * A.pitch + 4 * th * A.tw;
+    if (th > 1 && 8 * area > T::area) break;
+    const long long cost = (long long)((lines + th - 1) / th) *
+        ((th * A.tw + T::threads - 1) / T::threads * 520 + area / 15 + 150);
+    if (best < 0 || cost < best) { best = cost; A.th = th; }
+  }
+  A.ny = (lines + A.th - 1) / A.th;
+}
+template <int K, int S>
+__device__ __forceinline__ void adjoint_epilogue_body(const AdjointParams& A, float* sm) {
+  using T = AdjointTile<K, S>;
+  constexpr int c = T::c, NW = T::NW, SHIFT = T::SHIFT, NV = T::NV;
   const int tid = threadIdx.x, nthr = blockDim.x, plane = blockIdx.x, ch = plane % A.C;
-  constexpr int c = K / 2, NW = K + S;
   const int sH = S * A.H, sW = S * A.W, sh = S * A.h, sw = S * A.w, off = S * A.p;
   const float* g = A.g + (size_t)plane * sH * sW;
-  float kw[K * K], acc[K * K];
-#pragma unroll
-  for (int i = 0; i < K * K; ++i) { kw[i] = A.weight[(size_t)ch * K * K + i]; acc[i] = 0.f; }
-  const int pairs = (A.w + 1) / 2, total = A.h * pairs;
-  const float inv = 1.0f / (float)pairs;
-  // the window of a pair of cells starts (c - K + 1) mod 4 past a multiple of four columns: three 16-byte loads a row
-  constexpr int SHIFT = ((c - K + 1) % 4 + 4) % 4, NV = (SHIFT + NW + 3) / 4;
-  const bool quads = S % 2 == 0 && off % 4 == 0 && sW % 4 == 0 && ((size_t)A.g) % 16 == 0;
-  for (int it = tid; it < total; it += nthr) {
-    int my, px;
-    divmod_small(it, pairs, inv, my, px);
-    const int mx = 2 * px;
-    const bool two = mx + 1 < A.w;
-    float r0 = 0.f, r1 = 0.f;
-    if (A.r) {
-      const float2 rr = *(const float2*)(A.r + ((size_t)plane * A.h + my) * A.wp + mx);
-      r0 = rr.x;
-      if (two) r1 = rr.y;
+  const int nrow = T::rows(A.th), size = T::buffer(A), ntile = A.nx * A.ny;
+  float *kw = sm, *tiles = sm + T::taps;
+  // 16-byte copies where the columns of g and of the tile agree modulo 4
+  const bool quads = off % 4 == 0 && sW % 4 == 0 && (size_t)A.g % 16 == 0;
+  // a thread copies 16 bytes of every gstep-th row of a tile of g and 8 of every rstep-th row of r
+  const int chunks = A.pitch / 4, gj = tid / chunks, gq = tid - gj * chunks, gstep = nthr / chunks;
+  const int rj = tid / A.tw, rq = tid - rj * A.tw, rstep = nthr / A.tw;
+  auto load = [&](int t) {
+    float *buf = tiles + (t & 1) * size, *rbuf = buf + nrow * A.pitch;
+    const int ty = t / A.nx, cy = 2 * A.th * ty, cx = 2 * A.tw * (t - ty * A.nx);      // the tile's first cell
+    const int y0 = S * cy + c - K + 1, x0 = S * cx + c - K + 1 - SHIFT;
+    auto wrapped = [&](int i, int n) { return (i < 0 ? i + n : i >= n ? i - n : i) - off; };
+    if (quads) {     // the period is a multiple of four columns too: four columns are in g or not, together
+      const int x = wrapped(x0 + 4 * gq, sw);
+      const bool in = gj < gstep && (unsigned)x < (unsigned)sW;
+      const float* src = g + (in ? x : 0);
+      float* dst = buf + gj * A.pitch + 4 * gq;
+#pragma unroll 1
+      for (int j = gj < gstep ? gj : nrow; j < nrow; j += gstep, dst += gstep * A.pitch) {
+        const int y = wrapped(y0 + j, sh), near = y < 0 ? 0 : y < sH ? y : sH - 1;
+        fx_copy<16>(dst, src + (size_t)near * sW, in && y == near);
+      }
+    } else {
+      for (int i = tid & 31; i < A.pitch; i += 32) {
+        const int x = wrapped(x0 + i, sw);
+        const bool in = (unsigned)x < (unsigned)sW;
+        const float* src = g + (in ? x : 0);
+#pragma unroll 1
+        for (int j = tid >> 5; j < nrow; j += nthr >> 5) {
+          const int y = wrapped(y0 + j, sh), near = y < 0 ? 0 : y < sH ? y : sH - 1;
+          fx_copy<4>(buf + j * A.pitch + i, src + (size_t)near * sW, in && y == near);
+        }
+      }
     }
-    // columns S mx + S + c - i, i = 0 .. NW - 1 (the second cell starts S to the right)
-    int gx[NW];
+    if (!A.r) return;
+    const bool in = cx + 2 * rq < A.w;
+    const float* src = A.r + ((size_t)plane * A.h + cy) * A.wp + (in ? cx + 2 * rq : 0);
+    const int have = A.h - cy;
+#pragma unroll 1
+    for (int j = rj < rstep ? rj : 2 * A.th; j < 2 * A.th; j += rstep)
+      fx_copy<8>(rbuf + 2 * (A.tw * j + rq), src + (j < have ? j : 0) * A.wp, in && j < have);
+  };
+  constexpr int LEAD = T::LEAD, NP = T::NP, TAIL = T::TAIL, KP = T::KP;
+  float2 acc[K][NP];
+  float lead[K], tail[K];
 #pragma unroll
-    for (int i = 0; i < NW; ++i) {
-      int x = S * mx + S + c - i;
-      x = x < 0 ? x + sw : x >= sw ? x - sw : x;
-      x -= off;
-      gx[i] = (unsigned)x < (unsigned)sW ? x : -1;
-    }
-    const int lo = S * mx + c - K + 1 - off - SHIFT;    // first loaded column of the fast path
-    const bool fast = quads && lo >= 0 && lo + 4 * NV <= sW;
-    float v0 = 0.f, v1 = 0.f;
+  for (int a = 0; a < K; ++a) {
+    lead[a] = tail[a] = 0.f;
 #pragma unroll
-    for (int a = 0; a < K; ++a) {
-      int y = S * my - a + c;
-      y = y < 0 ? y + sh : y >= sh ? y - sh : y;
-      y -= off;
-      if ((unsigned)y >= (unsigned)sH) continue;
-      const float* row = g + (size_t)y * sW;
-      float win[NW];                                    // win[i]: column S mx + S + c - i
-      if (fast) {
-        float q[4 * NV];
+    for (int i = 0; i < NP; ++i) acc[a][i] = make_float2(0.f, 0.f);
+  }
+  for (int i = tid; i < K * K; i += nthr) {
+    const int a = i / K, b = i - a * K;
+    kw[a * KP + LEAD + K - 1 - b] = A.weight[(size_t)ch * K * K + i];
+  }
+  load(0);
+  for (int t = 0; t < ntile; ++t) {
+    fx_copies_done();
+    __syncthreads();                       // this tile is there, and every thread is done with the other buffer
+    if (t + 1 < ntile) load(t + 1);
+    const float* buf = tiles + (t & 1) * size;
+    const int ty = t / A.nx, tx = t - ty * A.nx;
+    for (int it = tid; it < A.th * A.tw; it += nthr) {
+      int iy, ix;
+      divmod_small(it, A.tw, A.inv_tw, iy, ix);
+      const int my = 2 * (A.th * ty + iy), mx = 2 * (A.tw * tx + ix);
+      if (my >= A.h || mx >= A.w) continue;
+      const bool right = mx + 1 < A.w, below = my + 1 < A.h;
+      float r[2][2] = {};
+      float2 v[2][2] = {};                   // sums over the even and the odd columns
+      if (A.r) {
+        const float* rp = buf + nrow * A.pitch + 4 * A.tw * iy + 2 * ix;
+        const float2 r0 = *(const float2*)rp, r1 = *(const float2*)(rp + 2 * A.tw);
+        r[0][0] = r0.x; r[1][0] = r1.x;
+        if (right) { r[0][1] = r0.y; r[1][1] = r1.y; }
+      }
+      const float* src = buf + 2 * S * (iy * A.pitch + ix);
 #pragma unroll
-        for (int i = 0; i < NV; ++i) {
-          const float4 t = __ldg((const float4*)(row + lo) + i);
-          q[4 * i] = t.x; q[4 * i + 1] = t.y; q[4 * i + 2] = t.z; q[4 * i + 3] = t.w;
+      for (int j = 0; j < K + S; ++j) {
+        float q[4 * NV];                   // row S my + c - K + 1 + j from column S mx + c - K + 1 - SHIFT on
+        if constexpr (S % 2 == 0) {
+#pragma unroll
+          for (int i = 0; i < NV; ++i) {
+            const float4 f = *(const float4*)(src + j * A.pitch + 4 * i);
+            q[4 * i] = f.x; q[4 * i + 1] = f.y; q[4 * i + 2] = f.z; q[4 * i + 3] = f.w;
+          }
+        } else {
+#pragma unroll
+          for (int i = SHIFT; i < SHIFT + NW; ++i) q[i] = src[j * A.pitch + i];
         }
 #pragma unroll
-        for (int i = 0; i < NW; ++i) win[i] = q[SHIFT + NW - 1 - i];
-      } else {
+        for (int d = 0; d < 2; ++d) {      // the upper and the lower two cells
+          const int a = K - 1 - j + S * d;
+          if (a < 0 || a >= K) continue;
+          const float* ka = kw + a * KP;
 #pragma unroll
-        for (int i = 0; i < NW; ++i) win[i] = gx[i] >= 0 ? row[gx[i]] : 0.f;
+          for (int x = 0; x < 2; ++x) {    // the left and the right one
+            const float* w = q + SHIFT + S * x;
+            const float2 rr = make_float2(r[d][x], r[d][x]);
+#pragma unroll
+            for (int i = 0; i < NP; ++i) {
+              const float2 f = make_float2(w[LEAD + 2 * i], w[LEAD + 2 * i + 1]);
+              v[d][x] = fx_fma2(*(const float2*)(ka + 2 * LEAD + 2 * i), f, v[d][x]);
+              acc[a][i] = fx_fma2(f, rr, acc[a][i]);
+            }
+            if constexpr (LEAD != 0) {
+              v[d][x].y = fmaf(ka[1], w[0], v[d][x].y);
+              lead[a] = fmaf(w[0], r[d][x], lead[a]);
+            }
+            if constexpr (TAIL != 0) {
+              v[d][x].x = fmaf(ka[LEAD + K - 1], w[K - 1], v[d][x].x);
+              tail[a] = fmaf(w[K - 1], r[d][x], tail[a]);
+            }
+          }
+        }
       }
+      float* o = A.v + ((size_t)plane * A.h + my) * A.w + mx;
 #pragma unroll
-      for (int b = 0; b < K; ++b) {
-        v0 = fmaf(kw[a * K + b], win[S + b], v0);
-        v1 = fmaf(kw[a * K + b], win[b], v1);
-        acc[a * K + b] = fmaf(win[S + b], r0, fmaf(win[b], r1, acc[a * K + b]));
+      for (int d = 0; d < 2; ++d) {
+        if (d && !below) break;
+        if (right && A.w % 2 == 0) *(float2*)(o + d * A.w) = make_float2(v[d][0].x + v[d][0].y, v[d][1].x + v[d][1].y);
+        else {
+          o[d * A.w] = v[d][0].x + v[d][0].y;
+          if (right) o[d * A.w + 1] = v[d][1].x + v[d][1].y;
+        }
       }
     }
-    float* o = A.v + ((size_t)plane * A.h + my) * A.w + mx;
-    o[0] = v0;
-    if (two) o[1] = v1;
   }
   if (!A.taps) return;
+  __syncthreads();
 #pragma unroll
   for (int t = 0; t < K * K; ++t) {
-    float x = acc[t];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if ((tid & 31) == 0) red[(tid >> 5) * K * K + t] = x;
+    const int a = t / K, e = K - 1 - (t - a * K) - LEAD;
+    tiles[t * T::sums + tid] = e < 0 ? lead[a] : e == 2 * NP ? tail[a] : e % 2 ? acc[a][e / 2].y : acc[a][e / 2].x;
   }
   __syncthreads();
-  for (int t = tid; t < K * K; t += nthr) {
+  for (int t0 = 0; t0 < K * K; t0 += nthr / 8) {          // eight threads a tap
+    const int t = t0 + (tid >> 3);
     float x = 0.f;
-    for (int i = 0; i < nthr / 32; ++i) x += red[i * K * K + t];
-    A.taps[(size_t)plane * K * K + t] = x;
+    if (t < K * K)
+      for (int i = tid & 7; i < nthr; i += 8) x += tiles[t * T::sums + i];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if (t < K * K && (tid & 7) == 0) A.taps[(size_t)plane * K * K + t] = x;
   }
 }
 // any tap count and scale
@@ -364,8 +478,6 @@ __device__ __forceinline__ Preimage preimage(int i, int n, int p, int mode) {
   return r;
 }
 __device__ __forceinline__ float pad_adjoint_at(const PadAdjointParams& A, const float* f, int y, int x) {
-  // away from the margins' images a source sample has one padded copy
-  if (y > A.p && y < A.H - 1 - A.p && x > A.p && x < A.W - 1 - A.p) return f[(size_t)(y + A.p) * A.w + x + A.p];
   const Preimage py = preimage(y, A.H, A.p, A.pad_mode), px = preimage(x, A.W, A.p, A.pad_mode);
   auto row = [&](int yy) {
     const float* q = f + (size_t)yy * A.w;
@@ -381,38 +493,95 @@ __device__ __forceinline__ float pad_adjoint_at(const PadAdjointParams& A, const
   if (py.e1 >= 0) v += row(py.e1);
   return v;
 }
+__device__ __forceinline__ float cell_sum(const PadAdjointParams& A, const float* g, int y, int x) {
+  const float* q = g + ((size_t)A.s * A.W * y + x) * A.s;
+  if (A.s == 2) {
+    const float *lo = q, *hi = q + 2 * A.W;
+    return (lo[0] + lo[1]) + (hi[0] + hi[1]);
+  }
+  float v = 0.f;
+  for (int a = 0; a < A.s; ++a)
+    for (int b = 0; b < A.s; ++b) v += q[(size_t)a * A.s * A.W + b];
+  return v;
+}
+// Bounds: the latency of the loads (f, g and gx once each).  Samples away from the margins' images have one padded copy: a thread does
+// four of them with all loads in flight.  The others -- 18 % of a 64 x 64 plane at p = 2, 39 % at p = 6 -- are numbered
+// by themselves (top and bottom bands, then the left and right ends of the rows between), so that the lanes of a warp that
+// walk through their copies all have copies to walk through.
+constexpr int kPadAdjointUnroll = 4;
 __device__ __forceinline__ void pad_adjoint_body(const PadAdjointParams& A) {
   const int plane = blockIdx.y;
   const float* f = A.f + (size_t)plane * A.h * A.w;
+  const float* g = A.g ? A.g + (size_t)plane * A.s * A.H * A.s * A.W : nullptr;
   float* out = A.gx + (size_t)plane * A.H * A.W;
   const int start = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
-  if (A.g && A.s == 2 && A.W % 2 == 0 && ((size_t)A.g) % 16 == 0 && ((size_t)A.gx) % 8 == 0) {
-    // two samples at a time: their eight values of g are two 16-byte loads
-    const int half = A.W / 2;
-    const float inv = 1.0f / (float)half;
-    const float* g = A.g + (size_t)plane * 4 * A.H * A.W;
-    for (int i = start; i < A.H * half; i += step) {
-      int y, xh;
-      divmod_small(i, half, inv, y, xh);
-      const float4 a = __ldg((const float4*)(g + (size_t)(2 * y) * 2 * A.W) + xh);
-      const float4 b = __ldg((const float4*)(g + (size_t)(2 * y + 1) * 2 * A.W) + xh);
-      const float v0 = pad_adjoint_at(A, f, y, 2 * xh) + ((a.x + a.y) + (b.x + b.y));
-      const float v1 = pad_adjoint_at(A, f, y, 2 * xh + 1) + ((a.z + a.w) + (b.z + b.w));
-      ((float2*)out)[i] = make_float2(v0, v1);
-    }
-    return;
-  }
+  const int m = A.p + 1;                                  // y <= p or y >= H - 1 - p: may have further copies
+  const int ih = A.H > 2 * m ? A.H - 2 * m : 0, iw = A.W > 2 * m ? A.W - 2 * m : 0;
   const float invW = 1.0f / (float)A.W;
-  for (int i = start; i < A.H * A.W; i += step) {
-    int y, x;
-    divmod_small(i, A.W, invW, y, x);
-    float v = pad_adjoint_at(A, f, y, x);
-    if (A.g) {
-      const float* g = A.g + ((size_t)plane * A.s * A.H + (size_t)A.s * y) * A.s * A.W + A.s * x;
-      for (int a = 0; a < A.s; ++a)
-        for (int b = 0; b < A.s; ++b) v += g[(size_t)a * A.s * A.W + b];
+  auto inner = [&](int y, int x) { return y >= m && y < A.H - m && x >= m && x < A.W - m; };
+  if (ih && iw) {
+    const int lo = m * A.W, hi = (A.H - m) * A.W;         // rows between the bands
+    if (g && A.s == 2 && A.W % 2 == 0 && (size_t)A.g % 16 == 0) {
+      // two samples at a time: their eight values of g are two 16-byte loads
+      const int half = A.W / 2;
+      const float inv = 1.0f / (float)half;
+      for (int i0 = lo / 2 + start; i0 < hi / 2; i0 += 2 * step) {
+        float4 a[2], b[2];
+        float2 v[2];
+        int y[2], x[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int i = i0 + u * step;
+          if (i >= hi / 2) continue;
+          divmod_small(i, half, inv, y[u], x[u]);
+          a[u] = __ldg((const float4*)(g + (size_t)(2 * y[u]) * 2 * A.W) + x[u]);
+          b[u] = __ldg((const float4*)(g + (size_t)(2 * y[u] + 1) * 2 * A.W) + x[u]);
+          const float* q = f + (size_t)(y[u] + A.p) * A.w + 2 * x[u] + A.p;
+          v[u] = make_float2(q[0], q[1]);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int i = i0 + u * step;
+          if (i >= hi / 2) continue;
+          if (inner(y[u], 2 * x[u])) out[2 * i] = v[u].x + ((a[u].x + a[u].y) + (b[u].x + b[u].y));
+          if (inner(y[u], 2 * x[u] + 1)) out[2 * i + 1] = v[u].y + ((a[u].z + a[u].w) + (b[u].z + b[u].w));
+        }
+      }
+    } else {
+      constexpr int U = kPadAdjointUnroll;
+      for (int i0 = lo + start; i0 < hi; i0 += U * step) {
+        float v[U];
+        int x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int i = i0 + u * step;
+          x[u] = 0;
+          if (i >= hi) continue;
+          int y;
+          divmod_small(i, A.W, invW, y, x[u]);
+          v[u] = f[(size_t)(y + A.p) * A.w + x[u] + A.p];
+          if (g && x[u] >= m && x[u] < A.W - m) v[u] += cell_sum(A, g, y, x[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (x[u] >= m && x[u] < A.W - m) out[i0 + u * step] = v[u];     // x stays 0 past the end
+      }
     }
-    out[i] = v;
+  }
+  const int band = ih && iw ? 2 * m * A.W : A.H * A.W, edges = band + (ih && iw ? 2 * m * ih : 0);
+  for (int e = start; e < edges; e += step) {
+    int y, x;
+    if (e < band) {
+      divmod_small(e, A.W, invW, y, x);
+      if (ih && iw && y >= m) y += ih;
+    } else {
+      const int q = (e - band) / (2 * m), i = e - band - q * 2 * m;
+      y = m + q;
+      x = i < m ? i : A.W - 2 * m + i;
+    }
+    float v = pad_adjoint_at(A, f, y, x);
+    if (g) v += cell_sum(A, g, y, x);
+    out[(size_t)y * A.W + x] = v;
   }
 }
 

@@ -12,9 +12,17 @@ __global__ void __launch_bounds__(128, 4) rows_bwd_kernel(const __grid_constant_
   rows_bwd_body<kAnyRadix, 0>(Q, smem);
 }
 template <int K, int S>
-__global__ void __launch_bounds__(256) adjoint_epilogue_kernel(const AdjointParams A) {
-  __shared__ float red[8 * K * K];
-  adjoint_epilogue_body<K, S>(A, red);
+__global__ void __launch_bounds__(256, AdjointTile<K, S>::blocks) adjoint_epilogue_kernel(const AdjointParams A) {
+  extern __shared__ float4 tiles[];
+  adjoint_epilogue_body<K, S>(A, (float*)tiles);
+}
+template <int K, int S>
+static int launch_adjoint(AdjointParams A, int planes, cudaStream_t st) {
+  plan_adjoint<K, S>(A);
+  const size_t smem = (size_t)AdjointTile<K, S>::floats(A) * sizeof(float);
+  CVB_CUDA(cudaFuncSetAttribute(adjoint_epilogue_kernel<K, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  adjoint_epilogue_kernel<K, S><<<planes, AdjointTile<K, S>::threads, smem, st>>>(A);
+  return CVB_OK;
 }
 __global__ void __launch_bounds__(256) adjoint_epilogue_any_kernel(const AdjointParams A) {
   __shared__ float red[8];
@@ -315,11 +323,12 @@ int run_bwd(const float* x, const float* g, const float* r, const void* table, c
     // the tap counts of the networks (2 at scale 2, 3, 5, 7) at the scales that have parameter gradients; others read g once
     // per tap
     switch (s * 16 + k) {
-#define X(KK, SS) case SS * 16 + KK: adjoint_epilogue_kernel<KK, SS><<<planes, 256, 0, st>>>(A); break;
+#define X(KK, SS) case SS * 16 + KK: rc = launch_adjoint<KK, SS>(A, planes, st); break;
       X(2, 2) X(3, 2) X(5, 2) X(7, 2) X(3, 3) X(5, 3) X(7, 3) X(3, 4) X(5, 4) X(7, 4)
 #undef X
       default: adjoint_epilogue_any_kernel<<<planes, 256, 0, st>>>(A);
     }
+    if (rc != CVB_OK) return rc;
     CVB_CUDA(cudaGetLastError());
     Q.x = A.v;
     Q.H = P.h; Q.W = P.w; Q.p = 0;

@@ -524,15 +524,22 @@ int emu_rp_backward(const float* x, const float* g, const float* r, float* gx, f
       AdjointParams A;
       A.g = g; A.r = r; A.weight = weight; A.v = (float*)v.get(); A.taps = (float*)tp.get();
       A.C = C; A.H = H; A.W = W; A.k = k; A.s = s; A.p = p; A.h = h; A.w = w; A.wp = P.wp;
-      emu::Guarded red(8 * k * k * 4);
-      auto go = [&](auto fn) { emu::launch(planes, 1, 1, 256, [&] { fn(A, (float*)red.get()); }); };
+      auto go = [&](int floats, auto fn) {
+        emu::Guarded sm((size_t)floats * 4);
+        emu::launch(planes, 1, 1, 256, [&] { fn(A, (float*)sm.get()); });
+        sm.check("shared memory");
+      };
       switch (s * 16 + k) {
-#define X(KK, SS) case SS * 16 + KK: go([](const AdjointParams& a, float* m) { adjoint_epilogue_body<KK, SS>(a, m); }); break;
+#define X(KK, SS)                                                                                         \
+  case SS * 16 + KK:                                                                                      \
+    plan_adjoint<KK, SS>(A);                                                                              \
+    go(AdjointTile<KK, SS>::floats(A), [](const AdjointParams& a, float* m) { adjoint_epilogue_body<KK, SS>(a, m); }); \
+    break;
         X(2, 2) X(3, 2) X(5, 2) X(7, 3) X(3, 4)
 #undef X
-        default: go([](const AdjointParams& a, float* m) { adjoint_epilogue_any(a, m); });
+        default: go(8, [](const AdjointParams& a, float* m) { adjoint_epilogue_any(a, m); });
       }
-      red.check("shared memory"); v.check("v"); tp.check("taps");
+      v.check("v"); tp.check("taps");
       Q.x = A.v; Q.H = h; Q.W = w; Q.p = 0; Q.pad_mode = 0;
       memcpy(taps, tp.get(), (size_t)planes * k * k * 4);
     }

@@ -213,6 +213,20 @@ def test_gradients_match_fp64_autograd(case):
         assert _rel(q, r) <= 2e-5
 
 
+@pytest.mark.parametrize("case", [
+    (1, 2, 20, 130, 5, 2, 2, "circular"),      # 67 items side by side: two tiles
+    (1, 1, 61, 36, 3, 2, 1, "replicate"),      # odd rows and columns of items, several tiles down, 16-byte copies
+    (2, 1, 19, 27, 7, 2, 0, "circular"),       # the windows wrap around; 4-byte copies
+    (1, 1, 18, 20, 7, 2, 0, "reflect"),        # the windows wrap around; 16-byte copies
+    (1, 1, 9, 138, 7, 4, 3, "constant"),       # the widest tiles
+    (1, 2, 12, 44, 3, 3, 4, "replicate"),      # odd scale, 16-byte copies
+    (1, 1, 2, 2, 2, 2, 0, "circular"),
+])
+def test_upsampling_gradients_across_tiles(case):
+    # the bound of test_gradients_match_fp64_autograd: the fp32 transforms' error, which the tiles leave as it is
+    test_gradients_match_fp64_autograd(case)
+
+
 @pytest.mark.parametrize("B,H,W", [(1, 4, 5), (3, 24, 31), (2, 16, 16), (1, 37, 64)])
 @pytest.mark.parametrize("alphas", [False, True])
 def test_block_and_its_gradients_match_the_layer_by_layer_block(monkeypatch, B, H, W, alphas):
