@@ -6,8 +6,8 @@
 //   g_z1 = g_t . gelu'(z1);  g_x = g_x1 + LN1'((W1 gamma1)^T g_z1)               DOWN
 // and every parameter gradient follows from four contractions over the pixels (wgrad_kernel), each 64 x 128 with the sums
 // of both operands:  g (x) gelu(z3),  xh2 (x) g_z3,  g_x1 (x) gelu(u),  xh1 (x) g_z1.
-// The contractions over channels run as in k_block_mlp.cu (two groups of 256 threads, TF32 hi + lo, operand in tensor
-// memory); those over pixels on the CUDA cores, where fp32 sums over a few thousand pixels keep their accuracy.
+// The contractions over channels run as in k_block_mlp.cu (two groups of 256 threads, operand in tensor memory) with TF32
+// hi + lo; those over pixels too, their sums in fp32 registers.
 #include "../../include/converse_b200.h"
 #include "cvb_internal.h"
 #include "cvb_mix.cuh"
@@ -200,11 +200,17 @@ static int launch_grad(const BlockGradParams& P, int sms, cudaStream_t st) {
 
 // ------------------------------------------------------------------ contractions over the pixels
 // out[p][q] = sum over pixels of P[p] Q[q], 64 x 128, and the sums of every P[p] and Q[q]; Q optionally through GELU.
-// A block takes 32-pixel tiles blockIdx.x, + gridDim.x, ...; the tile of all 192 channels sits in shared memory
-// [channel][pixel] and a thread owns the products of 4 x 8 channels (rows 16 apart: no bank conflicts), four pixels at a
-// time; the next tile is in registers meanwhile.  0.27 GFMA a contraction at 32768 pixels, 99 us for the four: FMA pipes 40 %
-// busy, the port to shared memory (twelve 16-byte reads per 128 FMAs a thread) 46 %, then waits for the loads.
-constexpr int kGPitch = 36, kGOut = kBlkC * kBlkM + kBlkC + kBlkM;
+// A block takes 32-pixel tiles blockIdx.x, + gridDim.x, ...: its threads split the 192 channels' values into TF32 hi + lo
+// (exact to 2^-22 of a value) in shared memory, channels as rows and pixels along K, and one tile's MMAs (Q in the 128 rows
+// of tensor memory, [P hi | P lo] side by side) run while the next is split.  The accumulators are read and added to fp32
+// sums in registers after every tile: the tensor cores cut what they add off instead of rounding it, which over four
+// additions stays below what rounding the sum of a block's thousand pixels costs: gradients of w1 to w4 of a block of
+// 8 x 64 x 64 are within 5.7e-7 to 8.5e-7 of fp64 (8.0e-7 to 1.1e-6 with fp32 products on the CUDA cores).  32768 pixels,
+// the four contractions: 50 us, 99 on the CUDA cores (which waited for the port to shared memory); 100 MB take 15 us.  The
+// erf of the GELUs, the split and its stores are the larger part of a tile.
+constexpr int kGOut = kBlkC * kBlkM + kBlkC + kBlkM;
+constexpr int kGThreads = 512, kGRows = 128, kGGroup = kGRows * 16 + 16;   // bytes of four pixels of 128 rows (+ 16: banks)
+constexpr int kGOperand = 8 * kGGroup, kGBuffer = 3 * kGOperand;           // Q hi, Q lo, [P hi | P lo]
 struct WgradParams {
   const float* p[4];
   const float* q[4];
@@ -212,69 +218,113 @@ struct WgradParams {
   float* part;          // [4][blocks][kGOut]
   int HW;
   long long npix;
+  int* status;
 };
-__global__ void __launch_bounds__(256, 2) wgrad_kernel(const __grid_constant__ WgradParams W) {
-  __shared__ __align__(16) float tile[192 * kGPitch];
+__global__ void __launch_bounds__(kGThreads, 2) wgrad_kernel(const __grid_constant__ WgradParams W) {
+  extern __shared__ __align__(128) char gsm[];
+  uint64_t* done = (uint64_t*)(gsm + 2 * kGBuffer);
+  uint32_t* holder = (uint32_t*)(done + 1);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, which = blockIdx.y;
-  const int tq = tid & 15, tp = tid >> 4;
-  const float *pp = W.p[which], *qp = W.q[which];
   const int HW = W.HW;
   const bool gelu = W.gelu[which] != 0;
-  float acc[4][8], sum = 0.f;
+  if (tid == 0) {
+    mbar_init(done, 1);
+    mbar_fence_init();
+  }
+  if (warp == 0) tc::tmem_alloc(holder, 128);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = *holder;
+  // this thread's part of the result: row q = 32 (warp & 3) + lane, sixteen columns p
+  const int p0 = 16 * (warp >> 2);
+  const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)p0;
+  float acc[16], sum[12], r[12];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 16; ++i) acc[i] = 0.f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  for (int i = 0; i < 12; ++i) sum[i] = 0.f;
   const long long ntiles = (W.npix + 31) / 32;
-  float r[24];
+  // channels warp, warp + 16, ... of P and then of Q at pixel `lane` of tile t
   auto load = [&](long long t) {
     const long long pix = t * 32 + lane;
     const bool in = t < ntiles && pix < W.npix;
-    const long long img = in ? pix / HW : 0;
+    const long long img = !in ? 0 : W.npix <= 0x7fffffff ? (unsigned)pix / (unsigned)HW : pix / HW;
     const int pos = in ? (int)(pix - img * HW) : 0;
-    const float* a = pp + ((size_t)img * kBlkC + warp) * HW + pos;
-    const float* b = qp + ((size_t)img * kBlkM + warp) * HW + pos;
+    const float* a = W.p[which] + ((size_t)img * kBlkC + warp) * HW + pos;
+    const float* b = W.q[which] + ((size_t)img * kBlkM + warp) * HW + pos;
+    const size_t step = (size_t)16 * HW;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) r[i] = in ? a[(size_t)(8 * i) * HW] : 0.f;
+    for (int i = 0; i < 4; ++i) r[i] = in ? a[i * step] : 0.f;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) r[8 + i] = in ? b[(size_t)(8 * i) * HW] : 0.f;
+    for (int i = 0; i < 8; ++i) r[4 + i] = in ? b[i * step] : 0.f;
+  };
+  bool ok = true;
+  uint32_t uses = 0;
+  auto drain = [&]() {
+    if (ok) ok = mbar_wait_bounded(done, uses & 1u, kWaitLimit);
+    uses += 1;
+    tc::fence_after_sync();
+#pragma unroll
+    for (int c = 0; c < 16; c += 8) {
+      uint32_t x[8], y[8];
+      tc::tmem_ld8(mine + (uint32_t)c, x);
+      tc::tmem_ld8(mine + 64u + (uint32_t)c, y);
+      tc::tmem_wait_ld();
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[c + j] += __uint_as_float(x[j]) + __uint_as_float(y[j]);
+    }
+    tc::fence_before_sync();
   };
   load(blockIdx.x);
-  for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    __syncthreads();
+  int it = 0;
+  for (long long t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
+    char* buf = gsm + (it & 1) * kGBuffer + (lane >> 2) * kGGroup + (lane & 3) * 4 + warp * 16;
 #pragma unroll
-    for (int i = 0; i < 24; ++i) tile[(warp + 8 * i) * kGPitch + lane] = i >= 8 && gelu ? gelu_erf(r[i]) : r[i];
-    __syncthreads();
-    load(t + gridDim.x);
-#pragma unroll 2
-    for (int x = 0; x < 32; x += 4) {
-      float4 a[4], b[8];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = *(const float4*)(tile + (tp + 16 * i) * kGPitch + x);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) b[j] = *(const float4*)(tile + (64 + tq + 16 * j) * kGPitch + x);
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          acc[i][j] = fmaf(a[i].w, b[j].w, fmaf(a[i].z, b[j].z, fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, acc[i][j]))));
+    for (int i = 0; i < 12; ++i) {
+      const float v = i >= 4 && gelu ? gelu_erf(r[i]) : r[i];
+      sum[i] += v;
+      float hi, lo;
+      tc::split_tf32(v, hi, lo);
+      char* dst = buf + (i < 4 ? 2 * kGOperand + i * 256 : (i - 4) * 256);      // 16 rows further
+      *(float*)dst = hi;
+      *(float*)(dst + (i < 4 ? 64 * 16 : kGOperand)) = lo;
     }
-    if (tid < 192) {
-      float s = 0.f;
+    load(t + gridDim.x);
+    tc::fence_proxy_async();
+    if (it > 0) drain();                       // the other buffer is free then, and so are the accumulators
+    __syncthreads();
+    if (warp == 0) {
+      tc::fence_after_sync();
+      const uint32_t e = tc::elect_one() & tc::from_first(ok ? 1u : 0u);
+      const char* base = gsm + (it & 1) * kGBuffer;
 #pragma unroll
-      for (int x = 0; x < 32; x += 4) {
-        const float4 a = *(const float4*)(tile + tid * kGPitch + x);
-        s += (a.x + a.y) + (a.z + a.w);
+      for (int ks = 0; ks < 4; ++ks) {
+        const uint64_t qh = tc::smem_desc(base + 2 * ks * kGGroup, kGGroup, 128);
+        const uint64_t ql = tc::smem_desc(base + kGOperand + 2 * ks * kGGroup, kGGroup, 128);
+        const uint64_t pb = tc::smem_desc(base + 2 * kGOperand + 2 * ks * kGGroup, kGGroup, 128);
+        tc::mma_tf32_elected(tmem, qh, pb, tc::idesc_tf32(128, 128, false, false), ks > 0 ? 1u : 0u, e);
+        tc::mma_tf32_elected(tmem + 64u, ql, pb, tc::idesc_tf32(128, 64, false, false), 1u, e);
       }
-      sum += s;
+      if (e) tc::mma_commit(done);
     }
   }
+  if (it > 0) drain();
+  if (!ok && W.status) atomicExch(W.status, 3);
   float* o = W.part + ((size_t)which * gridDim.x + blockIdx.x) * kGOut;
+  const int q = 32 * (warp & 3) + lane;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int j = 0; j < 16; ++j) o[(p0 + j) * kBlkM + q] = acc[j];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[(tp + 16 * i) * kBlkM + tq + 16 * j] = acc[i][j];
-  if (tid < 192) o[kBlkC * kBlkM + tid] = sum;
+  for (int i = 0; i < 12; ++i) {
+    float x = sum[i];
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) x += __shfl_xor_sync(0xffffffffu, x, k);
+    if (lane == 0) o[kBlkC * kBlkM + warp + 16 * i] = x;
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(tmem, 128);
 }
 // sums of the blocks' parts -> part of block 0
 __global__ void __launch_bounds__(128) wgrad_sum_kernel(float* part, int blocks) {
@@ -404,9 +454,11 @@ int run_block_grad(const cvb_block_bwd_args& A, size_t conv_ws, int sms, int* st
   const float* ps[4] = {A.g, at(b.xh2), at(b.gx1), at(b.xh1)};
   const float* qs[4] = {A.z3, at(b.gz3), A.u, gt};
   for (int i = 0; i < 4; ++i) { W.p[i] = ps[i]; W.q[i] = qs[i]; W.gelu[i] = i == 0 || i == 2; }
-  W.part = at(b.part); W.HW = HW; W.npix = npix;
+  W.part = at(b.part); W.HW = HW; W.npix = npix; W.status = status;
   const int blocks = wgrad_blocks(npix, sms);
-  wgrad_kernel<<<dim3(blocks, 4), 256, 0, st>>>(W);
+  constexpr int smem = 2 * kGBuffer + 16;
+  CVB_CUDA(cudaFuncSetAttribute(wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  wgrad_kernel<<<dim3(blocks, 4), kGThreads, smem, st>>>(W);
   CVB_CUDA(cudaGetLastError());
   wgrad_sum_kernel<<<dim3((kGOut + 127) / 128, 4), 128, 0, st>>>(W.part, blocks);
   CVB_CUDA(cudaGetLastError());

@@ -260,6 +260,12 @@ def test_block_and_its_gradients_match_the_layer_by_layer_block(monkeypatch, B, 
     assert _cabi.load().cvb_last_device_status(1) == 0
 
 
+@pytest.mark.parametrize("B,H,W", [(3, 41, 64), (5, 33, 47)])
+def test_block_gradients_over_several_tiles_of_pixels(monkeypatch, B, H, W):
+    """246 and 243 tiles of 32 pixels: three or four a block of the weight gradients, so that both operand buffers are reused."""
+    test_block_and_its_gradients_match_the_layer_by_layer_block(monkeypatch, B, H, W, True)
+
+
 def test_block_follows_its_parameters():
     from conversenet_b200 import ConverseBlock
     torch.manual_seed(3)
