@@ -72,11 +72,33 @@ inline size_t rows_smem(const Params& P) {
 // kernels built for small radices serve an axis whose two radices are small
 inline bool small_axis(const Axis& a) { return a.mp == 0 && a.r0 <= kSmallRadix && a.r1 <= kSmallRadix; }
 
-// Block size of the strip kernels: 256 threads where the blocks leave SMs idle (they then take half the passes over their
-// tile: 64 planes of 132 x 132) or where four tiles do not fit an SM's memory (520 x 520: 1451 us with 256 threads, 1600
-// with 128), else 128 (264 x 264: 324 us against 362).
-inline int strip_threads(size_t smem, int grid, int sms) {
-  return grid <= 2 * sms || 4 * (smem + 1024) > kSmemLimit + 1024 ? 256 : 128;
+// Block size of the strip kernels.  Without a matrix stage a stage of a tile is a number of register transforms that the
+// threads take in turns, so that a size that divides them badly leaves threads idle for most of the last turn (320 transforms:
+// three turns of 128 threads, two of 160), and a larger one fits an SM less often.  Every turn waits for its loads, whatever
+// the number of warps; so the size is chosen by the turns of a tile, each weighted with its radix (the ten stand for the
+// latency), times the rounds of blocks over the SMs (one at least).  The size to start from is 256 threads where the blocks
+// leave SMs idle or where four tiles do not fit an SM's memory, else 128 -- the only sizes of a kernel with a matrix stage --
+// and another has to win by a tenth.  Against the times of 96 to 256 threads on 60 kernels and shapes (100 to 512 points, 64 to
+// 1024 planes) the choice is within 4 % of the best on average, the start 18 %; the worst is 5 % slower than the start.
+// 1 x 64 planes of 240 x 160 75 -> 47 us, of 260 x 340 134 -> 85, rows of 1 x 128 planes of 244 x 324 61 -> 49.
+inline int strip_threads(const Params& P, bool rows, int grid, int sms) {
+  const Axis& a = rows ? P.ax : P.ay;
+  const size_t smem = rows ? rows_smem(P) : cols_smem(P);
+  const int start = grid <= 2 * sms || 4 * (smem + 1024) > kSmemLimit + 1024 ? 256 : 128;
+  if (a.mp) return start;
+  const int registers = small_axis(a) ? 80 : 128;        // of the kernels' launch bounds
+  auto turns = [](int n, int t) { return (n + t - 1) / t; };
+  int best = start;
+  double least = 1e30;
+  for (int t = 256; t >= 96; t -= 32) {
+    const int resident = (int)((kSmemLimit + 1024) / (smem + 1024)), fit = 65536 / (registers * t);
+    const double load = (double)grid / ((double)sms * (resident < fit ? resident : fit));
+    const double tile = rows ? 2.0 * turns(a.r1 * kLines, t) * (a.r0 + 10) + turns(a.r0 * kLines, t) * (2 * a.r1 + 10)
+                             : turns(a.r1 * kLines, t) * (a.r0 + 10) + turns(a.r0 / 2 + 1, t / (2 * kLines)) * (a.r1 + 10);
+    const double cost = tile * (load > 1.0 ? load : 1.0) * (t == start ? 1.0 : 1.1);
+    if (cost < least) { least = cost; best = t; }
+  }
+  return best;
 }
 
 inline size_t plane_smem(int h, int w, int k) {

@@ -246,7 +246,7 @@ static int strip(Params& P, int planes, int which, cudaStream_t st) {
   P.plane0 = 0; P.nplane = planes; P.status = status_ptr();
   if (takes_fix(P, which, sm_count())) return launch_fix(which, P, CVB_F32, sm_count(), st);
   const int gc = (planes * P.wc + kLines - 1) / kLines, gr = (planes * P.hh + kLines - 1) / kLines;
-  const int tc = strip_threads(cols_smem(P), gc, sm_count()), tr = strip_threads(rows_smem(P), gr, sm_count());
+  const int tc = strip_threads(P, false, gc, sm_count()), tr = strip_threads(P, true, gr, sm_count());
   if (which == 1)
     return P.ax.mp ? matrix_entry(P.ax.mp).rows(P, CVB_F32, tr, gr, rows_smem(P), st)
                    : launch_rows(P, small_axis(P.ax), tr, gr, rows_smem(P), st);
@@ -285,7 +285,7 @@ int run(Params& P, const Route& r, int io_dtype, void* workspace, size_t ws_byte
       P.r = P.rsave ? P.rsave + (size_t)p0 * P.h * P.wp
                     : (float*)((char*)workspace + (size_t)P.nplane * P.hh * P.wp * sizeof(float2));
     const int gc = (P.nplane * P.wc + kLines - 1) / kLines, gr = (P.nplane * P.hh + kLines - 1) / kLines;
-    const int tc = strip_threads(smem_c, gc, sm_count()), tr = strip_threads(smem_r, gr, sm_count());
+    const int tc = strip_threads(P, false, gc, sm_count()), tr = strip_threads(P, true, gr, sm_count());
     int rc = takes_fix(P, 0, sm_count()) ? launch_fix(0, P, io_dtype, sm_count(), st)
              : P.ay.mp ? matrix_entry(P.ay.mp).cols_fwd(P, io_dtype, tc, gc, smem_c, st)
              : f32   ? launch_cols_fwd_f32(P, sy, tc, gc, smem_c, st)

@@ -396,7 +396,7 @@ void strip(const Params& P, Kernel which, int sms) {
   const size_t bytes = which == kRows ? rows_smem(P) : cols_smem(P);
   if (bytes > kSmemLimit) throw std::runtime_error("shared memory");
   emu::Guarded sm(bytes);
-  int nthr = strip_threads(bytes, grid, sms);
+  int nthr = strip_threads(P, which == kRows, grid, sms);
   if (a.mp > 44 && nthr > 128) nthr = 128;           // k_rp_matrix.cu
   switch (a.mp) {
     case 0: strip_body<0, IO>(P, which, (float2*)sm.get(), nthr, grid); break;
@@ -464,6 +464,11 @@ extern "C" {
 
 const char* emu_rp_message() { return message.c_str(); }
 int emu_rp_plan(int n, int* r0, int* r1) { return axis_plan(n, *r0, *r1) ? matrix_width(*r0) : -1; }
+int emu_rp_threads(int planes, int h, int w, int rows, int sms) {
+  Params P;
+  if (!fill_params(P, nullptr, 1, planes, h, w, 3, 1, 0, 0)) return -1;
+  return strip_threads(P, rows, (planes * (rows ? P.hh : P.wc) + kLines - 1) / kLines, sms);
+}
 int emu_rp_one_block(int B, int C, int H, int W, int s, int p, int sms) {
   return route(B, C, H, W, s, p, sms, false, (size_t)64 << 20).one_block;
 }

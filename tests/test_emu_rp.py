@@ -82,6 +82,16 @@ def test_forward_matches_the_oracle(emu, case):
     assert orc.rel_l2(gelu, torch.nn.functional.gelu(torch.from_numpy(ref)).numpy()) <= 4e-6
 
 
+@pytest.mark.parametrize("H,W,sizes", [(69, 46, (128, 96)), (58, 50, (128, 192)), (29, 65, (96, 256)), (64, 23, (256, 96))])
+def test_strip_block_sizes(emu, H, W, sizes):
+    """Blocks of other sizes than a power of two: the last turn of a stage leaves any number of half warps without work."""
+    assert tuple(emu.emu_rp_threads(2, H, W, rows, 1) for rows in (0, 1)) == sizes
+    w, b, rng = _weights(2, 3, H + W)
+    x = rng.standard_normal((1, 2, H, W)).astype(np.float32)
+    ref = orc.converse2d_forward(x, w, b, 1, 0, "circular", 1e-5, dtype=np.float64)
+    assert orc.rel_l2(_forward(emu, x, w, b, 1, 0, "circular", multi=1, sms=1), ref) <= 2e-6   # as test_forward_matches_the_oracle
+
+
 FIXED = [
     # integer contractions (one SM: every tile count takes them): B, C, H, W, k, s, p, mode
     (1, 1, 132, 140, 3, 1, 1, "circular"),        # 134 x 142: the shortest axes, odd halves
