@@ -18,9 +18,8 @@
 //
 // One block per SM walks over tiles of 128 lines (= rows of the MMA = lanes of tensor memory).  A tile arrives in shared
 // memory as it is; thread t serves line t % 128: it folds a quarter of the line's q, cuts the four classes into digits and
-// writes them to tensor memory (256 columns), from where the MMAs read them.  All products of a digit of the line with the
-// constants' digits are one MMA: the constants' digits lie side by side along N in shared memory (36 to 60 KB), and so do the
-// accumulators.  Outputs come in chunks of 32 frequencies of one parity, cosines and sines (what 32 does not divide: 16 of
+// writes them to tensor memory (256 columns), from where the MMAs read them.  The constants' digits lie side by side
+// along N in shared memory (36 to 60 KB), and so do the accumulators; a pair of digits is an MMA.  Outputs come in chunks of 32 frequencies of one parity, cosines and sines (what 32 does not divide: 16 of
 // both parities), in the other 256 columns of tensor memory; a thread reads back eight frequencies of its line.  The warp
 // that is the last to have read a chunk issues the MMAs of the next one, which run while the values are finished and stored.
 // q >= 64 (lengths from 256 on: at most four) is added in fp32 there.
@@ -180,16 +179,19 @@ __device__ __forceinline__ void fix_digits(const float (&v)[Q], float scale, uin
   for (int d = 0; d < 4; ++d) fx_st(t + 16 * d, w[d]);
 }
 
-// the MMAs of n frequencies of one class: digits at column a (16 columns each), accumulators at column t
+// the MMAs of n frequencies of one class: digits at column a (16 columns each), accumulators at column t.  One for each pair of
+// digits (i, j), i + j <= 3, into the accumulator i + j: MMAs keep the order of their issue only among those of the same
+// accumulator and shape, so every MMA that meets an accumulator has its columns and no others.
 __device__ __forceinline__ void fix_issue(const int n, uint32_t t, uint32_t a, const unsigned char* from, uint32_t elected) {
-  auto b = fx_operand(from, 3 * n);
-  // digit i of the line with the constants' digits 0 .. min(2, 3 - i) goes to the accumulators i, i + 1, ..
+  const auto b0 = fx_operand(from, 3 * n);
 #pragma unroll
-  for (int kc = 0; kc < 2; ++kc, a += 8, b = fx_further(b, 96 * n)) {
-    fx_mma(t, a, b, 3 * n, kc > 0, elected);
-    fx_mma(t + 3 * n, a + 48, b, n, kc > 0, elected);
-    fx_mma(t + n, a + 16, b, 3 * n, true, elected);
-    fx_mma(t + 2 * n, a + 32, b, 2 * n, true, elected);
+  for (int kc = 0; kc < 2; ++kc, a += 8) {
+#pragma unroll
+    for (int p = 0; p < 9; ++p) {
+      // (the four that begin an accumulator first, neighbours on different ones)
+      const int i = p < 3 ? 0 : p == 3 ? 3 : p < 7 ? 1 : 2, j = p < 3 ? p : p == 3 ? 0 : p < 7 ? p - 4 : p - 7;
+      fx_mma(t + (i + j) * n, a + 16 * i, fx_further(b0, 96 * n * kc + 16 * n * j), n, kc > 0 || p > 3, elected);
+    }
   }
 }
 // chunk `it` of a pass: chunks of 32 (`full` per parity), then the rest of both parities; a whole warp

@@ -190,7 +190,9 @@ static inline unsigned max(unsigned a, unsigned b) { return a > b ? a : b; }
 #define __syncwarp() emu::wait(emu::Fiber::kWarp)
 
 // Tensor memory, the integer MMA (the second operand in rows of 16 bytes, eight rows a core matrix, K = 32), barriers in
-// shared memory and asynchronous copies of cvb_fix.cuh.  MMAs and copies happen at once.
+// shared memory and asynchronous copies of cvb_fix.cuh.  MMAs and copies happen at once.  On the GPU MMAs follow each other
+// in the order of their issue only where they have the same accumulator and shape; others may overtake one another until a
+// commit of theirs has been waited for, so that accumulators which overlap otherwise are an error here.
 #include <cstdint>
 #include <map>
 namespace cvb {
@@ -224,7 +226,9 @@ inline bool fx_wait(uint64_t* p, uint32_t parity) {
   }
   return true;
 }
-inline void fx_commit(uint64_t* p) { Barrier& b = barrier(p); --b.pending; settle(b); }
+struct Issued { uint32_t d; int n; };
+static std::vector<Issued> in_flight;      // since the last commit, which the kernel waits for before it issues again
+inline void fx_commit(uint64_t* p) { Barrier& b = barrier(p); --b.pending; settle(b); in_flight.clear(); }
 inline unsigned fx_count(unsigned* c) { return (*c)++; }
 inline uint32_t fx_elect() { return emu::fiber->lane == 0; }
 inline unsigned fx_from_first(unsigned v) { return (unsigned)emu::exchange(&emu::WarpSlots::i, (int)v, 0); }
@@ -245,6 +249,9 @@ inline void fx_mma(uint32_t d, uint32_t a, Operand o, int n, bool add, uint32_t 
   const unsigned char* b = o.at;
   const int brows = o.rows;
   if (n % 16 || n < 16 || n > 256 || d < 256 || d + n > 512 || a + 8 > 256 || (size_t)b % 16) throw std::runtime_error("MMA form");
+  for (const Issued& i : in_flight)
+    if ((i.d != d || i.n != n) && d < i.d + i.n && i.d < d + n) throw std::runtime_error("MMAs on overlapping accumulators have no order");
+  in_flight.push_back({d, n});
   for (int m = 0; m < 128; ++m) {
     const signed char* l = (const signed char*)&tensor_memory[m][a];
     for (int j = 0; j < n; ++j) {
