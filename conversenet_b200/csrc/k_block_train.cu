@@ -202,9 +202,9 @@ static int launch_grad(const BlockGradParams& P, int sms, cudaStream_t st) {
 // out[p][q] = sum over pixels of P[p] Q[q], 64 x 128, and the sums of every P[p] and Q[q]; Q optionally through GELU.
 // A block takes 32-pixel tiles blockIdx.x, + gridDim.x, ...: its threads split the 192 channels' values into TF32 hi + lo
 // (exact to 2^-22 of a value) in shared memory, channels as rows and pixels along K, and one tile's MMAs (Q in the 128 rows
-// of tensor memory, [P hi | P lo] side by side) run while the next is split.  The accumulators are read and added to fp32
-// sums in registers after every tile: the tensor cores cut what they add off instead of rounding it, which over four
-// additions stays below what rounding the sum of a block's thousand pixels costs: gradients of w1 to w4 of a block of
+// of tensor memory; hi hi in 64 columns, hi lo + lo hi in another 64) run while the next is split.  The accumulators are read
+// and added to fp32 sums in registers after every tile: the tensor cores cut what they add off instead of rounding it, which over
+// four additions (eight of the small products) stays below what rounding the sum of a block's thousand pixels costs: gradients of w1 to w4 of a block of
 // 8 x 64 x 64 are within 5.7e-7 to 8.5e-7 of fp64 (8.0e-7 to 1.1e-6 with fp32 products on the CUDA cores).  32768 pixels,
 // the four contractions: 50 us, 99 on the CUDA cores (which waited for the port to shared memory); 100 MB take 15 us.  The
 // erf of the GELUs, the split and its stores are the larger part of a tile.
@@ -302,9 +302,13 @@ __global__ void __launch_bounds__(kGThreads, 2) wgrad_kernel(const __grid_consta
       for (int ks = 0; ks < 4; ++ks) {
         const uint64_t qh = tc::smem_desc(base + 2 * ks * kGGroup, kGGroup, 128);
         const uint64_t ql = tc::smem_desc(base + kGOperand + 2 * ks * kGGroup, kGGroup, 128);
-        const uint64_t pb = tc::smem_desc(base + 2 * kGOperand + 2 * ks * kGGroup, kGGroup, 128);
-        tc::mma_tf32_elected(tmem, qh, pb, tc::idesc_tf32(128, 128, false, false), ks > 0 ? 1u : 0u, e);
-        tc::mma_tf32_elected(tmem + 64u, ql, pb, tc::idesc_tf32(128, 64, false, false), 1u, e);
+        const uint64_t ph = tc::smem_desc(base + 2 * kGOperand + 2 * ks * kGGroup, kGGroup, 128);
+        const uint64_t pl = tc::smem_desc(base + 2 * kGOperand + 2 * ks * kGGroup + 64 * 16, kGGroup, 128);
+        // (all of one shape: MMAs of another one on the same columns would have no order among them)
+        constexpr uint32_t idesc = tc::idesc_tf32(128, 64, false, false);
+        tc::mma_tf32_elected(tmem, qh, ph, idesc, ks > 0 ? 1u : 0u, e);
+        tc::mma_tf32_elected(tmem + 64u, qh, pl, idesc, ks > 0 ? 1u : 0u, e);
+        tc::mma_tf32_elected(tmem + 64u, ql, ph, idesc, 1u, e);
       }
       if (e) tc::mma_commit(done);
     }

@@ -260,6 +260,48 @@ def test_block_and_its_gradients_match_the_layer_by_layer_block(monkeypatch, B, 
     assert _cabi.load().cvb_last_device_status(1) == 0
 
 
+def _block_fp64(q, conv, mode, x):
+    """ConverseBlock in 64 bits: q the fourteen parameters of functional.block_parameters (None for absent alphas)."""
+    from conversenet_b200.autograd import spectral_forward
+    F = torch.nn.functional
+
+    def norm(v, w, b):
+        u = v.mean(1, keepdim=True)
+        return (v - u) / torch.sqrt((v - u).pow(2).mean(1, keepdim=True) + 1e-5) * w[:, None, None] + b[:, None, None]
+    t = F.gelu(F.conv2d(norm(x, q[0], q[1]), q[2], q[3]))
+    t = F.gelu(spectral_forward(t, conv[0], conv[1], 1, conv[2], mode, 1e-5))
+    x1 = x + (1.0 if q[6] is None else q[6]) * F.conv2d(t, q[4], q[5])
+    return x1 + (1.0 if q[13] is None else q[13]) * F.conv2d(F.gelu(F.conv2d(norm(x1, q[7], q[8]), q[9], q[10])), q[11], q[12])
+
+
+@pytest.mark.parametrize("B,H,W", [(1, 4, 5), (2, 64, 64), (5, 33, 47)])
+def test_block_gradients_match_fp64(B, H, W):
+    """Every gradient of a block against 64 bits: less than one tile of 32 pixels, one or two a block of the weight
+    gradients, several with a short last one."""
+    from conversenet_b200 import ConverseBlockAlphaVariant
+    from conversenet_b200 import _cabi, functional as CF
+    torch.manual_seed(H)
+    blk = ConverseBlockAlphaVariant(64, 64, 5, 1, 4, "replicate").cuda()
+    with torch.no_grad():
+        for q in blk.parameters():
+            if q.dim() == 1 or q.shape[-1] == 1 and q.shape[0] == 1:
+                q.add_(0.2 * torch.randn_like(q))
+    c1, c2 = blk.conv1, blk.conv2
+    params = list(CF.block_parameters(c1[0], c1[1], c1[5], blk.alpha1, c2[0], c2[1], c2[3], blk.alpha2)) + [c1[3].weight, c1[3].bias]
+    x = torch.randn(B, 64, H, W, device="cuda", requires_grad=True)
+    y = blk(x)
+    g = torch.randn_like(y)
+    got = [y] + list(torch.autograd.grad(y, [x] + params, g))
+    a = [t.detach().double().requires_grad_(True) for t in [x] + params]
+    ref = _block_fp64(a[1:15], (a[15], a[16], 4), "replicate", a[0])
+    want = [ref] + list(torch.autograd.grad(ref, a, g.double()))
+    assert _cabi.load().cvb_last_device_status(1) == 0
+    # TF32 hi + lo is within 2^-22 of a value and lo lo (2^-24) is left out: below the rounding of fp32 sums of as many
+    # pixels; a bit of the operands lost would be 1e-5
+    errors = [_rel(u, v) for u, v in zip(got, want)]
+    assert max(errors) <= 2e-6, errors
+
+
 @pytest.mark.parametrize("B,H,W", [(3, 41, 64), (5, 33, 47)])
 def test_block_gradients_over_several_tiles_of_pixels(monkeypatch, B, H, W):
     """246 and 243 tiles of 32 pixels: three or four a block of the weight gradients, so that both operand buffers are reused."""
