@@ -36,11 +36,14 @@ namespace cvb {
 
 // ---- packed weights: PRE | POST, each a multiple of 16 bytes: matrices as fp16 hi and lo (16 KB each), every row scaled by a
 // power of two to below 2^14, then fp32 vectors.  The factors that undo the scales of a row and of its operand are in the
-// vectors: 1 / (row scale x kNormScale) for what follows a LayerNorm (its values stay below 8), for W4 with the scale of the
-// hidden values, of which a bound follows from W3 and b3; t is scaled pixel by pixel.
+// vectors: 1 / (row scale x kNormScale) for what follows a LayerNorm (its values stay below 8), 1 / row scale for W2 and W4.  Every
+// hidden value has a scale of its own (a bound of it follows from its row of W3 and its b3), which W4's columns undo before
+// its rows are scaled: with one scale for all 128, a row of W3 2^20 times the others left these only their hi halves' bits.
+// t is scaled pixel by pixel.
 constexpr float kNormScale = 1024.f;
 constexpr int kPreFloats = kW + 2 * kBlkM;                      // W1; b1, undo1
-constexpr int kPostFloats = 3 * kW + 6 * kBlkC + 2 * kBlkM + 4; // W2, W3, W4; b2, a1, b4, a2, undo2, undo4; b3, undo3; hidden scale
+constexpr int kPostFloats = 3 * kW + 6 * kBlkC + 2 * kBlkM + kBlkM / 2; // W2, W3, W4; b2, a1, b4, a2, undo2, undo4; b3, undo3;
+                                                                // hidden scales (powers of two, as bf16)
 enum { kB2 = 0, kA1 = kBlkC, kB4 = 2 * kBlkC, kA2 = 3 * kBlkC, kUndo2 = 4 * kBlkC, kUndo4 = 5 * kBlkC, kB3 = 6 * kBlkC,
        kUndo3 = 6 * kBlkC + kBlkM, kHidden = 6 * kBlkC + 2 * kBlkM };
 size_t block_pack_bytes() { return (size_t)(kPreFloats + kPostFloats) * sizeof(float); }
@@ -60,7 +63,7 @@ __device__ __forceinline__ float to_2_14(float m) {
 
 // grid: 4 matrices x 16 slices.  The LayerNorm affine is folded into the weights that follow it.
 __global__ void __launch_bounds__(256) block_pack_kernel(const PackParams P) {
-  __shared__ float part[8];
+  __shared__ float hidden[kBlkM];
   const int which = blockIdx.x >> 4, slice = blockIdx.x & 15, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* post = P.out + kPreFloats;
   const float* w = which == 0 ? P.w1 : which == 1 ? P.w2 : which == 2 ? P.w3 : P.w4;
@@ -70,10 +73,8 @@ __global__ void __launch_bounds__(256) block_pack_kernel(const PackParams P) {
   float* vec = which == 0 ? P.out + kW : post + 3 * kW;
   const float* bias = which == 0 ? P.b1 : which == 1 ? P.b2 : which == 2 ? P.b3 : P.b4;
   const float* beta = which == 0 ? P.ln1_b : which == 2 ? P.ln2_b : nullptr;
-  // the hidden values' bound: |W3 . v + b3'| <= 8 |W3 row| + |b3'| for a normalised v of 64 values
-  float hidden = 1.f;
+  // the hidden values' bounds: |W3 . v + b3'| <= 8 |W3 row| + |b3'| for a normalised v of 64 values
   if (which == 3 || (which == 2 && slice == 0)) {
-    float most = 0.f;
     for (int n = warp; n < kBlkM; n += 8) {
       float q = 0.f, d = 0.f;
       for (int k = lane; k < kBlkC; k += 32) {
@@ -82,27 +83,31 @@ __global__ void __launch_bounds__(256) block_pack_kernel(const PackParams P) {
         d = fmaf(a, P.ln2_b[k], d);
       }
       for (int o = 16; o; o >>= 1) { q += __shfl_xor_sync(0xffffffffu, q, o); d += __shfl_xor_sync(0xffffffffu, d, o); }
-      most = fmaxf(most, 8.f * sqrtf(q) + fabsf(d + P.b3[n]));
+      const float most = 8.f * sqrtf(q) + fabsf(d + P.b3[n]);
+      if (lane == 0) hidden[n] = most > 0.f ? to_2_14(1.001f * most) : 0x1p100f;      // (of the rounding of the sums; no values at all)
     }
-    if (lane == 0) part[warp] = most;
     __syncthreads();
-    for (int i = 0; i < 8; ++i) most = fmaxf(most, part[i]);
-    hidden = to_2_14(1.001f * most);        // (of the rounding of the sums)
-    if (which == 2 && threadIdx.x == 0) vec[kHidden] = hidden;
+    if (which == 2 && threadIdx.x < kBlkM) {       // a thread's 32 of each 64 channels lie behind its other vectors' channels
+      const int n = threadIdx.x;
+      ((__nv_bfloat16*)(vec + kHidden))[(n & 32) * 2 + (n >> 6) * 32 + (n & 31)] = __float2bfloat16(hidden[n]);
+    }
   }
+  auto weight = [&](int n, int k) {
+    const float a = w[n * K + k];
+    return g ? a * g[k] : which == 3 ? a / hidden[k] : a;
+  };
   const int rows = N / 16;
   for (int r = warp; r < rows; r += 8) {
     const int n = slice * rows + r;
     float m = 0.f, d = 0.f;
     for (int k = lane; k < K; k += 32) {
-      const float a = w[n * K + k];
-      m = fmaxf(m, fabsf(g ? a * g[k] : a));
-      if (beta) d = fmaf(a, beta[k], d);
+      m = fmaxf(m, fabsf(weight(n, k)));
+      if (beta) d = fmaf(w[n * K + k], beta[k], d);
     }
     for (int o = 16; o; o >>= 1) { m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o)); d += __shfl_xor_sync(0xffffffffu, d, o); }
     const float f = to_2_14(m);
     for (int k = lane; k < K; k += 32) {
-      const float a = (g ? w[n * K + k] * g[k] : w[n * K + k]) * f;
+      const float a = weight(n, k) * f;
       const __half h = __float2half_rn(a);
       hi[pack_index16(N, n, k)] = h;
       hi[kW + pack_index16(N, n, k)] = __float2half_rn(a - __half2float(h));
@@ -112,7 +117,7 @@ __global__ void __launch_bounds__(256) block_pack_kernel(const PackParams P) {
     if (which == 0) { vec[n] = b; vec[kBlkM + n] = 1.f / (f * kNormScale); }
     if (which == 1) { vec[kB2 + n] = b; vec[kUndo2 + n] = 1.f / f; vec[kA1 + n] = P.a1 ? P.a1[n] : 1.f; }
     if (which == 2) { vec[kB3 + n] = b; vec[kUndo3 + n] = 1.f / (f * kNormScale); }
-    if (which == 3) { vec[kB4 + n] = b; vec[kUndo4 + n] = 1.f / f / hidden; vec[kA2 + n] = P.a2 ? P.a2[n] : 1.f; }
+    if (which == 3) { vec[kB4 + n] = b; vec[kUndo4 + n] = 1.f / f; vec[kA2 + n] = P.a2 ? P.a2[n] : 1.f; }
   }
 }
 
@@ -313,7 +318,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
           float a[32];
           tc::tmem_ld32(lane + (uint32_t)h0, a);
 #ifdef __CUDA_ARCH__
-          const float hs = vec[kHidden];
+          const uint32_t* hs = (const uint32_t*)(vh + kHidden) + h0 / 4;
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
             const float2 b = *(const float2*)(vh + kB3 + h0 + j), u = *(const float2*)(vh + kUndo3 + h0 + j);
@@ -324,7 +329,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
               zp[(size_t)j * HW] = za;
               zp[(size_t)(j + 1) * HW] = zb;
             }
-            v[j] = o.x * hs; v[j + 1] = o.y * hs;
+            v[j] = o.x * __uint_as_float(hs[j / 2] << 16); v[j + 1] = o.y * __uint_as_float(hs[j / 2] & 0xffff0000u);
           }
 #endif
         } else {                                    // 64 channels of t

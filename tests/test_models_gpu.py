@@ -298,3 +298,73 @@ def test_block_kernels_at_any_magnitude(B, H, W, dtype, t_kind):
     rel = lambda a, r: float((a.double() - r).norm() / r.norm())
     assert rel(pre, want_pre) <= bar and rel(post[~nan], want[~nan]) <= bar
     assert lib.cvb_last_device_status(1) == 0
+
+
+def _block_kernels_and_fp64(blk, x, t):
+    """Both 1x1 kernels of a block and what 64 bits give for x (B,64,H,W) and t (B,128,H,W): (pre, post), (pre, x1, post)."""
+    from conversenet_b200 import _cabi
+    from conversenet_b200 import functional as CF
+    F = torch.nn.functional
+    B, _, H, W = x.shape
+    with torch.no_grad():
+        c1, c2 = blk.conv1._modules, blk.conv2._modules
+        pack = blk._packed(CF.block_parameters(c1["0"], c1["1"], c1["5"], None, c2["0"], c2["1"], c2["3"], None))
+        eps, lib, st, io = c1["0"].eps, _cabi.load(), torch.cuda.current_stream().cuda_stream, int(x.dtype == torch.bfloat16)
+        pre, post = torch.empty_like(t), torch.empty_like(x)
+        assert lib.cvb_block_pre_fwd(x.data_ptr(), pre.data_ptr(), pack.data_ptr(), eps, B, H * W, io, st) == 0
+        assert lib.cvb_block_post_fwd(t.data_ptr(), x.data_ptr(), post.data_ptr(), pack.data_ptr(), eps, B, H * W, io, st) == 0
+
+        def conv(v, m):
+            return F.conv2d(v, m.weight.double(), m.bias.double())
+
+        def norm(v, m):
+            u = v.mean(1, keepdim=True)
+            s = (v - u).pow(2).mean(1, keepdim=True)
+            return (v - u) / torch.sqrt(s + eps) * m.weight.double()[:, None, None] + m.bias.double()[:, None, None]
+        x1 = x.double() + conv(t.double(), c1["5"])
+        want = (F.gelu(conv(norm(x.double(), c1["0"]), c1["1"])), x1, x1 + conv(F.gelu(conv(norm(x1, c2["0"]), c2["1"])), c2["3"]))
+    assert lib.cvb_last_device_status(1) == 0
+    return (pre, post), want
+
+
+def _worst_channel(a, r):
+    return float(((a.double() - r).pow(2).sum((0, 2, 3)) / r.pow(2).sum((0, 2, 3))).max().sqrt())
+
+
+@pytest.mark.parametrize("H, W", [(24, 32), (21, 25)])      # rows that are copied ahead, rows that are not
+@pytest.mark.parametrize("kind", ["a row of W3", "an entry of b3", "a row of zeros", "all rows", "the norms"])
+def test_block_kernels_on_uneven_weights(kind, H, W):
+    """A hidden channel may be 2^20 times the others (and its column of W4 as much smaller), rows and norms of any size."""
+    from conversenet_b200 import ConverseBlock
+    g = torch.Generator(device="cuda").manual_seed(H)
+    torch.manual_seed(H)
+    blk = ConverseBlock(64, 64, 3, 1, 1).cuda().eval()
+    w1, w2, w3, w4 = blk.conv1[1], blk.conv1[5], blk.conv2[1], blk.conv2[3]
+    with torch.no_grad():
+        w4.weight.mul_(100)           # (the second branch outweighs x1)
+        if kind == "a row of W3":
+            w3.weight[5] *= 2.0 ** 20
+            w3.bias[5] *= 2.0 ** 20
+            w4.weight[:, 5] *= 2.0 ** -20
+        elif kind == "an entry of b3":
+            w3.bias[70] = 2.0 ** 20
+            w4.weight[:, 70] *= 2.0 ** -20
+        elif kind == "a row of zeros":
+            w3.weight[9], w3.bias[9], w1.weight[3] = 0, 0, 0
+        elif kind == "all rows":
+            for m in (w1, w2, w3, w4):
+                f = torch.exp(4 * torch.randn(m.weight.size(0), device="cuda", generator=g))
+                m.weight.mul_(f[:, None, None, None])
+                m.bias.mul_(f)
+            w4.weight.div_(w3.weight.abs().amax((1, 2, 3))[None, :, None, None])
+        else:
+            for m in (blk.conv1[0], blk.conv2[0]):
+                m.weight.copy_(torch.exp(2 * torch.randn(64, device="cuda", generator=g)))
+                m.bias.copy_(torch.randn(64, device="cuda", generator=g))
+        x = torch.randn(2, 64, H, W, device="cuda", generator=g)
+        t = torch.nn.functional.gelu(torch.randn(2, 128, H, W, device="cuda", generator=g))
+    (pre, post), want = _block_kernels_and_fp64(blk, x, t)
+    live = want[0].pow(2).sum((0, 2, 3)) > 0
+    # 22 bits of each operand and fp32 sums of 64 and 128 products, in the worst channel
+    assert _worst_channel(pre[:, live], want[0][:, live]) <= 2e-6
+    assert _worst_channel(post, want[2]) <= 2e-6
