@@ -53,12 +53,12 @@ struct PackParams {
   float* out;
 };
 
-// the power of two that takes m to [2^13, 2^14) (1 for zero, infinities and NaN)
-__device__ __forceinline__ float to_2_14(float m) {
+// the power of two that takes m to [2^13, 2^14), at most 2^most (1 for zero, infinities and NaN)
+__device__ __forceinline__ float to_2_14(float m, int most) {
   const int e = (int)(__float_as_uint(m) >> 23);
   if (e == 0 || e >= 255) return 1.f;
-  const int f = 127 + 13 + 127 - e;      // (at most 2^100: its product with other scales stays finite)
-  return __uint_as_float((uint32_t)(f < 1 ? 1 : f > 227 ? 227 : f) << 23);
+  const int f = 127 + 13 + 127 - e;
+  return __uint_as_float((uint32_t)(f < 1 ? 1 : f > 127 + most ? 127 + most : f) << 23);
 }
 
 // grid: 4 matrices x 16 slices.  The LayerNorm affine is folded into the weights that follow it.
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256) block_pack_kernel(const PackParams P) {
       }
       for (int o = 16; o; o >>= 1) { q += __shfl_xor_sync(0xffffffffu, q, o); d += __shfl_xor_sync(0xffffffffu, d, o); }
       const float most = 8.f * sqrtf(q) + fabsf(d + P.b3[n]);
-      if (lane == 0) hidden[n] = most > 0.f ? to_2_14(1.001f * most) : 0x1p100f;      // (of the rounding of the sums; no values at all)
+      if (lane == 0) hidden[n] = most > 0.f ? to_2_14(1.001f * most, 100) : 0x1p100f;      // (1.001: sums are rounded; 2^100: W4's columns stay normal)
     }
     __syncthreads();
     if (which == 2 && threadIdx.x < kBlkM) {       // a thread's 32 of each 64 channels lie behind its other vectors' channels
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(256) block_pack_kernel(const PackParams P) {
       if (beta) d = fmaf(w[n * K + k], beta[k], d);
     }
     for (int o = 16; o; o >>= 1) { m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o)); d += __shfl_xor_sync(0xffffffffu, d, o); }
-    const float f = to_2_14(m);
+    const float f = to_2_14(m, 126);
     for (int k = lane; k < K; k += 32) {
       const float a = weight(n, k) * f;
       const __half h = __float2half_rn(a);
@@ -114,9 +114,9 @@ __global__ void __launch_bounds__(256) block_pack_kernel(const PackParams P) {
     }
     if (lane) continue;
     const float b = bias[n] + d;
-    if (which == 0) { vec[n] = b; vec[kBlkM + n] = 1.f / (f * kNormScale); }
+    if (which == 0) { vec[n] = b; vec[kBlkM + n] = 1.f / f / kNormScale; }
     if (which == 1) { vec[kB2 + n] = b; vec[kUndo2 + n] = 1.f / f; vec[kA1 + n] = P.a1 ? P.a1[n] : 1.f; }
-    if (which == 2) { vec[kB3 + n] = b; vec[kUndo3 + n] = 1.f / (f * kNormScale); }
+    if (which == 2) { vec[kB3 + n] = b; vec[kUndo3 + n] = 1.f / f / kNormScale; }
     if (which == 3) { vec[kB4 + n] = b; vec[kUndo4 + n] = 1.f / f; vec[kA2 + n] = P.a2 ? P.a2[n] : 1.f; }
   }
 }
@@ -307,7 +307,8 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
           tc::tmem_ld32(lane, a);
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
-            x1[j] = fmaf(vh[kA1 + j], fmaf(a[j] * undo, vh[kUndo2 + j], vh[kB2 + j]), COPIES ? v[j] : x1[j]);
+            // (both factors are powers of two: their product first, or a sum times one of them may overflow alone)
+            x1[j] = fmaf(vh[kA1 + j], fmaf(a[j], vh[kUndo2 + j] * undo, vh[kB2 + j]), COPIES ? v[j] : x1[j]);
             v[j] = x1[j];
             if (TRAIN && valid) P.x1[(op_out - (IO*)P.out) + (size_t)j * HW] = x1[j];
           }
@@ -349,7 +350,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) block_mix_kernel(const __grid_
           for (int j = 0; j < 32; ++j) most = fmaxf(most, fabsf(v[j]));
           mine()->x = most;
           mix_bar(g);
-          const int e = min(max((int)(__float_as_uint(fmaxf(most, other()->x)) >> 23), 32), 254);
+          const int e = min(max((int)(__float_as_uint(fmaxf(most, other()->x)) >> 23), 11), 254);
           if (ph == 0) {
             top = e;
           } else if (__any_sync(0xffffffffu, e > top + 4)) {       // it is larger still: the sums so far are scaled down

@@ -368,3 +368,19 @@ def test_block_kernels_on_uneven_weights(kind, H, W):
     # 22 bits of each operand and fp32 sums of 64 and 128 products, in the worst channel
     assert _worst_channel(pre[:, live], want[0][:, live]) <= 2e-6
     assert _worst_channel(post, want[2]) <= 2e-6
+
+
+@pytest.mark.parametrize("H, W", [(24, 32), (21, 25)])
+@pytest.mark.parametrize("t_size, w_size", [(2.0 ** 116, 2.0 ** -83), (2.0 ** 116, 2.0 ** -110), (2.0 ** -100, 2.0 ** 96), (2.0 ** -120, 2.0 ** 110)])
+def test_block_kernel_on_huge_and_tiny_values(t_size, w_size, H, W):
+    """t and W2 at the ends of fp32's range, their products within it."""
+    from conversenet_b200 import ConverseBlock
+    g = torch.Generator(device="cuda").manual_seed(H)
+    torch.manual_seed(W)
+    blk = ConverseBlock(64, 64, 3, 1, 1).cuda().eval()
+    with torch.no_grad():
+        blk.conv1[5].weight.mul_(w_size)
+        x = torch.randn(2, 64, H, W, device="cuda", generator=g)
+        t = torch.nn.functional.gelu(torch.randn(2, 128, H, W, device="cuda", generator=g)) * t_size
+    (_, post), want = _block_kernels_and_fp64(blk, x, t)
+    assert _worst_channel(post, want[2]) <= 2e-6
