@@ -13,8 +13,8 @@
 // accumulate exactly in 32-bit integers (tcgen05.mma kind::i8), one accumulator per weight 256^-(i + j), i + j <= 3; what
 // is left out lies 2^-32 below the largest value.  So the only roundings are those of the constants (2^-24), the folds and
 // the result: 1.8e-7 of a 268 x 268 plane's norm against fp64, where fp32 butterflies and dense stages are at 2.2e-7 or
-// more.  A line whose largest value is below 2^-87 loses precision gradually; one with an infinity or a NaN becomes NaN, and
-// with it, as in any transform, its plane.
+// more, whatever the magnitude of a line (one whose largest value is below 2^-87 takes its scale in two steps).  A line
+// with an infinity or a NaN becomes NaN, and with it, as in any transform, its plane.
 //
 // One block per SM walks over tiles of 128 lines (= rows of the MMA = lanes of tensor memory).  A tile arrives in shared
 // memory as it is; thread t serves line t % 128: it folds a quarter of the line's q, cuts the four classes into digits and
@@ -159,6 +159,11 @@ __host__ __device__ inline int fix_lines(int kind, const Params& P) {
   return P.nplane * (kind == kFixRows ? 2 * P.hh : fix_columns(kind, P));
 }
 
+// what a line's scale 2^(29 - exponent), 2^116 at most, lacks for its largest value (its bits) to reach 2^29
+__device__ __forceinline__ float fix_rest(unsigned largest) {
+  const int ex = (int)(largest >> 23);
+  return __uint_as_float((uint32_t)(127 + (ex < 1 ? 39 : ex < 40 ? 40 - ex : 0)) << 23);
+}
 // a thread's values of a class to tensor memory: Q / 4 columns of each digit
 template <int Q>
 __device__ __forceinline__ void fix_digits(const float (&v)[Q], float scale, uint32_t t) {
@@ -391,8 +396,16 @@ __device__ __forceinline__ void fix_body(const Params& P, unsigned char* smem) {
       // ---- digits ----
       int ex = (int)(*largest >> 23);
       const bool bad = ex >= 255;
+      const bool tiny = __any_sync(0xffffffffu, ex < 40 && *largest != 0);            // somewhere in the warp
       ex = ex < 40 ? 40 : ex > 254 ? 254 : ex;
       const float scale = __uint_as_float((uint32_t)(283 - ex) << 23);             // 2^(29 - exponent)
+      if (tiny) {
+        const float rest = fix_rest(*largest);
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int i = 0; i < QP; ++i) v[c][i] *= rest;
+      }
       // x = n / scale, constant = m * unit, the accumulators' lowest weight is 2^16
       const float undo = bad ? __uint_as_float(0x7fc00000u) : kTwice * (kFixUnit * 65536.f) * __uint_as_float((uint32_t)(ex - 29) << 23);
       if (q0 <= QH) {
@@ -437,6 +450,14 @@ __device__ __forceinline__ void fix_body(const Params& P, unsigned char* smem) {
           fx_ld_wait();
           fx_before_sync();
           fix_values<JP>(acc, undo, D);
+          if (tiny) {
+            const float back = 1.f / fix_rest(S.largest[(flip ^ 1) * kFixLines + line]);
+#pragma unroll
+            for (int i = 0; i < JP / 2; ++i) {
+              C[i] = fx_mul2(C[i], make_float2(back, back));
+              D[i] = fx_mul2(D[i], make_float2(back, back));
+            }
+          }
         }
         __syncwarp();
         if (it + 1 < chunks) {

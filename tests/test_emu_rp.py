@@ -124,14 +124,16 @@ def test_integer_contractions(emu, case):
 
 def test_integer_contractions_on_values_of_any_size(emu):
     """Lines are scaled one by one: planes of very different magnitudes, zeros, an infinity and a NaN do not meet."""
-    w, b, rng = _weights(6, 3, 7)
+    w, b, rng = _weights(8, 3, 7)
     w[:], b[:] = w[:, :1], b[:, :1]
-    x = np.repeat(rng.standard_normal((1, 1, 132, 140)).astype(np.float32), 6, axis=1)
+    x = np.repeat(rng.standard_normal((1, 1, 132, 140)).astype(np.float32), 8, axis=1)
+    x[:, 6] *= np.float32(2.0 ** -100)
+    x[:, 7] *= np.float32(2.0 ** -108)
     for c, f in enumerate((1.0, 2.0 ** -80, 2.0 ** 90, 0.0)):
         x[:, c] *= np.float32(f)
     x[0, 4, 60, 70], x[0, 5, 5, 9] = np.inf, np.nan
     out = _forward(emu, x, w, b, 1, 1, "circular", multi=1, sms=1)[0]
-    for c, f in ((1, 2.0 ** -80), (2, 2.0 ** 90)):
+    for c, f in ((1, 2.0 ** -80), (2, 2.0 ** 90), (6, 2.0 ** -100), (7, 2.0 ** -108)):
         assert np.array_equal(out[c] / np.float32(f), out[0])      # powers of two: not one bit differs
     assert not out[3].any() and not np.isfinite(out[4]).any() and np.isnan(out[5]).all()
 
