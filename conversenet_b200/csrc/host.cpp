@@ -110,15 +110,18 @@ at::Tensor f32(const at::Tensor& t) {
   return t.detach().to(at::kFloat).contiguous();
 }
 
-// `pairs`: `table` is the pair table and the pair kernels run; else the table of build_transfer for any batch, or the
-// real-plane one (both begin with what cvb_plane_fwd reads)
+// What `table` is and who reads it: the table of build_transfer for any batch (or one that serves this batch as well); the pair
+// table alone, for the pair kernels; the real-plane one (or one that begins with it), for the real planes where
+// cvb_takes_planes prefers them
+enum Form { kAnyBatch = 0, kPairTable = 1, kPlaneTable = 2 };
 at::Tensor forward(const at::Tensor& x, const at::Tensor& table, const at::Tensor& wf, int k, int s, int p, int mode,
-                   int gelu, at::Tensor out, bool pairs) {
+                   int gelu, at::Tensor out, int form) {
   const int B = (int)x.size(0), C = (int)x.size(1), H = (int)x.size(2), W = (int)x.size(3), io = io_type(x);
   if (!out.defined()) out = at::empty({B, C, (int64_t)H * s, (int64_t)W * s}, x.options().requires_grad(false));
   const size_t full = sizeof(float) * 2 * (size_t)C * (H + 2 * p) * (W + 2 * p);   // below that: no pair table in it
-  const bool planes = !pairs && api.takes_planes(B, C, H + 2 * p, W + 2 * p, s);
-  if ((size_t)table.numel() < full && !planes && (pairs || api.takes_pairs(B, H + 2 * p, W + 2 * p, s) == 2))
+  const bool pairs = form == kPairTable, planes = !pairs && api.takes_planes(B, C, H + 2 * p, W + 2 * p, s);
+  if ((size_t)table.numel() < full && !(planes && form == kPlaneTable) &&
+      (pairs || api.takes_pairs(B, H + 2 * p, W + 2 * p, s) == 2))
     throw Failed("the transfer table was built for another batch size");
   const size_t ws = pairs    ? api.pair_workspace_bytes(B, C, H, W, s, p)
                     : planes ? api.plane_workspace_bytes(B, C, H, W, s, p)
@@ -155,7 +158,7 @@ void want(Py_ssize_t n, Py_ssize_t m) {
   if (n != m) throw Failed("wrong number of arguments");
 }
 
-// converse2d(x, table, weight_f32, kernel_size, scale, padding, padding_mode, fuse_gelu, out or None, pairs)
+// converse2d(x, table, weight_f32, kernel_size, scale, padding, padding_mode, fuse_gelu, out or None, form)
 PyObject* py_converse2d(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     want(n, 10);
@@ -163,14 +166,13 @@ PyObject* py_converse2d(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (x0.dim() != 4) throw Failed("x must be (B,C,H,W)");
     const c10::cuda::CUDAGuard dev(x0.device());
     const at::Tensor &table = tensor(a[1], "table"), &wf = tensor(a[2], "weight");
-    const bool pairs = PyObject_IsTrue(a[9]);
-    const int k = (int)integer(a[3]), s = (int)integer(a[4]), p = (int)integer(a[5]), mode = pad_mode(a[6]);
+    const int k = (int)integer(a[3]), s = (int)integer(a[4]), p = (int)integer(a[5]), mode = pad_mode(a[6]), form = (int)integer(a[9]);
     const int gelu = PyObject_IsTrue(a[7]);
     at::Tensor out;
     if (a[8] != Py_None) out = tensor(a[8], "out");
     {
       const Unlocked unlocked;
-      out = forward(x0.is_contiguous() ? x0 : x0.contiguous(), table, wf, k, s, p, mode, gelu, std::move(out), pairs);
+      out = forward(x0.is_contiguous() ? x0 : x0.contiguous(), table, wf, k, s, p, mode, gelu, std::move(out), form);
     }
     return THPVariable_Wrap(std::move(out));
   });
@@ -363,7 +365,7 @@ PyObject* py_block_pack(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
-// block(x, table, weight_f32, pack, kernel_size, padding, padding_mode, eps1, eps2, pairs) -> ConverseBlock.forward(x)
+// block(x, table, weight_f32, pack, kernel_size, padding, padding_mode, eps1, eps2, form) -> ConverseBlock.forward(x)
 PyObject* py_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     want(n, 10);
@@ -374,7 +376,7 @@ PyObject* py_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int B = (int)x0.size(0), C = (int)x0.size(1), H = (int)x0.size(2), W = (int)x0.size(3), io = io_type(x0);
     const int k = (int)integer(a[4]), p = (int)integer(a[5]), mode = pad_mode(a[6]);
     const float eps1 = (float)real(a[7]), eps2 = (float)real(a[8]);
-    const bool pairs = PyObject_IsTrue(a[9]);
+    const int form = (int)integer(a[9]);
     at::Tensor out;
     {
       const Unlocked unlocked;
@@ -383,7 +385,7 @@ PyObject* py_block(PyObject*, PyObject* const* a, Py_ssize_t n) {
       void* st = stream(x);
       at::Tensor t = at::empty({B, 2 * C, H, W}, opt);
       check(api.block_pre(x.data_ptr(), t.data_ptr(), pack.data_ptr(), eps1, B, H * W, io, st), "cvb_block_pre_fwd");
-      t = forward(t, table, wf, k, 1, p, mode, 1, at::Tensor(), pairs);
+      t = forward(t, table, wf, k, 1, p, mode, 1, at::Tensor(), form);
       out = at::empty({B, C, H, W}, opt);
       check(api.block_post(t.data_ptr(), x.data_ptr(), out.data_ptr(), pack.data_ptr(), eps2, B, H * W, io, st),
             "cvb_block_post_fwd");
@@ -492,7 +494,7 @@ PyObject* py_block_train(PyObject*, PyObject* const* a, Py_ssize_t n) {
       x1 = at::empty({B, C, H, W}, opt), z3 = at::empty({B, 2 * C, H, W}, opt), out = at::empty({B, C, H, W}, opt);
       check(api.block_pre_train((const float*)x.data_ptr(), (float*)t1.data_ptr(), (float*)z1.data_ptr(), pack.data_ptr(), eps1,
                                 B, H * W, st), "cvb_block_pre_train");
-      forward(t1, table, wf, k, 1, p, mode, 0, u, false);
+      forward(t1, table, wf, k, 1, p, mode, 0, u, kPlaneTable);
       check(api.block_post_train((const float*)u.data_ptr(), (const float*)x.data_ptr(), (float*)out.data_ptr(),
                                  (float*)x1.data_ptr(), (float*)z3.data_ptr(), pack.data_ptr(), eps2, B, H * W, st),
             "cvb_block_post_train");

@@ -39,7 +39,8 @@ def converse2d_forward(x, table, weight_f32, kernel_size, scale, padding, paddin
                        out=None, pairs=False):
     """Fused pad -> solve -> crop (`models/util_converse.py:142-192`) on a CUDA tensor.  `pairs`: `table` is the pair
     table alone (see `build_transfer`)."""
-    return _cabi.host().converse2d(x, table, weight_f32, kernel_size, scale, padding, padding_mode, fuse_gelu, out, pairs)
+    return _cabi.host().converse2d(x, table, weight_f32, kernel_size, scale, padding, padding_mode, fuse_gelu, out,
+                                   1 if pairs else 0)
 
 
 def build_pair_transfer(weight, bias, eps, h, w):

@@ -166,8 +166,9 @@ class Converse2D(nn.Module):
             return F.gelu(out) if fuse_gelu else out
         if pairs == 2:      # real planes may be faster all the same
             pairs = host.takes_pairs(shape[0], h, w, self.scale, shape[1])
-        table, wf = self._table_for(h, w, x.device, 1 if pairs else 2)
-        return host.converse2d(x, table, wf, self.kernel_size, self.scale, p, self.padding_mode, fuse_gelu, None, pairs)
+        which = 1 if pairs else 2
+        table, wf = self._table_for(h, w, x.device, which)
+        return host.converse2d(x, table, wf, self.kernel_size, self.scale, p, self.padding_mode, fuse_gelu, None, which)
 
 
 def _with_gelu(conv, x):
@@ -279,9 +280,9 @@ class ConverseBlock(nn.Module):
         conv._check_backend()
         shape, p, host = x.shape, conv.padding, _cabi.host()
         h, w = shape[2] + 2 * p, shape[3] + 2 * p
-        pairs = host.takes_pairs(shape[0], h, w, 1, conv.in_channels)
-        table, wf = conv._table_for(h, w, x.device, 1 if pairs else 2)
-        return host.block(x, table, wf, pack, conv.kernel_size, p, conv.padding_mode, c1["0"].eps, c2["0"].eps, pairs)
+        which = 1 if host.takes_pairs(shape[0], h, w, 1, conv.in_channels) else 2
+        table, wf = conv._table_for(h, w, x.device, which)
+        return host.block(x, table, wf, pack, conv.kernel_size, p, conv.padding_mode, c1["0"].eps, c2["0"].eps, which)
 
     def _forward_fixed_order(self, x, conv, alpha1, alpha2):
         # (see `fixed_order`)

@@ -90,6 +90,21 @@ def test_integer_contractions(case):
     assert _cabi.load().cvb_last_device_status(1) == 0      # no bounded wait has run out
 
 
+def test_a_table_of_another_batch_is_refused():
+    """The real-plane table that one image reads is not what full pairs of planes of 268 x 268 read."""
+    from conversenet_b200 import Converse2D
+    from conversenet_b200 import functional as CF
+    m = Converse2D(64, 64, 3, padding=6, padding_mode="circular").cuda()
+    table, wf = CF.build_transfer(m.weight, m.bias, 1, 1e-5, 268, 268, batch=1)
+    for B in (2, 8):                # (from 128 planes on the modules themselves keep that table)
+        with pytest.raises(RuntimeError, match="another batch size"):
+            CF.converse2d_forward(torch.randn(B, 64, 256, 256, device="cuda"), table, wf, 3, 1, 6, "circular")
+    table, wf = CF.build_transfer(m.weight, m.bias, 1, 1e-5, 268, 268)
+    x = torch.randn(2, 64, 256, 256, device="cuda")
+    with torch.no_grad():
+        assert torch.equal(CF.converse2d_forward(x, table, wf, 3, 1, 6, "circular"), m(x))
+
+
 def test_integer_contractions_keep_planes_apart():
     from conversenet_b200 import Converse2D
     g = torch.Generator(device="cuda").manual_seed(3)
