@@ -195,7 +195,7 @@ class Converse2DFunction(torch.autograd.Function):
         if ctx.needs_input_grad[1] or ctx.needs_input_grad[2]:
             kept = _cabi.host().train_forward(x, table, wf, kernel_size, scale, padding, padding_mode)
         if kept is None:
-            out = CF.converse2d_forward(x, table, wf, kernel_size, scale, padding, padding_mode)
+            out = _cabi.host().converse2d(x, table, wf, kernel_size, scale, padding, padding_mode, False, None, 2)
         else:
             out, r = kept
         ctx.save_for_backward(x, weight, bias, table, r)

@@ -407,18 +407,20 @@ PyObject* py_train_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int k = (int)integer(a[3]), s = (int)integer(a[4]), p = (int)integer(a[5]), mode = pad_mode(a[6]);
     if (!api.bwd_workspace_bytes(B, C, H, W, k, s, p, 0, 1)) Py_RETURN_NONE;
     at::Tensor out, r;
-    int rc;
-    {
+    int rc = CVB_OK;
+    if (s == 1) {        // nothing to keep
+      const Unlocked unlocked;
+      out = forward(x0.is_contiguous() ? x0 : x0.contiguous(), table, wf, k, s, p, mode, 0, at::Tensor(), kPlaneTable);
+    } else {
       const Unlocked unlocked;
       const at::Tensor x = x0.is_contiguous() ? x0 : x0.contiguous();
       at::Tensor w;
       out = at::empty({B, C, (int64_t)H * s, (int64_t)W * s}, x.options().requires_grad(false));
-      if (s > 1) r = at::empty({B, C, H + 2 * p, (W + 2 * p + 1) / 2 * 2}, x.options().dtype(at::kFloat).requires_grad(false));
+      r = at::empty({B, C, H + 2 * p, (W + 2 * p + 1) / 2 * 2}, x.options().dtype(at::kFloat).requires_grad(false));
       const size_t ws = api.train_workspace_bytes(B, C, H, W, s, p);
       if (ws) w = bytes_like(x, ws);
       rc = api.fwd_train(x.data_ptr(), out.data_ptr(), table.data_ptr(), (const float*)wf.data_ptr(),
-                         s > 1 ? (float*)r.data_ptr() : nullptr, B, C, H, W, k, s, p, mode, io, ws ? w.data_ptr() : nullptr, ws,
-                         stream(x));
+                         (float*)r.data_ptr(), B, C, H, W, k, s, p, mode, io, ws ? w.data_ptr() : nullptr, ws, stream(x));
       if (rc != CVB_ERR_UNSUPPORTED_SIZE) check(rc, "cvb_converse2d_fwd_train");
     }
     if (rc == CVB_ERR_UNSUPPORTED_SIZE) Py_RETURN_NONE;

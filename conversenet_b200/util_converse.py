@@ -156,7 +156,7 @@ class Converse2D(nn.Module):
             raise RuntimeError("x must be (B,%d,H,W)" % self.in_channels)
         p, host = self.padding, _cabi.host()
         h, w = shape[2] + 2 * p, shape[3] + 2 * p
-        pairs = host.takes_pairs(shape[0], h, w, self.scale)
+        pairs = host.takes_pairs(shape[0], h, w, self.scale, shape[1])
         if torch.is_grad_enabled() and (x.requires_grad or self.weight.requires_grad or self.bias.requires_grad):
             # differentiable route (the reference is differentiable through torch.fft, converse2d.cpp:223)
             # its gradients read the real-plane table; so does the forward, but for the multi-pass pair kernels
@@ -164,8 +164,6 @@ class Converse2D(nn.Module):
             out = Converse2DFunction.apply(x, self.weight, self.bias, table, wf, self.kernel_size, self.scale,
                                            self.padding, self.padding_mode, self.eps)
             return F.gelu(out) if fuse_gelu else out
-        if pairs == 2:      # real planes may be faster all the same
-            pairs = host.takes_pairs(shape[0], h, w, self.scale, shape[1])
         which = 1 if pairs else 2
         table, wf = self._table_for(h, w, x.device, which)
         return host.converse2d(x, table, wf, self.kernel_size, self.scale, p, self.padding_mode, fuse_gelu, None, which)
@@ -251,7 +249,7 @@ class ConverseBlock(nn.Module):
         pack = self._packed(params)
         p, eps1, eps2, host = conv.padding, c1["0"].eps, c2["0"].eps, _cabi.host()
         h, w = x.shape[2] + 2 * p, x.shape[3] + 2 * p
-        table, wf = conv._table_for(h, w, x.device, 0 if host.takes_pairs(x.shape[0], h, w, 1) == 2 else 2)
+        table, wf = conv._table_for(h, w, x.device, 0 if host.takes_pairs(x.shape[0], h, w, 1, conv.in_channels) == 2 else 2)
         x = x.contiguous()
         kept = host.block_train(x, table, wf, pack, conv.kernel_size, p, conv.padding_mode, eps1, eps2)
         if kept is None:

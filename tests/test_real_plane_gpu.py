@@ -105,6 +105,28 @@ def test_a_table_of_another_batch_is_refused():
         assert torch.equal(CF.converse2d_forward(x, table, wf, 3, 1, 6, "circular"), m(x))
 
 
+def test_training_at_268_reads_one_table():
+    """Full pairs of planes of 268 x 268, 128 of them or more: the integer contractions with and without gradients, and of
+    the two tables the one that they and the backward read; fewer planes: the pair kernels and both tables."""
+    from conversenet_b200 import Converse2D, ConverseBlock, _cabi
+    torch.manual_seed(5)
+    bytes_of = lambda C: _cabi.load().cvb_plane_transfer_bytes(C, 268, 268)
+    x = torch.randn(2, 64, 256, 256, device="cuda")
+    for C, alone in ((64, True), (8, False)):
+        m = Converse2D(C, C, 7, padding=6, padding_mode="circular").cuda()
+        y = m(x[:, :C])
+        assert ({t.numel() for t, _ in m._tables.values()} == {bytes_of(C)}) == alone
+        m.weight.requires_grad_(False), m.bias.requires_grad_(False)
+        z = m(x[:, :C].clone().requires_grad_(True))
+        with torch.no_grad():
+            assert torch.equal(m(x[:, :C]), y) and torch.equal(z, y)
+    blk = ConverseBlock(64, 64, 7, 1, 6, "circular").cuda()
+    y = blk(x)
+    assert {t.numel() for t, _ in blk.conv1[3]._tables.values()} == {bytes_of(128)}
+    with torch.no_grad():
+        assert _rel(blk(x), y) <= 1e-6
+
+
 def test_integer_contractions_keep_planes_apart():
     from conversenet_b200 import Converse2D
     g = torch.Generator(device="cuda").manual_seed(3)
