@@ -557,24 +557,28 @@ int emu_rp_backward(const float* x, const float* g, const float* r, float* gx, f
     }
     set_vec(Q, true);
     strip<float>(Q, kColsFwd, sms);
-    BwdParams R;
-    R.P = Q; R.wx = (const float2*)wx.get(); R.D = (float2*)d.get(); R.nseg = nseg; R.solve = 1;
-    const size_t tile = ((size_t)P.pitch * kLines + 1) & ~(size_t)1;
-    emu::Guarded sm(3 * tile * sizeof(float2) + (P.ax.mp ? matrix_entries(P.ax.r0) : 0) * sizeof(float));
-    const int rows = (P.hh + kLines - 1) / kLines;
-    switch (P.ax.mp) {
-      case 0: emu::launch(rows, C, nseg, 128, [&] { rows_bwd_body<kAnyRadix, 0>(R, (float2*)sm.get()); }); break;
+    if (!D) {          // dL/dx alone
+      strip<float>(Q, kRows, sms);
+    } else {
+      BwdParams R;
+      R.P = Q; R.wx = (const float2*)wx.get(); R.D = (float2*)d.get(); R.nseg = nseg; R.solve = 1;
+      const size_t tile = ((size_t)P.pitch * kLines + 1) & ~(size_t)1;
+      emu::Guarded sm(3 * tile * sizeof(float2) + (P.ax.mp ? matrix_entries(P.ax.r0) : 0) * sizeof(float));
+      const int rows = (P.hh + kLines - 1) / kLines;
+      switch (P.ax.mp) {
+        case 0: emu::launch(rows, C, nseg, 128, [&] { rows_bwd_body<kAnyRadix, 0>(R, (float2*)sm.get()); }); break;
 #define CVB_RP_X(M) case M: emu::launch(rows, C, nseg, 128, [&] { rows_bwd_body<kMatrixR1, M>(R, (float2*)sm.get()); }); break;
-        CVB_RP_EACH_WIDTH(CVB_RP_X)
+          CVB_RP_EACH_WIDTH(CVB_RP_X)
 #undef CVB_RP_X
-    }
-    sm.check("shared memory"); d.check("D"); wg.check("the workspace");
-    const float2* dd = (const float2*)d.get();
-    const size_t n = (size_t)C * w * P.hh;
-    for (size_t i = 0; i < n; ++i) {
-      double a = 0, b = 0;
-      for (int sg = 0; sg < nseg; ++sg) { a += dd[sg * n + i].x; b += dd[sg * n + i].y; }
-      D[2 * i] = (float)a; D[2 * i + 1] = (float)b;
+      }
+      sm.check("shared memory"); d.check("D"); wg.check("the workspace");
+      const float2* dd = (const float2*)d.get();
+      const size_t n = (size_t)C * w * P.hh;
+      for (size_t i = 0; i < n; ++i) {
+        double a = 0, b = 0;
+        for (int sg = 0; sg < nseg; ++sg) { a += dd[sg * n + i].x; b += dd[sg * n + i].y; }
+        D[2 * i] = (float)a; D[2 * i + 1] = (float)b;
+      }
     }
     const bool direct = s == 1 && p == 0;
     Params O = Q;

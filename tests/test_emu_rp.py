@@ -197,6 +197,43 @@ def test_gradient_kernels_match_fp64_autograd(emu, case):
                 assert bool((torch.from_numpy(taps[:, :, a, c]).double() - want).abs().le(2e-6 * most).all())
 
 
+@pytest.mark.parametrize("case", [
+    # integer contractions (one SM: every tile count takes them): columns of a zero-extended or strided cotangent, rows with
+    # the conjugated multiplier (dL/dx alone: the parameters' rows have a kernel of their own), columns back without a crop
+    (1, 1, 132, 140, 3, 1, 1, "circular"),        # 134 x 142
+    (2, 1, 130, 131, 5, 1, 2, "replicate"),       # 134 x 135: columns alone; tiles across planes
+    (1, 1, 20, 134, 3, 1, 0, "circular"),         # rows alone, no padding
+    (1, 1, 256, 140, 5, 1, 1, "reflect"),         # 258 x 142: one q above 64
+    (1, 1, 128, 264, 3, 1, 2, "constant"),        # 132 x 268: four q above 64
+    (1, 1, 132, 32, 3, 2, 1, "circular"),         # 134 x 34 by 2
+])
+@pytest.mark.parametrize("params", [False, True])
+def test_gradients_through_the_integer_contractions(emu, case, params):
+    from conversenet_b200.autograd import _Cotangent, _pad, spectral_forward
+    B, C, H, W, k, s, p, mode = case
+    w, b, rng = _weights(C, k, H * W)
+    x = rng.standard_normal((B, C, H, W)).astype(np.float32)
+    g = rng.standard_normal((B, C, H * s, W * s)).astype(np.float32)
+    r = _forward(emu, x, w, b, s, p, mode, keep=True, multi=1, sms=1)[1]
+    h, wd = H + 2 * p, W + 2 * p
+    hh = h // 2 + 1
+    gx, D, taps = np.zeros_like(x), np.zeros((C, wd, hh, 2), np.float32) if params else None, np.zeros((B, C, k, k), np.float32)
+    wf, bf = np.ascontiguousarray(w.reshape(C, k, k)), np.ascontiguousarray(b.reshape(C))
+    _check(emu, emu.emu_rp_backward(_ptr(x), _ptr(g), _ptr(r), _ptr(gx), _ptr(D), _ptr(taps), _ptr(wf), _ptr(bf), B, C, H, W, k, s,
+                                    p, PAD[mode], ctypes.c_float(1e-5), 1, 1))
+    X, Wt, Bt = (torch.from_numpy(a).double().requires_grad_(True) for a in (x, w, b))
+    ref, = torch.autograd.grad(spectral_forward(X, Wt, Bt, s, p, mode, 1e-5), X, torch.from_numpy(g).double())
+    # test_integer_contractions' bound; the padding's adjoint and the correlation add a few fp32 sums
+    assert orc.rel_l2(gx, ref.numpy()) <= 6e-7
+    if not params:
+        return
+    cot = _Cotangent(torch.from_numpy(g), torch.from_numpy(wf), k, s, p)
+    q = (cot.g_full if s == 1 else cot.v).double()
+    d = (torch.fft.fft2(_pad(torch.from_numpy(x).double(), p, mode)) * torch.fft.fft2(q).conj()).sum(0)[:, :hh]
+    got = torch.view_as_complex(torch.from_numpy(D).double()).transpose(1, 2) / 4
+    assert float((got - d).abs().pow(2).sum().sqrt() / d.abs().pow(2).sum().sqrt()) <= 2e-6
+
+
 def test_routes_and_shared_memory(emu):
     one = lambda n, planes: emu.emu_rp_one_block(1, planes, n, n, 1, 0, SMS)
     assert [one(76, 64), one(108, 1), one(110, 98), one(110, 99), one(132, 99), one(132, 64)] == [1, 1, 0, 1, 1, 0]

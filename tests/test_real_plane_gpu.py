@@ -250,6 +250,36 @@ def test_gradients_match_fp64_autograd(case):
         assert _rel(q, r) <= 2e-5
 
 
+@pytest.mark.parametrize("params", [False, True])       # dL/dx alone sends the rows through the contractions as well
+@pytest.mark.parametrize("case", [
+    (1, 96, 132, 140, 3, 1, 1, "circular"),    # 134 x 142
+    (2, 24, 250, 232, 3, 1, 4, "reflect"),     # 258 x 240: columns alone
+    (1, 64, 256, 256, 7, 1, 6, "replicate"),   # 268 x 268
+    (1, 96, 242, 131, 3, 2, 1, "constant"),    # 244 x 133 by 2
+    (1, 3, 200, 192, 5, 1, 1, "circular"),     # 202 x 194: wide dense stages, any number of planes
+])
+def test_gradients_through_the_integer_contractions(case, params):
+    from conversenet_b200 import Converse2D, _cabi
+    from conversenet_b200.autograd import spectral_forward
+    B, C, H, W, k, s, p, mode = case
+    torch.manual_seed(H + W)
+    m = Converse2D(C, C, k, scale=s, padding=p, padding_mode=mode).cuda()
+    with torch.no_grad():
+        m.bias.add_(torch.randn_like(m.bias) + 4.0)
+    m.requires_grad_(params)
+    x = torch.randn(B, C, H, W, device="cuda", requires_grad=True)
+    of = [x, m.weight, m.bias] if params else [x]
+    y = m(x)
+    g = torch.randn_like(y)
+    got = torch.autograd.grad(y, of, g)
+    a = [t.detach().double().requires_grad_(True) for t in (x, m.weight, m.bias)]
+    ref = torch.autograd.grad(spectral_forward(*a, s, p, mode, 1e-5), a[:len(of)], g.double())
+    assert _rel(got[0], ref[0]) <= 6e-7          # tests/test_emu_rp.py
+    for q, r in zip(got[1:], ref[1:]):
+        assert _rel(q, r) <= 2e-6                # sums over every pixel, the chain rule in 64 bits
+    assert _cabi.load().cvb_last_device_status(1) == 0
+
+
 @pytest.mark.parametrize("case", [
     (1, 2, 20, 130, 5, 2, 2, "circular"),      # 67 items side by side: two tiles
     (1, 1, 61, 36, 3, 2, 1, "replicate"),      # odd rows and columns of items, several tiles down, 16-byte copies
