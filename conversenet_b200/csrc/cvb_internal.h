@@ -1,6 +1,7 @@
 // Internal glue between the translation units of libconverse_b200.so.
 #pragma once
 #include "cvb_kernels.cuh"
+#include "cvb_plan.h"
 
 namespace cvb {
 
@@ -28,13 +29,14 @@ int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cu
   CVB_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
   return CVB_OK;
 }
-// dynamic shared memory beyond 48 KB has to be allowed
+// Dynamic shared memory beyond 48 KB has to be allowed.  The limit belongs to the kernel and not to the launch: it is always
+// all there is (none of these kernels has static shared memory), since a smaller call's size, set by another thread between
+// this one and the launch, would make the launch fail.
 template <typename... P>
 int allow_smem(void (*kernel)(P...), size_t smem) {
-  return smem <= 48 * 1024 ? CVB_OK : [&]() -> int {
-    CVB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    return CVB_OK;
-  }();
+  if (smem <= 48 * 1024) return CVB_OK;
+  CVB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit));
+  return CVB_OK;
 }
 #endif
 

@@ -14,7 +14,7 @@ __global__ void __launch_bounds__(512, 1) smem_dynamic_kernel(const FwdParams P)
 namespace {
 template <typename IO>
 int launch_t(const FwdParams& P, size_t smem, cudaStream_t st) {
-  CVB_CUDA(cudaFuncSetAttribute(smem_dynamic_kernel<IO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (const int rc = allow_smem(smem_dynamic_kernel<IO>, smem)) return rc;
   int nthr = CVB_TUNE("CVB_THREADS", 0);
   if (nthr <= 0) {
     // enough threads for the stage with the fewest butterflies, at most 512
@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(512, 1) smem_xspec_kernel(const XspecParams Q)
 int launch_xspec(const XspecParams& Q, cudaStream_t st) {
   const size_t smem = xspec_smem_bytes(Q.h, Q.w, Q.direct);
   if (Q.direct) CVB_CUDA(cudaMemsetAsync(Q.out, 0, (size_t)Q.C * Q.h * Q.w * sizeof(float2), st));
-  CVB_CUDA(cudaFuncSetAttribute(smem_xspec_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (const int rc = allow_smem(smem_xspec_kernel, smem)) return rc;
   const int by = Q.w * (Q.h / Q.py.radix[0]), bx = Q.h * (Q.w / Q.px.radix[0]);
   int nthr = ((by > bx ? by : bx) + 31) / 32 * 32;
   if (nthr < 64) nthr = 64;

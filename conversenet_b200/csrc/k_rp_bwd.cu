@@ -20,7 +20,7 @@ template <int K, int S>
 static int launch_adjoint(AdjointParams A, int planes, cudaStream_t st) {
   plan_adjoint<K, S>(A);
   const size_t smem = (size_t)AdjointTile<K, S>::floats(A) * sizeof(float);
-  CVB_CUDA(cudaFuncSetAttribute(adjoint_epilogue_kernel<K, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (const int rc = allow_smem(adjoint_epilogue_kernel<K, S>, smem)) return rc;
   adjoint_epilogue_kernel<K, S><<<planes, AdjointTile<K, S>::threads, smem, st>>>(A);
   return CVB_OK;
 }
@@ -350,7 +350,8 @@ int run_bwd(const float* x, const float* g, const float* r, const void* table, c
       rc = matrix_bwd(P.ax.mp)(R, grid, smem, st);
       if (rc != CVB_OK) return rc;
     } else {
-      CVB_CUDA(cudaFuncSetAttribute(rows_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      rc = allow_smem(rows_bwd_kernel, smem);
+      if (rc != CVB_OK) return rc;
       rows_bwd_kernel<<<grid, 128, smem, st>>>(R);
       CVB_CUDA(cudaGetLastError());
     }
@@ -388,13 +389,15 @@ int run_bwd(const float* x, const float* g, const float* r, const void* table, c
     switch (s * 16 + k) {
 #define X(KK, SS)                                                                                                  \
       case SS * 16 + KK:                                                                                           \
-        CVB_CUDA(cudaFuncSetAttribute(chain_kernel<KK, SS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+        rc = allow_smem(chain_kernel<KK, SS>, smem);                                                               \
+        if (rc != CVB_OK) return rc;                                                                               \
         chain_kernel<KK, SS><<<grid, 256, smem, st>>>(T);                                                          \
         break;
       CVB_CHAIN_CASES(X)
 #undef X
       default:
-        CVB_CUDA(cudaFuncSetAttribute(chain_kernel<0, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        rc = allow_smem(chain_kernel<0, 0>, smem);
+        if (rc != CVB_OK) return rc;
         chain_kernel<0, 0><<<grid, 256, smem, st>>>(T);
     }
     CVB_CUDA(cudaGetLastError());

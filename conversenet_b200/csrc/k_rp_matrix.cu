@@ -57,7 +57,7 @@ int CVB_CAT(launch_matrix_cols_inv, CVB_MP)(const Params& P, int io_dtype, int t
 }
 
 int CVB_CAT(launch_matrix_rows_bwd, CVB_MP)(const BwdParams& Q, dim3 grid, size_t smem, cudaStream_t st) {
-  CVB_CUDA(cudaFuncSetAttribute(matrix_rows_bwd_kernel<CVB_MP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (const int rc = allow_smem(matrix_rows_bwd_kernel<CVB_MP>, smem)) return rc;
   matrix_rows_bwd_kernel<CVB_MP><<<grid, 128, smem, st>>>(Q);
   CVB_CUDA(cudaGetLastError());
   return CVB_OK;

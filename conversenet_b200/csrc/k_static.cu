@@ -41,7 +41,7 @@ template <typename IO>
 int launch_p(const FwdParams& P, size_t smem, int blocks, cudaStream_t st) {
   auto kernel = P.hh ? smem_persistent_kernel<IO, CVB_RY0, CVB_RY1, CVB_RX0, CVB_RX1, CVB_NT, CVB_MB, true>
                      : smem_persistent_kernel<IO, CVB_RY0, CVB_RY1, CVB_RX0, CVB_RX1, CVB_NT, CVB_MB, false>;
-  CVB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (const int rc = allow_smem(kernel, smem)) return rc;
   kernel<<<blocks, CVB_NT, smem, st>>>(P);
   CVB_CUDA(cudaGetLastError());
   return CVB_OK;

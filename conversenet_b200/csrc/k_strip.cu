@@ -139,9 +139,9 @@ int launch_t(const FwdParams& P, void* workspace, size_t ws_bytes, cudaStream_t 
     return CVB_OK;
   }
   if (g.smem_col > kSmemLimit || g.smem_row > kSmemLimit) return CVB_ERR_UNSUPPORTED_SIZE;
-  CVB_CUDA(cudaFuncSetAttribute(strip_colfwd_kernel<IO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem_col));
-  CVB_CUDA(cudaFuncSetAttribute(strip_colinv_kernel<IO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem_col));
-  CVB_CUDA(cudaFuncSetAttribute(strip_rowmid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem_row));
+  if (const int rc = allow_smem(strip_colfwd_kernel<IO>, g.smem_col)) return rc;
+  if (const int rc = allow_smem(strip_colinv_kernel<IO>, g.smem_col)) return rc;
+  if (const int rc = allow_smem(strip_rowmid_kernel, g.smem_row)) return rc;
   StripParams SP;
   SP.f = P;
   SP.ws = (float2*)workspace;

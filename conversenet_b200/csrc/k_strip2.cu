@@ -35,7 +35,7 @@ namespace {
 template <typename K>
 int launch_k(K kernel, const StripParams& SP0, int nstrips, size_t smem, cudaStream_t st) {
   const StripParams& SP = SP0;
-  CVB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (const int rc = allow_smem(kernel, smem)) return rc;
   kernel<<<dim3(nstrips, SP.npair), kThreads, smem, st>>>(SP);
   CVB_CUDA(cudaGetLastError());
   return CVB_OK;
@@ -43,7 +43,7 @@ int launch_k(K kernel, const StripParams& SP0, int nstrips, size_t smem, cudaStr
 template <typename K>
 int resident_blocks(K kernel, size_t smem) {
   int n = 0;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+  if (allow_smem(kernel, smem) != CVB_OK ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kThreads, smem) != cudaSuccess || n < 1) {
     (void)cudaGetLastError();
     n = 2;

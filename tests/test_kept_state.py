@@ -309,3 +309,35 @@ def test_a_captured_graph_holds_the_tables_it_reads():
     filler += [torch.full((n,), float("nan"), device="cuda") for n in (1 << 10, 1 << 14, 50000, 1 << 17) for _ in range(32)]
     assert torch.equal(g(x), ref)
     del filler
+
+
+@pytest.mark.gpu
+def test_kernels_at_several_sizes_from_several_threads():
+    """The same kernels launched with more and with less shared memory at the same time: a small call must not take the
+    permission for more from a large one that is about to launch."""
+    import threading
+    from conversenet_b200 import Converse2D
+    failures = []
+
+    def work(k, s, p, sizes):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                m = Converse2D(4, 4, k, scale=s, padding=p, padding_mode="circular").cuda()
+                xs = [torch.randn(1, 4, h, w, device="cuda", requires_grad=True) for h, w in sizes]
+                for _ in range(120):
+                    for x in xs:
+                        y = m(x)
+                        torch.autograd.grad(y, (x, m.weight), y.detach())
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:
+            failures.append(e)
+    # scale 2: tiles of the adjoint epilogue, dense and register rows; scale 1: integer contractions (202 = 101 x 2, 254 = 127 x 2,
+    # taken at any number of planes), strip kernels
+    jobs = [(5, 2, 2, [(16, 16), (24, 300)]), (5, 2, 2, [(60, 200), (20, 20)]), (3, 1, 1, [(200, 200), (252, 252)]),
+            (3, 1, 1, [(252, 200), (200, 252)]), (3, 1, 2, [(160, 300), (196, 116)]), (3, 1, 2, [(116, 196), (300, 160)])]
+    threads = [threading.Thread(target=work, args=j) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures[0]
