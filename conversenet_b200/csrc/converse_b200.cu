@@ -183,9 +183,11 @@ static bool takes_static_pairs(int B, int h, int w) {
 static bool takes_multipass_pairs(int B, int h, int w, int s) {
   return s == 1 && full_pairs(B) && dual_tables(h, w) && !(B == 5 && three_stage_axis(h));
 }
-// Of those, the ones whose real planes are faster all the same when the caller has the table for them: 268 x 268, whose
-// 67-point stages run as integer contractions (cvb_fix.cuh): 8 x 128 planes 956 us against 1063, 2 x 128 255 against 276,
-// with a tenth of the rounding error.  From 128 planes on: smaller batches keep the one table that they always had.
+// Of those, the ones that run on real planes all the same when the caller has the table for them: 268 x 268 (of the pair lengths
+// the one that has integer contractions too), whose 67-point stages then keep a tenth of the rounding error (1.8e-7 against 2 to
+// 4e-6 of the TF32 products).  Pairs / real planes, us: 2 x 32 planes 71 / 71, 2 x 48 133 / 133, 2 x 64 152 / 139, 2 x 96 204 / 209, 2 x 128
+// 256 / 281, 8 x 128 971 / 1063: no slower up to 128 planes, up to 14 % slower above, which is the price of the accuracy.  From
+// 128 planes on: smaller batches keep the one table that they always had.
 static bool takes_contractions(int B, int C, int h, int w, int s) {
   return takes_multipass_pairs(B, h, w, s) && gemm_axis(h) && gemm_axis(w) && rp::fix_length(h) && rp::fix_length(w) &&
          (long long)B * C >= 128;

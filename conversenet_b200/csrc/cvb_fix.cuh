@@ -18,21 +18,25 @@
 //
 // One block per SM walks over tiles of 128 lines (= rows of the MMA = lanes of tensor memory).  A tile arrives in shared
 // memory as it is; thread t serves line t % 128: it folds a quarter of the line's q, cuts the four classes into digits and
-// writes them to tensor memory (256 columns), from where the MMAs read them.  The constants' digits lie side by side
-// along N in shared memory (36 to 60 KB), and so do the accumulators; a pair of digits is an MMA.  Outputs come in chunks of 32 frequencies of one parity, cosines and sines (what 32 does not divide: 16 of
-// both parities), in the other 256 columns of tensor memory; a thread reads back eight frequencies of its line.  The warp
-// that is the last to have read a chunk issues the MMAs of the next one, which run while the values are finished and stored.
+// writes them to tensor memory (256 columns), from where the MMAs read them.  The constants' digits lie side by side along N
+// in shared memory (36 to 60 KB), and so do the accumulators; a pair of digits is an MMA.  Outputs come in chunks of 32
+// frequencies of one parity, cosines and sines (what 32 does not divide: 16 of both parities), in the other 256 columns of tensor
+// memory; a thread reads back eight frequencies of its line.  The warp that is the last to have read a chunk issues the MMAs of
+// the next one, which run while the values are finished and stored.
 // q >= 64 (lengths from 256 on: at most four) is added in fp32 there.
 // Columns: the next tile is copied to shared memory as soon as the last one is folded.  Rows: the forward transform, the
 // multiplier and the transform back follow each other on a tile that stays in shared memory.
 //
-// What bounds it: a chain per chunk (MMAs issued, their latency, tensor memory read, converted) of about 2200 cycles at four
-// warps a scheduler; the integer units issue about half of it.  A tile of columns of 268 takes 15 000 to 17 000 cycles, the
-// two passes of a tile of rows 50 000 (table and exchange with the workspace included).  1 x 128 planes of 268 x 268: 126 us,
-// with the matrix stages 155; 244 x 244 99 / 137; 178 x 178 74 / 122; 254 x 254 (R0 = 127) 100 / 287.
-// Tried on the way (1 x 128 planes of 268 x 268): digits in shared memory 180 us; MMAs issued by a divergent lane instead of a
-// whole warp with one lane elected 152; 1024 threads of 64 registers 139; cosines and sines as chunks of their own 203 (with
-// spills); the MMA loops unrolled 135 (instruction fetch).
+// What bounds it: a chain per chunk (MMAs issued one after the other, their latency, tensor memory read, converted) at four warps a
+// scheduler; half of the issue slots and a tenth of the tensor pipe are used.  1 x 128 planes of 268 x 268: 140 us, with the
+// matrix stages 156; 244 x 244 105 / 138; 178 x 178 77 / 120; 254 x 254 (R0 = 127) 106 / 287.
+// A digit of the line times several of the constants' as one MMA 3 n, 2 n and n columns wide, four a K step instead of nine, took
+// 126, 99, 74 and 100 us, but those overlap in accumulators without the same shape, and nothing orders such MMAs.  Tried with it:
+// pairs of accumulators 2 n wide with zeros beside the constants' digits, six a K step 144 us (columns cost more than MMAs);
+// cosines and sines by turns 138 against 140, 1 % slower at other lengths.
+// Tried on the way (against the 126 us): digits in shared memory 180 us; MMAs issued by a divergent lane instead of a whole warp with
+// one lane elected 152; 1024 threads of 64 registers 139; cosines and sines as chunks of their own 203 (with spills); the MMA
+// loops unrolled 135 (instruction fetch).
 #pragma once
 #include "cvb_rp.cuh"
 #ifdef __CUDACC__
@@ -132,6 +136,9 @@ __device__ __forceinline__ float2 fx_mul2(float2 a, float2 b) {
 #endif
 
 // ------------------------------------------------------------------ geometry
+// Up to 270: tensor memory holds the digits of that many points.  From 130: where the measurements begin that takes_fix
+// (cvb_rp_plan.h) rests on.  The kernel itself is right from 66 on and faster than the matrix stages from about 94 points along
+// columns and 118 along rows (128 planes of 122 x 122 34 / 46 us, of 94 x 94 32 / 35; 256 of 300 x 94 124 / 117).
 __host__ __device__ constexpr bool fix_length(int n) { return n % 2 == 0 && n >= 130 && n <= 270; }
 __host__ __device__ constexpr int fix_rows(int n) { return (n / 4 + 16) & ~15; }       // frequencies of a parity, padded
 __host__ __device__ constexpr int fix_operand(int n) { return 768 * fix_rows(n); }     // bytes: 2 parities x 2 x 3 digits x 64
@@ -253,7 +260,8 @@ struct FixBlock {
   }
 };
 
-// Columns: slice `sl` of `ns` of a tile on its way to shared memory
+// Columns: slice `sl` of `ns` of a tile on its way to shared memory: fp32 and the spectra by asynchronous copies, bf16 by plain
+// loads and stores (the copies do not convert)
 template <int KIND, typename IO, bool EXTRA>
 __device__ __forceinline__ void fix_load(const Params& P, unsigned char* smem, int tile, int sl, int ns) {
   const FixBlock<KIND, EXTRA> S(P, smem);

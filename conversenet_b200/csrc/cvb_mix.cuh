@@ -55,8 +55,12 @@ __device__ __forceinline__ void mix_mma(uint32_t tmem, const float* b_hi, int k0
   }
 }
 
-// ---- the forward's operands: fp16 hi + lo (22 bits, as TF32 hi + lo, at twice the rate and half the space), which need the
-// values of a row scaled by a power of two to below 2^14: both halves are normal numbers then, whatever the row's size.
+// ---- the forward's operands: fp16 hi + lo, at twice the rate of TF32 hi + lo and half the space.  The values of a row are
+// scaled by a power of two, the largest to below 2^14.  A value then keeps 22 bits, as TF32 hi + lo does, down to 2^-3 (its lo
+// half is a normal number), and an absolute error of 2^-25 below: 2^-39 of the bound of a row of weights or of a hidden channel,
+// 2^-38 of a LayerNorm's bound of 8 (which a pixel whose channels differ by far less than eps comes nowhere near), 2^-35 of a
+// pixel's largest value of t.  TF32 would keep 22 bits of values smaller still; a sum in fp32 would not show them
+// unless the other operand makes up for it.
 // half index of element (n, k) of an operand with N rows (K-major core matrices of 8 x 8, no swizzle)
 __host__ __device__ constexpr int pack_index16(int N, int n, int k) {
   return (n >> 3) * 64 + (n & 7) * 8 + (k & 7) + ((k >> 3) & 1) * (N / 8) * 64 + (k >> 4) * (N / 8) * 128;

@@ -227,7 +227,10 @@ struct AdjointParams {
 template <int K, int S>
 struct AdjointTile {
   static constexpr int c = K / 2, NW = K + S, SHIFT = ((c - K + 1) % 4 + 4) % 4, NV = (SHIFT + NW + 3) / 4;
-  static constexpr int threads = 256, sums = threads + 8, blocks = K < 7 && K * S < 20 ? 3 : 2, area = 216 * 1024 / blocks;    // an SM's blocks; their tiles
+  // Blocks of an SM: three leave a thread 80 registers, which up to five taps a side take with 24 bytes spilled at most; at scale
+  // 4 five taps would spill 64 bytes and seven taps 356 to 496 at any scale (none and 40 to 56 with 128 registers).  `area`: bytes
+  // that a block's two tiles may take.
+  static constexpr int threads = 256, sums = threads + 8, blocks = K < 7 && K * S < 20 ? 3 : 2, area = 216 * 1024 / blocks;
   __host__ __device__ static int rows(int th) { return 2 * S * th + K - S; }
   __host__ __device__ static int floats(const AdjointParams& A) {
     const int t = 2 * buffer(A), red = K * K * sums;
@@ -241,7 +244,7 @@ struct AdjointTile {
 };
 // At most 64 items side by side (524 floats a row at scale 4: two tiles of one item's rows always fit); as many rows of items
 // as make the walk shortest by a rough count of a block's cycles -- 520 for every 256 items, 15 floats copied per cycle, 150
-// a tile -- in at most 56 KB, so that blocks overlap on an SM.
+// a tile -- as fit 36 KB a tile where three blocks share an SM, 54 KB where two do.
 template <int K, int S>
 inline void plan_adjoint(AdjointParams& A) {
   using T = AdjointTile<K, S>;

@@ -130,11 +130,12 @@ inline bool fill_params(Params& P, const void* table, int B, int C, int H, int W
 
 // Strip kernels (kFixFwd, kFixRows, kFixInv) that run as integer contractions (cvb_fix.cuh): along axes that would need a
 // matrix stage, from the number of lines on that gives 55 of 100 SMs a tile (a launch takes as long with fewer).  Matrix
-// stage / contractions on all three kernels, us, planes of N x N: 244 48 planes (91 tiles) 70.7 / 51.9, 32 planes 43.6 / 50.6;
-// 80 planes (153 tiles, two rounds) 112 / 93; 128 planes of 268 155 / 125, 218 157 / 94, 178 122 / 74, 134 49.4 / 38.5; 64
-// planes of 134 (67 tiles) 34.9 / 38.4.  Wide matrix stages (R0 > 88) lose to any number of lines: 8 planes of 202 54.8 / 47.
-// The narrowest (R0 = 37, 41) keep the rows below 240: 128 planes of 164 64.4 with the columns alone, 71.7 with all three;
-// 246 105 / 101.  Register radices stay: 128 planes of 264 79 / 124.
+// stage / contractions on all three kernels, us, planes of N x N: 244 48 planes (91 tiles) 68.3 / 55.1, 32 planes 42.6 / 51 or
+// more; 80 planes (153 tiles, two rounds) 114 / 101; 128 planes of 268 156 / 142, 218 157 / 100, 178 120 / 79.5, 134 48.8 / 40.7;
+// 64 planes of 134 (67 tiles) 33.8 / 38 or more.  Wide matrix stages (R0 > 88) lose to any number of lines: 8 planes of 202
+// 53.5 / 49.7.  The narrowest (R0 = 37, 41) keep the rows below 240: matrix stages / columns alone / all three, 128 planes of 164
+// 71.4 / 69.1 / 77.9, 222 110 / 99.0 / 101, 246 126 / 108.5 / 108.3 (512 planes 513 / 434 / 428).  Register radices
+// stay: 128 planes of 264 79 / 124.
 inline bool takes_fix(const Params& P, int kind, int sms) {
   const Axis& a = kind == kFixRows ? P.ax : P.ay;
   if (!a.fix || (kind == kFixRows && a.mp <= 20 && a.n < 240)) return false;
@@ -182,8 +183,8 @@ inline Route route(int B, int C, int H, int W, int s, int p, int sms, bool force
   if (n > 0) {                            // chunks of equal size, as many as
     const int least = (planes + (int)n - 1) / (int)n;
     const bool fy = fix_axis(h, a), fx = fix_axis(w, c);
-    // rounds of tiles that the integer contractions take for m planes: 4 x 128 planes of 268 x 268, 512 us in four chunks
-    // (two rounds a kernel each), 561 in three (2.4, that is three)
+    // rounds of tiles that the integer contractions take for m planes: 4 x 128 planes of 268 x 268 in four chunks (two rounds
+    // a kernel each) take 0.91 of the time in three (2.4, that is three)
     auto rounds = [&](int m) {
       auto of = [&](long long lines) { return (int)((lines + (long long)kFixLines * sms - 1) / ((long long)kFixLines * sms)); };
       return (fy ? 2 * of((long long)m * (w + 1)) : 0) + (fx ? 2 * of(2LL * m * (h / 2 + 1)) : 0);

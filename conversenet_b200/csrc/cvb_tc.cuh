@@ -2,12 +2,17 @@
 // shared-memory matrix descriptors, the instruction descriptor, TMEM allocation, MMA issue,
 // commit to an mbarrier and TMEM loads.  Device-only inline PTX for sm_100a.
 //
-// Operands are fp32 in shared memory read as TF32.  To keep fp32 accuracy every product is
-// split: a = a_hi + a_lo with a_hi = tf32(a), and D += a_hi*b_hi + a_hi*b_lo + a_lo*b_hi
-// (three MMAs, error ~2^-21 per product).
+// To keep fp32 accuracy a product is split: a = a_hi + a_lo with a_hi rounded to the operand's
+// type, and D += a_hi*b_hi + a_hi*b_lo + a_lo*b_hi (three MMAs, error ~2^-21 per product): TF32
+// in the weight and channel gradients, the layer-wise kernels and the tensor-core pair kernels,
+// fp16 in the block kernels (cvb_mix.cuh, which scales its operands for it).  The integer
+// contractions split into signed bytes (cvb_fix.cuh).  Operand A lies in shared or in tensor
+// memory, B in shared memory.
+// MMAs keep the order of their issue only among those of the same accumulator and shape: no two
+// between two waits may overlap in any other way.
 //
-// Shared-memory layout used for both operands: K-major, no swizzle ("core matrix" = 8 rows of
-// 16 bytes, 128 contiguous bytes).  Element (mn, k) of an operand sits at
+// Shared-memory layout of a 32-bit operand: K-major, no swizzle ("core matrix" = 8 rows of
+// 16 bytes, 128 contiguous bytes; others: as many elements as 16 bytes hold).  Element (mn, k) sits at
 //       float index = (mn / 8) * SBO_f + (mn % 8) * 4 + k % 4 + ((k / 4) % 2) * LBO_f + (k / 8) * KSTEP_f
 // SBO = stride between 8-row groups, LBO = stride between the two 4-wide K halves of one MMA
 // (K = 8 per instruction, 32 bytes per row); checked on a B200 with index-valued operands.

@@ -17,9 +17,10 @@
 // 32 channels x 32 pixels; others are loaded pixel by pixel (any image size and alignment, fp32 or bf16).
 //
 // fp16 hi + lo keeps 22 bits of a value like TF32 hi + lo, with K = 16 an MMA instead of 8 and half the space, as long as the
-// values lie high enough in fp16's range: rows of weights and pixels are scaled by powers of two.  A LayerNorm's values stay
-// below 8, the hidden ones below a bound that follows from the weights; t has any size, so a pixel takes its scale from its
-// first 64 channels, and if the others are more than 32 times as large its sums so far are scaled down in tensor memory.
+// values lie high enough in fp16's range (cvb_mix.cuh states the bound): rows of weights, hidden channels and pixels are scaled
+// by powers of two.  A LayerNorm's values stay below 8, each hidden channel below a bound that follows from its weights; t has
+// any size that fp32 has, so a pixel takes its scale from its first 64 channels, and if the others are more than 32 times as
+// large its sums so far are scaled down in tensor memory.
 // With TF32 (twice as many MMAs, whose 46 cycles at least the two groups wait for together, and waits for one operand buffer)
 // 8 x 256 x 256 pixels took 103 us PRE and 232 POST, with fp16 93 and 199, with the copies ahead 81 and 164; against fp64
 // PRE's error went from 5.9e-7 to 3.6e-7, POST's from 1.0e-6 to 5.8e-7.

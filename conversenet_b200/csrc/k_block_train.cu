@@ -207,7 +207,8 @@ static int launch_grad(const BlockGradParams& P, int sms, cudaStream_t st) {
 // four additions (eight of the small products) stays below what rounding the sum of a block's thousand pixels costs: gradients of w1 to w4 of a block of
 // 8 x 64 x 64 are within 5.7e-7 to 8.5e-7 of fp64 (8.0e-7 to 1.1e-6 with fp32 products on the CUDA cores).  32768 pixels,
 // the four contractions: 50 us, 99 on the CUDA cores (which waited for the port to shared memory); 100 MB take 15 us.  The
-// erf of the GELUs, the split and its stores are the larger part of a tile.
+// erf of the GELUs, the split and its stores are the larger part of a tile.  An infinity among the operands makes the sums that it meets
+// NaN (hi - hi), not infinite.
 constexpr int kGOut = kBlkC * kBlkM + kBlkC + kBlkM;
 constexpr int kGThreads = 512, kGRows = 128, kGGroup = kGRows * 16 + 16;   // bytes of four pixels of 128 rows (+ 16: banks)
 constexpr int kGOperand = 8 * kGGroup, kGBuffer = 3 * kGOperand;           // Q hi, Q lo, [P hi | P lo]

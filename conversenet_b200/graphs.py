@@ -1,6 +1,6 @@
 """CUDA-graph replay of a network's forward.
 
-A forward is many launches: ConverseDnCNN issues about 100 kernels on one 256 x 256 image and 700 on eight
+A forward is many launches: ConverseDnCNN issues about 100 kernels on one 256 x 256 image and 350 on eight
 (chunks of the multi-pass kernels), and on small images the host needs longer to enqueue them than the GPU
 needs to run them.  `GraphedForward` captures one forward (this package's kernels, PyTorch's few 1x1 convolutions and copies, and the
 allocations between them) in a CUDA graph with static input and output buffers and replays it: one
