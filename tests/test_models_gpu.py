@@ -332,9 +332,10 @@ def _worst_channel(a, r):
 
 
 @pytest.mark.parametrize("H, W", [(24, 32), (21, 25)])      # rows that are copied ahead, rows that are not
-@pytest.mark.parametrize("kind", ["a row of W3", "an entry of b3", "a row of zeros", "all rows", "the norms"])
+@pytest.mark.parametrize("kind", ["a row of W3", "an entry of b3", "a row of zeros", "all rows", "the norms", "channels of t"])
 def test_block_kernels_on_uneven_weights(kind, H, W):
-    """A hidden channel may be 2^20 times the others (and its column of W4 as much smaller), rows and norms of any size."""
+    """A hidden channel may be 2^20 times the others (and its column of W4 as much smaller), rows and norms of any size, channels
+    of t 2^11 apart."""
     from conversenet_b200 import ConverseBlock
     g = torch.Generator(device="cuda").manual_seed(H)
     torch.manual_seed(H)
@@ -363,6 +364,9 @@ def test_block_kernels_on_uneven_weights(kind, H, W):
                 m.bias.copy_(torch.randn(64, device="cuda", generator=g))
         x = torch.randn(2, 64, H, W, device="cuda", generator=g)
         t = torch.nn.functional.gelu(torch.randn(2, 128, H, W, device="cuda", generator=g))
+        if kind == "channels of t":       # (22 bits reach down to 2^-13 of a pixel's largest value)
+            t[:, 1::2] *= 2.0 ** -11
+            w2.weight[:, 1::2] *= 2.0 ** 11
     (pre, post), want = _block_kernels_and_fp64(blk, x, t)
     live = want[0].pow(2).sum((0, 2, 3)) > 0
     # 22 bits of each operand and fp32 sums of 64 and 128 products, in the worst channel
