@@ -165,8 +165,9 @@ int cvb_build_plane_transfer(const float* weight, const float* bias, int C, int 
 
 /*
  * The same operator on one real plane after the other with that table, whatever the batch.  cvb_takes_planes: 1 for batches
- * that cvb_takes_pairs answers 2 for although the real planes are the faster ones, so that a caller that knows its batch
- * keeps the real-plane table and calls cvb_plane_fwd; else 0.
+ * that cvb_takes_pairs answers 2 for although the real planes are the better ones (a tenth of the rounding error; 9 % faster
+ * at 128 planes, up to 14 % slower above), so that a caller that knows its batch keeps the real-plane table and calls
+ * cvb_plane_fwd; else 0.
  */
 int cvb_takes_planes(int B, int C, int h, int w, int s);
 size_t cvb_plane_workspace_bytes(int B, int C, int H, int W, int s, int p);
